@@ -413,9 +413,10 @@ def _flux(ll, l, r, rr, nx, nz, gx, gz, jst):
 
 
 def _ode(u, x, w, mach, aoa):
-    """R of every cell from its nine states u (9, 4, M, N) and its corners x, w (4, 2, M, N)."""
+    """R of every cell of a group of G equal grids from its nine states u (9, 4, M, G, N) and its
+    corners x, w (4, 2, M, G, N); mach and aoa (radian) have G values."""
     M = u.shape[2]
-    m = torch.arange(M, device=u.device)[:, None].expand(u.shape[2:])
+    m = torch.arange(M, device=u.device)[:, None, None].expand(u.shape[2:])
     c, b, bb, f, ff, i, ii, o, oo = u
 
     def edge(p, q):
@@ -428,9 +429,10 @@ def _ode(u, x, w, mach, aoa):
     nx, nz, gx, gz = n_i
     proj = (nx * (c[1] - gx * c[0]) + nz * (c[2] - gz * c[0])) / (nx * nx + nz * nz)
     wall = torch.stack([c[0], c[1] - 2 * nx * proj, c[2] - 2 * nz * proj, c[3]])
-    speed, a = mach * math.sqrt(1.4), math.radians(aoa)
+    speed = mach[:, None] * math.sqrt(1.4)
     one = torch.ones_like(c[0])
-    far = 2 * torch.stack([one, one * speed * math.cos(a), one * speed * math.sin(a),
+    far = 2 * torch.stack([one, one * speed * torch.cos(aoa)[:, None],
+                           one * speed * torch.sin(aoa)[:, None],
                            one * (2.5 + speed * speed / 2)]) - c
     i = torch.where(m == 0, wall, i)
     o = torch.where(m == M - 1, far, o)
@@ -443,36 +445,52 @@ def _ode(u, x, w, mach, aoa):
 
 
 def _stencil(U):
-    """(4, M, N) -> (9, 4, M, N); rows past the radial ends hold the end's state."""
+    """(4, M, G, N) -> (9, 4, M, G, N); rows past the radial ends hold the end's state."""
     M = U.shape[1]
     at = torch.arange(M, device=U.device)
-    return torch.stack([torch.roll(U[:, (at + dm).clamp(0, M - 1)], -dn, 2) for dm, dn in SLOTS])
+    return torch.stack([torch.roll(U[:, (at + dm).clamp(0, M - 1)], -dn, 3) for dm, dn in SLOTS])
 
 
 def _corners(X):
-    return torch.stack([X[:, :-1, :-1], X[:, :-1, 1:], X[:, 1:, 1:], X[:, 1:, :-1]])
-
-
-def _ode_of(one):
-    return lambda U, X, V, mach: _ode(_stencil(U), _corners(X), _corners(V), mach, one["aoa"])
+    return torch.stack([X[:, :-1, :, :-1], X[:, :-1, :, 1:], X[:, 1:, :, 1:], X[:, 1:, :, :-1]])
 
 
 def _forces(U, X):
     p = _pressure(U[:, 0])
-    a, b = X[:, 0, :-1], X[:, 0, 1:]
+    a, b = X[:, 0, :, :-1], X[:, 0, :, 1:]
     return torch.stack([p * (b[1] - a[1]), p * (a[0] - b[0])])
 
 
-def _primal(one):
-    return (one["U"], one["dX"], one["V"], torch.tensor(one["mach"], dtype=F64, device="cuda"))
+def _groups(inputs: list[dict]) -> list[dict]:
+    """The instances of each grid size together: arrays (var, M, G, N), offsets of the parts."""
+    found: dict = {}
+    cells = verts = 0
+    for k, one in enumerate(inputs):
+        g = found.setdefault((one["M"], one["N"]), {"ids": [], "cells": [], "verts": []})
+        g["ids"].append(k)
+        g["cells"].append(4 * cells)
+        g["verts"].append(2 * verts)
+        cells += one["M"] * one["N"]
+        verts += (one["M"] + 1) * (one["N"] + 1)
+    out = []
+    for (M, N), g in found.items():
+        part = [inputs[k] for k in g["ids"]]
+        vec = lambda v: torch.tensor(v, dtype=F64, device="cuda")  # noqa: E731
+        aoa = vec([math.radians(i["aoa"]) for i in part])
+        args = (*(torch.stack([i[k] for i in part], 2) for k in ("U", "dX", "V")),
+                vec([i["mach"] for i in part]))
+        f = lambda U, X, V, mach, aoa=aoa: _ode(  # noqa: E731
+            _stencil(U), _corners(X), _corners(V), mach, aoa)
+        out.append(dict(g, M=M, N=N, aoa=aoa, args=args, f=f))
+    return out
 
 
-def _unpack(v, offset: int, shape, per_complex: bool = True):
-    """The instance's part of a packed vector as (var, M, N), complex where interleaved."""
+def _unpack(v, offsets, shape, per_complex: bool = True):
+    """The group's parts of a packed vector as (var, M, G, N), complex where interleaved."""
     n = math.prod(shape)
     if per_complex:
         v = torch.view_as_complex(v.view(-1, 2))
-    return v[offset:offset + n].reshape(shape[2], shape[1], shape[0]).permute(2, 1, 0)
+    return torch.stack([v[o:o + n].reshape(*reversed(shape)).permute(2, 1, 0) for o in offsets], 2)
 
 
 def _real_imag(fn, d):
@@ -480,51 +498,61 @@ def _real_imag(fn, d):
     return torch.complex(fn(d.real.contiguous()), fn(d.imag.contiguous()))
 
 
-def _jacobians(one):
-    """The six Jacobians in the package's packed layouts, and d(odes)/d(states) as (4,4,M,N,9)."""
-    U, X, V, mach = _primal(one)
+def _packed(a) -> torch.Tensor:
+    """One instance's array in the package's layout (first index fastest), interleaved."""
+    a = a.permute(*reversed(range(a.ndim))).contiguous().reshape(-1)
+    return torch.view_as_real(a).reshape(-1) if a.is_complex() else a
+
+
+def _each(a, dim: int) -> list:
+    """A group's array as one packed vector per instance (the group's dimension is `dim`)."""
+    return [_packed(a.select(dim, g)) for g in range(a.shape[dim])]
+
+
+def _jacobians(group, U=None):
+    """The six Jacobians per instance of the group, and d(odes)/d(states) as (4,4,M,G,N,9)."""
+    U, X, V, mach = (group["args"][0] if U is None else U), *group["args"][1:]
+    aoa, M = group["aoa"], group["M"]
     u, x, w = _stencil(U), _corners(X), _corners(V)
-    M, N = one["M"], one["N"]
 
     def columns(fn, at, var):
         cols = []
         for j in range(var):
-            t = torch.zeros_like(at[0])
-            t[j] = 1.0
-            cols.append([])
             for s in range(at.shape[0]):
-                full = torch.zeros_like(at)
-                full[s] = t
-                cols[-1].append(torch.func.jvp(fn, (at,), (full,))[1])
-        # (var, slots, 4, M, N) -> (4, var, M, N, slots)
-        return torch.stack([torch.stack(c) for c in cols]).permute(2, 0, 3, 4, 1)
+                t = torch.zeros_like(at)
+                t[s, j] = 1.0
+                cols.append(torch.func.jvp(fn, (at,), (t,))[1])
+        # (var * slots, 4, M, G, N) -> (4, var, M, G, N, slots)
+        c = torch.stack(cols)
+        return c.reshape(var, at.shape[0], *c.shape[1:]).permute(2, 0, 3, 4, 5, 1)
 
-    Ju = columns(lambda t: _ode(t, x, w, mach, one["aoa"]), u, 4)
+    Ju = columns(lambda t: _ode(t, x, w, mach, aoa), u, 4)
+    rows = torch.arange(M, device=U.device)
     for s, (dm, _) in enumerate(SLOTS):
-        rows = torch.arange(M, device=U.device)
-        Ju[:, :, ((rows + dm < 0) | (rows + dm >= M)).nonzero()[:, 0], :, s] = 0.0
-    Jx = columns(lambda t: _ode(u, t, w, mach, one["aoa"]), x, 2)
-    Jv = columns(lambda t: _ode(u, x, t, mach, one["aoa"]), w, 2)
-    Jm = torch.func.jvp(lambda t: _ode(u, x, w, t, one["aoa"]), (mach,),
-                        (torch.ones_like(mach),))[1]
-    fx = torch.stack([X[:, 0, :-1], X[:, 0, 1:]])                    # (2 ends, 2, N)
-    wall = U[:, :1]
+        Ju[:, :, (rows + dm < 0) | (rows + dm >= M), :, :, s] = 0.0
+    Jx = columns(lambda t: _ode(u, t, w, mach, aoa), x, 2)
+    Jv = columns(lambda t: _ode(u, x, t, mach, aoa), w, 2)
+    Jm = torch.func.jvp(lambda t: _ode(u, x, w, t, aoa), (mach,), (torch.ones_like(mach),))[1]
+    ends = torch.stack([X[:, 0, :, :-1], X[:, 0, :, 1:]])              # (2 ends, 2, G, N)
+    wall = U[:, 0]
 
     def force(s, e):
-        p = _pressure(s[:, 0])
+        p = _pressure(s)
         return torch.stack([p * (e[1][1] - e[0][1]), p * (e[0][0] - e[1][0])])
 
-    unit = lambda a, *at: torch.zeros_like(a).index_put(  # noqa: E731
-        tuple(torch.tensor(i, device=a.device) for i in at), torch.ones((), dtype=F64, device=a.device))
-    JFu = torch.stack([torch.func.jvp(lambda t: force(t, fx), (wall,), (unit(wall, k),))[1]
-                       for k in range(4)])                             # (4, 2, N)
-    JFx = torch.stack([torch.stack([torch.func.jvp(lambda t: force(wall, t), (fx,),
-                                                   (unit(fx, e, k),))[1] for k in range(2)])
-                       for e in range(2)])                             # (ends, comp, 2, N)
-    order = lambda a: a.permute(*reversed(range(a.ndim))).contiguous().reshape(-1)  # noqa: E731
-    return {"mach": order(Jm), "states": order(Ju), "vertices": order(Jx), "velocities": order(Jv),
-            "forces_states": order(JFu.permute(1, 0, 2)),
-            "forces_vertices": order(JFx.permute(2, 1, 3, 0))}, Ju
+    def unit(a, *at):
+        t = torch.zeros_like(a)
+        t[at] = 1.0
+        return t
+
+    JFu = torch.stack([torch.func.jvp(lambda t: force(t, ends), (wall,), (unit(wall, k),))[1]
+                       for k in range(4)], 1)                           # (2, 4, G, N)
+    JFx = torch.stack([torch.stack([torch.func.jvp(lambda t: force(wall, t), (ends,),
+                                                   (unit(ends, e, k),))[1] for k in range(2)], 1)
+                       for e in range(2)], -1)                          # (2, 2, G, N, ends)
+    return {"mach": _each(Jm, 2), "states": _each(Ju, 3), "vertices": _each(Jx, 3),
+            "velocities": _each(Jv, 3), "forces_states": _each(JFu, 2),
+            "forces_vertices": _each(JFx, 2)}, Ju
 
 
 class _Elimination:
@@ -536,19 +564,17 @@ class _Elimination:
         K, P = self.K, self.P
         n = torch.arange(N, device=Ju.device)
         blocks = {}
-        for s, (dm, dn) in enumerate(SLOTS):
-            nn = (n + dn) % N
-            for m in range(max(0, -dm), min(M, M - dm)):
-                B = blocks.setdefault((m, m + dm), torch.zeros(N, 4, N, 4, dtype=dtype,
-                                                               device=Ju.device))
-                B[n, :, nn, :] += Ju[:, :, m, :, s].permute(2, 0, 1).to(dtype)
+        for s, (dm, dn) in enumerate(SLOTS):  # all rings' blocks of one offset at a time
+            B = blocks.setdefault(dm, torch.zeros(M, N, 4, N, 4, dtype=dtype, device=Ju.device))
+            B[:, n, :, (n + dn) % N, :] += Ju[..., s].permute(3, 2, 0, 1).to(dtype)
         eye = torch.eye(K, dtype=dtype, device=Ju.device)
         get = {}
-        for (a, b), B in blocks.items():
-            B = B.reshape(K, K)
-            if a == b:
+        for dm, B in blocks.items():
+            B = B.reshape(M, K, K)
+            if dm == 0:
                 B = B - (shift if dtype == C128 else shift.real) * eye
-            get[(b, a) if adjoint else (a, b)] = B.conj().T if adjoint else B
+            for m in range(max(0, -dm), min(M, M - dm)):
+                get[(m + dm, m) if adjoint else (m, m + dm)] = B[m].conj().T if adjoint else B[m]
         zero = torch.zeros(K, K, dtype=dtype, device=Ju.device)
 
         def pair(p, q):
@@ -601,152 +627,156 @@ class _Elimination:
         return x.reshape(-1, self.N, 4)[:self.M].permute(2, 0, 1)
 
 
-def _packed_complex(a) -> torch.Tensor:
-    return torch.view_as_real(_flat(a)).reshape(-1)
-
-
 def exact(case: dict, seed: int):
     kind = case["kind"]
-    if kind in ("resolvent", "ptc", "response"):  # block eliminations: about 40 TFLOP/s at most
+    if kind in ("resolvent", "ptc", "response"):
         M, N = _sizes(case)[0]
         runs = {"resolvent": 2, "ptc": case.get("steps", 0), "response": case.get("shifts", 0) + 1}
-        if runs[kind] * M * (8 * N) ** 3 > 4e11:
+        if runs[kind] * M * (2e9 + (8 * N) ** 3) > 1e12:  # over some 15 seconds of eliminations
             return None
     inputs = _inputs(case, seed)
     extra = _extra(case, inputs, seed)
-    parts = []
-    cells = verts = 0
-    for k, one in enumerate(inputs):
-        parts.append(_exact_one(kind, case, one, extra, k, cells, verts))
-        cells += 4 * one["M"] * one["N"]
-        verts += 2 * (one["M"] + 1) * (one["N"] + 1)
-    if kind in ("dropin", "second_order", "resolvent", "ptc", "response"):
-        return parts[0]
-    if isinstance(parts[0], dict):
-        return {k: torch.cat([p[k] for p in parts]) for k in parts[0]}
-    if isinstance(parts[0], list):
-        return [torch.cat([p[k] for p in parts]) for k in range(len(parts[0]))]
-    return torch.cat(parts)
+    groups = _groups(inputs)
+    if kind in ("dropin", "second_order", "response"):
+        parts = {"dropin": _exact_dropin, "second_order": _exact_second_order,
+                 "response": _exact_response}[kind](case, groups[0], extra)
+        return {k: v.cpu().numpy() for k, v in parts.items()}
+    if kind == "ptc":
+        return _exact_ptc(case, groups[0])
+    if kind == "resolvent":
+        return _exact_resolvent(case, groups[0], extra)
+    outputs: dict = {}
+    for g in groups:  # the instances' parts in their order
+        for key, parts in _exact_group(kind, g, extra).items():
+            outputs.setdefault(key, [None] * len(inputs))
+            for k, part in zip(g["ids"], parts):
+                outputs[key][k] = part
+    out = {k: torch.cat(v) for k, v in outputs.items()}
+    if kind in ("residual", "tangent"):
+        return out["R"]
+    if kind == "gradient":
+        return [out["R"], out["U"], out["X"], out["V"], out["mach"].cpu()]
+    return out
 
 
-def _exact_one(kind, case, one, extra, index, cells, verts):
-    M, N = one["M"], one["N"]
-    f, args = _ode_of(one), _primal(one)
-    U, X, V, mach = args
+def _pullback(f, args, w):
+    """The four reverse products with a complex cotangent."""
+    pull = torch.func.vjp(f, *args)[1]
+    return [torch.complex(a, b) for a, b in zip(pull(w.real.contiguous()),
+                                                pull(w.imag.contiguous()))]
+
+
+def _exact_group(kind, g, extra) -> dict:
+    f, args, M, N = g["f"], g["args"], g["M"], g["N"]
     su, sx = (4, M, N), (2, M + 1, N + 1)
     if kind == "residual":
-        return _flat(f(*args))
+        return {"R": _each(f(*args), 2)}
     if kind == "gradient":
         R, pull = torch.func.vjp(f, *args)
-        g = pull(_unpack(extra["w"], cells, su, False))
-        return [_flat(R), *[_flat(v) for v in g[:3]], g[3].reshape(1).cpu()]
-    if kind in ("tangent", "products"):
-        d = (_unpack(extra["dU"], cells, su), _unpack(extra["dX"], verts, sx),
-             _unpack(extra["dV"], verts, sx),
-             torch.view_as_complex(extra["dMa"].view(-1, 2))[index])
-        jvp = lambda t: torch.func.jvp(f, args, t)[1]  # noqa: E731
-        zero = tuple(torch.zeros_like(a) for a in args)
-        along = []
-        for part in ("real", "imag"):
-            along.append([jvp(tuple(getattr(d[j], part).contiguous() if j == k else zero[j]
-                                    for j in range(4))) for k in range(4)])
-        each = [torch.complex(a, b) for a, b in zip(*along)]
-        if kind == "tangent":
-            return _packed_complex(sum(each))
-        w = _unpack(extra["w"], cells, su)
-        pull = torch.func.vjp(f, *args)[1]
-        gr, gi = pull(w.real.contiguous()), pull(w.imag.contiguous())
-        rev = [torch.complex(a, b) for a, b in zip(gr, gi)]
-        names = ("states", "vertices", "velocities")
-        out = {f"{n}_fwd": _packed_complex(v) for n, v in zip(names, each)}
-        out |= {f"{n}_rev": _packed_complex(v) for n, v in zip(names, rev)}
-        out["mach_fwd"] = _packed_complex(each[3])
-        out["mach_rev"] = torch.view_as_real(rev[3].reshape(1)).reshape(-1)
-        return out
+        d = pull(_unpack(extra["w"], g["cells"], su, False))
+        return {"R": _each(R, 2), "U": _each(d[0], 2), "X": _each(d[1], 2), "V": _each(d[2], 2),
+                "mach": list(d[3].reshape(-1, 1))}
     if kind == "linearize":
-        return _jacobians(one)[0]
-    if kind == "dropin":
-        w, dU, dX = extra["w"], extra["dU"], extra["dX"]
-        jvp = lambda k: lambda t: torch.func.jvp(  # noqa: E731
-            f, args, tuple(t if j == k else torch.zeros_like(a) for j, a in enumerate(args)))[1]
-        pull = torch.func.vjp(f, *args)[1]
-        rev = [torch.complex(a, b) for a, b in zip(pull(w.real.contiguous()),
-                                                   pull(w.imag.contiguous()))]
-        zU, zX = torch.zeros_like(U), torch.zeros_like(X)
-        dF = (_real_imag(lambda t: torch.func.jvp(_forces, (U, X), (zU, t))[1], dX)
-              + _real_imag(lambda t: torch.func.jvp(_forces, (U, X), (t, zX))[1], dU))
-        out = {"odes": f(*args), "forces": _forces(U, X),
-               "rhs": _real_imag(jvp(1), dX) + _real_imag(jvp(2), 0.1j * dX), "d_forces": dF,
-               "rev": rev[0], "rev_x": rev[1]}
-        return {k: v.cpu().numpy() for k, v in out.items()}
-    if kind == "second_order":
-        w, dU = extra["w"], extra["dU"]
-
-        def inner(wr, d):
-            """The gradients of <wr, dR/dU d> with respect to U, the Mach number and X."""
-            def scalar(U, X, mach):
-                return (wr * torch.func.jvp(lambda t: f(t, X, V, mach), (U,), (d,))[1]).sum()
-            return torch.func.grad(scalar, argnums=(0, 2, 1))(U, X, mach)
-
-        wr, wi = w.real.contiguous(), -w.imag.contiguous()
-        dr, di = dU.real.contiguous(), dU.imag.contiguous()
-        rr, ri, ir, ii = inner(wr, dr), inner(wr, di), inner(wi, dr), inner(wi, di)
-        out = [torch.complex(rr[k] - ii[k], ri[k] + ir[k]) for k in range(3)]
-        return {"uu": out[0].cpu().numpy(), "um": out[1].reshape(1).cpu().numpy(),
-                "ux": out[2].cpu().numpy()}
-    if kind == "resolvent":
-        Ju = _jacobians(one)[1]
-        s = complex(case["re"], case["im"])
-        x = _Elimination(Ju, s, False).solve(_unpack(extra["b"], 0, su))
-        y = _Elimination(Ju, s, True).solve(_unpack(extra["c"], 0, su))
-        return [_packed_complex(x), _packed_complex(y)]
-    if kind == "ptc":
-        return _exact_ptc(case, one, f, args)
-    return _exact_response(case, one, args)
+        return _jacobians(g)[0]
+    d = (_unpack(extra["dU"], g["cells"], su), _unpack(extra["dX"], g["verts"], sx),
+         _unpack(extra["dV"], g["verts"], sx),
+         torch.view_as_complex(extra["dMa"].view(-1, 2))[g["ids"]])
+    along = lambda *t: torch.func.jvp(f, args, t)[1]  # noqa: E731
+    if kind == "tangent":
+        return {"R": _each(torch.complex(along(*(v.real.contiguous() for v in d)),
+                                         along(*(v.imag.contiguous() for v in d))), 2)}
+    zero = [torch.zeros_like(a) for a in args]
+    names = ("states", "vertices", "velocities", "mach")
+    out = {}
+    for k, name in enumerate(names):
+        one = lambda t, k=k: along(*zero[:k], t, *zero[k + 1:])  # noqa: E731
+        out[f"{name}_fwd"] = _each(_real_imag(one, d[k]), 2)
+    rev = _pullback(f, args, _unpack(extra["w"], g["cells"], su))
+    for name, v in zip(names[:3], rev):
+        out[f"{name}_rev"] = _each(v, 2)
+    out["mach_rev"] = list(torch.view_as_real(rev[3]))
+    return out
 
 
-def _exact_ptc(case, one, f, args):
+def _exact_dropin(case, g, extra) -> dict:
+    f, args = g["f"], g["args"]
     U, X, V, mach = args
-    norms, rels, norm0 = [], [], None
-    for step in range(case["steps"]):
-        R = f(U, X, V, mach)
-        norm = float(R.abs().max())
-        norm0 = norm if norm0 is None else norm0
-        norms.append(norm)
-        rels.append(norm / norm0)
-        J, Ju = _jacobians(dict(one, U=U))
-        shift = rels[-1] / 0.1
-        U = U + _Elimination(Ju, complex(shift), False, F64).solve(-R)
-    return {"U": _flat(U), "R": _flat(R), "J": J["states"], "norms": norms, "rel_norms": rels}
+    w, dU, dX = (extra[k][:, :, None] for k in ("w", "dU", "dX"))
+    zU, zX, zm = torch.zeros_like(U), torch.zeros_like(X), torch.zeros_like(mach)
+    rhs = (_real_imag(lambda t: torch.func.jvp(f, args, (zU, t, zX, zm))[1], dX)
+           + _real_imag(lambda t: torch.func.jvp(f, args, (zU, zX, t, zm))[1], 0.1j * dX))
+    dF = (_real_imag(lambda t: torch.func.jvp(_forces, (U, X), (zU, t))[1], dX)
+          + _real_imag(lambda t: torch.func.jvp(_forces, (U, X), (t, zX))[1], dU))
+    rev = _pullback(f, args, w)
+    return {"odes": f(*args)[:, :, 0], "forces": _forces(U, X)[:, 0], "rhs": rhs[:, :, 0],
+            "d_forces": dF[:, 0], "rev": rev[0][:, :, 0], "rev_x": rev[1][:, :, 0]}
 
 
-def _exact_response(case, one, args):
+def _exact_second_order(case, g, extra) -> dict:
+    f, (U, X, V, mach) = g["f"], g["args"]
+    w, dU = extra["w"][:, :, None], extra["dU"][:, :, None]
+
+    def inner(wr, d):
+        """The gradients of <wr, dR/dU d> with respect to U, the Mach number and X."""
+        def scalar(U, X, mach):
+            return (wr * torch.func.jvp(lambda t: f(t, X, V, mach), (U,), (d,))[1]).sum()
+        return torch.func.grad(scalar, argnums=(0, 2, 1))(U, X, mach)
+
+    wr, wi = w.real.contiguous(), -w.imag.contiguous()  # the cotangent enters conjugated
+    dr, di = dU.real.contiguous(), dU.imag.contiguous()
+    rr, ri, ir, ii = inner(wr, dr), inner(wr, di), inner(wi, dr), inner(wi, di)
+    uu, um, ux = (torch.complex(rr[k] - ii[k], ri[k] + ir[k]) for k in range(3))
+    return {"uu": uu[:, :, 0], "um": um, "ux": ux[:, :, 0]}
+
+
+def _exact_resolvent(case, g, extra) -> list:
+    Ju = _jacobians(g)[1][:, :, :, 0]
+    s, shape = complex(case["re"], case["im"]), (4, g["M"], g["N"])
+    x = _Elimination(Ju, s, False).solve(_unpack(extra["b"], [0], shape)[:, :, 0])
+    y = _Elimination(Ju, s, True).solve(_unpack(extra["c"], [0], shape)[:, :, 0])
+    return [_packed(x), _packed(y)]
+
+
+def _exact_ptc(case, g) -> dict:
+    U, X, V, mach = g["args"]
+    norms, rels = [], []
+    for _ in range(case["steps"]):
+        R = g["f"](U, X, V, mach)
+        norms.append(float(R.abs().max()))
+        rels.append(norms[-1] / norms[0])
+        J, Ju = _jacobians(g, U)
+        dU = _Elimination(Ju[:, :, :, 0], complex(rels[-1] / 0.1), False, F64).solve(-R[:, :, 0])
+        U = U + dU[:, :, None]
+    return {"U": _packed(U[:, :, 0]), "R": _packed(R[:, :, 0]), "J": J["states"][0],
+            "norms": norms, "rel_norms": rels}
+
+
+def _exact_response(case, g, extra) -> dict:
+    f, args = g["f"], g["args"]
     U, X, V, mach = args
-    f = _ode_of(one)
-    Ju = _jacobians(one)[1]
-    q = one["mach"] ** 2 * 1.4 / 2
+    Ju = _jacobians(g)[1][:, :, :, 0]
+    ma = float(mach)
+    q = ma**2 * 1.4 / 2
     dX = torch.stack([X[1], -(X[0] - 0.25)])
-    zU, zX = torch.zeros_like(U), torch.zeros_like(X)
-    zero = torch.zeros_like(mach)
-    rx = torch.func.jvp(f, args, (zU, dX, zX, zero))[1].to(C128)
-    rv = torch.func.jvp(f, args, (zU, zX, dX, zero))[1].to(C128)
+    zU, zX, zm = torch.zeros_like(U), torch.zeros_like(X), torch.zeros_like(mach)
+    rx = torch.func.jvp(f, args, (zU, dX, zX, zm))[1][:, :, 0].to(C128)
+    rv = torch.func.jvp(f, args, (zU, zX, dX, zm))[1][:, :, 0].to(C128)
     F = _forces(U, X)
     dFx = torch.func.jvp(_forces, (U, X), (zU, dX))[1].to(C128)
-    px = (X[0, 0, :-1] + X[0, 0, 1:]) / 2 - 0.25
-    pz = (X[1, 0, :-1] + X[1, 0, 1:]) / 2
-    gx, gz = -F[1] / q, F[0] / q                       # d c_m / d(points) at fixed forces
-    mid = (dX[:, 0, :-1] + dX[:, 0, 1:]) / 2
-    cm_x = (gx * mid[0] + gz * mid[1]).sum()
+    along = lambda t: torch.func.jvp(_forces, (U, X), (t, zX))[1]  # noqa: E731
+    px = (X[0, 0, :, :-1] + X[0, 0, :, 1:]) / 2 - 0.25
+    pz = (X[1, 0, :, :-1] + X[1, 0, :, 1:]) / 2
+    mid = (dX[:, 0, :, :-1] + dX[:, 0, :, 1:]) / 2
+    cm_x = ((F[0] * mid[1] - F[1] * mid[0]) / q).sum()  # the arm's change at fixed forces
     cl, cm = [], []
     for k in _reduced_frequencies(case):
-        s = 1j * k * one["mach"] * math.sqrt(1.4) / 0.5
+        s = 1j * k * ma * math.sqrt(1.4) / 0.5
         dU = -_Elimination(Ju, s, False).solve(rx + s * rv)
-        dF = dFx + _real_imag(lambda t: torch.func.jvp(_forces, (U, X), (t, zX))[1], dU)
-        cl.append(complex((dF[1] / q).sum()))
-        cm.append(complex(((pz * dF[0] - px * dF[1]) / q).sum() + cm_x))
-    pull_F = torch.func.vjp(_forces, U, X)[1]
-    g = torch.stack([torch.zeros_like(F[0]), torch.full_like(F[1], 1.0 / q)])
-    gU, gX = pull_F(g)
-    lam = _Elimination(Ju, 0j, True, F64).solve(gU)
-    grad = gX - torch.func.vjp(f, *args)[1](lam)[1]
-    return {"cl": np.array(cl), "cm": np.array(cm), "grad": grad.cpu().numpy()}
+        dF = dFx + _real_imag(along, dU[:, :, None])
+        cl.append((dF[1] / q).sum())
+        cm.append(((pz * dF[0] - px * dF[1]) / q).sum() + cm_x)
+    gU, gX = torch.func.vjp(_forces, U, X)[1](
+        torch.stack([torch.zeros_like(F[0]), torch.full_like(F[1], 1.0 / q)]))
+    lam = _Elimination(Ju, 0j, True, F64).solve(gU[:, :, 0])
+    grad = gX - torch.func.vjp(f, *args)[1](lam[:, :, None])[1]
+    return {"cl": torch.stack(cl), "cm": torch.stack(cm), "grad": grad[:, :, 0]}
