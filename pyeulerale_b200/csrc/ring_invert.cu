@@ -1,0 +1,440 @@
+// Gauss-Jordan inversion of a ring's K x K diagonal block (ringlu.cu) with partial pivoting, as
+// one cooperative launch: the block's columns are spread over CTAs, NC columns per CTA, each
+// thread keeping its rows of them in registers from the first pivot to the last.
+//
+// What bounds it is the chain of K pivot steps, not arithmetic: a panel on one SM and its update
+// on all of them, as two launches per panel, spent 27 us per 16 steps on the panel and as much
+// again on loading it, the update and two launch gaps. Here a panel never leaves its CTA's
+// registers: CTA p eliminates its columns (search for the largest remaining entry, one barrier
+// per step), hands each group of four finished steps to a publishing warp, which copies them to
+// global memory and raises a flag with the pivot rows in it, and every other CTA applies the
+// group to its own columns as a rank-4 update, so that CTA p + 1 begins its pivots about 2.5 us
+// after CTA p's last one. NC = 16 real or 8 complex columns: a block of K = 512 occupies 32 (64)
+// SMs. Measured per block (one or two blocks at a time): K = 128 complex 88 us, real 67; 256: 205
+// and 145; 512: 562 and 360; 1024: 2250 and 1170. With the two launches per panel a ring of
+// K = 512 took 1150 us, of K = 128 about 300 us, complex.
+//
+// The waits are polls of a flag in global memory by CTAs of one cooperative launch (all are
+// resident); each gives up after kPollLimit polls, records it in info and ends the launch's
+// work on that system.
+
+#include "ring_invert.cuh"
+
+#include <cuComplex.h>
+
+#include <algorithm>
+#include <string>
+
+#include "../../include/euler_b200.h"
+
+namespace eb {
+
+int fail(int code, const char* msg);
+int check_launch(const char* what);
+
+namespace rl {
+namespace {
+
+constexpr int kMaxRows = 1024;
+constexpr int kMaxWarps = 16;
+constexpr int kPollLimit = 1 << 22;  // about three seconds
+
+__device__ __forceinline__ double mul(double a, double b) { return a * b; }
+__device__ __forceinline__ cuDoubleComplex mul(cuDoubleComplex a, cuDoubleComplex b) {
+  return make_cuDoubleComplex(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double neg(double a) { return -a; }
+__device__ __forceinline__ cuDoubleComplex neg(cuDoubleComplex a) {
+  return make_cuDoubleComplex(-a.x, -a.y);
+}
+// c + a b
+__device__ __forceinline__ double fmadd(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ cuDoubleComplex fmadd(cuDoubleComplex a, cuDoubleComplex b,
+                                                 cuDoubleComplex c) {
+  return make_cuDoubleComplex(fma(a.x, b.x, fma(-a.y, b.y, c.x)),
+                              fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
+// c - a b
+__device__ __forceinline__ double fmsub(double a, double b, double c) { return fma(-a, b, c); }
+__device__ __forceinline__ cuDoubleComplex fmsub(cuDoubleComplex a, cuDoubleComplex b,
+                                                 cuDoubleComplex c) {
+  return make_cuDoubleComplex(fma(-a.x, b.x, fma(a.y, b.y, c.x)),
+                              fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
+}
+// 1 / a of a normal number: the hardware's approximation (error e below 2^-19) and one step of
+// the third-order Newton iteration y (1 + e + e^2), without the branches of a division, so that
+// it runs in the shadow of the pivot search.
+__device__ __forceinline__ double recip(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ cuDoubleComplex recip(cuDoubleComplex a) {
+  const double d = recip(a.x * a.x + a.y * a.y);
+  return make_cuDoubleComplex(a.x * d, -a.y * d);
+}
+// a non-negative number ordered like the modulus
+__device__ __forceinline__ double size_of(double a) { return fabs(a); }
+__device__ __forceinline__ double size_of(cuDoubleComplex a) { return a.x * a.x + a.y * a.y; }
+template <class T>
+__device__ __forceinline__ T zero_of();
+template <>
+__device__ __forceinline__ double zero_of<double>() {
+  return 0.0;
+}
+template <>
+__device__ __forceinline__ cuDoubleComplex zero_of<cuDoubleComplex>() {
+  return make_cuDoubleComplex(0.0, 0.0);
+}
+// Loads past L1: the panels are written by other SMs during the launch.
+__device__ __forceinline__ double load_l2(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ cuDoubleComplex load_l2(const cuDoubleComplex* p) {
+  const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+  return make_cuDoubleComplex(v.x, v.y);
+}
+
+__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_release(unsigned long long* p, unsigned long long v) {
+  asm volatile("fence.acq_rel.gpu;\n st.release.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v)
+               : "memory");
+}
+// Barrier `id` of `n` threads (a multiple of 32): wait, or arrive without waiting.
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  asm volatile("barrier.cta.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("barrier.cta.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
+}
+
+constexpr int kSub = 4;  // steps published together
+// The word published for a group of kSub steps: the launch's epoch, whether the steps found
+// their pivots, and the pivot rows (ten bits each).
+__device__ __forceinline__ unsigned long long pack(int epoch, bool ok, const int* piv) {
+  unsigned long long w = ((unsigned long long)epoch << 1) | (ok ? 1ull : 0ull);
+#pragma unroll
+  for (int k = 0; k < kSub; ++k) w = (w << 10) | (unsigned long long)(ok ? piv[k] : 0);
+  return w;
+}
+__device__ __forceinline__ bool is_epoch(unsigned long long w, int epoch) {
+  return (w >> (10 * kSub + 1)) == (unsigned long long)epoch;
+}
+__device__ __forceinline__ bool is_ok(unsigned long long w) { return (w >> (10 * kSub)) & 1ull; }
+__device__ __forceinline__ int row_of(unsigned long long w, int k) {
+  return (int)((w >> (10 * (kSub - 1 - k))) & 0x3FFull);
+}
+
+template <class T, int NC>
+struct Shared {
+  T cand[2][kMaxWarps][NC];      // each warp's best row of a step
+  T cand_inv[2][kMaxWarps];      // the reciprocal of its pivot entry
+  unsigned cand_key[2][kMaxWarps];
+  T rows[kSub][NC];              // the pivot rows of a group of steps in this CTA's columns
+  unsigned long long word;       // the group's published word (0: the wait gave up)
+  int own[NC];                   // this CTA's own pivot rows
+  int ok;                        // its own steps found their pivots so far
+  int stop;
+};
+
+// Grid: (ceil(K / NC), systems); block: the compute threads, ceil(K / ROWS) rounded up to whole
+// warps, and one warp that publishes. Compute thread t holds rows t + r nt (r < ROWS) of the
+// CTA's columns j NC .. j NC + NC - 1. Steps follow the in-place Gauss-Jordan elimination with
+// implicit row pivoting: a group of steps with pivot rows P turns every other column c into
+// A[:, c] (rows P zeroed) + A'[:, group] A[P, c], and after the last step the working array W
+// holds Dinv[pos(i), perm[k]] = W[i, k] with pos(i) the step that chose row i.
+template <class T, int NC, int ROWS, int Threads>
+__global__ void __launch_bounds__(Threads + 32, 1)
+    k_ring_invert(int K, int z0, int chains, char* base, int64_t stride, InvertAt at, int epoch) {
+  constexpr bool kReal = sizeof(T) == sizeof(double);
+  constexpr int nt = Threads, kWarps = Threads / 32;  // compute threads and warps
+  constexpr int kStepBar = 1, kGroupBar = 2;  // kGroupBar + q: group q of this CTA's steps
+  constexpr int kGroups = NC / kSub;
+  extern __shared__ __align__(16) unsigned char ri_smem[];
+  Shared<T, NC>& S = *reinterpret_cast<Shared<T, NC>*>(ri_smem);
+  T* stage = reinterpret_cast<T*>(ri_smem + sizeof(Shared<T, NC>));  // NC columns of K
+  const int z = z0 + blockIdx.y, chain = z % chains;
+  char* ws = base + stride * (z / chains);
+  auto place = [&](const At& a) { return ws + a.off + a.chain * chain; };
+  const T* in = reinterpret_cast<const T*>(place(at.in));
+  T* pub = reinterpret_cast<T*>(place(at.pub));
+  unsigned long long* flags = reinterpret_cast<unsigned long long*>(place(at.flags));
+  int* info = reinterpret_cast<int*>(place(at.info));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j = blockIdx.x, panels = gridDim.x, c0 = j * NC, width = min(NC, K - c0);
+  if (tid == 0) {  // info may be set during this launch: one thread's view is the CTA's
+    S.stop = *info;
+    S.ok = 1;
+  }
+  __syncthreads();
+  if (S.stop != 0) return;
+  if (warp == kWarps) {  // the publishing warp: copies the groups from shared memory
+    const int words = kSub * K * (int)sizeof(T) / 16;
+    for (int q = 0; q < width / kSub; ++q) {
+      bar_sync(kGroupBar + q, nt + 32);
+      if (S.stop != 0) return;
+      const double2* from = reinterpret_cast<const double2*>(stage + (size_t)K * kSub * q);
+      double2* to = reinterpret_cast<double2*>(pub + (size_t)K * (c0 + kSub * q));
+#pragma unroll 8
+      for (int i = lane; i < words; i += 32) __stcg(to + i, from[i]);
+      __syncwarp();
+      if (lane == 0) store_release(flags + c0 / kSub + q, pack(epoch, S.ok != 0, S.own + kSub * q));
+      if (S.ok == 0) return;
+    }
+    bar_arrive(kGroupBar + kGroups, nt + 32);
+    return;
+  }
+  T a[ROWS][NC];
+  bool left[ROWS];  // rows not chosen yet
+  int pos[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const int i = tid + r * nt;
+    left[r] = i < K;
+    pos[r] = 0;
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+      a[r][k] = i < K && k < width ? in[(size_t)K * (c0 + k) + i] : zero_of<T>();
+  }
+  // this thread's best remaining entry of column a[.][0]: its key (ordered like the modulus to
+  // one part in 2^10, the row in the low ten bits; 0: none) and its reciprocal
+  unsigned mine = 0u;
+  T inv_mine = zero_of<T>();
+  auto candidate = [&]() {
+    T pivot = a[0][0];
+    mine = 0u;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const unsigned key = left[r] ? ((unsigned)__double2hiint(size_of(a[r][0])) & ~0x3FFu) |
+                                         (unsigned)(kMaxRows - 1 - (tid + r * nt))
+                                   : 0u;
+      if (r == 0 || key > mine) {
+        mine = key;
+        pivot = a[r][0];
+      }
+    }
+    inv_mine = recip(pivot);
+  };
+  for (int p = 0; p < panels; ++p) {
+    if (p == j) {
+      // A rolled loop: each CTA runs it once, so unrolled steps would all be fetched cold (the
+      // unrolled form took 950 cycles per step). The columns rotate by one per step instead: the
+      // step's column is a[.][0], its result goes to the last place.
+      candidate();
+      bool ok = true;
+#pragma unroll 1
+      for (int jj = 0; jj < width; ++jj) {
+        const int par = jj & 1;
+        const unsigned best = __reduce_max_sync(0xffffffffu, mine);
+        if (mine == best) {  // this thread's row is the warp's best: stage it
+          // (best = 0, no row left: every lane stages, and the step fails if all warps say so)
+          const int brow = kMaxRows - 1 - (int)(best & 0x3FFu);
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+            if (brow == tid + r * nt) {
+#pragma unroll
+              for (int k = 0; k < NC; ++k) S.cand[par][warp][k] = a[r][k];
+            }
+          S.cand_inv[par][warp] = inv_mine;
+          S.cand_key[par][warp] = best;
+        }
+        bar_sync(kStepBar, nt);
+        unsigned kb = 0u;
+#pragma unroll
+        for (int q = 0; q < kWarps; ++q) kb = max(kb, S.cand_key[par][q]);
+        const int prow = kMaxRows - 1 - (int)(kb & 0x3FFu);
+        const unsigned size = kb & ~0x3FFu;
+        ok = size != 0u && size < 0x7FF00000u && prow < K;
+        if (!ok) {  // the same in every compute thread
+          if (tid == 0) {
+            S.ok = 0;
+            atomicExch(info, 1);
+          }
+          bar_arrive(kGroupBar + jj / kSub, nt + 32);
+          break;
+        }
+        const int w = (prow % nt) >> 5;  // the warp that holds row prow
+        const T inv = S.cand_inv[par][w];
+        const T* row = S.cand[par][w];
+        if (tid == 0) S.own[jj] = prow;
+        T f[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) f[r] = mul(a[r][0], inv);
+        if (warp == w) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+            if (tid + r * nt == prow) {  // the pivot row becomes inv times itself
+              left[r] = false;
+              pos[r] = c0 + jj;
+              f[r] = neg(inv);
+#pragma unroll
+              for (int k = 1; k < NC; ++k) a[r][k] = zero_of<T>();
+            }
+        }
+        // the next step's column first: its search runs under the other columns' updates
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) a[r][0] = fmsub(f[r], row[1], a[r][1]);
+        candidate();
+#pragma unroll
+        for (int k = 2; k < NC; ++k) {
+          const T b = row[k];
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) a[r][k - 1] = fmsub(f[r], b, a[r][k]);
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) a[r][NC - 1] = neg(f[r]);
+        if (jj % kSub == kSub - 1) {  // hand the group's columns to the other CTAs
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) {
+            const int i = tid + r * nt;
+            if (i < K) {
+#pragma unroll
+              for (int k = 0; k < kSub; ++k)
+                stage[K * (jj - (kSub - 1) + k) + i] = a[r][NC - kSub + k];
+            }
+          }
+          bar_arrive(kGroupBar + jj / kSub, nt + 32);
+        }
+      }
+      if (!ok) return;
+      continue;
+    }
+    const int groups = min(NC, K - p * NC) / kSub;
+    for (int q = 0; q < groups; ++q) {
+      const int g0 = p * NC + q * kSub;  // the group's first step
+      if (warp == 0) {
+        unsigned long long w = 0ull;
+        int n = 0;
+        for (; n < kPollLimit; ++n) {
+          w = load_acquire(flags + g0 / kSub);
+          if (is_epoch(w, epoch)) break;
+        }
+        if (lane == 0) {
+          if (n == kPollLimit) atomicExch(info, 2);
+          S.word = n < kPollLimit && is_ok(w) ? w : 0ull;
+        }
+      }
+      bar_sync(kStepBar, nt);
+      const unsigned long long word = S.word;
+      if (word == 0ull) {  // the publishing warp of this CTA ends as well
+        if (tid == 0) S.stop = 1;
+        for (int o = 0; p < j && o < 1; ++o) bar_arrive(kGroupBar, nt + 32);
+        return;
+      }
+      T g[ROWS][kSub];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int i = tid + r * nt;
+#pragma unroll
+        for (int k = 0; k < kSub; ++k)
+          g[r][k] = i < K ? load_l2(pub + (size_t)K * (g0 + k) + i) : zero_of<T>();
+      }
+#pragma unroll
+      for (int k = 0; k < kSub; ++k) {
+        const int piv = row_of(word, k);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+          if (tid + r * nt == piv) {
+            left[r] = false;
+            pos[r] = g0 + k;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              S.rows[k][c] = a[r][c];
+              a[r][c] = zero_of<T>();
+            }
+          }
+      }
+      bar_sync(kStepBar, nt);
+#pragma unroll
+      for (int k = 0; k < kSub; ++k)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const T b = S.rows[k][c];
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) a[r][c] = fmadd(g[r][k], b, a[r][c]);
+        }
+    }
+  }
+  bar_sync(kGroupBar + kGroups, nt + 32);  // the publishing warp has read stage
+  // the inverse's columns: rows in the order of their steps, through shared memory. (Only the
+  // last panel can be narrow; its rotation leaves column k at place NC - width + k.)
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (tid + r * nt < K) {
+#pragma unroll
+      for (int k = 0; k < NC; ++k)
+        if (k >= NC - width) stage[(size_t)K * (k - (NC - width)) + pos[r]] = a[r][k];
+    }
+  bar_sync(kStepBar, nt);
+  cuDoubleComplex* out = reinterpret_cast<cuDoubleComplex*>(place(at.out));
+  for (int k = 0; k < width; ++k) {
+    const size_t col = (size_t)K * S.own[k];
+    for (int i = tid; i < K; i += nt) {
+      const T v = stage[(size_t)K * k + i];
+      if constexpr (kReal) {
+        out[col + i] = make_cuDoubleComplex(v, 0.0);
+        reinterpret_cast<double*>(place(at.real))[col + i] = v;
+      } else {
+        out[col + i] = v;
+      }
+    }
+  }
+}
+
+template <class T, int NC, int ROWS, int Threads>
+int launch(int K, int n_shifts, int chains, char* base, int64_t stride, const InvertAt& at,
+           int epoch, cudaStream_t st) {
+  auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
+  constexpr int threads = Threads + 32;
+  const int smem = (int)(sizeof(Shared<T, NC>) + sizeof(T) * NC * (size_t)K);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+      cudaSuccess)
+    return check_launch("ring_invert attribute");
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+    return check_launch("ring_invert occupancy");
+  const int panels = (K + NC - 1) / NC, systems = n_shifts * chains;
+  const int fit = sms * per_sm / panels;  // systems whose CTAs are resident together
+  if (fit < 1) return fail(EB_ERR_CUDA, "ring_invert: the device cannot hold one block's CTAs");
+  for (int z0 = 0; z0 < systems; z0 += fit) {
+    const dim3 grid(panels, std::min(fit, systems - z0));
+    void* args[] = {(void*)&K,      (void*)&z0, (void*)&chains, (void*)&base,
+                    (void*)&stride, (void*)&at, (void*)&epoch};
+    if (cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(threads), args, smem, st) !=
+        cudaSuccess)
+      return check_launch("ring_invert");
+  }
+  return EB_OK;
+}
+
+}  // namespace
+
+int ring_invert(int K, int n_shifts, int chains, char* base, int64_t stride, const InvertAt& at,
+                int epoch, bool real, cudaStream_t st) {
+  if (K < 4 || K > kMaxRows || K % 4 != 0 || n_shifts < 1 || chains < 1 || epoch < 1)
+    return fail(EB_ERR_ARG, "ring_invert: bad sizes");
+  auto run = [&](auto kernel) { return kernel(K, n_shifts, chains, base, stride, at, epoch, st); };
+  // Rows per thread: 128 compute threads (one warp per scheduler: the step's latency grows with the
+  // warps that share one) as long as a thread's rows fit its registers; above K = 512 more
+  // threads, which caps them (K = 1024 real: 1174 us at four rows, 1262 at two; complex: 2246 us at
+  // two rows and 512 threads, 2453 at four and 256).
+  if (real)
+    return K <= 128   ? run(launch<double, 16, 1, 128>)
+           : K <= 256 ? run(launch<double, 16, 2, 128>)
+           : K <= 512 ? run(launch<double, 16, 4, 128>)
+           : K <= 768 ? run(launch<double, 16, 3, 256>)
+                      : run(launch<double, 16, 4, 256>);
+  return K <= 128   ? run(launch<cuDoubleComplex, 8, 1, 128>)
+         : K <= 256 ? run(launch<cuDoubleComplex, 8, 2, 128>)
+         : K <= 512 ? run(launch<cuDoubleComplex, 8, 4, 128>)
+         : K <= 768 ? run(launch<cuDoubleComplex, 8, 3, 256>)
+                    : run(launch<cuDoubleComplex, 8, 2, 512>);
+}
+
+}  // namespace rl
+}  // namespace eb

@@ -31,13 +31,15 @@
 // launch count per ring does not grow with the number of shifts. All device memory comes from
 // the caller's workspace.
 //
-// Gauss-Jordan inversion (blocked, nb columns per panel, implicit row pivoting): the panel
-// kernel runs the nb elimination steps on the panel columns in shared memory (pivot = largest
-// modulus among the rows not yet chosen; in-place storage of the transformation); the update
-// kernel applies the panel's transformation to all other columns as a rank-nb update
+// Gauss-Jordan inversion (implicit row pivoting: the pivot is the largest modulus among the rows
+// not yet chosen; in-place storage of the transformation). For a few shifts one cooperative
+// launch keeps the whole block in the registers of its CTAs (ring_invert.cu). For many shifts
+// the blocked form: the panel kernel runs nb elimination steps on the panel columns, the update
+// kernel applies the panel's transformation to the other columns of a block as a rank-nb update
 // A[:, c] += G R[:, c], R = the panel's pivot rows, G = panel columns minus the unit vectors of
-// the pivot rows. After K steps the working array W holds T P (T = product of the elementary
-// transformations), and the inverse is Dinv[j, p_k] = W[p_j, k] (one permuting copy).
+// the pivot rows, and the block's combined update goes to the rest of the matrix as ZGEMMs. After
+// K steps the working array W holds T P (T = product of the elementary transformations), and the
+// inverse is Dinv[j, p_k] = W[p_j, k] (one permuting copy).
 
 #include <cuda_runtime.h>
 
@@ -51,6 +53,7 @@
 #include "../../include/euler_b200.h"
 #include "dense.cuh"
 #include "physics.cuh"
+#include "ring_invert.cuh"
 
 namespace eb {
 
@@ -98,31 +101,28 @@ int lane_stream(cudaStream_t st, cudaStream_t& out, int lane = 0) {
 
 inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Panel width of the Gauss-Jordan inversion: the largest of 16, 8, 4 that divides K (= 4N) and
-// keeps a thread's panel rows (K / 512 rounded up, at most 2) within 16 complex registers.
-inline int panel_width(int K) {
-  if (K > 1024) return 0;
-  const int rows = (K + 511) / 512;
-  for (int nb = 16; nb >= 4; nb /= 2)
-    if (K % nb == 0 && rows * nb <= 16) return nb;
-  return 0;
-}
+// Rings of at most 1024 unknowns are supported.
+inline bool ring_supported(int K) { return K <= 1024; }
 
-// Width of the Gauss-Jordan column blocks whose trailing update is one ZGEMM (when it divides
-// K and a stream's group has at least kGjBlockMinShifts shifts; otherwise every panel updates
-// the whole block itself). On the 129x129 grid (K = 512) the blocked form takes 0.175 instead
-// of 0.200 ms per ring and shift with 16 shifts per group (0.180 without the look-ahead of
-// invert_ring), breaks even at 4 and stays 8 % slower with one shift even with the look-ahead:
-// the single shift's thin ZGEMMs and extra launches cost more than its streaming passes.
+// Blocked inversion: panels of 16 columns (8 where a panel thread holds two rows), column
+// blocks whose trailing update is one ZGEMM.
+inline int panel_width(int K) { return K <= 512 ? 16 : 8; }
 constexpr int kGjBlock = 64;
+// The blocked form needs whole column blocks and enough shifts per stream to fill the GPU with
+// its panels (one SM per shift): with one shift of the 129x129 grid (K = 512) it took 1.25 ms
+// per ring, with 16 per stream 0.175 ms per ring and shift; the cooperative launch takes 0.56 ms
+// per inversion, two shifts at a time (ring_invert.cu).
 constexpr int kGjBlockMinShifts = 8;
+inline bool blocked_inversion(int K, int shifts_per_stream) {
+  return K % kGjBlock == 0 && shifts_per_stream >= kGjBlockMinShifts;
+}
 
 struct Layout {
   int M, N, K;
   size_t blk;   // bytes of one K x K complex block
   size_t bdr;   // bytes of one ring's block diagonal (N real 4 x 4 blocks)
   size_t off_D, off_L1, off_C1, off_B2, off_C2, off_T, off_L2, off_Rp, off_perm, off_info,
-      off_acc, off_shift;
+      off_flags, off_acc, off_shift;
   size_t off_y, off_x, off_r, off_w;
   size_t total;
 };
@@ -150,6 +150,7 @@ Layout plan(int M, int N) {
   L.off_Rp = take(sizeof(cuDoubleComplex) * (size_t)kGjBlock * L.K);
   L.off_perm = take(sizeof(int) * (size_t)L.K);
   L.off_info = take(sizeof(int) * 4);
+  L.off_flags = take(sizeof(uint64_t) * kInvertFlags);
   L.off_acc = take(sizeof(double) * 2);
   L.off_shift = take(sizeof(double) * 2);
   const size_t vec = sizeof(cuDoubleComplex) * (size_t)L.K * M;
@@ -693,6 +694,7 @@ struct Group {
   char* base;
   int64_t stride;  // bytes
   int S;
+  bool blocked = false;  // how its rings are inverted (see invert_ring)
   int64_t es() const { return stride / (int64_t)sizeof(cuDoubleComplex); }
   cuDoubleComplex* blk(size_t off, int m) const {
     return reinterpret_cast<cuDoubleComplex*>(base + off + L.blk * (size_t)m);
@@ -706,7 +708,7 @@ int check_group(const eb_batch* b, int n_shifts, const void* ws, int64_t stride,
   if (b->n_inst != 1 || b->d_table) return fail(EB_ERR_ARG, "ringlu: single instance only");
   if (n_shifts < 1 || n_shifts > 65535 || !ws) return fail(EB_ERR_ARG, "ringlu: bad shifts or workspace");
   const int M = b->single.M, N = b->single.N;
-  if (M < 4 || N < 5 || panel_width(4 * N) == 0) return fail(EB_ERR_ARG, "ringlu: unsupported grid size");
+  if (M < 4 || N < 5 || !ring_supported(4 * N)) return fail(EB_ERR_ARG, "ringlu: unsupported grid size");
   L = plan(M, N);
   if (stride < (int64_t)L.total || stride % 256 != 0)
     return fail(EB_ERR_ARG, "ringlu: workspace stride too small or not a multiple of 256");
@@ -726,33 +728,27 @@ void gj_pass(const Group& g, int j0, int c_lo, int c_hi, size_t off_in, size_t o
                                                     off_out, g.L.off_perm, g.L.off_info);
 }
 
-void gj_pass_any(const Group& g, int nb, int rows, int j0, int c_lo, int c_hi, size_t in,
-                 size_t out, cudaStream_t st) {
-  if (rows == 1) {
-    if (nb == 16) gj_pass<16, 1>(g, j0, c_lo, c_hi, in, out, st);
-    else if (nb == 8) gj_pass<8, 1>(g, j0, c_lo, c_hi, in, out, st);
-    else gj_pass<4, 1>(g, j0, c_lo, c_hi, in, out, st);
-  } else {
-    if (nb == 8) gj_pass<8, 2>(g, j0, c_lo, c_hi, in, out, st);
-    else gj_pass<4, 2>(g, j0, c_lo, c_hi, in, out, st);
-  }
+void gj_pass_any(const Group& g, int nb, int j0, int c_lo, int c_hi, size_t in, size_t out,
+                 cudaStream_t st) {
+  if (nb == 16) gj_pass<16, 1>(g, j0, c_lo, c_hi, in, out, st);  // K <= 512
+  else gj_pass<8, 2>(g, j0, c_lo, c_hi, in, out, st);
 }
 
-// D_m <- D_m^-1 for every shift by Gauss-Jordan with implicit row pivoting (ping-pong between
-// D_m and the scratch block T). In the blocked form the columns go in blocks of kGjBlock:
-// the panels of a block update only the block's columns (an even number of passes, so the
-// block ends in D_m), and the rest of D_m takes the block's combined rank-kGjBlock update as
-// strided-batched ZGEMMs (tensor-core DMMA) instead of kGjBlock / nb streaming passes.
+// D_m <- D_m^-1 for every shift by Gauss-Jordan with implicit row pivoting: for a few shifts one
+// cooperative launch (ring_invert.cu), for many the blocked form, whose columns go in blocks of
+// kGjBlock: the panels of a block update only the block's columns (ping-pong with the scratch
+// block T, an even number of passes, so the block ends in D_m), and the rest of D_m takes the
+// block's combined rank-kGjBlock update as strided-batched ZGEMMs (tensor-core DMMA).
 int invert_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
-  const int K = L.K, nb = panel_width(K), rows = (K + kPanelThreads - 1) / kPanelThreads;
+  const int K = L.K, nb = panel_width(K);
   const size_t buf[2] = {g.boff(L.off_D, m), L.off_T};
-  const int passes = K / nb;
-  const bool blocked = K % kGjBlock == 0 && (kGjBlock / nb) % 2 == 0 && g.S >= kGjBlockMinShifts;
-  if (!blocked) {
-    for (int p = 0; p < passes; ++p)
-      gj_pass_any(g, nb, rows, p * nb, 0, K, buf[p & 1], buf[(p + 1) & 1], st);
-  } else {
+  if (!g.blocked) {
+    const InvertAt at{{(int64_t)buf[0], 0}, {(int64_t)L.off_T, 0}, {(int64_t)buf[0], 0}, {},
+                      {(int64_t)L.off_flags, 0}, {(int64_t)L.off_info, 0}};
+    return ring_invert(K, g.S, 1, g.base, g.stride, at, m + 1, false, st);
+  }
+  {
     // Look-ahead: the block's update of the next block's columns runs on st, right before the
     // next block's panels; its update of every other column runs on the side stream, under
     // those panels. st waits for the side stream before it moves the next pivot rows (which
@@ -773,7 +769,7 @@ int invert_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
     bool side_busy = false;
     for (int b0 = 0; b0 < K; b0 += kGjBlock) {
       for (int q = 0; q < kGjBlock / nb; ++q)
-        gj_pass_any(g, nb, rows, b0 + q * nb, b0, b0 + kGjBlock, buf[q & 1], buf[(q + 1) & 1], st);
+        gj_pass_any(g, nb, b0 + q * nb, b0, b0 + kGjBlock, buf[q & 1], buf[(q + 1) & 1], st);
       if (K == kGjBlock) break;
       if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
         return check_launch("ringlu side join");
@@ -792,12 +788,10 @@ int invert_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
     if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
       return check_launch("ringlu side join");
   }
-  const size_t W = blocked ? buf[0] : buf[passes & 1];
-  const size_t other = blocked ? buf[1] : buf[(passes + 1) & 1];
+  const size_t W = buf[0], other = buf[1];
   k_gj_permute<<<dim3(std::min(K, 1024), g.S), 256, sizeof(int) * K, st>>>(K, g.base, g.stride, W, other,
                                                                           L.off_perm, L.off_info);
-  if (other != buf[0] &&
-      cudaMemcpy2DAsync(g.base + buf[0], g.stride, g.base + other, g.stride, L.blk, g.S,
+  if (cudaMemcpy2DAsync(g.base + buf[0], g.stride, g.base + other, g.stride, L.blk, g.S,
                         cudaMemcpyDeviceToDevice, st) != cudaSuccess)
     return check_launch("ringlu inverse copy");
   return EB_OK;
@@ -1065,7 +1059,7 @@ using namespace eb::rl;
 extern "C" {
 
 int64_t eb_ringlu_workspace_bytes(int M, int N) {
-  if (M < 4 || N < 5 || panel_width(4 * N) == 0) return -1;
+  if (M < 4 || N < 5 || !ring_supported(4 * N)) return -1;
   return (int64_t)plan(M, N).total;
 }
 
@@ -1085,7 +1079,7 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   for (int s = 0; s < n_shifts; ++s) {
     char* w = g.base + (int64_t)s * g.stride;
     cudaMemsetAsync(w, 0, L.off_T, st);  // the stored super-blocks and block diagonals
-    cudaMemsetAsync(w + L.off_info, 0, sizeof(int) * 4, st);
+    cudaMemsetAsync(w + L.off_info, 0, L.off_acc - L.off_info, st);  // and the panel flags
     k_assemble<<<grid_for((int64_t)M * N * 9, 256), 256, 0, st>>>(
         M, N, J[s], reinterpret_cast<const double*>(w + L.off_shift),
         reinterpret_cast<cuDoubleComplex*>(w + L.off_D), reinterpret_cast<cuDoubleComplex*>(w + L.off_L1),
@@ -1093,7 +1087,8 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
         reinterpret_cast<double*>(w + L.off_C2));
   }
   if ((rc = check_launch("ringlu assemble")) != EB_OK) return rc;
-  if (n_shifts == 1) {
+  if (!blocked_inversion(L.K, (n_shifts + 1) / 2)) {
+    // one stream: the inversions are cooperative launches, which never run two at a time here
     for (int m = 0; m < M; ++m)
       if ((rc = factor_ring(g, m, st, 2)) != EB_OK) return rc;
     return EB_OK;
@@ -1104,8 +1099,8 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   if ((rc = lane_stream(st, s2, 1)) != EB_OK) return rc;
   const Handle& lane = g_handle[1];
   const int s1 = (n_shifts + 1) / 2;
-  const Group g1{L, g.base, g.stride, s1};
-  const Group g2{L, g.base + (int64_t)s1 * g.stride, g.stride, n_shifts - s1};
+  const Group g1{L, g.base, g.stride, s1, true};
+  const Group g2{L, g.base + (int64_t)s1 * g.stride, g.stride, n_shifts - s1, true};
   cudaEventRecord(lane.start, st);
   cudaStreamWaitEvent(lane.stream, lane.start, 0);
   for (int m = 0; m < M; ++m) {
@@ -1519,7 +1514,7 @@ int ptc_stream(cudaStream_t& out) {
 extern "C" {
 
 int64_t eb_ptc_workspace_bytes(int M, int N, int max_steps) {
-  if (M < 4 || N < 5 || panel_width(4 * N) == 0 || max_steps < 1) return -1;
+  if (M < 4 || N < 5 || !ring_supported(4 * N) || max_steps < 1) return -1;
   return (int64_t)ptc_plan(M, N, max_steps).total;
 }
 
@@ -1539,7 +1534,7 @@ int eb_ptc_run(const eb_batch* b, const double* X, const double* V, double* U, d
     return fail(EB_ERR_ARG, "ptc: workspace not 256-byte aligned");
   if (max_steps < 1 || !(ser > 0) || !(rtol >= 0)) return fail(EB_ERR_ARG, "ptc: bad options");
   const int M = b->single.M, N = b->single.N;
-  if (M < 4 || N < 5 || panel_width(4 * N) == 0) return fail(EB_ERR_ARG, "ptc: unsupported grid size");
+  if (M < 4 || N < 5 || !ring_supported(4 * N)) return fail(EB_ERR_ARG, "ptc: unsupported grid size");
   const PtcLayout P = ptc_plan(M, N, max_steps);
   if (workspace_bytes < (int64_t)P.total) return fail(EB_ERR_ARG, "ptc: workspace too small");
   // the loop runs on a stream of its own, after the work queued on the caller's stream (and
