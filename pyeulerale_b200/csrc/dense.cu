@@ -39,6 +39,28 @@ constexpr int kGemmThreads = 128;
 constexpr int kPadM = kBM + 4;
 constexpr int kPadK = kBK + 4;
 
+// Operands of batch entry z: strided from three bases, or entry z % n of workspace z / n.
+struct Operands {
+  const char *a, *b;
+  char* c;
+  int64_t sa, sb, sc;  // bytes
+  Products set;        // set.n == 0: strided
+  template <class T>
+  __device__ __forceinline__ void of(int64_t z, const T*& A, const T*& B, T*& C) const {
+    int64_t oa = sa * z, ob = sb * z, oc = sc * z;
+    if (set.n > 0) {
+      const int64_t s = z / set.n;
+      const int e = (int)(z % set.n);
+      oa = sa * s + set.a[e];
+      ob = sb * s + set.b[e];
+      oc = sc * s + set.c[e];
+    }
+    A = reinterpret_cast<const T*>(a + oa);
+    B = reinterpret_cast<const T*>(b + ob);
+    C = reinterpret_cast<T*>(c + oc);
+  }
+};
+
 struct GemmSmem {
   double ar[2][kBK][kPadM], ai[2][kBK][kPadM];
   double br[2][kBN][kPadK], bi[2][kBN][kPadK];
@@ -104,15 +126,13 @@ __device__ __forceinline__ void store_slice(GemmSmem& S, int buf, const double2 
 }
 
 __global__ void __launch_bounds__(kGemmThreads)
-    k_zgemm_nn(int M, int N, int K, double alpha, const double2* A, int lda, int64_t sa,
-               const double2* B, int ldb, int64_t sb, double beta, double2* C, int ldc,
-               int64_t sc) {
+    k_zgemm_nn(int M, int N, int K, double alpha, Operands ops, int lda, int ldb, double beta,
+               int ldc) {
   extern __shared__ __align__(16) unsigned char zg_smem[];
   GemmSmem& S = *reinterpret_cast<GemmSmem*>(zg_smem);
-  const int64_t z = blockIdx.z;
-  A += sa * z;
-  B += sb * z;
-  C += sc * z;
+  const double2 *A, *B;
+  double2* C;
+  ops.of(blockIdx.z, A, B, C);
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // the warp's 32 x 32 sub-tile
@@ -218,17 +238,15 @@ __device__ __forceinline__ void cp_async_wait() {
 
 template <int BN, int Stages>
 __global__ void __launch_bounds__(kGemmThreads)
-    k_zgemm_nn_async(int M, int N, int K, double alpha, const double2* A, int lda, int64_t sa,
-                     const double2* B, int ldb, int64_t sb, double beta, double2* C, int ldc,
-                     int64_t sc) {
+    k_zgemm_nn_async(int M, int N, int K, double alpha, Operands ops, int lda, int ldb,
+                     double beta, int ldc) {
   constexpr int NJ = BN / 16;                        // 8-column fragments per warp
   constexpr int kBPerT = kBK * BN / kGemmThreads;   // B elements per thread and slice
   extern __shared__ __align__(16) unsigned char zg_smem[];
   AsyncSmem<BN, Stages>& S = *reinterpret_cast<AsyncSmem<BN, Stages>*>(zg_smem);
-  const int64_t z = blockIdx.z;
-  A += sa * z;
-  B += sb * z;
-  C += sc * z;
+  const double2 *A, *B;
+  double2* C;
+  ops.of(blockIdx.z, A, B, C);
   const int tid = threadIdx.x;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
   const int lane = tid & 31, warp = tid >> 5;
@@ -318,10 +336,10 @@ __global__ void __launch_bounds__(kGemmThreads)
 
 }  // namespace
 
-int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A, int lda,
-                     int64_t stride_a, const cuDoubleComplex* B, int ldb, int64_t stride_b,
-                     double beta, cuDoubleComplex* C, int ldc, int64_t stride_c, int batch,
-                     cudaStream_t st, int variant) {
+namespace {
+
+int launch_zgemm(int M, int N, int K, double alpha, double beta, const Operands& ops, int lda,
+                 int ldb, int ldc, int batch, int variant, cudaStream_t st) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (variant < 0) {  // the default, or EB_ZGEMM=v<k> (measurements of the variants in place)
     const char* e = std::getenv("EB_ZGEMM");
@@ -338,149 +356,203 @@ int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A
       cudaSuccess)
     return check_launch("zgemm attribute");
   const dim3 grid((M + kBM - 1) / kBM, (N + bn - 1) / bn, batch);
-  kernel<<<grid, kGemmThreads, smem, st>>>(
-      M, N, K, alpha, reinterpret_cast<const double2*>(A), lda, stride_a,
-      reinterpret_cast<const double2*>(B), ldb, stride_b, beta, reinterpret_cast<double2*>(C),
-      ldc, stride_c);
+  kernel<<<grid, kGemmThreads, smem, st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
   return check_launch("zgemm");
+}
+
+}  // namespace
+
+int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A, int lda,
+                     int64_t stride_a, const cuDoubleComplex* B, int ldb, int64_t stride_b,
+                     double beta, cuDoubleComplex* C, int ldc, int64_t stride_c, int batch,
+                     cudaStream_t st, int variant) {
+  constexpr int64_t kB = sizeof(cuDoubleComplex);
+  const Operands ops{reinterpret_cast<const char*>(A), reinterpret_cast<const char*>(B),
+                     reinterpret_cast<char*>(C), kB * stride_a, kB * stride_b, kB * stride_c, {}};
+  return launch_zgemm(M, N, K, alpha, beta, ops, lda, ldb, ldc, batch, variant, st);
+}
+
+int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st) {
+  const Operands ops{base, base, base, stride, stride, stride, set};
+  return launch_zgemm(M, N, K, alpha, beta, ops, lda, ldb, ldc, workspaces * set.n, -1, st);
 }
 
 namespace {
 
-// y = alpha A x + beta y: a CTA of 256 threads takes 32 rows; thread (r, g) sums the columns
-// j = g (mod 8) of row r (a warp reads 32 consecutive rows of one column), the eight partial sums
-// of a row are added in a fixed order through shared memory.
-__global__ void __launch_bounds__(256) k_zgemv_n(int n, double alpha, const double2* A, int lda,
-                                                 int64_t sa, const double2* x, int64_t sx,
-                                                 double beta, double2* y, int64_t sy) {
-  __shared__ double2 part[8][32];
-  const int64_t z = blockIdx.y;
-  A += sa * z;
-  x += sx * z;
-  y += sy * z;
-  const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + r;
+// (Bd v)[i] or (Bd^T v)[i] for one entry i of a block diagonal of real 4 x 4 blocks.
+__device__ __forceinline__ double2 bd_entry(const double* bd, const double2* v, int i, bool trans) {
+  const double* b = bd + 16 * (i >> 2);
+  const double2* u = v + (i & ~3);
+  const int r = i & 3;
+  double2 o = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double w = trans ? b[k + 4 * r] : b[r + 4 * k];
+    o.x = fma(w, u[k].x, o.x);
+    o.y = fma(w, u[k].y, o.y);
+  }
+  return o;
+}
+
+template <class T>
+__device__ __forceinline__ T* place(char* ws, int64_t off) {
+  return reinterpret_cast<T*>(ws + off);
+}
+
+// y[i] of one row: the sum of the products, the block-diagonal term and the previous y.
+__device__ __forceinline__ void finish_row(const SweepTerm& t, char* ws, int i, double sr,
+                                           double si, bool trans) {
+  double2* y = place<double2>(ws, t.y) + i;
+  double2 o = make_double2(sr, si);
+  if (t.add) {
+    o.x += y->x;
+    o.y += y->y;
+  }
+  if (t.bd >= 0) {
+    const double2 b = bd_entry(place<const double>(ws, t.bd), place<const double2>(ws, t.v), i, trans);
+    o.x -= b.x;
+    o.y -= b.y;
+  }
+  *y = o;
+}
+
+// Sweep step, op(A) = A. What bounds a step is latency: a few dependent loads and one launch, so
+// a product is spread thin, eight rows per CTA (K = 512: 64 CTAs of 64 KB each; with 32 rows per
+// CTA each of 16 SMs streamed 256 KB). Thread (r, g) sums the columns j = g (mod 32) of row r;
+// the partial sums are added in a fixed order. Grid: (row groups x terms, workspaces).
+__global__ void __launch_bounds__(256) k_sweep_n(int n, char* base, int64_t stride,
+                                                 SweepTerms terms) {
+  __shared__ double2 part[8][8];
+  const SweepTerm t = terms.t[blockIdx.x % terms.n];
+  const int group = blockIdx.x / terms.n;
+  char* ws = base + stride * blockIdx.y;
+  const int r = threadIdx.x & 7, g = threadIdx.x >> 3, lane = threadIdx.x & 31;
+  const int i = group * 8 + r;
   double sr = 0.0, si = 0.0;
-  if (i < n) {
+  if (i < n && t.a >= 0) {
+    const double2* A = place<const double2>(ws, t.a) + i;
+    const double2* x = place<const double2>(ws, t.x);
     constexpr int kUnroll = 8;  // column loads in flight per thread (ldg_inflight)
     int j = g;
-    for (; j + 8 * (kUnroll - 1) < n; j += 8 * kUnroll) {
+    for (; j + 32 * (kUnroll - 1) < n; j += 32 * kUnroll) {
       double2 a[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(A + i + (int64_t)lda * (j + 8 * u));
+      for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(A + (int64_t)n * (j + 32 * u));
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        const double2 v = x[j + 8 * u];
+        const double2 v = x[j + 32 * u];
         sr = fma(a[u].x, v.x, fma(-a[u].y, v.y, sr));
         si = fma(a[u].x, v.y, fma(a[u].y, v.x, si));
       }
     }
-    for (; j < n; j += 8) {
-      const double2 a = A[i + (int64_t)lda * j], v = x[j];
+    for (; j < n; j += 32) {
+      const double2 a = ldg_inflight(A + (int64_t)n * j), v = x[j];
       sr = fma(a.x, v.x, fma(-a.y, v.y, sr));
       si = fma(a.x, v.y, fma(a.y, v.x, si));
     }
   }
-  part[g][r] = make_double2(sr, si);
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+    si += __shfl_xor_sync(0xffffffffu, si, o);
+  }
+  if (lane < 8) part[threadIdx.x >> 5][lane] = make_double2(sr, si);
   __syncthreads();
-  if (g == 0 && i < n) {
+  if (threadIdx.x < 8 && i < n) {
     double tr = 0.0, ti = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      tr += part[k][r].x;
-      ti += part[k][r].y;
+      tr += part[k][threadIdx.x].x;
+      ti += part[k][threadIdx.x].y;
     }
-    double2 out = make_double2(alpha * tr, alpha * ti);
-    if (beta != 0.0) {
-      out.x = fma(beta, y[i].x, out.x);
-      out.y = fma(beta, y[i].y, out.y);
-    }
-    y[i] = out;
+    finish_row(t, ws, i, t.alpha * tr, t.alpha * ti, false);
   }
 }
 
-// y = alpha A^H x + beta y: one warp per output j (column j of A, read by the lanes in
-// consecutive rows), a fixed shuffle tree adds the lanes' partial sums.
-__global__ void __launch_bounds__(256) k_zgemv_c(int n, double alpha, const double2* A, int lda,
-                                                 int64_t sa, const double2* x, int64_t sx,
-                                                 double beta, double2* y, int64_t sy) {
-  const int64_t z = blockIdx.y;
-  A += sa * z;
-  x += sx * z;
-  y += sy * z;
+// Sweep step, op(A) = A^H: one warp per output (a column of A), the vectors in shared memory; a
+// fixed shuffle tree adds the lanes' partial sums. Grid: (groups of eight outputs x terms,
+// workspaces).
+__global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stride,
+                                                 SweepTerms terms) {
+  extern __shared__ __align__(16) unsigned char sw_smem[];
+  double2* xs = reinterpret_cast<double2*>(sw_smem);  // x, then Bd2^T v2
+  const SweepTerm t = terms.t[blockIdx.x % terms.n];
+  const int group = blockIdx.x / terms.n;
+  char* ws = base + stride * blockIdx.y;
   const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int j = group * 8 + (threadIdx.x >> 5);
+  for (int i = threadIdx.x; i < n; i += 256) {
+    if (t.a >= 0) xs[i] = place<const double2>(ws, t.x)[i];
+    if (t.a2 >= 0)
+      xs[n + i] = bd_entry(place<const double>(ws, t.bd2), place<const double2>(ws, t.v2), i, true);
+  }
+  __syncthreads();
   if (j >= n) return;
-  const double2* col = A + (int64_t)lda * j;
   double sr = 0.0, si = 0.0;
-  constexpr int kUnroll = 8;  // row loads in flight per lane (ldg_inflight)
-  int i = lane;
-  for (; i + 32 * (kUnroll - 1) < n; i += 32 * kUnroll) {  // conj(a) v
-    double2 a[kUnroll];
+  auto dot = [&](const double2* col, const double2* v, double alpha) {
+    double tr = 0.0, ti = 0.0;
+    constexpr int kUnroll = 8;  // row loads in flight per lane (ldg_inflight)
+    int i = lane;
+    for (; i + 32 * (kUnroll - 1) < n; i += 32 * kUnroll) {  // conj(a) v
+      double2 a[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(col + i + 32 * u);
+      for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(col + i + 32 * u);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const double2 v = x[i + 32 * u];
-      sr = fma(a[u].x, v.x, fma(a[u].y, v.y, sr));
-      si = fma(a[u].x, v.y, fma(-a[u].y, v.x, si));
+      for (int u = 0; u < kUnroll; ++u) {
+        const double2 w = v[i + 32 * u];
+        tr = fma(a[u].x, w.x, fma(a[u].y, w.y, tr));
+        ti = fma(a[u].x, w.y, fma(-a[u].y, w.x, ti));
+      }
     }
-  }
-  for (; i < n; i += 32) {
-    const double2 a = col[i], v = x[i];
-    sr = fma(a.x, v.x, fma(a.y, v.y, sr));
-    si = fma(a.x, v.y, fma(-a.y, v.x, si));
-  }
+    for (; i < n; i += 32) {
+      const double2 a = ldg_inflight(col + i), w = v[i];
+      tr = fma(a.x, w.x, fma(a.y, w.y, tr));
+      ti = fma(a.x, w.y, fma(-a.y, w.x, ti));
+    }
+    sr = fma(alpha, tr, sr);
+    si = fma(alpha, ti, si);
+  };
+  if (t.a >= 0) dot(place<const double2>(ws, t.a) + (int64_t)n * j, xs, t.alpha);
+  if (t.a2 >= 0) dot(place<const double2>(ws, t.a2) + (int64_t)n * j, xs + n, -1.0);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     sr += __shfl_xor_sync(0xffffffffu, sr, o);
     si += __shfl_xor_sync(0xffffffffu, si, o);
   }
-  if (lane == 0) {
-    double2 out = make_double2(alpha * sr, alpha * si);
-    if (beta != 0.0) {
-      out.x = fma(beta, y[j].x, out.x);
-      out.y = fma(beta, y[j].y, out.y);
-    }
-    y[j] = out;
-  }
+  if (lane == 0) finish_row(t, ws, j, sr, si, true);
 }
 
-// C = alpha A B + beta C with A n x n and B, C n x nr (nr <= kMaxRhs right-hand sides): the
-// multi-right-hand-side form of k_zgemv_n (one read of A serves all nr columns). A cluster of
+// The sweep step over nr right-hand sides (one read of A serves all of them). A cluster of
 // kSkCluster CTAs takes 32 rows: CTA c of the cluster sums the columns of its contiguous share,
 // thread (r, g) of its 256 the columns j = g (mod 8) of that share for row r and every
 // right-hand side, with eight column loads in flight; the eight warps' partial sums are added
 // in a fixed order in shared memory, and the cluster's leader adds the CTAs' partial sums in
-// rank order through distributed shared memory and writes C. Spreading a product over the
+// rank order through distributed shared memory and writes y. Spreading a product over the
 // cluster puts eight SMs' loads in flight where one CTA per 32 rows left each SM streaming
-// its 256 KB share alone. Batch entry z (grid z) uses A + zmap[z] sa etc. (zmap == nullptr: z
-// itself); entries z >= *n_batch exit (the whole cluster alike). With bd != nullptr the
-// epilogue also subtracts Bd V, Bd being n / 4 real 4 x 4 blocks (column-major) at
-// bd + zmap[z] bd_stride bytes and V (n x nr, leading dimension ldc) at V + zmap[z] sv: the ring
-// LU's block-diagonal coupling, fused into the product that precedes it.
+// its 256 KB share alone. Grid: (row groups x terms, cluster, workspaces); workspaces from
+// *n_active on exit (the whole cluster alike).
 constexpr int kMaxRhs = 8;
 constexpr int kSkCluster = 8;
 
 __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
-    k_zgemm_skinny(int n, int nr, double alpha, const double2* A, int lda, int64_t sa,
-                   const double2* B, int ldb, int64_t sb, double beta, double2* C, int ldc,
-                   int64_t sc, const int* zmap, const int* n_batch, const char* bd,
-                   int64_t bd_stride, const double2* V, int64_t sv) {
+    k_sweep_multi(int n, int nr, const char* base, int64_t stride, char* vectors, int64_t vstride,
+                  const int* zmap, const int* n_active, SweepTerms terms) {
   extern __shared__ __align__(16) unsigned char sk_smem[];
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  if (n_batch && (int)blockIdx.z >= *n_batch) return;  // uniform over the cluster
-  const int64_t z = zmap ? zmap[blockIdx.z] : blockIdx.z;
-  A += sa * z;
-  B += sb * z;
-  C += sc * z;
-  const double* Bd = bd ? reinterpret_cast<const double*>(bd + bd_stride * z) : nullptr;
-  if (V) V += sv * z;
+  if ((int)blockIdx.z >= *n_active) return;  // uniform over the cluster
+  const SweepTerm t = terms.t[blockIdx.x % terms.n];
+  const int group = blockIdx.x / terms.n;
+  const int64_t z = zmap[blockIdx.z];
+  const char* ws = base + stride * z;
+  char* vs = vectors + vstride * z;
+  const double2* A = reinterpret_cast<const double2*>(ws + t.a);
+  const double2* B = place<const double2>(vs, t.x);
   const int rank = (int)cluster.block_rank();
   const int share = (((n + kSkCluster - 1) / kSkCluster) + 7) / 8 * 8;  // columns per CTA
   const int j0 = rank * share, j1 = min(n, j0 + share);
-  const int cols = max(j1 - j0, 0);
+  const int cols = t.a >= 0 ? max(j1 - j0, 0) : 0;
   double2* Bs = reinterpret_cast<double2*>(sk_smem);  // cols x nr (this CTA's rows of B)
   double2* part = Bs + (size_t)share * nr;            // 8 x 32 x nr, then the CTA's 32 x nr
   const int total = cols * nr;
@@ -491,7 +563,7 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
       const int e = e0 + 256 * u + (int)threadIdx.x;
       if (e < total) {
         const int q = e / cols, j = e - q * cols;
-        b[u] = ldg_inflight(B + j0 + j + (int64_t)ldb * q);
+        b[u] = ldg_inflight(B + j0 + j + (int64_t)n * q);
       }
     }
 #pragma unroll
@@ -502,7 +574,7 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
   }
   __syncthreads();
   const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + r;
+  const int i = group * 32 + r;
   double sr[kMaxRhs], si[kMaxRhs];
 #pragma unroll
   for (int q = 0; q < kMaxRhs; ++q) sr[q] = si[q] = 0.0;
@@ -513,7 +585,7 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
       double2 a[kUnroll];
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u)
-        a[u] = ldg_inflight(A + i + (int64_t)lda * (j0 + j + 8 * u));
+        a[u] = ldg_inflight(A + i + (int64_t)n * (j0 + j + 8 * u));
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u)
 #pragma unroll
@@ -526,7 +598,7 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
         }
     }
     for (; j < cols; j += 8) {
-      const double2 a = A[i + (int64_t)lda * (j0 + j)];
+      const double2 a = A[i + (int64_t)n * (j0 + j)];
 #pragma unroll
       for (int q = 0; q < kMaxRhs; ++q) {
         if (q < nr) {
@@ -557,7 +629,7 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
   if (rank == 0) {
     for (int e = threadIdx.x; e < 32 * nr; e += 256) {
       const int q = e >> 5, rr = e & 31;
-      const int row = blockIdx.x * 32 + rr;
+      const int row = group * 32 + rr;
       double tr = 0.0, ti = 0.0;
       for (int c = 0; c < kSkCluster; ++c) {
         const double2* other = cluster.map_shared_rank(mine, c);
@@ -566,22 +638,17 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
         ti += v.y;
       }
       if (row < n) {
-        double2* out = C + row + (int64_t)ldc * q;
-        double2 o = make_double2(alpha * tr, alpha * ti);
-        if (beta != 0.0) {
-          o.x = fma(beta, out->x, o.x);
-          o.y = fma(beta, out->y, o.y);
+        double2* out = place<double2>(vs, t.y) + row + (int64_t)n * q;
+        double2 o = make_double2(t.alpha * tr, t.alpha * ti);
+        if (t.add) {
+          o.x += out->x;
+          o.y += out->y;
         }
-        if (Bd) {  // - Bd V for row = 4 blk + rr4
-          const int blk = row >> 2, rr4 = row & 3;
-          const double* b = Bd + 16 * blk;
-          const double2* v = V + (int64_t)ldc * q + 4 * blk;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const double bk = b[rr4 + 4 * k];
-            o.x = fma(-bk, v[k].x, o.x);
-            o.y = fma(-bk, v[k].y, o.y);
-          }
+        if (t.bd >= 0) {
+          const double2 b = bd_entry(reinterpret_cast<const double*>(ws + t.bd),
+                                     place<const double2>(vs, t.v) + (int64_t)n * q, row, false);
+          o.x -= b.x;
+          o.y -= b.y;
         }
         *out = o;
       }
@@ -592,42 +659,32 @@ __global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
 
 }  // namespace
 
-int zgemv_batched(int conj_trans, int n, double alpha, const cuDoubleComplex* A, int lda,
-                  int64_t stride_a, const cuDoubleComplex* x, int64_t stride_x, double beta,
-                  cuDoubleComplex* y, int64_t stride_y, int batch, cudaStream_t st) {
-  if (n <= 0 || batch <= 0) return 0;
-  const double2* a = reinterpret_cast<const double2*>(A);
-  const double2* v = reinterpret_cast<const double2*>(x);
-  double2* w = reinterpret_cast<double2*>(y);
+int sweep_product(int conj_trans, int n, char* base, int64_t stride, int workspaces,
+                  const SweepTerms& terms, cudaStream_t st) {
+  if (n <= 0 || workspaces <= 0 || terms.n <= 0) return 0;
+  const dim3 grid((n + 7) / 8 * terms.n, workspaces);
   if (conj_trans)
-    k_zgemv_c<<<dim3((n + 7) / 8, batch), 256, 0, st>>>(n, alpha, a, lda, stride_a, v, stride_x,
-                                                        beta, w, stride_y);
+    k_sweep_h<<<grid, 256, 2 * sizeof(double2) * (size_t)n, st>>>(n, base, stride, terms);
   else
-    k_zgemv_n<<<dim3((n + 31) / 32, batch), 256, 0, st>>>(n, alpha, a, lda, stride_a, v,
-                                                          stride_x, beta, w, stride_y);
-  return check_launch("zgemv");
+    k_sweep_n<<<grid, 256, 0, st>>>(n, base, stride, terms);
+  return check_launch("sweep product");
 }
 
-int zgemm_skinny_batched(int n, int nr, double alpha, const cuDoubleComplex* A, int lda,
-                         int64_t stride_a, const cuDoubleComplex* B, int ldb, int64_t stride_b,
-                         double beta, cuDoubleComplex* C, int ldc, int64_t stride_c, int batch,
-                         const int* zmap, const int* n_batch, cudaStream_t st, const void* bd,
-                         int64_t bd_stride, const cuDoubleComplex* V, int64_t stride_v) {
-  if (bd && n % 4 != 0) return fail(EB_ERR_ARG, "zgemm_skinny: block diagonal needs n % 4 == 0");
-  if (n <= 0 || batch <= 0 || nr <= 0) return 0;
-  if (nr > kMaxRhs) return fail(EB_ERR_ARG, "zgemm_skinny: too many right-hand sides");
+int sweep_product_multi(int n, int nr, char* base, int64_t stride, char* vectors, int64_t vstride,
+                        int workspaces, const int* zmap, const int* n_active,
+                        const SweepTerms& terms, cudaStream_t st) {
+  if (n % 4 != 0) return fail(EB_ERR_ARG, "sweep: block diagonals need n % 4 == 0");
+  if (n <= 0 || workspaces <= 0 || nr <= 0 || terms.n <= 0) return 0;
+  if (nr > kMaxRhs) return fail(EB_ERR_ARG, "sweep: too many right-hand sides");
   const int share = (((n + kSkCluster - 1) / kSkCluster) + 7) / 8 * 8;
   const size_t smem = sizeof(double2) * ((size_t)share * nr + 9 * 32 * (size_t)nr);
-  if (smem > 200 * 1024) return fail(EB_ERR_ARG, "zgemm_skinny: right-hand sides too large");
-  if (cudaFuncSetAttribute(k_zgemm_skinny, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (smem > 200 * 1024) return fail(EB_ERR_ARG, "sweep: right-hand sides too large");
+  if (cudaFuncSetAttribute(k_sweep_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
-    return check_launch("zgemm_skinny attribute");
-  k_zgemm_skinny<<<dim3((n + 31) / 32, kSkCluster, batch), 256, smem, st>>>(
-      n, nr, alpha, reinterpret_cast<const double2*>(A), lda, stride_a,
-      reinterpret_cast<const double2*>(B), ldb, stride_b, beta, reinterpret_cast<double2*>(C),
-      ldc, stride_c, zmap, n_batch, static_cast<const char*>(bd), bd_stride,
-      reinterpret_cast<const double2*>(V), stride_v);
-  return check_launch("zgemm_skinny");
+    return check_launch("sweep attribute");
+  k_sweep_multi<<<dim3((n + 31) / 32 * terms.n, kSkCluster, workspaces), 256, smem, st>>>(
+      n, nr, base, stride, vectors, vstride, zmap, n_active, terms);
+  return check_launch("sweep product");
 }
 
 }  // namespace dense

@@ -23,25 +23,47 @@ int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A
                      double beta, cuDoubleComplex* C, int ldc, int64_t stride_c, int batch,
                      cudaStream_t st, int variant = -1);
 
-// y_z = alpha op(A_z) x_z + beta y_z for z < batch, A_z square n x n column-major (lda),
-// op(A) = A (conj_trans = 0) or A^H (conj_trans = 1); alpha, beta real; beta == 0 does not
-// read y. x and y contiguous; strides in elements.
-int zgemv_batched(int conj_trans, int n, double alpha, const cuDoubleComplex* A, int lda,
-                  int64_t stride_a, const cuDoubleComplex* x, int64_t stride_x, double beta,
-                  cuDoubleComplex* y, int64_t stride_y, int batch, cudaStream_t st);
+// Products inside a set of workspaces: entry e < n of workspace s multiplies the matrices at
+// byte offsets a[e], b[e], c[e] of base + stride s.
+struct Products {
+  int n = 0;
+  int64_t a[4], b[4], c[4];
+  void add(int64_t pa, int64_t pb, int64_t pc) {
+    a[n] = pa;
+    b[n] = pb;
+    c[n++] = pc;
+  }
+};
+// C = alpha A B + beta C for every entry of every workspace (complex).
+int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st);
 
-// C_z = alpha A_z B_z + beta C_z with A_z n x n and B_z, C_z n x nr (nr <= 8 right-hand
-// sides), column-major; batch entry z uses A + zmap[z] stride_a (etc.; zmap == nullptr: z), and
-// entries z >= *n_batch (device int; n_batch == nullptr: all) do nothing. beta == 0 does not
-// read C. With bd != nullptr, C_z also takes - Bd_z V_z: Bd_z = n / 4 real column-major 4 x 4
-// blocks at (const char*) bd + zmap[z] bd_stride, V_z (n x nr, leading dimension ldc) at
-// V + zmap[z] stride_v. Returns an EB_* status.
-int zgemm_skinny_batched(int n, int nr, double alpha, const cuDoubleComplex* A, int lda,
-                         int64_t stride_a, const cuDoubleComplex* B, int ldb, int64_t stride_b,
-                         double beta, cuDoubleComplex* C, int ldc, int64_t stride_c, int batch,
-                         const int* zmap, const int* n_batch, cudaStream_t st,
-                         const void* bd = nullptr, int64_t bd_stride = 0,
-                         const cuDoubleComplex* V = nullptr, int64_t stride_v = 0);
+// One matrix-vector product of a triangular sweep, as byte offsets into a workspace:
+// y = [y +] alpha op(A) x - Bd v - op(A2) (Bd2 v2), with op(A) = A and Bd, Bd2 as they are, or
+// op(A) = A^H and Bd, Bd2 transposed. A, A2: n x n complex, column-major; Bd, Bd2: n / 4 real
+// column-major 4 x 4 blocks (negative offset: term absent).
+struct SweepTerm {
+  int64_t a = -1, x = -1, y = -1;
+  int64_t bd = -1, v = -1;
+  int64_t a2 = -1, bd2 = -1, v2 = -1;
+  double alpha = 0.0;
+  int add = 0;
+};
+struct SweepTerms {
+  int n = 0;
+  SweepTerm t[4];
+  void add(const SweepTerm& s) { t[n++] = s; }
+};
+// The products of one sweep step for every workspace (they may run in any order).
+int sweep_product(int conj_trans, int n, char* base, int64_t stride, int workspaces,
+                  const SweepTerms& terms, cudaStream_t st);
+
+// The same step over nr <= 8 right-hand sides per workspace (op(A) = A; no second matrix): x, y
+// and v are byte offsets into vectors + vstride z, blocks of n x nr columns; workspaces
+// z = zmap[0 .. *n_active - 1] only (device arrays).
+int sweep_product_multi(int n, int nr, char* base, int64_t stride, char* vectors, int64_t vstride,
+                        int workspaces, const int* zmap, const int* n_active,
+                        const SweepTerms& terms, cudaStream_t st);
 
 }  // namespace dense
 }  // namespace eb

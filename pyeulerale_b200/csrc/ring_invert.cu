@@ -148,7 +148,7 @@ struct Shared {
 // holds Dinv[pos(i), perm[k]] = W[i, k] with pos(i) the step that chose row i.
 template <class T, int NC, int ROWS, int Threads>
 __global__ void __launch_bounds__(Threads + 32, 1)
-    k_ring_invert(int K, int z0, int chains, char* base, int64_t stride, InvertAt at, int epoch) {
+    k_ring_invert(int K, int z0, char* base, int64_t stride, InvertAt at, int epoch) {
   constexpr bool kReal = sizeof(T) == sizeof(double);
   constexpr int nt = Threads, kWarps = Threads / 32;  // compute threads and warps
   constexpr int kStepBar = 1, kGroupBar = 2;  // kGroupBar + q: group q of this CTA's steps
@@ -156,9 +156,8 @@ __global__ void __launch_bounds__(Threads + 32, 1)
   extern __shared__ __align__(16) unsigned char ri_smem[];
   Shared<T, NC>& S = *reinterpret_cast<Shared<T, NC>*>(ri_smem);
   T* stage = reinterpret_cast<T*>(ri_smem + sizeof(Shared<T, NC>));  // NC columns of K
-  const int z = z0 + blockIdx.y, chain = z % chains;
-  char* ws = base + stride * (z / chains);
-  auto place = [&](const At& a) { return ws + a.off + a.chain * chain; };
+  char* ws = base + stride * (z0 + blockIdx.y);
+  auto place = [&](size_t off) { return ws + off; };
   const T* in = reinterpret_cast<const T*>(place(at.in));
   T* pub = reinterpret_cast<T*>(place(at.pub));
   unsigned long long* flags = reinterpret_cast<unsigned long long*>(place(at.flags));
@@ -385,8 +384,8 @@ __global__ void __launch_bounds__(Threads + 32, 1)
 }
 
 template <class T, int NC, int ROWS, int Threads>
-int launch(int K, int n_shifts, int chains, char* base, int64_t stride, const InvertAt& at,
-           int epoch, cudaStream_t st) {
+int launch(int K, int systems, char* base, int64_t stride, const InvertAt& at, int epoch,
+           cudaStream_t st) {
   auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
   constexpr int threads = Threads + 32;
   const int smem = (int)(sizeof(Shared<T, NC>) + sizeof(T) * NC * (size_t)K);
@@ -398,12 +397,12 @@ int launch(int K, int n_shifts, int chains, char* base, int64_t stride, const In
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
     return check_launch("ring_invert occupancy");
-  const int panels = (K + NC - 1) / NC, systems = n_shifts * chains;
+  const int panels = (K + NC - 1) / NC;
   const int fit = sms * per_sm / panels;  // systems whose CTAs are resident together
   if (fit < 1) return fail(EB_ERR_CUDA, "ring_invert: the device cannot hold one block's CTAs");
   for (int z0 = 0; z0 < systems; z0 += fit) {
     const dim3 grid(panels, std::min(fit, systems - z0));
-    void* args[] = {(void*)&K,      (void*)&z0, (void*)&chains, (void*)&base,
+    void* args[] = {(void*)&K,      (void*)&z0, (void*)&base,
                     (void*)&stride, (void*)&at, (void*)&epoch};
     if (cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(threads), args, smem, st) !=
         cudaSuccess)
@@ -414,11 +413,11 @@ int launch(int K, int n_shifts, int chains, char* base, int64_t stride, const In
 
 }  // namespace
 
-int ring_invert(int K, int n_shifts, int chains, char* base, int64_t stride, const InvertAt& at,
-                int epoch, bool real, cudaStream_t st) {
-  if (K < 4 || K > kMaxRows || K % 4 != 0 || n_shifts < 1 || chains < 1 || epoch < 1)
+int ring_invert(int K, int systems, char* base, int64_t stride, const InvertAt& at, int epoch,
+                bool real, cudaStream_t st) {
+  if (K < 4 || K > kMaxRows || K % 4 != 0 || systems < 1 || epoch < 1)
     return fail(EB_ERR_ARG, "ring_invert: bad sizes");
-  auto run = [&](auto kernel) { return kernel(K, n_shifts, chains, base, stride, at, epoch, st); };
+  auto run = [&](auto kernel) { return kernel(K, systems, base, stride, at, epoch, st); };
   // Rows per thread: 128 compute threads (one warp per scheduler: the step's latency grows with the
   // warps that share one) as long as a thread's rows fit its registers; above K = 512 more
   // threads, which caps them (K = 1024 real: 1174 us at four rows, 1262 at two; complex: 2246 us at

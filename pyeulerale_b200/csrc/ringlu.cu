@@ -5,16 +5,19 @@
 // pentadiagonal with K x K super-blocks: the diagonal block D_m is periodic block-pentadiagonal
 // in the angular index (slots c, b, bb, f, ff), the off-diagonal blocks B1_m (slot i), B2_m
 // (slot ii), C1_m (slot o) and C2_m (slot oo) start block diagonal. Block Gaussian elimination
-// over the rings (pivoting inside each diagonal super-block) factors it exactly:
+// over the rings (pivoting inside each diagonal super-block) factors it exactly.
 //   A = Lt Ut,  Lt = I + sum L_a[m] (block (m, m-a)),  Ut = blockdiag(D_m) + sum C_b[m] (m, m+b),
 // with, at ring m,
 //   Dinv_m = D_m^-1                      (Gauss-Jordan inversion with partial pivoting)
 //   L1[m+1] = B1'[m+1] Dinv_m,  L2[m+2] = B2[m+2] Dinv_m
-//   D[m+1] -= L1[m+1] C1'[m],   B1'[m+2] -= L2[m+2] C1'[m]
-//   D[m+2] -= L2[m+2] C2[m],    C1'[m+1] -= L1[m+1] C2[m]
+//   D[m+1] -= L1[m+1] C1'[m],   B1'[m+2] = B1[m+2] - L2[m+2] C1'[m]
+//   D[m+2] -= L2[m+2] C2[m],    C1'[m+1] = C1[m+1] - L1[m+1] C2[m]
 // (primes: blocks already updated by earlier rings). B2 and C2 are never updated, so they stay
 // block diagonal and the products with them are block-row / block-column scalings instead of
-// dense GEMMs: a ring costs one inversion and three dense complex GEMMs of order K.
+// dense GEMMs: a ring costs one inversion and three dense complex GEMMs of order K. (The other
+// direction, from the far field inwards, is not stable at small shifts: on a 129x129 grid it
+// leaves residuals of 1e-6 where this one leaves 1e-11, so the rings cannot be eliminated from
+// both ends at once.)
 // Storage per ring: Dinv_m, L1[m] and C1'[m] as dense super-blocks, B2 and C2 as their N real
 // 4 x 4 diagonal blocks. L2[m+2] is only needed while ring m is eliminated (one scratch block):
 // the solves apply it as B2[m+2] (Dinv_m y), one dense product with the stored inverse.
@@ -26,10 +29,9 @@
 //
 // Batching: the shifts of one call share the instance and the Jacobian; shift s has its own
 // workspace at base + s * stride. Every step of the elimination is one launch for all shifts
-// (grid dimension = shift), the dense GEMMs and GEMVs are the library's own strided-batched
-// kernels (dense.cu: complex GEMM on the FP64 tensor cores, GEMV), so the
-// launch count per ring does not grow with the number of shifts. All device memory comes from
-// the caller's workspace.
+// (grid dimension = shift), the dense products are the library's own kernels (dense.cu: complex
+// GEMM on the FP64 tensor cores, sweep products), so the launch count per ring does not grow
+// with the number of shifts. All device memory comes from the caller's workspace.
 //
 // Gauss-Jordan inversion (implicit row pivoting: the pivot is the largest modulus among the rows
 // not yet chosen; in-place storage of the transformation). For a few shifts one cooperative
@@ -117,12 +119,13 @@ inline bool blocked_inversion(int K, int shifts_per_stream) {
   return K % kGjBlock == 0 && shifts_per_stream >= kGjBlockMinShifts;
 }
 
+// Byte offsets in a workspace.
 struct Layout {
   int M, N, K;
   size_t blk;   // bytes of one K x K complex block
   size_t bdr;   // bytes of one ring's block diagonal (N real 4 x 4 blocks)
-  size_t off_D, off_L1, off_C1, off_B2, off_C2, off_T, off_L2, off_Rp, off_perm, off_info,
-      off_flags, off_acc, off_shift;
+  size_t off_D, off_L1, off_C1, off_B1d, off_C1d, off_B2, off_C2, off_T, off_L2, off_Rp, off_perm,
+      off_info, off_flags, off_acc, off_shift;
   size_t off_y, off_x, off_r, off_w;
   size_t total;
 };
@@ -143,6 +146,8 @@ Layout plan(int M, int N) {
   L.off_D = take(L.blk * M);
   L.off_L1 = take(L.blk * M);
   L.off_C1 = take(L.blk * M);
+  L.off_B1d = take(L.bdr * M);
+  L.off_C1d = take(L.bdr * M);
   L.off_B2 = take(L.bdr * M);
   L.off_C2 = take(L.bdr * M);
   L.off_T = take(L.blk);
@@ -162,12 +167,12 @@ Layout plan(int M, int N) {
   return L;
 }
 
-// Scatters the 4x4 blocks of the nine-slot Jacobian into the ring super-blocks
-// (column-major K x K) and subtracts the shift on the diagonal; the ii / oo blocks (B2, C2)
-// go to the rings' block diagonals (ring m, cell n: 16 doubles at 16 (m N + n), column-major).
+// Scatters the 4x4 blocks of the nine-slot Jacobian: the couplings within a ring, minus the shift
+// on the diagonal, into the (zeroed) ring super-blocks D (column-major K x K), the couplings to
+// other rings into the rings' block diagonals (ring m, cell n: 16 doubles at 16 (m N + n),
+// column-major).
 __global__ void k_assemble(int M, int N, const double* J, const double* shift,
-                           cuDoubleComplex* D, cuDoubleComplex* B1, double* B2,
-                           cuDoubleComplex* C1, double* C2) {
+                           cuDoubleComplex* D, double* B1, double* C1, double* B2, double* C2) {
   const double sr = shift[0], si = shift[1];
   const int64_t cells = (int64_t)M * N;
   const int K = 4 * N;
@@ -180,18 +185,13 @@ __global__ void k_assemble(int M, int N, const double* J, const double* shift,
     const int m = (int)(c % M), n = (int)(c / M);
     if (!slot_active(s, m, M)) continue;
     const double* J16 = J + slot_stride * s + 16 * c;
-    if (s == kII || s == kOO) {
-      double* bd = (s == kII ? B2 : C2) + 16 * ((int64_t)m * N + n);
+    if (s == kI || s == kO || s == kII || s == kOO) {
+      double* bd = (s == kI ? B1 : s == kO ? C1 : s == kII ? B2 : C2) + 16 * ((int64_t)m * N + n);
       for (int e = 0; e < 16; ++e) bd[e] = J16[e];
       continue;
     }
     const int nn = wrap(n + slot_dn(s), N);
-    cuDoubleComplex* T;
-    switch (s) {
-      case kI: T = B1 + blk * m; break;
-      case kO: T = C1 + blk * m; break;
-      default: T = D + blk * m; break;
-    }
+    cuDoubleComplex* T = D + blk * m;
     for (int i = 0; i < 4; ++i)
       for (int r = 0; r < 4; ++r) {
         double v = J16[r + 4 * i];
@@ -219,15 +219,19 @@ __device__ __forceinline__ cuDoubleComplex cfms(cuDoubleComplex a, cuDoubleCompl
   return make_cuDoubleComplex(fma(-a.x, b.x, fma(a.y, b.y, acc.x)), fma(-a.x, b.y, fma(-a.y, b.x, acc.y)));
 }
 
-// Per-shift pointer into the workspace.
+// The workspaces of a launch, one per shift.
+struct Systems {
+  char* base;
+  int64_t stride;
+};
+// A place in the workspace of shift blockIdx.y.
 template <class T>
-__device__ __forceinline__ T* at(char* ws0, int64_t stride, size_t off) {
-  return reinterpret_cast<T*>(ws0 + stride * blockIdx.y + off);
+__device__ __forceinline__ T* at(const Systems& g, size_t off) {
+  return reinterpret_cast<T*>(g.base + g.stride * blockIdx.y + off);
 }
 
 // Gauss-Jordan panel: elimination steps j0 .. j0+NB-1 on the panel columns of the K x K block
-// `in` (byte offset off_in of each shift's workspace), result written to the same columns of
-// `out` (grid: 1 x n_shifts, 512 threads). Thread t keeps rows t + 512 r (r < ROWS) of the panel
+// `in`, result written to the same columns of `out` (grid: 1 x shifts, 512 threads). Thread t keeps rows t + 512 r (r < ROWS) of the panel
 // in registers. A step: every warp finds its best row among the rows not chosen yet (largest
 // modulus, ties to the smaller row) and stages it in shared memory; after one barrier every
 // warp reduces the warp candidates itself, so all threads know the pivot row p and its values,
@@ -248,17 +252,16 @@ constexpr int kPanelThreads = 512;
 constexpr int kMaxK = 1024;
 template <int NB, int ROWS>
 __global__ void __launch_bounds__(kPanelThreads, 1)
-    k_gj_panel(int K, int j0, char* ws0, int64_t stride, size_t off_in, size_t off_out,
-               size_t off_perm, size_t off_info) {
+    k_gj_panel(int K, int j0, Systems sys, size_t off_in, size_t off_out, size_t off_perm, size_t off_info) {
   constexpr int kWarps = kPanelThreads / 32;
   __shared__ cuDoubleComplex cand[2][kWarps][NB];
   __shared__ cuDoubleComplex cand_inv[2][kWarps];  // 1 / (the candidate's pivot value)
   __shared__ unsigned long long cand_key[2][kWarps];
   __shared__ unsigned char chosen[kMaxK];
-  const cuDoubleComplex* in = at<cuDoubleComplex>(ws0, stride, off_in);
-  cuDoubleComplex* out = at<cuDoubleComplex>(ws0, stride, off_out);
-  int* perm = at<int>(ws0, stride, off_perm);
-  int* info = at<int>(ws0, stride, off_info);
+  const cuDoubleComplex* in = at<cuDoubleComplex>(sys, off_in);
+  cuDoubleComplex* out = at<cuDoubleComplex>(sys, off_out);
+  int* perm = at<int>(sys, off_perm);
+  int* info = at<int>(sys, off_info);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (*info != 0) return;  // an earlier panel met a singular pivot
   for (int i = tid; i < K; i += kPanelThreads) chosen[i] = 0;
@@ -388,9 +391,8 @@ constexpr int kUpdRowsT = 64;
 constexpr int kUpdColsT = 32;
 template <int NB>
 __global__ void __launch_bounds__(256, 3) k_gj_update(int K, int j0, int c_lo, int c_hi,
-                                                   char* ws0, int64_t stride, size_t off_in,
-                                                   size_t off_out, size_t off_perm,
-                                                   size_t off_info) {
+                                                   Systems sys, size_t off_in, size_t off_out,
+                                                   size_t off_perm, size_t off_info) {
   constexpr int kPer = kUpdRowsT * kUpdColsT / 256;  // outputs per thread
   constexpr int kGI = (NB * kUpdRowsT + 255) / 256, kRI = (NB * kUpdColsT + 255) / 256;
   __shared__ cuDoubleComplex G[NB][kUpdRowsT];
@@ -398,9 +400,9 @@ __global__ void __launch_bounds__(256, 3) k_gj_update(int K, int j0, int c_lo, i
   const int ctiles = (c_hi - c_lo + kUpdColsT - 1) / kUpdColsT;
   const int c0 = c_lo + (blockIdx.x % ctiles) * kUpdColsT;
   const int r0 = (blockIdx.x / ctiles) * kUpdRowsT;
-  const cuDoubleComplex* in = at<cuDoubleComplex>(ws0, stride, off_in);
-  cuDoubleComplex* out = at<cuDoubleComplex>(ws0, stride, off_out);
-  const int* perm = at<int>(ws0, stride, off_perm);
+  const cuDoubleComplex* in = at<cuDoubleComplex>(sys, off_in);
+  cuDoubleComplex* out = at<cuDoubleComplex>(sys, off_out);
+  const int* perm = at<int>(sys, off_perm);
   const int tid = threadIdx.x;
   const int r = tid % kUpdRowsT, row = r0 + r, cb = tid / kUpdRowsT;
   // All of this thread's loads first: its inputs (columns cb, cb + 4, ...), its elements of the
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(256, 3) k_gj_update(int K, int j0, int c_lo, i
     const int col = c0 + cb + 4 * q;
     acc[q] = row < K && col < c_hi ? in[(size_t)K * col + row] : make_cuDoubleComplex(0.0, 0.0);
   }
-  int bad = *at<int>(ws0, stride, off_info) != 0;
+  int bad = *at<int>(sys, off_info) != 0;
   int pg[kGI];
 #pragma unroll
   for (int q = 0; q < kGI; ++q) {
@@ -471,16 +473,15 @@ __global__ void __launch_bounds__(256, 3) k_gj_update(int K, int j0, int c_lo, i
 // columns into R (BW x K, column-major) and zeroes them in W, which turns the update into
 // W[:, c] += W[:, block] R[:, c], one strided-batched ZGEMM per column range. Grid: K columns
 // x shifts; skipped when a panel met a singular pivot (the factorisation then fails anyway).
-__global__ void __launch_bounds__(64) k_gj_take_pivot_rows(int K, int b0, int BW, char* ws0,
-                                                          int64_t stride, size_t off_W,
-                                                          size_t off_R, size_t off_perm,
+__global__ void __launch_bounds__(64) k_gj_take_pivot_rows(int K, int b0, int BW, Systems sys,
+                                                          size_t off_W, size_t off_R, size_t off_perm,
                                                           size_t off_info) {
   const int c = blockIdx.x;
   if (c >= b0 && c < b0 + BW) return;
-  if (*at<int>(ws0, stride, off_info) != 0) return;
-  cuDoubleComplex* W = at<cuDoubleComplex>(ws0, stride, off_W);
-  cuDoubleComplex* R = at<cuDoubleComplex>(ws0, stride, off_R);
-  const int* perm = at<int>(ws0, stride, off_perm);
+  if (*at<int>(sys, off_info) != 0) return;
+  cuDoubleComplex* W = at<cuDoubleComplex>(sys, off_W);
+  cuDoubleComplex* R = at<cuDoubleComplex>(sys, off_R);
+  const int* perm = at<int>(sys, off_perm);
   for (int k = threadIdx.x; k < BW; k += blockDim.x) {
     const int p = perm[b0 + k];
     if (p < 0 || p >= K) continue;
@@ -491,14 +492,14 @@ __global__ void __launch_bounds__(64) k_gj_take_pivot_rows(int K, int b0, int BW
 
 // Dinv[j, perm[k]] = W[perm[j], k]: the inverse from the Gauss-Jordan working array (W at
 // off_W, result at off_out; grid: column groups x shifts).
-__global__ void __launch_bounds__(256) k_gj_permute(int K, char* ws0, int64_t stride, size_t off_W,
-                                                    size_t off_out, size_t off_perm, size_t off_info) {
+__global__ void __launch_bounds__(256) k_gj_permute(int K, Systems sys, size_t off_W, size_t off_out,
+                                                    size_t off_perm, size_t off_info) {
   extern __shared__ int pm[];
   __shared__ int bad;
-  const cuDoubleComplex* W = at<cuDoubleComplex>(ws0, stride, off_W);
-  cuDoubleComplex* out = at<cuDoubleComplex>(ws0, stride, off_out);
-  const int* perm = at<int>(ws0, stride, off_perm);
-  if (threadIdx.x == 0) bad = *at<int>(ws0, stride, off_info);
+  const cuDoubleComplex* W = at<cuDoubleComplex>(sys, off_W);
+  cuDoubleComplex* out = at<cuDoubleComplex>(sys, off_out);
+  const int* perm = at<int>(sys, off_perm);
+  if (threadIdx.x == 0) bad = *at<int>(sys, off_info);
   __syncthreads();
   for (int i = threadIdx.x; i < K; i += blockDim.x) {
     pm[i] = perm[i];
@@ -513,16 +514,41 @@ __global__ void __launch_bounds__(256) k_gj_permute(int K, char* ws0, int64_t st
   }
 }
 
-// Block-diagonal left product: X = Bd S, Bd the N real 4 x 4 blocks at off_bd (one ring's
-// block diagonal), S the K x K block at off_S, X the K x K block at off_X.
-// Grid: N row blocks x shifts.
-__global__ void __launch_bounds__(256) k_bd_left(int K, char* ws0, int64_t stride, size_t off_bd,
-                                                 size_t off_S, size_t off_X) {
-  __shared__ double bd[16];
-  const double* B = at<const double>(ws0, stride, off_bd);
-  const cuDoubleComplex* S = at<cuDoubleComplex>(ws0, stride, off_S);
-  cuDoubleComplex* X = at<cuDoubleComplex>(ws0, stride, off_X);
+__device__ __forceinline__ cuDoubleComplex from_real(double v) {
+  return make_cuDoubleComplex(v, 0.0);
+}
+
+// One column of a dense K x K block from its N real 4 x 4 diagonal blocks: entry r of column c.
+__device__ __forceinline__ double bd_at(const double* bd, int r, int c) {
+  return (r >> 2) == (c >> 2) ? bd[16 * (r >> 2) + (r & 3) + 4 * (c & 3)] : 0.0;
+}
+
+// X = the dense block of a block diagonal, two of them (blockIdx.z). Grid: K columns x shifts x 2.
+__global__ void __launch_bounds__(256) k_bd_fill(int K, Systems sys, size_t bd0, size_t x0,
+                                                 size_t bd1, size_t x1) {
+  const double* bd = at<const double>(sys, blockIdx.z ? bd1 : bd0);
+  cuDoubleComplex* X = at<cuDoubleComplex>(sys, blockIdx.z ? x1 : x0) + (size_t)K * blockIdx.x;
+  for (int r = threadIdx.x; r < K; r += blockDim.x) X[r] = from_real(bd_at(bd, r, blockIdx.x));
+}
+
+// Before the products of a step (blockIdx.z): 0: X = Bd S (Bd the N real 4 x 4 blocks at bd);
+// 1: F = the dense block of the block diagonal at fbd. Grid: N x shifts x 2.
+__global__ void __launch_bounds__(256) k_bd_left(int K, Systems sys, size_t off_bd, size_t off_S, size_t off_X,
+                                                 size_t off_fbd, size_t off_F) {
   const int n = blockIdx.x;
+  if (blockIdx.z == 1) {  // columns 4 n .. 4 n + 3
+    const double* bd = at<const double>(sys, off_fbd);
+    cuDoubleComplex* F = at<cuDoubleComplex>(sys, off_F);
+    for (int e = threadIdx.x; e < 4 * K; e += blockDim.x) {
+      const int r = e % K, c = 4 * n + e / K;
+      F[(size_t)K * c + r] = from_real(bd_at(bd, r, c));
+    }
+    return;
+  }
+  __shared__ double bd[16];
+  const double* B = at<const double>(sys, off_bd);
+  const cuDoubleComplex* S = at<cuDoubleComplex>(sys, off_S);
+  cuDoubleComplex* X = at<cuDoubleComplex>(sys, off_X);
   if (threadIdx.x < 16) bd[threadIdx.x] = B[16 * n + threadIdx.x];
   __syncthreads();
   for (int c = threadIdx.x; c < K; c += blockDim.x) {
@@ -538,16 +564,23 @@ __global__ void __launch_bounds__(256) k_bd_left(int K, char* ws0, int64_t strid
   }
 }
 
-// Block-diagonal right products: Y -= X Bd for two (X, Y) pairs selected by blockIdx.z, Bd the
-// N real 4 x 4 blocks at off_bd. Grid: N column blocks x shifts x 2.
-__global__ void __launch_bounds__(256) k_bd_right(int K, char* ws0, int64_t stride, size_t off_bd,
-                                                  size_t off_X0, size_t off_Y0, size_t off_X1,
-                                                  size_t off_Y1) {
+// After the products of a step (blockIdx.z): 0: Y -= X Bd; 1: Y1 = F - X1 Bd, F the dense block of
+// the block diagonal at fbd, Bd the N real 4 x 4 blocks at bd; 2: the step's L1 (X1) to its
+// slot. Grid: N column blocks x shifts x 3.
+__global__ void __launch_bounds__(256) k_bd_right(int K, Systems sys, size_t off_bd, size_t off_X, size_t off_Y,
+                                                  size_t off_X1, size_t off_Y1, size_t off_fbd, size_t off_L) {
   __shared__ double bd[16];
-  const double* B = at<const double>(ws0, stride, off_bd);
-  const cuDoubleComplex* X = at<cuDoubleComplex>(ws0, stride, blockIdx.z ? off_X1 : off_X0);
-  cuDoubleComplex* Y = at<cuDoubleComplex>(ws0, stride, blockIdx.z ? off_Y1 : off_Y0);
-  const int n = blockIdx.x;
+  const int n = blockIdx.x, z = blockIdx.z;
+  const cuDoubleComplex* X = at<cuDoubleComplex>(sys, z == 0 ? off_X : off_X1);
+  if (z == 2) {
+    cuDoubleComplex* L = at<cuDoubleComplex>(sys, off_L);
+    for (int e = threadIdx.x; e < 4 * K; e += blockDim.x)
+      L[(size_t)K * 4 * n + e] = X[(size_t)K * 4 * n + e];
+    return;
+  }
+  const double* B = at<const double>(sys, off_bd);
+  cuDoubleComplex* Y = at<cuDoubleComplex>(sys, z == 0 ? off_Y : off_Y1);
+  const double* fbd = z == 1 ? at<const double>(sys, off_fbd) : nullptr;
   if (threadIdx.x < 16) bd[threadIdx.x] = B[16 * n + threadIdx.x];
   __syncthreads();
   for (int r = threadIdx.x; r < K; r += blockDim.x) {
@@ -557,7 +590,7 @@ __global__ void __launch_bounds__(256) k_bd_right(int K, char* ws0, int64_t stri
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       cuDoubleComplex* y = Y + (size_t)K * (4 * n + c) + r;
-      cuDoubleComplex acc = *y;
+      cuDoubleComplex acc = fbd ? from_real(bd_at(fbd, r, 4 * n + c)) : *y;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const double b = bd[q + 4 * c];
@@ -569,28 +602,13 @@ __global__ void __launch_bounds__(256) k_bd_right(int K, char* ws0, int64_t stri
   }
 }
 
-// Block-diagonal vector product of the solves: out -= Bd v (trans = 0) or out -= Bd^T v
-// (trans = 1; the blocks are real, so Bd^H = Bd^T), or out = -(...) when `assign` is set. Bd:
-// N real 4 x 4 blocks at off_bd; v, out: K complex at off_v, off_out. Grid: blocks x shifts.
-__global__ void __launch_bounds__(128) k_bd_vec(int N, char* ws0, int64_t stride, size_t off_bd,
-                                                size_t off_v, size_t off_out, int trans,
-                                                int assign) {
-  const double* B = at<const double>(ws0, stride, off_bd);
-  const cuDoubleComplex* v = at<cuDoubleComplex>(ws0, stride, off_v);
-  cuDoubleComplex* out = at<cuDoubleComplex>(ws0, stride, off_out);
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 4 * N; e += gridDim.x * blockDim.x) {
-    const int n = e >> 2, r = e & 3;
-    const double* b = B + 16 * n;
-    const cuDoubleComplex* vn = v + 4 * n;
-    cuDoubleComplex acc = assign ? make_cuDoubleComplex(0.0, 0.0) : out[e];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double bi = trans ? b[i + 4 * r] : b[r + 4 * i];
-      acc.x = fma(-bi, vn[i].x, acc.x);
-      acc.y = fma(-bi, vn[i].y, acc.y);
-    }
-    out[e] = acc;
-  }
+// The step's L1 to its slot. Grid: any x shifts.
+__global__ void __launch_bounds__(256) k_copy_block(int K, Systems sys, size_t off_X, size_t off_Y) {
+  const cuDoubleComplex* X = at<cuDoubleComplex>(sys, off_X);
+  cuDoubleComplex* Y = at<cuDoubleComplex>(sys, off_Y);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)K * K;
+       e += (int64_t)gridDim.x * blockDim.x)
+    Y[e] = X[e];
 }
 
 // Reference layout (4, M, N) <-> ring layout [m][n][v].
@@ -694,12 +712,8 @@ struct Group {
   char* base;
   int64_t stride;  // bytes
   int S;
-  bool blocked = false;  // how its rings are inverted (see invert_ring)
-  int64_t es() const { return stride / (int64_t)sizeof(cuDoubleComplex); }
-  cuDoubleComplex* blk(size_t off, int m) const {
-    return reinterpret_cast<cuDoubleComplex*>(base + off + L.blk * (size_t)m);
-  }
-  size_t boff(size_t off, int m) const { return off + L.blk * (size_t)m; }
+  bool blocked = false;  // how its rings are inverted (see invert)
+  Systems systems() const { return Systems{base, stride}; }
 };
 
 int check_group(const eb_batch* b, int n_shifts, const void* ws, int64_t stride, Layout& L) {
@@ -718,180 +732,201 @@ int check_group(const eb_batch* b, int n_shifts, const void* ws, int64_t stride,
 
 // Panel steps j0 .. j0 + NB - 1 (in -> out) and their update of the columns [c_lo, c_hi).
 template <int NB, int ROWS>
-void gj_pass(const Group& g, int j0, int c_lo, int c_hi, size_t off_in, size_t off_out,
-             cudaStream_t st) {
-  const int K = g.L.K;
+void gj_pass(const Group& g, int j0, int c_lo, int c_hi, size_t in, size_t out, cudaStream_t st) {
+  const Layout& L = g.L;
+  const int K = L.K;
   const int tiles = ((c_hi - c_lo + kUpdColsT - 1) / kUpdColsT) * ((K + kUpdRowsT - 1) / kUpdRowsT);
-  k_gj_panel<NB, ROWS><<<dim3(1, g.S), kPanelThreads, 0, st>>>(K, j0, g.base, g.stride, off_in, off_out,
-                                                               g.L.off_perm, g.L.off_info);
-  k_gj_update<NB><<<dim3(tiles, g.S), 256, 0, st>>>(K, j0, c_lo, c_hi, g.base, g.stride, off_in,
-                                                    off_out, g.L.off_perm, g.L.off_info);
+  k_gj_panel<NB, ROWS><<<dim3(1, g.S), kPanelThreads, 0, st>>>(K, j0, g.systems(), in, out, L.off_perm,
+                                                              L.off_info);
+  k_gj_update<NB><<<dim3(tiles, g.S), 256, 0, st>>>(K, j0, c_lo, c_hi, g.systems(), in, out,
+                                                    L.off_perm, L.off_info);
 }
 
-void gj_pass_any(const Group& g, int nb, int j0, int c_lo, int c_hi, size_t in, size_t out,
-                 cudaStream_t st) {
-  if (nb == 16) gj_pass<16, 1>(g, j0, c_lo, c_hi, in, out, st);  // K <= 512
-  else gj_pass<8, 2>(g, j0, c_lo, c_hi, in, out, st);
-}
-
-// D_m <- D_m^-1 for every shift by Gauss-Jordan with implicit row pivoting: for a few shifts one
-// cooperative launch (ring_invert.cu), for many the blocked form, whose columns go in blocks of
-// kGjBlock: the panels of a block update only the block's columns (ping-pong with the scratch
-// block T, an even number of passes, so the block ends in D_m), and the rest of D_m takes the
-// block's combined rank-kGjBlock update as strided-batched ZGEMMs (tensor-core DMMA).
-int invert_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
+// D <- D^-1 for every shift by Gauss-Jordan with implicit row pivoting (D: a K x K block's
+// place): for a few shifts one cooperative launch (ring_invert.cu), for many the blocked form,
+// whose columns go in blocks of kGjBlock: the panels of a block update only the block's columns
+// (ping-pong with the scratch block T, an even number of passes, so the block ends in D), and the
+// rest of D takes the block's combined rank-kGjBlock update as ZGEMMs (tensor-core DMMA).
+int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
   const int K = L.K, nb = panel_width(K);
-  const size_t buf[2] = {g.boff(L.off_D, m), L.off_T};
   if (!g.blocked) {
-    const InvertAt at{{(int64_t)buf[0], 0}, {(int64_t)L.off_T, 0}, {(int64_t)buf[0], 0}, {},
-                      {(int64_t)L.off_flags, 0}, {(int64_t)L.off_info, 0}};
-    return ring_invert(K, g.S, 1, g.base, g.stride, at, m + 1, false, st);
+    const InvertAt where{D, L.off_T, D, 0, L.off_flags, L.off_info};
+    return ring_invert(K, g.S, g.base, g.stride, where, epoch, false, st);
   }
-  {
-    // Look-ahead: the block's update of the next block's columns runs on st, right before the
-    // next block's panels; its update of every other column runs on the side stream, under
-    // those panels. st waits for the side stream before it moves the next pivot rows (which
-    // reads and zeroes rows of those columns and overwrites R) and at the end.
-    cudaStream_t hs = nullptr;
-    int rc = lane_stream(st, hs, side_lane);
-    if (rc != EB_OK) return rc;
-    Handle& side = g_handle[side_lane];
-    const int64_t es = g.es();
-    cuDoubleComplex* W = g.blk(L.off_D, m);
-    cuDoubleComplex* Rp = reinterpret_cast<cuDoubleComplex*>(g.base + L.off_Rp);
-    auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int b0) {
-      if (c_hi <= c_lo) return EB_OK;
-      return dense::zgemm_nn_batched(K, c_hi - c_lo, kGjBlock, 1.0, W + (size_t)K * b0, K, es,
-                                     Rp + (size_t)kGjBlock * c_lo, kGjBlock, es, 1.0,
-                                     W + (size_t)K * c_lo, K, es, g.S, hh);
-    };
-    bool side_busy = false;
-    for (int b0 = 0; b0 < K; b0 += kGjBlock) {
-      for (int q = 0; q < kGjBlock / nb; ++q)
-        gj_pass_any(g, nb, b0 + q * nb, b0, b0 + kGjBlock, buf[q & 1], buf[(q + 1) & 1], st);
-      if (K == kGjBlock) break;
-      if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
-        return check_launch("ringlu side join");
-      k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, kGjBlock, g.base, g.stride, buf[0],
-                                                        L.off_Rp, L.off_perm, L.off_info);
-      const int n0 = b0 + kGjBlock, n1 = std::min(K, b0 + 2 * kGjBlock);  // the next block
-      if ((rc = update(st, n0, n1, b0)) != EB_OK) return rc;
-      if (cudaEventRecord(side.start, st) != cudaSuccess ||
-          cudaStreamWaitEvent(side.stream, side.start, 0) != cudaSuccess)
-        return check_launch("ringlu side fork");
-      if ((rc = update(hs, 0, b0, b0)) != EB_OK) return rc;
-      if ((rc = update(hs, n1, K, b0)) != EB_OK) return rc;
-      if (cudaEventRecord(side.done, side.stream) != cudaSuccess) return check_launch("ringlu side");
-      side_busy = true;
+  // Look-ahead: the block's update of the next block's columns runs on st, right before the
+  // next block's panels; its update of every other column runs on the side stream, under
+  // those panels. st waits for the side stream before it moves the next pivot rows (which
+  // reads and zeroes rows of those columns and overwrites R) and at the end.
+  cudaStream_t hs = nullptr;
+  int rc = lane_stream(st, hs, side_lane);
+  if (rc != EB_OK) return rc;
+  Handle& side = g_handle[side_lane];
+  constexpr int64_t kB = sizeof(cuDoubleComplex);
+  auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int b0) {
+    if (c_hi <= c_lo) return EB_OK;
+    dense::Products p;
+    p.add(D + kB * K * b0, L.off_Rp + kB * kGjBlock * c_lo, D + kB * K * c_lo);
+    return dense::zgemm_set(K, c_hi - c_lo, kGjBlock, 1.0, 1.0, g.base, g.stride, g.S, p, K,
+                            kGjBlock, K, hh);
+  };
+  bool side_busy = false;
+  for (int b0 = 0; b0 < K; b0 += kGjBlock) {
+    for (int q = 0; q < kGjBlock / nb; ++q) {
+      const size_t in = q & 1 ? L.off_T : D, out = q & 1 ? D : L.off_T;
+      if (nb == 16) gj_pass<16, 1>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
+      else gj_pass<8, 2>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
     }
+    if (K == kGjBlock) break;
     if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
       return check_launch("ringlu side join");
+    k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, kGjBlock, g.systems(), D, L.off_Rp,
+                                                      L.off_perm, L.off_info);
+    const int n0 = b0 + kGjBlock, n1 = std::min(K, b0 + 2 * kGjBlock);  // the next block
+    if ((rc = update(st, n0, n1, b0)) != EB_OK) return rc;
+    if (cudaEventRecord(side.start, st) != cudaSuccess ||
+        cudaStreamWaitEvent(side.stream, side.start, 0) != cudaSuccess)
+      return check_launch("ringlu side fork");
+    if ((rc = update(hs, 0, b0, b0)) != EB_OK) return rc;
+    if ((rc = update(hs, n1, K, b0)) != EB_OK) return rc;
+    if (cudaEventRecord(side.done, side.stream) != cudaSuccess) return check_launch("ringlu side");
+    side_busy = true;
   }
-  const size_t W = buf[0], other = buf[1];
-  k_gj_permute<<<dim3(std::min(K, 1024), g.S), 256, sizeof(int) * K, st>>>(K, g.base, g.stride, W, other,
-                                                                          L.off_perm, L.off_info);
-  if (cudaMemcpy2DAsync(g.base + buf[0], g.stride, g.base + other, g.stride, L.blk, g.S,
-                        cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-    return check_launch("ringlu inverse copy");
+  if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
+    return check_launch("ringlu side join");
+  k_gj_permute<<<dim3(std::min(K, 1024), g.S), 256, sizeof(int) * K, st>>>(
+      K, g.systems(), D, L.off_T, L.off_perm, L.off_info);
+  k_copy_block<<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(K, g.systems(),
+                                                                               L.off_T, D);
   return EB_OK;
+}
+
+// The dense couplings of ring 0.
+int begin_rings(const Group& g, cudaStream_t st) {
+  const Layout& L = g.L;
+  k_bd_fill<<<dim3(L.K, g.S, 2), 256, 0, st>>>(L.K, g.systems(), L.off_B1d + L.bdr,
+                                               L.off_L1 + L.blk, L.off_C1d, L.off_C1);
+  return check_launch("ringlu couplings");
 }
 
 // One ring of the block elimination for every shift of the group.
 int factor_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
   const int M = L.M, K = L.K, N = L.N;
-  const int64_t es = g.es();
-  int rc = invert_ring(g, m, st, side_lane);
-  if (rc != EB_OK) return rc;
-  if (m + 1 < M) {
-    // T = L1[m+1] = B1'[m+1] Dinv_m;  D[m+1] -= T C1'[m]
-    if ((rc = dense::zgemm_nn_batched(K, K, K, 1.0, g.blk(L.off_L1, m + 1), K, es,
-                                      g.blk(L.off_D, m), K, es, 0.0, g.blk(L.off_T, 0), K, es,
-                                      g.S, st)) != EB_OK)
-      return rc;
-    if ((rc = dense::zgemm_nn_batched(K, K, K, -1.0, g.blk(L.off_T, 0), K, es,
-                                      g.blk(L.off_C1, m), K, es, 1.0, g.blk(L.off_D, m + 1), K,
-                                      es, g.S, st)) != EB_OK)
-      return rc;
-  }
+  auto D = [&](int r) { return L.off_D + L.blk * r; };
+  auto B = [&](int r) { return L.off_L1 + L.blk * r; };
+  auto C = [&](int r) { return L.off_C1 + L.blk * r; };
+  auto products = [&](double alpha, double beta, const dense::Products& p) {
+    return dense::zgemm_set(K, K, K, alpha, beta, g.base, g.stride, g.S, p, K, K, K, st);
+  };
+  int rc = invert(g, D(m), m + 1, st, side_lane);
+  if (rc != EB_OK || m + 1 == M) return rc;
+  dense::Products t;  // T = L1[m+1] = B1'[m+1] Dinv_m
+  t.add(B(m + 1), D(m), L.off_T);
+  if ((rc = products(1.0, 0.0, t)) != EB_OK) return rc;
+  dense::Products p;
+  p.add(L.off_T, C(m), D(m + 1));  // D[m+1] -= T C1'[m]
   if (m + 2 < M) {
-    // L2[m+2] = B2[m+2] Dinv_m (scratch);  B1'[m+2] -= L2[m+2] C1'[m]
-    k_bd_left<<<dim3(N, g.S), 256, 0, st>>>(K, g.base, g.stride, L.off_B2 + L.bdr * (m + 2),
-                                            g.boff(L.off_D, m), L.off_L2);
-    if ((rc = dense::zgemm_nn_batched(K, K, K, -1.0, g.blk(L.off_L2, 0), K, es,
-                                      g.blk(L.off_C1, m), K, es, 1.0, g.blk(L.off_L1, m + 2), K,
-                                      es, g.S, st)) != EB_OK)
-      return rc;
-    // D[m+2] -= L2[m+2] C2[m];  C1'[m+1] -= L1[m+1] C2[m]
-    k_bd_right<<<dim3(N, g.S, 2), 256, 0, st>>>(K, g.base, g.stride, L.off_C2 + L.bdr * m,
-                                                L.off_L2, g.boff(L.off_D, m + 2),
-                                                L.off_T, g.boff(L.off_C1, m + 1));
+    // L2[m+2] = B2[m+2] Dinv_m (scratch);  B1'[m+2] = B1[m+2] - L2[m+2] C1'[m]
+    k_bd_left<<<dim3(N, g.S, 2), 256, 0, st>>>(K, g.systems(), L.off_B2 + L.bdr * (m + 2), D(m),
+                                               L.off_L2, L.off_B1d + L.bdr * (m + 2), B(m + 2));
+    p.add(L.off_L2, C(m), B(m + 2));
   }
-  if (m + 1 < M &&
-      cudaMemcpy2DAsync(g.blk(L.off_L1, m + 1), g.stride, g.blk(L.off_T, 0), g.stride, L.blk, g.S,
-                        cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-    return check_launch("ringlu L1 copy");
-  return EB_OK;
+  if ((rc = products(-1.0, 1.0, p)) != EB_OK) return rc;
+  if (m + 2 < M)  // D[m+2] -= L2[m+2] C2[m];  C1'[m+1] = C1[m+1] - T C2[m];  L1[m+1] = T
+    k_bd_right<<<dim3(N, g.S, 3), 256, 0, st>>>(K, g.systems(), L.off_C2 + L.bdr * m, L.off_L2,
+                                                D(m + 2), L.off_T, C(m + 1),
+                                                L.off_C1d + L.bdr * (m + 1), B(m + 1));
+  else
+    k_copy_block<<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(
+        K, g.systems(), L.off_T, B(m + 1));
+  return check_launch("ringlu step");
 }
+
+// The triangular sweeps with the stored factors, as steps of matrix-vector products on ring
+// vectors (`step` takes the terms of one step, which are independent).
+struct Sweep {
+  const Layout& L;
+  size_t y, x, w;  // ring vectors: right-hand sides, solutions, Dinv y of the finished rings
+  size_t vec;      // bytes of one ring vector
+
+  int64_t D(int m) const { return (int64_t)(L.off_D + L.blk * m); }
+  int64_t B(int m) const { return (int64_t)(L.off_L1 + L.blk * m); }
+  int64_t C(int m) const { return (int64_t)(L.off_C1 + L.blk * m); }
+  int64_t bd(size_t off, int m) const { return (int64_t)(off + L.bdr * m); }
+  int64_t at(size_t v, int m) const { return (int64_t)(v + vec * m); }
+  dense::SweepTerm term(int64_t a, int64_t in, int64_t out, double alpha, int add) const {
+    dense::SweepTerm t;
+    t.a = a;
+    t.x = in;
+    t.y = out;
+    t.alpha = alpha;
+    t.add = add;
+    return t;
+  }
+  template <class Step>
+  int one(Step step, const dense::SweepTerm& t) const {
+    dense::SweepTerms s;
+    s.add(t);
+    return step(s);
+  }
+
+  // X = A^-1 Y. A = Lt Ut with L2[m] = B2[m] Dinv_{m-2}, so the forward sweep keeps w[m] = Dinv_m
+  // y[m] of the finished rings (formed beside the next ring's step) and subtracts B2[m] w[m-2].
+  template <class Step>
+  int forward(Step step) const {
+    const int M = L.M;
+    int rc;
+    for (int m = 1; m < M; ++m) {  // Lt z = b (z in y)
+      dense::SweepTerms s;
+      dense::SweepTerm t = term(B(m), at(y, m - 1), at(y, m), -1.0, 1);
+      if (m >= 2) t.bd = bd(L.off_B2, m), t.v = at(w, m - 2);
+      s.add(t);
+      if (m + 1 < M) s.add(term(D(m - 1), at(y, m - 1), at(w, m - 1), 1.0, 0));
+      if ((rc = step(s)) != EB_OK) return rc;
+    }
+    for (int m = M - 1; m >= 0; --m) {  // Ut x = z
+      if (m + 1 < M) {
+        dense::SweepTerm t = term(C(m), at(x, m + 1), at(y, m), -1.0, 1);
+        if (m + 2 < M) t.bd = bd(L.off_C2, m), t.v = at(x, m + 2);
+        if ((rc = one(step, t)) != EB_OK) return rc;
+      }
+      if ((rc = one(step, term(D(m), at(y, m), at(x, m), 1.0, 0))) != EB_OK) return rc;
+    }
+    return EB_OK;
+  }
+
+  // X = A^-H Y; the adjoint sweep applies L2[m+2]^H as Dinv_m^H (B2[m+2]^T x[m+2]).
+  template <class Step>
+  int adjoint(Step step) const {
+    const int M = L.M;
+    int rc;
+    for (int m = 0; m < M; ++m) {  // Ut^H z = b (z in x)
+      if (m >= 1) {
+        dense::SweepTerm t = term(C(m - 1), at(x, m - 1), at(y, m), -1.0, 1);
+        if (m >= 2) t.bd = bd(L.off_C2, m - 2), t.v = at(x, m - 2);
+        if ((rc = one(step, t)) != EB_OK) return rc;
+      }
+      if ((rc = one(step, term(D(m), at(y, m), at(x, m), 1.0, 0))) != EB_OK) return rc;
+    }
+    for (int m = M - 2; m >= 0; --m) {  // Lt^H x = z
+      dense::SweepTerm t = term(B(m + 1), at(x, m + 1), at(x, m), -1.0, 1);
+      if (m + 2 < M) t.a2 = D(m), t.bd2 = bd(L.off_B2, m + 2), t.v2 = at(x, m + 2);
+      if ((rc = one(step, t)) != EB_OK) return rc;
+    }
+    return EB_OK;
+  }
+};
 
 // Ring-ordered triangular solves with the stored factors for every shift: y (ring layout)
 // holds the right-hand sides on entry; the solutions are left in x (w: scratch vectors).
-// A = Lt Ut with L2[m] = B2[m] Dinv_{m-2}, so the forward sweep keeps w[m] = Dinv_m y[m] of the
-// finished rings and subtracts B2[m] w[m-2]; the adjoint sweep applies L2[m+2]^H as
-// Dinv_m^H (B2[m+2]^T x[m+2]).
 int ring_solve(const Group& g, bool adjoint, cudaStream_t stream) {
   const Layout& L = g.L;
-  const int M = L.M, K = L.K, N = L.N;
-  const int64_t es = g.es();
-  cuDoubleComplex* y = reinterpret_cast<cuDoubleComplex*>(g.base + L.off_y);
-  cuDoubleComplex* x = reinterpret_cast<cuDoubleComplex*>(g.base + L.off_x);
-  cuDoubleComplex* w = reinterpret_cast<cuDoubleComplex*>(g.base + L.off_w);
-  auto yv = [&](int m) { return y + (size_t)K * m; };
-  auto xv = [&](int m) { return x + (size_t)K * m; };
-  auto wv = [&](int m) { return w + (size_t)K * m; };
-  const size_t vb = sizeof(cuDoubleComplex) * (size_t)K;  // bytes of one ring vector
-  const int kN = 0, kH = 1;  // op(A) = A, A^H
-  auto gemv = [&](int op, double alpha, const cuDoubleComplex* A, const cuDoubleComplex* v,
-                  double beta, cuDoubleComplex* out) {
-    return dense::zgemv_batched(op, K, alpha, A, K, es, v, es, beta, out, es, g.S, stream);
+  const Sweep sweep{L, L.off_y, L.off_x, L.off_w, sizeof(cuDoubleComplex) * (size_t)L.K};
+  auto step = [&](const dense::SweepTerms& t) {
+    return dense::sweep_product(adjoint, L.K, g.base, g.stride, g.S, t, stream);
   };
-  const dim3 bdg((4 * N + 127) / 128, g.S);
-  // out -= Bd v (trans: Bd^T v), ring vectors given by workspace offsets; assign: out = -Bd v
-  auto bdvec = [&](size_t off_bd, size_t off_v, size_t off_out, int trans, int assign) {
-    k_bd_vec<<<bdg, 128, 0, stream>>>(N, g.base, g.stride, off_bd, off_v, off_out, trans, assign);
-  };
-  int st = EB_OK;
-  auto run = [&](int s) {
-    if (s != EB_OK) st = s;
-  };
-  if (!adjoint) {
-    for (int m = 0; m < M; ++m) {  // Lt z = b (z in y), w[m] = Dinv_m z[m]
-      if (m >= 1) run(gemv(kN, -1.0, g.blk(L.off_L1, m), yv(m - 1), 1.0, yv(m)));
-      if (m >= 2) bdvec(L.off_B2 + L.bdr * m, L.off_w + vb * (m - 2), L.off_y + vb * m, 0, 0);
-      if (m + 2 < M) run(gemv(kN, 1.0, g.blk(L.off_D, m), yv(m), 0.0, wv(m)));
-    }
-    for (int m = M - 1; m >= 0; --m) {  // Ut x = z
-      if (m + 1 < M) run(gemv(kN, -1.0, g.blk(L.off_C1, m), xv(m + 1), 1.0, yv(m)));
-      if (m + 2 < M) bdvec(L.off_C2 + L.bdr * m, L.off_x + vb * (m + 2), L.off_y + vb * m, 0, 0);
-      run(gemv(kN, 1.0, g.blk(L.off_D, m), yv(m), 0.0, xv(m)));
-    }
-  } else {
-    for (int m = 0; m < M; ++m) {  // Ut^H z = b (z in x)
-      if (m >= 1) run(gemv(kH, -1.0, g.blk(L.off_C1, m - 1), xv(m - 1), 1.0, yv(m)));
-      if (m >= 2) bdvec(L.off_C2 + L.bdr * (m - 2), L.off_x + vb * (m - 2), L.off_y + vb * m, 1, 0);
-      run(gemv(kH, 1.0, g.blk(L.off_D, m), yv(m), 0.0, xv(m)));
-    }
-    for (int m = M - 1; m >= 0; --m) {  // Lt^H x = z
-      if (m + 1 < M) run(gemv(kH, -1.0, g.blk(L.off_L1, m + 1), xv(m + 1), 1.0, xv(m)));
-      if (m + 2 < M) {  // x[m] -= Dinv_m^H (B2[m+2]^T x[m+2]), with w[m] = -B2[m+2]^T x[m+2]
-        bdvec(L.off_B2 + L.bdr * (m + 2), L.off_x + vb * (m + 2), L.off_w + vb * m, 1, 1);
-        run(gemv(kH, 1.0, g.blk(L.off_D, m), wv(m), 1.0, xv(m)));
-      }
-    }
-  }
-  if (st != EB_OK) return st;
-  return check_launch("ring solve");
+  return adjoint ? sweep.adjoint(step) : sweep.forward(step);
 }
 
 // ---- many right-hand sides per factorisation (the anchored GMRES preconditioner) ----------
@@ -961,37 +996,14 @@ int ring_solve_multi(const Group& g, int nr, cuDoubleComplex* Y, cuDoubleComplex
                      cuDoubleComplex* W, int64_t mstride, const int* zmap, const int* n_active,
                      cudaStream_t st) {
   const Layout& L = g.L;
-  const int M = L.M, K = L.K;
-  const int64_t es = g.es();
-  auto blk = [&](cuDoubleComplex* base, int m) { return base + (size_t)K * nr * m; };
-  int rc = EB_OK;
-  // C = alpha A B + beta C [- Bd V: the block-diagonal coupling at off_bd, fused into the
-  // product's epilogue]
-  auto gemm = [&](double alpha, const cuDoubleComplex* A, const cuDoubleComplex* B, double beta,
-                  cuDoubleComplex* C, size_t off_bd = 0, const cuDoubleComplex* V = nullptr) {
-    if (rc == EB_OK)
-      rc = dense::zgemm_skinny_batched(K, nr, alpha, A, K, es, B, K, mstride, beta, C, K,
-                                       mstride, g.S, zmap, n_active, st,
-                                       V ? g.base + off_bd : nullptr, g.stride, V, mstride);
-  };
-  for (int m = 0; m < M; ++m) {  // Lt z = b (z in Y), W[m] = Dinv_m z[m]
-    if (m >= 2)
-      gemm(-1.0, g.blk(L.off_L1, m), blk(Y, m - 1), 1.0, blk(Y, m), L.off_B2 + L.bdr * m,
-           blk(W, m - 2));
-    else if (m == 1)
-      gemm(-1.0, g.blk(L.off_L1, m), blk(Y, m - 1), 1.0, blk(Y, m));
-    if (m + 2 < M) gemm(1.0, g.blk(L.off_D, m), blk(Y, m), 0.0, blk(W, m));
-  }
-  for (int m = M - 1; m >= 0; --m) {  // Ut x = z
-    if (m + 2 < M)
-      gemm(-1.0, g.blk(L.off_C1, m), blk(X, m + 1), 1.0, blk(Y, m), L.off_C2 + L.bdr * m,
-           blk(X, m + 2));
-    else if (m + 1 < M)
-      gemm(-1.0, g.blk(L.off_C1, m), blk(X, m + 1), 1.0, blk(Y, m));
-    gemm(1.0, g.blk(L.off_D, m), blk(Y, m), 0.0, blk(X, m));
-  }
-  if (rc != EB_OK) return rc;
-  return check_launch("ring solve multi");
+  constexpr int64_t kB = sizeof(cuDoubleComplex);
+  char* base = reinterpret_cast<char*>(std::min(Y, std::min(X, W)));
+  auto off = [&](cuDoubleComplex* v) { return (size_t)(reinterpret_cast<char*>(v) - base); };
+  const Sweep sweep{L, off(Y), off(X), off(W), (size_t)kB * L.K * nr};
+  return sweep.forward([&](const dense::SweepTerms& t) {
+    return dense::sweep_product_multi(L.K, nr, g.base, g.stride, base, kB * mstride, g.S, zmap,
+                                      n_active, t, st);
+  });
 }
 
 // out = A_{anchor(s)}^-1 in for the systems of one instance (the anchored GMRES preconditioner):
@@ -1076,19 +1088,27 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   const Layout& L = g.L;
   const int M = L.M, N = L.N, n_shifts = g.S;
   int rc = EB_OK;
+  constexpr int kMost = 16000;  // four products per shift and launch, within the grid's limit
+  if (n_shifts > kMost) {
+    for (int s = 0; s < n_shifts && rc == EB_OK; s += kMost)
+      rc = issue_factor(Group{L, g.base + (int64_t)s * g.stride, g.stride,
+                              std::min(kMost, n_shifts - s)}, J + s, st);
+    return rc;
+  }
   for (int s = 0; s < n_shifts; ++s) {
     char* w = g.base + (int64_t)s * g.stride;
-    cudaMemsetAsync(w, 0, L.off_T, st);  // the stored super-blocks and block diagonals
-    cudaMemsetAsync(w + L.off_info, 0, L.off_acc - L.off_info, st);  // and the panel flags
+    cudaMemsetAsync(w + L.off_D, 0, L.blk * M, st);
+    cudaMemsetAsync(w + L.off_info, 0, L.off_acc - L.off_info, st);  // and the inversions' flags
     k_assemble<<<grid_for((int64_t)M * N * 9, 256), 256, 0, st>>>(
         M, N, J[s], reinterpret_cast<const double*>(w + L.off_shift),
-        reinterpret_cast<cuDoubleComplex*>(w + L.off_D), reinterpret_cast<cuDoubleComplex*>(w + L.off_L1),
-        reinterpret_cast<double*>(w + L.off_B2), reinterpret_cast<cuDoubleComplex*>(w + L.off_C1),
+        reinterpret_cast<cuDoubleComplex*>(w + L.off_D), reinterpret_cast<double*>(w + L.off_B1d),
+        reinterpret_cast<double*>(w + L.off_C1d), reinterpret_cast<double*>(w + L.off_B2),
         reinterpret_cast<double*>(w + L.off_C2));
   }
   if ((rc = check_launch("ringlu assemble")) != EB_OK) return rc;
   if (!blocked_inversion(L.K, (n_shifts + 1) / 2)) {
     // one stream: the inversions are cooperative launches, which never run two at a time here
+    if ((rc = begin_rings(g, st)) != EB_OK) return rc;
     for (int m = 0; m < M; ++m)
       if ((rc = factor_ring(g, m, st, 2)) != EB_OK) return rc;
     return EB_OK;
@@ -1103,6 +1123,7 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   const Group g2{L, g.base + (int64_t)s1 * g.stride, g.stride, n_shifts - s1, true};
   cudaEventRecord(lane.start, st);
   cudaStreamWaitEvent(lane.stream, lane.start, 0);
+  if ((rc = begin_rings(g1, st)) != EB_OK || (rc = begin_rings(g2, s2)) != EB_OK) return rc;
   for (int m = 0; m < M; ++m) {
     if ((rc = factor_ring(g1, m, st, 2)) != EB_OK) return rc;
     if ((rc = factor_ring(g2, m, s2, 3)) != EB_OK) return rc;
@@ -1206,13 +1227,12 @@ int eb_ringlu_factor_many(const eb_batch* b, const double* const* J, int n_shift
   if ((rc = run_factor(g, J, st)) != EB_OK) return rc;
   if ((rc = check_launch("ringlu factor")) != EB_OK) return rc;
   std::vector<int> info(n_shifts);
-  for (int s = 0; s < n_shifts; ++s)
-    if (cudaMemcpyAsync(&info[s], g.base + (int64_t)s * g.stride + L.off_info, sizeof(int),
-                        cudaMemcpyDeviceToHost, st) != cudaSuccess)
-      return check_launch("ringlu info");
+  if (cudaMemcpy2DAsync(info.data(), sizeof(int), g.base + L.off_info, g.stride, sizeof(int),
+                        n_shifts, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    return check_launch("ringlu info");
   if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch("ringlu info");
-  for (int s = 0; s < n_shifts; ++s)
-    if (info[s] != 0) return fail(EB_ERR_NAN, "ringlu: singular or non-finite ring block");
+  for (int i : info)
+    if (i != 0) return fail(EB_ERR_NAN, "ringlu: singular or non-finite ring block");
   return EB_OK;
 }
 
