@@ -338,6 +338,93 @@ __global__ void __launch_bounds__(kGemmThreads)
 
 namespace {
 
+// ---- real matrices ----------------------------------------------------------------------------
+// The cp.async ring on 64 x 32 tiles with real elements: a copy moves two (the dimensions are
+// multiples of 4, so a pair never straddles an edge), pitches 4 modulo 16 doubles keep the
+// fragment loads of each half-warp on distinct banks. K = 512: 128 tiles per product, two
+// products (or shifts) fill the SMs.
+constexpr int kRealBN = 32, kRealStages = 3;
+struct RealSmem {
+  double a[kRealStages][kBK][kPadM];
+  double b[kRealStages][kRealBN][kPadK];
+};
+
+__global__ void __launch_bounds__(kGemmThreads)
+    k_dgemm_nn(int M, int N, int K, double alpha, Operands ops, int lda, int ldb, double beta,
+               int ldc) {
+  constexpr int BN = kRealBN, Stages = kRealStages, NJ = BN / 16;
+  extern __shared__ __align__(16) unsigned char dg_smem[];
+  RealSmem& S = *reinterpret_cast<RealSmem*>(dg_smem);
+  const double *A, *B;
+  double* C;
+  ops.of(blockIdx.z, A, B, C);
+  const int tid = threadIdx.x;
+  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+  const int lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
+  const int fr = lane >> 2, fc = lane & 3;
+  double acc[4][NJ][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int slices = (K + kBK - 1) / kBK;
+  auto issue = [&](int s) {  // slice s into buffer s % Stages (one commit group per call)
+    if (s < slices) {
+      const int buf = s % Stages, k0 = s * kBK;
+#pragma unroll
+      for (int q = 0; q < kBM * kBK / 2 / kGemmThreads; ++q) {
+        const int e = tid + kGemmThreads * q, m = 2 * (e % (kBM / 2)), k = e / (kBM / 2);
+        const int gm = m0 + m, gk = k0 + k;
+        const bool ok = gm < M && gk < K;
+        cp_async16(&S.a[buf][k][m], ok ? A + gm + (int64_t)lda * gk : A, ok);
+      }
+#pragma unroll
+      for (int q = 0; q < kBK * BN / 2 / kGemmThreads; ++q) {
+        const int e = tid + kGemmThreads * q, k = 2 * (e % (kBK / 2)), n = e / (kBK / 2);
+        const int gk = k0 + k, gn = n0 + n;
+        const bool ok = gk < K && gn < N;
+        cp_async16(&S.b[buf][n][k], ok ? B + gk + (int64_t)ldb * gn : B, ok);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < Stages - 1; ++s) issue(s);
+  for (int s = 0; s < slices; ++s) {
+    cp_async_wait<Stages - 2>();
+    __syncthreads();
+    issue(s + Stages - 1);
+    const int buf = s % Stages;
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 4) {
+      double a[4], b[NJ];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = S.a[buf][kk + fc][wm + 8 * i + fr];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) b[j] = S.b[buf][wn + 8 * j + fr][kk + fc];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma884(acc[i][j], a[i], b[j]);
+    }
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int gm = m0 + wm + 8 * i + fr, gn = n0 + wn + 8 * j + 2 * fc + h;
+        if (gm < M && gn < N) {
+          double* c = C + gm + (int64_t)ldc * gn;
+          const double v = alpha * acc[i][j][h];
+          *c = beta != 0.0 ? fma(beta, *c, v) : v;
+        }
+      }
+}
+
 int launch_zgemm(int M, int N, int K, double alpha, double beta, const Operands& ops, int lda,
                  int ldb, int ldc, int batch, int variant, cudaStream_t st) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
@@ -376,6 +463,19 @@ int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_
               int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st) {
   const Operands ops{base, base, base, stride, stride, stride, set};
   return launch_zgemm(M, N, K, alpha, beta, ops, lda, ldb, ldc, workspaces * set.n, -1, st);
+}
+
+int dgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || workspaces * set.n <= 0) return 0;
+  if ((M | N | K | lda | ldb | ldc) % 4 != 0) return fail(EB_ERR_ARG, "dgemm: sizes must be multiples of 4");
+  const Operands ops{base, base, base, stride, stride, stride, set};
+  if (cudaFuncSetAttribute(k_dgemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(RealSmem)) != cudaSuccess)
+    return check_launch("dgemm attribute");
+  const dim3 grid((M + kBM - 1) / kBM, (N + kRealBN - 1) / kRealBN, workspaces * set.n);
+  k_dgemm_nn<<<grid, kGemmThreads, sizeof(RealSmem), st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
+  return check_launch("dgemm");
 }
 
 namespace {

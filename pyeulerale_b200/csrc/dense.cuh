@@ -38,6 +38,10 @@ struct Products {
 int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
               int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st);
 
+// The same with real matrices; the dimensions and leading dimensions are multiples of 4.
+int dgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st);
+
 // One matrix-vector product of a triangular sweep, as byte offsets into a workspace:
 // y = [y +] alpha op(A) x - Bd v - op(A2) (Bd2 v2), with op(A) = A and Bd, Bd2 as they are, or
 // op(A) = A^H and Bd, Bd2 transposed. A, A2: n x n complex, column-major; Bd, Bd2: n / 4 real

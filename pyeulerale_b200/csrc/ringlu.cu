@@ -124,7 +124,7 @@ struct Layout {
   int M, N, K;
   size_t blk;   // bytes of one K x K complex block
   size_t bdr;   // bytes of one ring's block diagonal (N real 4 x 4 blocks)
-  size_t off_D, off_L1, off_C1, off_B1d, off_C1d, off_B2, off_C2, off_T, off_L2, off_Rp, off_perm,
+  size_t off_D, off_L1, off_C1, off_B1d, off_C1d, off_B2, off_C2, off_T, off_L2, off_Cr, off_Br, off_Rp, off_perm,
       off_info, off_flags, off_acc, off_shift;
   size_t off_y, off_x, off_r, off_w;
   size_t total;
@@ -152,6 +152,8 @@ Layout plan(int M, int N) {
   L.off_C2 = take(L.bdr * M);
   L.off_T = take(L.blk);
   L.off_L2 = take(L.blk);
+  L.off_Cr = take(L.blk);
+  L.off_Br = take(L.blk);
   L.off_Rp = take(sizeof(cuDoubleComplex) * (size_t)kGjBlock * L.K);
   L.off_perm = take(sizeof(int) * (size_t)L.K);
   L.off_info = take(sizeof(int) * 4);
@@ -167,10 +169,34 @@ Layout plan(int M, int N) {
   return L;
 }
 
+// A scalar of type T (the imaginary part of a real one is dropped).
+template <class T>
+__device__ __forceinline__ T scalar(double re, double im = 0.0);
+template <>
+__device__ __forceinline__ double scalar<double>(double re, double) {
+  return re;
+}
+template <>
+__device__ __forceinline__ cuDoubleComplex scalar<cuDoubleComplex>(double re, double im) {
+  return make_cuDoubleComplex(re, im);
+}
+__device__ __forceinline__ cuDoubleComplex complex_of(double v) {
+  return make_cuDoubleComplex(v, 0.0);
+}
+__device__ __forceinline__ cuDoubleComplex complex_of(cuDoubleComplex v) { return v; }
+// acc + w x for a real w
+__device__ __forceinline__ double axpy(double w, double x, double acc) { return fma(w, x, acc); }
+__device__ __forceinline__ cuDoubleComplex axpy(double w, cuDoubleComplex x, cuDoubleComplex acc) {
+  return make_cuDoubleComplex(fma(w, x.x, acc.x), fma(w, x.y, acc.y));
+}
+
 // Scatters the 4x4 blocks of the nine-slot Jacobian: the couplings within a ring, minus the shift
 // on the diagonal, into the (zeroed) ring super-blocks D (column-major K x K), the couplings to
 // other rings into the rings' block diagonals (ring m, cell n: 16 doubles at 16 (m N + n),
 // column-major).
+// T: the scalar type of D, whose blocks are blk complex elements apart either way (real numbers, of
+// a real shift, fill the first half of a block's place).
+template <class T>
 __global__ void k_assemble(int M, int N, const double* J, const double* shift,
                            cuDoubleComplex* D, double* B1, double* C1, double* B2, double* C2) {
   const double sr = shift[0], si = shift[1];
@@ -191,7 +217,7 @@ __global__ void k_assemble(int M, int N, const double* J, const double* shift,
       continue;
     }
     const int nn = wrap(n + slot_dn(s), N);
-    cuDoubleComplex* T = D + blk * m;
+    T* out = reinterpret_cast<T*>(D + blk * m);
     for (int i = 0; i < 4; ++i)
       for (int r = 0; r < 4; ++r) {
         double v = J16[r + 4 * i];
@@ -200,7 +226,7 @@ __global__ void k_assemble(int M, int N, const double* J, const double* shift,
           v -= sr;
           w = -si;
         }
-        T[(int64_t)(4 * nn + i) * K + (4 * n + r)] = make_cuDoubleComplex(v, w);
+        out[(int64_t)(4 * nn + i) * K + (4 * n + r)] = scalar<T>(v, w);
       }
   }
 }
@@ -514,101 +540,110 @@ __global__ void __launch_bounds__(256) k_gj_permute(int K, Systems sys, size_t o
   }
 }
 
-__device__ __forceinline__ cuDoubleComplex from_real(double v) {
-  return make_cuDoubleComplex(v, 0.0);
-}
-
 // One column of a dense K x K block from its N real 4 x 4 diagonal blocks: entry r of column c.
 __device__ __forceinline__ double bd_at(const double* bd, int r, int c) {
   return (r >> 2) == (c >> 2) ? bd[16 * (r >> 2) + (r & 3) + 4 * (c & 3)] : 0.0;
 }
 
-// X = the dense block of a block diagonal, two of them (blockIdx.z). Grid: K columns x shifts x 2.
+// The kernels below work on blocks of scalar type T. Where a block is also part of the factors,
+// which are complex whatever T is, a real launch writes it a second time as complex numbers.
+
+// X = the dense block of a block diagonal, two of them (blockIdx.z); Z1: the second one as complex
+// numbers (real T). Grid: K columns x shifts x 2.
+template <class T>
 __global__ void __launch_bounds__(256) k_bd_fill(int K, Systems sys, size_t bd0, size_t x0,
-                                                 size_t bd1, size_t x1) {
+                                                 size_t bd1, size_t x1, size_t z1) {
   const double* bd = at<const double>(sys, blockIdx.z ? bd1 : bd0);
-  cuDoubleComplex* X = at<cuDoubleComplex>(sys, blockIdx.z ? x1 : x0) + (size_t)K * blockIdx.x;
-  for (int r = threadIdx.x; r < K; r += blockDim.x) X[r] = from_real(bd_at(bd, r, blockIdx.x));
+  T* X = at<T>(sys, blockIdx.z ? x1 : x0) + (size_t)K * blockIdx.x;
+  cuDoubleComplex* Z = at<cuDoubleComplex>(sys, z1) + (size_t)K * blockIdx.x;
+  for (int r = threadIdx.x; r < K; r += blockDim.x) {
+    const double v = bd_at(bd, r, blockIdx.x);
+    X[r] = scalar<T>(v);
+    if (sizeof(T) == sizeof(double) && blockIdx.z) Z[r] = complex_of(v);
+  }
 }
 
 // Before the products of a step (blockIdx.z): 0: X = Bd S (Bd the N real 4 x 4 blocks at bd);
 // 1: F = the dense block of the block diagonal at fbd. Grid: N x shifts x 2.
-__global__ void __launch_bounds__(256) k_bd_left(int K, Systems sys, size_t off_bd, size_t off_S, size_t off_X,
-                                                 size_t off_fbd, size_t off_F) {
+template <class T>
+__global__ void __launch_bounds__(256) k_bd_left(int K, Systems sys, size_t off_bd, size_t off_S,
+                                                 size_t off_X, size_t off_fbd, size_t off_F) {
   const int n = blockIdx.x;
   if (blockIdx.z == 1) {  // columns 4 n .. 4 n + 3
     const double* bd = at<const double>(sys, off_fbd);
-    cuDoubleComplex* F = at<cuDoubleComplex>(sys, off_F);
+    T* F = at<T>(sys, off_F);
     for (int e = threadIdx.x; e < 4 * K; e += blockDim.x) {
       const int r = e % K, c = 4 * n + e / K;
-      F[(size_t)K * c + r] = from_real(bd_at(bd, r, c));
+      F[(size_t)K * c + r] = scalar<T>(bd_at(bd, r, c));
     }
     return;
   }
   __shared__ double bd[16];
   const double* B = at<const double>(sys, off_bd);
-  const cuDoubleComplex* S = at<cuDoubleComplex>(sys, off_S);
-  cuDoubleComplex* X = at<cuDoubleComplex>(sys, off_X);
+  const T* S = at<T>(sys, off_S);
+  T* X = at<T>(sys, off_X);
   if (threadIdx.x < 16) bd[threadIdx.x] = B[16 * n + threadIdx.x];
   __syncthreads();
   for (int c = threadIdx.x; c < K; c += blockDim.x) {
-    const cuDoubleComplex* s = S + (size_t)K * c + 4 * n;
-    const cuDoubleComplex s0 = s[0], s1 = s[1], s2 = s[2], s3 = s[3];
-    cuDoubleComplex* x = X + (size_t)K * c + 4 * n;
+    const T* s = S + (size_t)K * c + 4 * n;
+    const T sv[4] = {s[0], s[1], s[2], s[3]};
+    T* x = X + (size_t)K * c + 4 * n;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const double b0 = bd[r], b1 = bd[r + 4], b2 = bd[r + 8], b3 = bd[r + 12];
-      x[r] = make_cuDoubleComplex(fma(b3, s3.x, fma(b2, s2.x, fma(b1, s1.x, b0 * s0.x))),
-                                  fma(b3, s3.y, fma(b2, s2.y, fma(b1, s1.y, b0 * s0.y))));
+      T acc = scalar<T>(0.0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc = axpy(bd[r + 4 * k], sv[k], acc);
+      x[r] = acc;
     }
   }
 }
 
 // After the products of a step (blockIdx.z): 0: Y -= X Bd; 1: Y1 = F - X1 Bd, F the dense block of
-// the block diagonal at fbd, Bd the N real 4 x 4 blocks at bd; 2: the step's L1 (X1) to its
-// slot. Grid: N column blocks x shifts x 3.
-__global__ void __launch_bounds__(256) k_bd_right(int K, Systems sys, size_t off_bd, size_t off_X, size_t off_Y,
-                                                  size_t off_X1, size_t off_Y1, size_t off_fbd, size_t off_L) {
+// the block diagonal at fbd, Bd the N real 4 x 4 blocks at bd (Z1: the same as complex numbers,
+// real T); 2: the step's L1 (X1) to its place L. Grid: N column blocks x shifts x 3.
+template <class T>
+__global__ void __launch_bounds__(256) k_bd_right(int K, Systems sys, size_t off_bd, size_t off_X,
+                                                  size_t off_Y, size_t off_X1, size_t off_Y1,
+                                                  size_t off_Z1, size_t off_fbd, size_t off_L) {
   __shared__ double bd[16];
   const int n = blockIdx.x, z = blockIdx.z;
-  const cuDoubleComplex* X = at<cuDoubleComplex>(sys, z == 0 ? off_X : off_X1);
+  const T* X = at<T>(sys, z == 0 ? off_X : off_X1);
   if (z == 2) {
     cuDoubleComplex* L = at<cuDoubleComplex>(sys, off_L);
     for (int e = threadIdx.x; e < 4 * K; e += blockDim.x)
-      L[(size_t)K * 4 * n + e] = X[(size_t)K * 4 * n + e];
+      L[(size_t)K * 4 * n + e] = complex_of(X[(size_t)K * 4 * n + e]);
     return;
   }
   const double* B = at<const double>(sys, off_bd);
-  cuDoubleComplex* Y = at<cuDoubleComplex>(sys, z == 0 ? off_Y : off_Y1);
+  T* Y = at<T>(sys, z == 0 ? off_Y : off_Y1);
+  cuDoubleComplex* Z = at<cuDoubleComplex>(sys, off_Z1);
   const double* fbd = z == 1 ? at<const double>(sys, off_fbd) : nullptr;
   if (threadIdx.x < 16) bd[threadIdx.x] = B[16 * n + threadIdx.x];
   __syncthreads();
   for (int r = threadIdx.x; r < K; r += blockDim.x) {
-    cuDoubleComplex x[4];
+    T x[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) x[q] = X[(size_t)K * (4 * n + q) + r];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      cuDoubleComplex* y = Y + (size_t)K * (4 * n + c) + r;
-      cuDoubleComplex acc = fbd ? from_real(bd_at(fbd, r, 4 * n + c)) : *y;
+      const size_t e = (size_t)K * (4 * n + c) + r;
+      T acc = fbd ? scalar<T>(bd_at(fbd, r, 4 * n + c)) : Y[e];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double b = bd[q + 4 * c];
-        acc.x = fma(-x[q].x, b, acc.x);
-        acc.y = fma(-x[q].y, b, acc.y);
-      }
-      *y = acc;
+      for (int q = 0; q < 4; ++q) acc = axpy(-bd[q + 4 * c], x[q], acc);
+      Y[e] = acc;
+      if (sizeof(T) == sizeof(double) && fbd) Z[e] = complex_of(acc);
     }
   }
 }
 
-// The step's L1 to its slot. Grid: any x shifts.
+// Y = X as complex numbers. Grid: any x shifts.
+template <class T>
 __global__ void __launch_bounds__(256) k_copy_block(int K, Systems sys, size_t off_X, size_t off_Y) {
-  const cuDoubleComplex* X = at<cuDoubleComplex>(sys, off_X);
+  const T* X = at<T>(sys, off_X);
   cuDoubleComplex* Y = at<cuDoubleComplex>(sys, off_Y);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)K * K;
        e += (int64_t)gridDim.x * blockDim.x)
-    Y[e] = X[e];
+    Y[e] = complex_of(X[e]);
 }
 
 // Reference layout (4, M, N) <-> ring layout [m][n][v].
@@ -712,6 +747,7 @@ struct Group {
   char* base;
   int64_t stride;  // bytes
   int S;
+  bool real = false;     // every shift is real: the elimination runs in real numbers
   bool blocked = false;  // how its rings are inverted (see invert)
   Systems systems() const { return Systems{base, stride}; }
 };
@@ -751,8 +787,8 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
   const Layout& L = g.L;
   const int K = L.K, nb = panel_width(K);
   if (!g.blocked) {
-    const InvertAt where{D, L.off_T, D, 0, L.off_flags, L.off_info};
-    return ring_invert(K, g.S, g.base, g.stride, where, epoch, false, st);
+    const InvertAt where{D, L.off_T, D, L.off_L2 + L.blk / 2, L.off_flags, L.off_info};
+    return ring_invert(K, g.S, g.base, g.stride, where, epoch, g.real, st);
   }
   // Look-ahead: the block's update of the next block's columns runs on st, right before the
   // next block's panels; its update of every other column runs on the side stream, under
@@ -796,50 +832,70 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
     return check_launch("ringlu side join");
   k_gj_permute<<<dim3(std::min(K, 1024), g.S), 256, sizeof(int) * K, st>>>(
       K, g.systems(), D, L.off_T, L.off_perm, L.off_info);
-  k_copy_block<<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(K, g.systems(),
-                                                                               L.off_T, D);
+  k_copy_block<cuDoubleComplex><<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(
+      K, g.systems(), L.off_T, D);
   return EB_OK;
 }
 
+// The operands of the elimination. Complex elimination: each block in its place among the factors.
+// Real elimination (a quarter of the arithmetic): real numbers in the first half of a diagonal
+// block's place until it is inverted, in scratch for the rest (T and L2 in the first halves of
+// their places, the inverse in the second half of L2's, the couplings alternating between the
+// halves of Cr and Br); the factors are stored as complex numbers all the same, so the solves do
+// not depend on it.
+struct Blocks {
+  const Layout& L;
+  bool real;
+  size_t D(int m) const { return L.off_D + L.blk * m; }
+  size_t Dinv(int m) const { return real ? L.off_L2 + L.blk / 2 : D(m); }
+  size_t B(int m) const { return real ? L.off_Br + (m & 1) * (L.blk / 2) : stored_B(m); }
+  size_t C(int m) const { return real ? L.off_Cr + (m & 1) * (L.blk / 2) : stored_C(m); }
+  size_t stored_B(int m) const { return L.off_L1 + L.blk * m; }
+  size_t stored_C(int m) const { return L.off_C1 + L.blk * m; }
+};
+
 // The dense couplings of ring 0.
+template <class T>
 int begin_rings(const Group& g, cudaStream_t st) {
   const Layout& L = g.L;
-  k_bd_fill<<<dim3(L.K, g.S, 2), 256, 0, st>>>(L.K, g.systems(), L.off_B1d + L.bdr,
-                                               L.off_L1 + L.blk, L.off_C1d, L.off_C1);
+  const Blocks b{L, g.real};
+  k_bd_fill<T><<<dim3(L.K, g.S, 2), 256, 0, st>>>(L.K, g.systems(), L.off_B1d + L.bdr, b.B(1),
+                                                  L.off_C1d, b.C(0), b.stored_C(0));
   return check_launch("ringlu couplings");
 }
 
 // One ring of the block elimination for every shift of the group.
+template <class T>
 int factor_ring(const Group& g, int m, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
+  const Blocks b{L, g.real};
   const int M = L.M, K = L.K, N = L.N;
-  auto D = [&](int r) { return L.off_D + L.blk * r; };
-  auto B = [&](int r) { return L.off_L1 + L.blk * r; };
-  auto C = [&](int r) { return L.off_C1 + L.blk * r; };
   auto products = [&](double alpha, double beta, const dense::Products& p) {
-    return dense::zgemm_set(K, K, K, alpha, beta, g.base, g.stride, g.S, p, K, K, K, st);
+    return g.real ? dense::dgemm_set(K, K, K, alpha, beta, g.base, g.stride, g.S, p, K, K, K, st)
+                  : dense::zgemm_set(K, K, K, alpha, beta, g.base, g.stride, g.S, p, K, K, K, st);
   };
-  int rc = invert(g, D(m), m + 1, st, side_lane);
+  int rc = invert(g, b.D(m), m + 1, st, side_lane);
   if (rc != EB_OK || m + 1 == M) return rc;
   dense::Products t;  // T = L1[m+1] = B1'[m+1] Dinv_m
-  t.add(B(m + 1), D(m), L.off_T);
+  t.add(b.B(m + 1), b.Dinv(m), L.off_T);
   if ((rc = products(1.0, 0.0, t)) != EB_OK) return rc;
   dense::Products p;
-  p.add(L.off_T, C(m), D(m + 1));  // D[m+1] -= T C1'[m]
+  p.add(L.off_T, b.C(m), b.D(m + 1));  // D[m+1] -= T C1'[m]
   if (m + 2 < M) {
     // L2[m+2] = B2[m+2] Dinv_m (scratch);  B1'[m+2] = B1[m+2] - L2[m+2] C1'[m]
-    k_bd_left<<<dim3(N, g.S, 2), 256, 0, st>>>(K, g.systems(), L.off_B2 + L.bdr * (m + 2), D(m),
-                                               L.off_L2, L.off_B1d + L.bdr * (m + 2), B(m + 2));
-    p.add(L.off_L2, C(m), B(m + 2));
+    k_bd_left<T><<<dim3(N, g.S, 2), 256, 0, st>>>(K, g.systems(), L.off_B2 + L.bdr * (m + 2),
+                                                  b.Dinv(m), L.off_L2,
+                                                  L.off_B1d + L.bdr * (m + 2), b.B(m + 2));
+    p.add(L.off_L2, b.C(m), b.B(m + 2));
   }
   if ((rc = products(-1.0, 1.0, p)) != EB_OK) return rc;
   if (m + 2 < M)  // D[m+2] -= L2[m+2] C2[m];  C1'[m+1] = C1[m+1] - T C2[m];  L1[m+1] = T
-    k_bd_right<<<dim3(N, g.S, 3), 256, 0, st>>>(K, g.systems(), L.off_C2 + L.bdr * m, L.off_L2,
-                                                D(m + 2), L.off_T, C(m + 1),
-                                                L.off_C1d + L.bdr * (m + 1), B(m + 1));
+    k_bd_right<T><<<dim3(N, g.S, 3), 256, 0, st>>>(
+        K, g.systems(), L.off_C2 + L.bdr * m, L.off_L2, b.D(m + 2), L.off_T, b.C(m + 1),
+        b.stored_C(m + 1), L.off_C1d + L.bdr * (m + 1), b.stored_B(m + 1));
   else
-    k_copy_block<<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(
-        K, g.systems(), L.off_T, B(m + 1));
+    k_copy_block<T><<<dim3(grid_for((int64_t)K * K, 256) / 4 + 1, g.S), 256, 0, st>>>(
+        K, g.systems(), L.off_T, b.stored_B(m + 1));
   return check_launch("ringlu step");
 }
 
@@ -1092,26 +1148,31 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   if (n_shifts > kMost) {
     for (int s = 0; s < n_shifts && rc == EB_OK; s += kMost)
       rc = issue_factor(Group{L, g.base + (int64_t)s * g.stride, g.stride,
-                              std::min(kMost, n_shifts - s)}, J + s, st);
+                              std::min(kMost, n_shifts - s), g.real}, J + s, st);
     return rc;
   }
   for (int s = 0; s < n_shifts; ++s) {
     char* w = g.base + (int64_t)s * g.stride;
-    cudaMemsetAsync(w + L.off_D, 0, L.blk * M, st);
+    if (cudaMemset2DAsync(w + L.off_D, L.blk, 0, g.real ? L.blk / 2 : L.blk, M, st) != cudaSuccess)
+      return check_launch("ringlu zero");
     cudaMemsetAsync(w + L.off_info, 0, L.off_acc - L.off_info, st);  // and the inversions' flags
-    k_assemble<<<grid_for((int64_t)M * N * 9, 256), 256, 0, st>>>(
+    auto assemble = g.real ? k_assemble<double> : k_assemble<cuDoubleComplex>;
+    assemble<<<grid_for((int64_t)M * N * 9, 256), 256, 0, st>>>(
         M, N, J[s], reinterpret_cast<const double*>(w + L.off_shift),
         reinterpret_cast<cuDoubleComplex*>(w + L.off_D), reinterpret_cast<double*>(w + L.off_B1d),
         reinterpret_cast<double*>(w + L.off_C1d), reinterpret_cast<double*>(w + L.off_B2),
         reinterpret_cast<double*>(w + L.off_C2));
   }
   if ((rc = check_launch("ringlu assemble")) != EB_OK) return rc;
-  if (!blocked_inversion(L.K, (n_shifts + 1) / 2)) {
+  if (g.real || !blocked_inversion(L.K, (n_shifts + 1) / 2)) {
     // one stream: the inversions are cooperative launches, which never run two at a time here
-    if ((rc = begin_rings(g, st)) != EB_OK) return rc;
-    for (int m = 0; m < M; ++m)
-      if ((rc = factor_ring(g, m, st, 2)) != EB_OK) return rc;
-    return EB_OK;
+    auto all = [&](auto begin, auto ring) {
+      int code = begin(g, st);
+      for (int m = 0; m < M && code == EB_OK; ++m) code = ring(g, m, st, 2);
+      return code;
+    };
+    return g.real ? all(begin_rings<double>, factor_ring<double>)
+                  : all(begin_rings<cuDoubleComplex>, factor_ring<cuDoubleComplex>);
   }
   // Two halves of the shifts on two streams, ring by ring: one half's latency-bound
   // Gauss-Jordan panels overlap the other half's GEMMs on the rest of the GPU.
@@ -1119,14 +1180,16 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
   if ((rc = lane_stream(st, s2, 1)) != EB_OK) return rc;
   const Handle& lane = g_handle[1];
   const int s1 = (n_shifts + 1) / 2;
-  const Group g1{L, g.base, g.stride, s1, true};
-  const Group g2{L, g.base + (int64_t)s1 * g.stride, g.stride, n_shifts - s1, true};
+  const Group g1{L, g.base, g.stride, s1, false, true};
+  const Group g2{L, g.base + (int64_t)s1 * g.stride, g.stride, n_shifts - s1, false,
+                 true};
   cudaEventRecord(lane.start, st);
   cudaStreamWaitEvent(lane.stream, lane.start, 0);
-  if ((rc = begin_rings(g1, st)) != EB_OK || (rc = begin_rings(g2, s2)) != EB_OK) return rc;
+  using Z = cuDoubleComplex;
+  if ((rc = begin_rings<Z>(g1, st)) != EB_OK || (rc = begin_rings<Z>(g2, s2)) != EB_OK) return rc;
   for (int m = 0; m < M; ++m) {
-    if ((rc = factor_ring(g1, m, st, 2)) != EB_OK) return rc;
-    if ((rc = factor_ring(g2, m, s2, 3)) != EB_OK) return rc;
+    if ((rc = factor_ring<Z>(g1, m, st, 2)) != EB_OK) return rc;
+    if ((rc = factor_ring<Z>(g2, m, s2, 3)) != EB_OK) return rc;
   }
   cudaEventRecord(lane.done, lane.stream);
   cudaStreamWaitEvent(st, lane.done, 0);
@@ -1139,11 +1202,12 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
 // per thread (least recently used first out). EB_RINGLU_GRAPHS=0 turns capture off.
 struct GraphKey {
   int device, M, N, S;
+  bool real;
   const char* base;
   int64_t stride;
   std::vector<const double*> J;
   bool operator==(const GraphKey& o) const {
-    return device == o.device && M == o.M && N == o.N && S == o.S && base == o.base &&
+    return device == o.device && M == o.M && N == o.N && S == o.S && real == o.real && base == o.base &&
            stride == o.stride && J == o.J;
   }
 };
@@ -1166,7 +1230,7 @@ int run_factor(const Group& g, const double* const* J, cudaStream_t st) {
   if (!graphs_enabled()) return issue_factor(g, J, st);
   int dev = 0;
   cudaGetDevice(&dev);
-  GraphKey key{dev, g.L.M, g.L.N, g.S, g.base, g.stride, std::vector<const double*>(J, J + g.S)};
+  GraphKey key{dev, g.L.M, g.L.N, g.S, g.real, g.base, g.stride, std::vector<const double*>(J, J + g.S)};
   GraphEntry* e = nullptr;
   for (auto& x : g_graphs)
     if (x.key == key) e = &x;
@@ -1219,7 +1283,9 @@ int eb_ringlu_factor_many(const eb_batch* b, const double* const* J, int n_shift
   for (int s = 0; s < n_shifts; ++s)
     if (!J[s]) return fail(EB_ERR_ARG, "ringlu: null Jacobian");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const Group g{L, static_cast<char*>(workspace), workspace_stride, n_shifts};
+  bool real = true;
+  for (int s = 0; s < n_shifts; ++s) real = real && shifts[2 * s + 1] == 0.0;
+  const Group g{L, static_cast<char*>(workspace), workspace_stride, n_shifts, real};
   for (int s = 0; s < n_shifts; ++s)
     if (cudaMemcpyAsync(g.base + (int64_t)s * g.stride + L.off_shift, shifts + 2 * s,
                         2 * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess)
@@ -1482,7 +1548,7 @@ int issue_ptc_step(const eb_batch* b, const PtcLayout& P, char* ws, const double
   const int64_t cells = (int64_t)M * N;
   PtcCtl* ctl = reinterpret_cast<PtcCtl*>(ws + P.off_ctl);
   char* lw = ws + P.off_lu;
-  const Group g{P.lu, lw, (int64_t)P.lu.total, 1};
+  const Group g{P.lu, lw, (int64_t)P.lu.total, 1, true};  // (the step's shifts are real)
   double* shift = reinterpret_cast<double*>(lw + P.lu.off_shift);
   cuDoubleComplex* y = reinterpret_cast<cuDoubleComplex*>(lw + P.lu.off_y);
   cuDoubleComplex* x = reinterpret_cast<cuDoubleComplex*>(lw + P.lu.off_x);
