@@ -31,7 +31,7 @@ NVCC_FLAGS = [
 # exact free stream), and only uncontracted evaluation keeps equal inputs bitwise equal across
 # the differently inlined call sites. The residual itself is continuous there and keeps FMA.
 PER_FILE_FLAGS = {"jacobians.cu": ["-fmad=false"], "second_order.cu": ["-fmad=false"],
-                  "jac_tiled.cu": ["-fmad=false"]}
+                  "jac_cells.cu": ["-fmad=false"]}
 # The library links only the CUDA runtime: its dense products are its own kernels (dense.cu).
 LINK_FLAGS = []
 

@@ -1,0 +1,434 @@
+// d(odes)/d(states), d(odes)/d(vertices), d(odes)/d(velocities) and d(odes)/d(mach)
+// (eb_compute_odes_wrt_*, replacing the complex-step procedures of
+// src/spatial_discretization.f90:552-593, 666-750, 933-993, 1087-1143): one thread per cell, each
+// of its four faces differentiated in closed form (jac_faces.cuh).
+//
+// A cell's outputs (nine 4 x 4 blocks, or four corners' 4 x 2 blocks) are what bounds these
+// kernels: 1152 or 256 bytes per cell against about 1200 FP64 operations. Threads are the cells in
+// their order in memory (radial index fastest), so a warp's 32 blocks of one slot are contiguous
+// whatever the grid's sizes; each warp passes them through shared memory and writes them in
+// whole 512-byte rows (written by the threads themselves, a store touched 32 lines for 16 bytes
+// each). A block sum keeps the reference's face order, ((F_b + F_f) + F_i) + F_o.
+//
+// Measured on 282,000 cells of uneven grids: states 567 us before (dual numbers, tiles staged in
+// shared memory, at one CTA per SM), vertices 594 us, velocities 263 us, mach 34 us.
+
+#include "autotune.cuh"
+#include "common.cuh"
+#include "jac_faces.cuh"
+
+namespace eb {
+namespace {
+
+// A warp's outputs of D doubles per cell, in rows padded by 16 bytes, so that the threads' 16-byte
+// accesses to their own rows fall on distinct banks.
+template <int D>
+struct WarpRows {
+  double2 v[32][D / 2 + 1];
+};
+
+// Thread `lane` hands over `mine`; the warp writes the rows of its first `valid` cells to `out`
+// (the first cell's place).
+template <int D>
+__device__ __forceinline__ void write_rows(WarpRows<D>& S, const double (&mine)[D], int lane,
+                                           int valid, double* out) {
+#pragma unroll
+  for (int e = 0; e < D / 2; ++e) S.v[lane][e] = make_double2(mine[2 * e], mine[2 * e + 1]);
+  __syncwarp();
+  constexpr int kPer = D / 2;
+  double2* o = reinterpret_cast<double2*>(out);
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int f = 32 * e + lane;
+    if (f < valid * kPer) o[f] = S.v[f / kPer][f % kPer];
+  }
+  __syncwarp();
+}
+
+struct CellAt {  // a cell's place in its instance
+  int m, n;
+  int64_t M, N;
+  const double *U, *X, *V;
+
+  __device__ __forceinline__ State state(int dm, int dn) const {
+    int c = n + dn;
+    c = c < 0 ? c + (int)N : c >= (int)N ? c - (int)N : c;
+    const double2* q = reinterpret_cast<const double2*>(U + 4 * (m + dm + M * c));
+    const double2 a = __ldg(q), b = __ldg(q + 1);
+    return make_state(a.x, a.y, b.x, b.y);
+  }
+  // The corners in the order backward-inward, forward-inward, forward-outward, backward-outward.
+  __device__ __forceinline__ double2 corner(const double* A, int k) const {
+    const int64_t v = m + (k >= 2) + (M + 1) * (n + (k == 1 || k == 2));
+    return __ldg(reinterpret_cast<const double2*>(A + 2 * v));
+  }
+};
+
+struct CellGeometry {
+  double2 x[4];
+  FaceGeometry b, f, i, o;  // faces between corners 3-0, 1-2, 0-1 and 2-3 (outward normals)
+  double cross;     // signed area times 2
+
+  __device__ __forceinline__ explicit CellGeometry(const CellAt& at) {
+    double2 w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      x[k] = at.corner(at.X, k);
+      w[k] = at.V ? at.corner(at.V, k) : make_double2(0.0, 0.0);
+    }
+    auto edge = [&](int p, int q) {
+      return FaceGeometry{x[q].y - x[p].y, x[p].x - x[q].x, (w[p].x + w[q].x) / 2.0,
+                  (w[p].y + w[q].y) / 2.0};
+    };
+    i = edge(0, 1);
+    f = edge(1, 2);
+    o = edge(2, 3);
+    b = edge(3, 0);
+    cross = (x[2].x - x[0].x) * (x[3].y - x[1].y) - (x[2].y - x[0].y) * (x[3].x - x[1].x);
+  }
+  __device__ __forceinline__ double inv_area() const { return 1.0 / (abs_c(cross) / 2.0); }
+  __device__ __forceinline__ Wall wall() const { return make_wall(i.nx, i.nz, i.gx, i.gz); }
+};
+
+// The radial line of a cell, boundary rows included (make_ode's five cases, f90:401-436): the
+// inner face has the line (o, c, i, ii), the outer one (i, c, o, oo), with ghost states past the
+// ends and the dissipation off on the faces whose line would reach past a ghost.
+struct RadialLine {
+  State i, o, ii, oo;
+  bool diss_i, diss_o;
+  __device__ __forceinline__ RadialLine(const CellAt& at, const State& c, const CellGeometry& g,
+                                        const Instance& in) {
+    const int m = at.m, M = (int)at.M;
+    diss_i = m >= 2;
+    diss_o = m <= M - 3;
+    i = m > 0 ? at.state(-1, 0) : wall_ghost_of(c, g.wall());
+    o = m < M - 1 ? at.state(1, 0) : farfield_ghost_of(c, in);
+    ii = diss_i ? at.state(-2, 0) : c;
+    oo = diss_o ? at.state(2, 0) : c;
+  }
+};
+
+__device__ __forceinline__ void clear(double (&a)[16]) {
+#pragma unroll
+  for (int e = 0; e < 16; ++e) a[e] = 0.0;
+}
+
+// Calls body(local cell, lane, valid cells of the warp) for the cells of this thread's instance.
+// Whole warps stay in the loop together; the body's cell is clamped to the instance.
+template <class Body>
+__device__ __forceinline__ void for_cells(const Instance& in, Body body) {
+  const int64_t cells = (int64_t)in.M * in.N;
+  const int lane = threadIdx.x & 31;
+  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); first < cells;
+       first += (int64_t)gridDim.x * blockDim.x) {
+    const int valid = (int)min((int64_t)32, cells - first);
+    body(first, min(first + lane, cells - 1), lane, valid);
+  }
+}
+
+__device__ __forceinline__ CellAt cell_at(const Instance& in, int64_t local, const double* X,
+                                          const double* V, const double* U) {
+  return CellAt{(int)(local % in.M), (int)(local / in.M), in.M, in.N, U + 4 * in.cell_offset,
+                X + 2 * in.vert_offset, V ? V + 2 * in.vert_offset : nullptr};
+}
+
+template <int Warps>
+__global__ void __launch_bounds__(32 * Warps, 12 / Warps)
+    k_jac_states_cells(Table t, const double* X, const double* V, const double* U, double* J) {
+  __shared__ WarpRows<16> rows[Warps];
+  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
+  WarpRows<16>& S = rows[threadIdx.x >> 5];
+  const int64_t slot = 16 * (int64_t)in.M * in.N;
+  for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
+    const CellAt at = cell_at(in, local, X, V, U);
+    const int m = at.m, M = in.M;
+    const CellGeometry geo(at);
+    const double s = -geo.inv_area();
+    double* out = J + 144 * in.cell_offset + 16 * first;
+    auto store = [&](int k, double (&a)[16], bool active) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) a[e] = active ? s * a[e] : 0.0;
+      write_rows(S, a, lane, valid, out + slot * k);
+    };
+    double centre[16], a[16];
+    clear(centre);
+    const State c = at.state(0, 0);
+    {  // angular faces: b (line f, c, b, bb), then f (line b, c, f, ff)
+      const State fw = at.state(0, 1), bw = at.state(0, -1);
+      double Qb[4], gb, c4b;  // face b's block of its outer state f
+      {
+        const State bb = at.state(0, -2);
+        const FaceDerivatives d(fw, c, bw, bb, geo.b, true, in);
+        add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
+        clear(a);
+        add_outer(a, d.Q, d.g_rr, d.c4, bb);
+        store(kBB, a, true);
+        clear(a);
+        add_block(a, d.of<false>(bw), bw, d.nx, d.nz, d.vr);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) Qb[k] = d.Q[k];
+        gb = d.g_ll;
+        c4b = d.c4;
+      }
+      const State ff = at.state(0, 2);
+      const FaceDerivatives d(bw, c, fw, ff, geo.f, true, in);
+      add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
+      add_outer(a, d.Q, d.g_ll, -d.c4, bw);
+      store(kB, a, true);
+      clear(a);
+      add_outer(a, Qb, gb, -c4b, fw);
+      add_block(a, d.of<false>(fw), fw, d.nx, d.nz, d.vr);
+      store(kF, a, true);
+      clear(a);
+      add_outer(a, d.Q, d.g_rr, d.c4, ff);
+      store(kFF, a, true);
+    }
+    // radial faces: i (line o, c, i, ii), then o (line i, c, o, oo); a ghost's block goes to the
+    // cell itself, through the ghost's derivative
+    const RadialLine line(at, c, geo, in);
+    double Qi[4], gi, c4i;  // face i's block of its outer state o
+    {
+      const FaceDerivatives d(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+      add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
+      clear(a);
+      add_outer(a, d.Q, d.g_rr, d.c4, line.ii);
+      store(kII, a, m > 1);
+      clear(a);
+      add_block(a, d.of<false>(line.i), line.i, d.nx, d.nz, d.vr);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) Qi[k] = d.Q[k];
+      gi = d.g_ll;
+      c4i = d.c4;
+    }
+    const FaceDerivatives d(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+    if (m == 0) through_wall(centre, a, geo.wall());
+    if (m == M - 1) {  // face i's outer state is the far-field ghost: minus its block
+      double e[16];
+      clear(e);
+      add_outer(e, Qi, gi, -c4i, line.o);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) centre[k] -= e[k];
+    }
+    add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
+    if (m == 0) {
+      double e[16];
+      clear(e);
+      add_outer(e, d.Q, d.g_ll, -d.c4, line.i);
+      through_wall(centre, e, geo.wall());
+    }
+    add_outer(a, d.Q, d.g_ll, -d.c4, line.i);
+    store(kI, a, m > 0);
+    clear(a);
+    add_outer(a, d.Q, d.g_rr, d.c4, line.oo);
+    store(kOO, a, m < M - 2);
+    clear(a);
+    add_block(a, d.of<false>(line.o), line.o, d.nx, d.nz, d.vr);
+    if (m == M - 1) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) centre[k] -= a[k];
+    }
+    add_outer(a, Qi, gi, -c4i, line.o);
+    store(kO, a, m < M - 1);
+    store(kC, centre, true);
+  });
+}
+
+// The derivative of the wall ghost's momentum by the wall's normal (x then z) or grid velocity,
+// contracted with dF_k by the momentum: e1, e2 -> the derivatives of F_k.
+__device__ __forceinline__ double2 ghost_by_normal(const Wall& w, const State& c, double e1,
+                                                   double e2) {
+  const double mx = c.u[1] - w.gx * c.u[0], mz = c.u[2] - w.gz * c.u[0];
+  const double t = w.nx * mx + w.nz * mz, en = fma(e1, w.nx, e2 * w.nz);
+  const double q = 2.0 * w.inn, r = q * en;
+  return make_double2(fma(r, 2.0 * t * w.nx * w.inn - mx, -q * t * e1),
+                      fma(r, 2.0 * t * w.nz * w.inn - mz, -q * t * e2));
+}
+__device__ __forceinline__ double2 ghost_by_velocity(const Wall& w, const State& c, double e1,
+                                                     double e2) {
+  const double a = 2.0 * w.inn * c.u[0] * fma(e1, w.nx, e2 * w.nz);
+  return make_double2(a * w.nx, a * w.nz);
+}
+
+// d(odes)/d(vertices) (Velo = false) or d(odes)/d(velocities): four corners' 4 x 2 blocks.
+template <bool Velo>
+__global__ void __launch_bounds__(128, 3)
+    k_jac_corners_cells(Table t, const double* X, const double* V, const double* U, double* J) {
+  __shared__ WarpRows<8> rows[4];
+  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
+  WarpRows<8>& S = rows[threadIdx.x >> 5];
+  const int64_t slot = 8 * (int64_t)in.M * in.N;
+  for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
+    const CellAt at = cell_at(in, local, X, V, U);
+    const int m = at.m;
+    const CellGeometry geo(at);
+    const double ia = geo.inv_area();
+    const State c = at.state(0, 0);
+    // per face (b, f, i, o): dF_k by its normal, or by its grid velocity
+    double gx[4][4], gz[4][4], sum[4];
+    auto face = [&](int q, const State& ll, const State& r, const State& rr, const FaceGeometry& f,
+                    bool diss) {
+      if constexpr (Velo) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double a = -0.5 * (c.u[k] + r.u[k]);
+          gx[q][k] = a * f.nx;
+          gz[q][k] = a * f.nz;
+        }
+      } else {
+        const FaceDerivatives d(ll, c, r, rr, f, diss, in);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          gx[q][k] = d.by_normal<true>(c, r, f, k);
+          gz[q][k] = d.by_normal<false>(c, r, f, k);
+          const double v = d.flux(ll, c, r, rr, k);
+          sum[k] = q == 0 ? v : sum[k] + v;
+        }
+      }
+    };
+    {
+      const State fw = at.state(0, 1), bw = at.state(0, -1);
+      if constexpr (Velo) {
+        face(0, c, bw, c, geo.b, true);
+        face(1, c, fw, c, geo.f, true);
+      } else {
+        face(0, fw, bw, at.state(0, -2), geo.b, true);
+        face(1, bw, fw, at.state(0, 2), geo.f, true);
+      }
+    }
+    const RadialLine line(at, c, geo, in);
+    face(2, line.o, line.i, line.ii, geo.i, line.diss_i);
+    face(3, line.i, line.o, line.oo, geo.o, line.diss_o);
+    if (m == 0) {  // the wall ghost is on both radial lines and moves with the inner face
+      const Wall w = geo.wall();
+      double e[16], dp[4];
+      clear(e);
+      const FaceDerivatives di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+      add_block(e, di.of<false>(line.i), line.i, di.nx, di.nz, di.vr);
+      const FaceDerivatives dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+      grad_p(line.i, dp);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // face o's outer block: Q g_ll (x) dp - c4 I
+        const double q = dO.Q[k] * dO.g_ll;
+        const double e1 = e[k + 4] + fma(q, dp[1], k == 1 ? -dO.c4 : 0.0);
+        const double e2 = e[k + 8] + fma(q, dp[2], k == 2 ? -dO.c4 : 0.0);
+        const double2 a = Velo ? ghost_by_velocity(w, c, e1, e2) : ghost_by_normal(w, c, e1, e2);
+        gx[2][k] += a.x;
+        gz[2][k] += a.y;
+      }
+    }
+    double* out = J + 32 * in.cell_offset + 8 * first;
+    const double sa = geo.cross < 0.0 ? -0.5 : 0.5;  // the area by the cross product
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      // corner k ends face `into` and begins face `from` (corners 0-1: i, 1-2: f, 2-3: o, 3-0: b)
+      const int from = k == 0 ? 2 : k == 1 ? 1 : k == 2 ? 3 : 0;
+      const int into = k == 0 ? 0 : k == 1 ? 2 : k == 2 ? 1 : 3;
+      double a[8];
+      if constexpr (Velo) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          a[r] = -ia * 0.5 * (gx[from][r] + gx[into][r]);
+          a[r + 4] = -ia * 0.5 * (gz[from][r] + gz[into][r]);
+        }
+      } else {
+        // cross = (x2 - x0) (z3 - z1) - (z2 - z0) (x3 - x1), by corner k's coordinates
+        const double2 p = geo.x[(k + 1) & 3], q = geo.x[(k + 3) & 3];
+        double ax = p.y - q.y, az = q.x - p.x;
+        ax *= sa;
+        az *= sa;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {  // the normal of the face p -> q is (z_q - z_p, x_p - x_q)
+          const double R = -sum[r] * ia;
+          a[r] = -ia * fma(R, ax, gz[from][r] - gz[into][r]);
+          a[r + 4] = -ia * fma(R, az, gx[into][r] - gx[from][r]);
+        }
+      }
+      write_rows(S, a, lane, valid, out + slot * k);
+    }
+  });
+}
+
+// d(odes)/d(mach): zero but for the far-field row, whose ghost 2 U_inf - U depends on the Mach
+// number. Blocks of the grid's first part write the zeros (rows of whole warps), the rest take the
+// far-field cells, one thread each (with a thread per cell, every warp that held a far-field cell
+// ran its four faces for one lane).
+__global__ void __launch_bounds__(128)
+    k_jac_mach_cells(Table t, int zero_blocks, const double* X, const double* V, const double* U,
+                     double* J) {
+  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
+  const int64_t cells = (int64_t)in.M * in.N;
+  double* Ji = J + 4 * in.cell_offset;
+  if ((int)blockIdx.x < zero_blocks) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 2 * cells;
+         e += (int64_t)zero_blocks * blockDim.x)
+      if ((e >> 1) % in.M != in.M - 1) reinterpret_cast<double2*>(Ji)[e] = make_double2(0.0, 0.0);
+    return;
+  }
+  for (int n = (blockIdx.x - zero_blocks) * blockDim.x + threadIdx.x; n < in.N;
+       n += (gridDim.x - zero_blocks) * blockDim.x) {
+    const int64_t local = in.M - 1 + (int64_t)in.M * n;
+    const CellAt at = cell_at(in, local, X, V, U);
+    const CellGeometry geo(at);
+    const State c = at.state(0, 0);
+    const RadialLine line(at, c, geo, in);
+    const FaceDerivatives di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+    const FaceDerivatives dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+    double e[16];
+    clear(e);
+    add_outer(e, di.Q, di.g_ll, -di.c4, line.o);
+    add_block(e, dO.of<false>(line.o), line.o, dO.nx, dO.nz, dO.vr);
+    const double root = sqrt_(kGamma), speed = in.mach * root;
+    const double d[4] = {0.0, 2.0 * root * in.cos_aoa, 2.0 * root * in.sin_aoa, 2.0 * speed * root};
+    const double s = -geo.inv_area();
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      Ji[4 * local + k] = s * fma(e[k + 4], d[1], fma(e[k + 8], d[2], e[k + 12] * d[3]));
+  }
+}
+
+template <int Warps>
+int launch_states(const eb_batch* b, const Table& t, const double* X, const double* V,
+                  const double* U, double* J, cudaStream_t st) {
+  dim3 grid;
+  if (int rc = per_instance_grid(b, false, 1, 32 * Warps, grid)) return rc;
+  k_jac_states_cells<Warps><<<grid, 32 * Warps, 0, st>>>(t, X, V, U, J);
+  return check_launch("compute_odes_wrt_states");
+}
+
+}  // namespace
+
+int launch_jac_states(const eb_batch* b, const double* X, const double* V, const double* U,
+                      double* J, cudaStream_t st) {
+  const Table t = make_table(b);
+  static const char* const kNames[2] = {"width 4 (warps per CTA)", "width 2 (warps per CTA)"};
+  return tune::launch_tuned("jac_states_tiled", b->n_cells, b->max_dim, 2, 0, kNames, st,
+                            [&](int v) {
+                              return v == 0 ? launch_states<4>(b, t, X, V, U, J, st)
+                                            : launch_states<2>(b, t, X, V, U, J, st);
+                            });
+}
+
+int launch_jac_corners(const eb_batch* b, bool velocities, const double* X, const double* V,
+                       const double* U, double* J, cudaStream_t st) {
+  const Table t = make_table(b);
+  dim3 grid;
+  if (int rc = per_instance_grid(b, false, 1, 128, grid)) return rc;
+  if (velocities) k_jac_corners_cells<true><<<grid, 128, 0, st>>>(t, X, V, U, J);
+  else k_jac_corners_cells<false><<<grid, 128, 0, st>>>(t, X, V, U, J);
+  return check_launch(velocities ? "compute_odes_wrt_velocities" : "compute_odes_wrt_vertices");
+}
+
+int launch_jac_mach(const eb_batch* b, const double* X, const double* V, const double* U,
+                    double* J, cudaStream_t st) {
+  const Table t = make_table(b);
+  dim3 grid;
+  if (int rc = per_instance_grid(b, false, 1, 512, grid)) return rc;
+  const int N = b->n_inst > 1 || b->d_table ? b->max_dim : b->single.N;
+  const int zero_blocks = (int)grid.x;
+  grid.x += (N + 127) / 128;
+  k_jac_mach_cells<<<grid, 128, 0, st>>>(t, zero_blocks, X, V, U, J);
+  return check_launch("compute_odes_wrt_mach");
+}
+
+}  // namespace eb
