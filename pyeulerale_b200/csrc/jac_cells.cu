@@ -133,7 +133,7 @@ __device__ __forceinline__ CellAt cell_at(const Instance& in, int64_t local, con
 }
 
 template <int Warps>
-__global__ void __launch_bounds__(32 * Warps, 12 / Warps)
+__global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
     k_jac_states_cells(Table t, const double* X, const double* V, const double* U, double* J) {
   __shared__ WarpRows<16> rows[Warps];
   const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;

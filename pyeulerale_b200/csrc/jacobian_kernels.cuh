@@ -36,7 +36,9 @@ struct SeededStates {
 
 // d(odes)/d(states) blocks (compute_odes_wrt_states, f90:666-750). B = double gives the
 // Jacobian; B = Dual<double,2> with a direction gives its directional derivatives. Each slot's
-// block sums only the faces that read that slot (others contribute exactly zero).
+// block sums only the faces that read that slot (others contribute exactly zero). Grid z: slots
+// (one block of threads per slot: with a thread per cell alone, a 128 x 128 grid leaves an SM four
+// warps, and one of its blocks runs up to sixteen face evaluations one after the other).
 template <class B, int Dir>
 __global__ void __launch_bounds__(128) k_jac_states(Table t, int64_t n_cells, const double* X,
                                                     const double* V, const double* U,
@@ -61,7 +63,7 @@ __global__ void __launch_bounds__(128) k_jac_states(Table t, int64_t n_cells, co
     const B area_b = lift<B>(geo.area);
     const int64_t slot_stride = 16 * (int64_t)in.M * in.N;
     const int64_t base = 144 * in.cell_offset + 16 * local;
-    for (int s = 0; s < 9; ++s) {
+    for (int s = blockIdx.z; s < 9; s += gridDim.z) {
       const int64_t o = base + slot_stride * s;
       if (!slot_active(s, p.m, in.M)) {
         for (int e = 0; e < 16; ++e) store_b<B>(lift<B>(0.0), o + e, J, Jre, Jim);
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(128) k_jac_states(Table t, int64_t n_cells, co
   }
 }
 
-// d(odes)/d(vertices) or d(odes)/d(velocities) blocks (f90:933-993, 1087-1143).
+// d(odes)/d(vertices) or d(odes)/d(velocities) blocks (f90:933-993, 1087-1143). Grid z: corners.
 template <class B, int Dir, bool Velo>
 __global__ void __launch_bounds__(128) k_jac_vertexlike(Table t, int64_t n_cells,
                                                         const double* X, const double* V,
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(128) k_jac_vertexlike(Table t, int64_t n_cells
     typed_corners<TVb, B>(p.w, dir.xr, dir.xi, Dir == kDirVelocities, wo);
     const int64_t slot_stride = 8 * (int64_t)in.M * in.N;
     const int64_t base = 32 * in.cell_offset + 8 * local;
-    for (int k = 0; k < 4; ++k) {
+    for (int k = blockIdx.z; k < 4; k += gridDim.z) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if constexpr (Velo) {

@@ -44,6 +44,7 @@ int eb_compute_odes_wrt_states_untiled(const eb_batch* b, const double* X, const
   const Table t = make_table(b);
   dim3 jgrid;
   if (int rc = per_instance_grid(b, false, 1, 128, jgrid)) return rc;
+  jgrid.z = 9;
   k_jac_states<double, kDirNone><<<jgrid, 128, 0, EB_STREAM(stream)>>>(
       t, b->n_cells, X, V, U, nullptr, J, nullptr, nullptr);
   return check_launch("compute_odes_wrt_states_untiled");

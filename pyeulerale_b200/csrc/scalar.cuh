@@ -74,6 +74,9 @@ EB_HD double value(const Dual<T, K>& x) {
   return value(x.v);
 }
 
+// Quotients and roots keep their values' division; the derivatives share one reciprocal per operand
+// (a division per component made up most of the nested duals' time).
+
 // ---- Dual (op) Dual ------------------------------------------------------------------------
 template <class T, int K>
 EB_HD Dual<T, K> operator+(const Dual<T, K>& a, const Dual<T, K>& b) {
@@ -111,8 +114,9 @@ template <class T, int K>
 EB_HD Dual<T, K> operator/(const Dual<T, K>& a, const Dual<T, K>& b) {
   Dual<T, K> r;
   r.v = a.v / b.v;
+  const T inv = 1.0 / b.v;
 #pragma unroll
-  for (int i = 0; i < K; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) / b.v;
+  for (int i = 0; i < K; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * inv;
   return r;
 }
 
@@ -165,16 +169,18 @@ template <class T, int K, class S, EB_LOWER(S, T)>
 EB_HD Dual<T, K> operator/(const Dual<T, K>& a, const S& b) {
   Dual<T, K> r;
   r.v = a.v / b;
+  const S inv = 1.0 / b;
 #pragma unroll
-  for (int i = 0; i < K; ++i) r.d[i] = a.d[i] / b;
+  for (int i = 0; i < K; ++i) r.d[i] = a.d[i] * inv;
   return r;
 }
 template <class T, int K, class S, EB_LOWER(S, T)>
 EB_HD Dual<T, K> operator/(const S& a, const Dual<T, K>& b) {
   Dual<T, K> r;
   r.v = a / b.v;
+  const T slope = -r.v * (1.0 / b.v);
 #pragma unroll
-  for (int i = 0; i < K; ++i) r.d[i] = -(r.v * b.d[i]) / b.v;
+  for (int i = 0; i < K; ++i) r.d[i] = slope * b.d[i];
   return r;
 }
 #undef EB_LOWER
@@ -185,9 +191,9 @@ template <class T, int K>
 EB_HD Dual<T, K> sqrt_(const Dual<T, K>& a) {
   Dual<T, K> r;
   r.v = sqrt_(a.v);
-  T two_r = 2.0 * r.v;
+  const T slope = 0.5 / r.v;
 #pragma unroll
-  for (int i = 0; i < K; ++i) r.d[i] = a.d[i] / two_r;
+  for (int i = 0; i < K; ++i) r.d[i] = a.d[i] * slope;
   return r;
 }
 

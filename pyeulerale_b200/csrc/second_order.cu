@@ -47,6 +47,7 @@ int eb_odes_wrt_states_dir(const eb_batch* b, const double* X, const double* V,
   const Table t = make_table(b);
   dim3 jgrid;
   if (int rc = per_instance_grid(b, false, 1, 128, jgrid)) return rc;
+  jgrid.z = 9;
   EB_DIR_DISPATCH(k_jac_states, t, b->n_cells, X, V, U, d, nullptr, J_re, J_im);
   return check_launch("odes_wrt_states_dir");
 }
@@ -60,6 +61,7 @@ int eb_odes_wrt_vertices_dir(const eb_batch* b, const double* X, const double* V
   const Table t = make_table(b);
   dim3 g;
   if (int rc = per_instance_grid(b, false, 1, 128, g)) return rc;
+  g.z = 4;
   cudaStream_t s = EB_STREAM(stream);
   switch (dir_kind) {
     case kDirStates:
