@@ -40,6 +40,48 @@ def _torch():
     return torch
 
 
+class _Staging:
+    """Pinned host buffers between the host arrays and the device, one ring per solver.
+
+    A transfer from ordinary host memory waits for the driver's own copies; through a pinned buffer
+    the host writes (or reads) the values once, in whatever layout its array has, and the transfer
+    runs on the stream. A buffer is written again only after its previous transfer has finished.
+    """
+
+    def __init__(self, torch, count: int = 4) -> None:
+        self._torch = torch
+        self._ring = [[None, torch.cuda.Event()] for _ in range(count)]
+        self._next = 0
+
+    def _buffer(self, n: int):
+        slot = self._ring[self._next]
+        self._next = (self._next + 1) % len(self._ring)
+        slot[1].synchronize()
+        if slot[0] is None or slot[0].numel() < n:
+            slot[0] = self._torch.empty(n, dtype=self._torch.float64, pin_memory=True)
+        return slot[0][:n], slot[1]
+
+    def to_device(self, array: np.ndarray, dtype, dst=None):
+        """``array`` as ``dtype`` in Fortran order on the device (flat float64, in ``dst`` if given)."""
+        n = array.size * (2 if dtype is complex else 1)
+        buf, event = self._buffer(n)
+        buf.numpy().view(dtype).reshape(array.shape, order="F")[...] = array
+        if dst is None:
+            dst = self._torch.empty(n, dtype=self._torch.float64, device="cuda")
+        dst.copy_(buf, non_blocking=True)
+        event.record()
+        return dst
+
+    def to_host(self, src, dtype, out: np.ndarray) -> np.ndarray:
+        """Flat float64 device values, as ``dtype`` in Fortran order, into ``out``."""
+        buf, event = self._buffer(src.numel())
+        buf.copy_(src, non_blocking=True)
+        event.record()
+        event.synchronize()
+        out[...] = buf.numpy().view(dtype).reshape(out.shape, order="F")
+        return out
+
+
 class SpatialDiscretization:
     """Spatial discretization of the compressible 2D Euler equations around a moving airfoil.
 
@@ -117,6 +159,7 @@ class SpatialDiscretization:
         self._dJF_u = torch.zeros(8 * N, **f64)
         self._dJF_x = torch.zeros(8 * N, **f64)
         self._mirrors: dict[str, np.ndarray] = {}
+        self._staging = _Staging(torch)
         self._lu_stale = True
         self.set_free_stream_state()
 
@@ -258,30 +301,19 @@ class SpatialDiscretization:
                                   self._coefficient_length, self._coefficient_center)
         return _lib.single_batch(inst)
 
-    def _h2d(self, dst, array: np.ndarray) -> None:
-        torch = self._torch
-        src = np.ascontiguousarray(np.asarray(array).ravel(order="F"))
-        if np.iscomplexobj(src):
-            src = src.view(np.float64)
-        dst.copy_(torch.from_numpy(src.astype(np.float64, copy=False)))
-
     def _upload(self, velocities: bool = True) -> None:
-        self._h2d(self._dX, self._vertices.real)
+        self._staging.to_device(self._vertices.real, float, self._dX)
         if velocities:
-            self._h2d(self._dV, self._velocities.real)
-        self._h2d(self._dU, self._states.real)
+            self._staging.to_device(self._velocities.real, float, self._dV)
+        self._staging.to_device(self._states.real, float, self._dU)
 
     def _cvec(self, array: np.ndarray):
         """Complex host array -> interleaved device float64 vector."""
-        torch = self._torch
-        src = np.ascontiguousarray(np.asarray(array, dtype=complex).ravel(order="F"))
-        return torch.from_numpy(src.view(np.float64)).to("cuda")
+        return self._staging.to_device(np.asarray(array), complex)
 
-    @staticmethod
-    def _store(out: np.ndarray, dev, shape: tuple) -> np.ndarray:
-        host = dev.cpu().numpy().view(np.complex128)
-        out[...] = np.reshape(host, shape, order="F")
-        return out
+    def _store(self, out: np.ndarray, dev, shape: tuple) -> np.ndarray:
+        """Interleaved complex device vector -> host array ``out`` of that shape."""
+        return self._staging.to_host(dev, complex, out)
 
     def _stream(self) -> int:
         return self._torch.cuda.current_stream().cuda_stream
@@ -294,22 +326,19 @@ class SpatialDiscretization:
     def set_free_stream_state(self) -> None:
         """Sets ``states`` to free-stream (core.py:265-268)."""
         self._call("eb_set_free_stream_state", ptr(self._dU))
-        host = self._dU.cpu().numpy()
-        self._states[...] = np.reshape(host, self._states.shape, order="F")
+        self._staging.to_host(self._dU, float, self._states)
 
     def compute_odes(self) -> None:
         """Computes ``odes`` from ``states``, ``vertices`` and ``velocities`` (core.py:270-276)."""
         self._upload()
         self._call("eb_compute_odes", ptr(self._dX), ptr(self._dV), ptr(self._dU), ptr(self._dR))
-        host = self._dR.cpu().numpy()
-        self._odes[...] = np.reshape(host, self._odes.shape, order="F")
+        self._staging.to_host(self._dR, float, self._odes)
 
     def compute_forces(self) -> None:
         """Computes ``forces`` from ``states`` and ``vertices`` (core.py:601-608)."""
         self._upload(velocities=False)
         self._call("eb_compute_forces", ptr(self._dX), ptr(self._dU), ptr(self._dF), None)
-        host = self._dF.cpu().numpy()
-        self._forces[...] = np.reshape(host, self._forces.shape, order="F")
+        self._staging.to_host(self._dF, float, self._forces)
 
     def linearize(self) -> None:
         """Computes the Jacobians on the device (core.py:278-292)."""
@@ -332,7 +361,7 @@ class SpatialDiscretization:
         y = torch.empty(2 * out_numel, dtype=torch.float64, device="cuda")
         self._call(name, ptr(jac), ptr(x), ptr(y))
         if out is None:
-            out = np.asfortranarray(np.empty(out_shape, dtype=complex))
+            out = np.empty(out_shape, dtype=complex, order="F")
         return self._store(out, y, out_shape)
 
     def apply_odes_wrt_mach_fwd(self, d_mach: np.ndarray, d_odes: np.ndarray | None = None):
@@ -508,9 +537,9 @@ class SpatialDiscretization:
         y_im = torch.empty_like(y_re)
         self._call(apply_rev, ptr(J_re), ptr(w), ptr(y_re))
         self._call(apply_rev, ptr(J_im), ptr(w), ptr(y_im))
-        a = y_re.cpu().numpy().view(np.complex128)
-        b = y_im.cpu().numpy().view(np.complex128)
-        return np.asfortranarray(np.reshape(a + 1j * b, out_shape, order="F"))
+        y_re[0::2] -= y_im[1::2]  # y_re + i y_im
+        y_re[1::2] += y_im[0::2]
+        return self._store(np.empty(out_shape, dtype=complex, order="F"), y_re, out_shape)
 
     def _grad_out(self, out, shape, result):
         if out is not None:
@@ -719,7 +748,7 @@ class SpatialDiscretization:
             self._check_array(pressure_coefficients, shape=shape,
                               dtype=np.dtypes.Float64DType())
         else:
-            pressure_coefficients = np.asfortranarray(np.empty(dtype=float, shape=shape))
+            pressure_coefficients = np.empty(dtype=float, shape=shape, order="F")
         torch = self._torch
         self._upload(velocities=False)
         cp = torch.empty(self._nc(), dtype=torch.float64, device="cuda")
@@ -735,7 +764,7 @@ class SpatialDiscretization:
         if d_pressure_coefficients is not None:
             self._check_array(d_pressure_coefficients, shape=shape)
         else:
-            d_pressure_coefficients = np.asfortranarray(np.empty(dtype=complex, shape=shape))
+            d_pressure_coefficients = np.empty(dtype=complex, shape=shape, order="F")
         torch = self._torch
         self._upload(velocities=False)
         dcp = torch.empty(2 * self._nc(), dtype=torch.float64, device="cuda")
