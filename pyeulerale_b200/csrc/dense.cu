@@ -14,7 +14,6 @@
 // both), with no register staging; it issues the same MMAs in the same order, so the two
 // variants give identical results.
 
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -623,138 +622,105 @@ __global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stri
   if (lane == 0) finish_row(t, ws, j, sr, si, true);
 }
 
-// The sweep step over nr right-hand sides (one read of A serves all of them). A cluster of
-// kSkCluster CTAs takes 32 rows: CTA c of the cluster sums the columns of its contiguous share,
-// thread (r, g) of its 256 the columns j = g (mod 8) of that share for row r and every
-// right-hand side, with eight column loads in flight; the eight warps' partial sums are added
-// in a fixed order in shared memory, and the cluster's leader adds the CTAs' partial sums in
-// rank order through distributed shared memory and writes y. Spreading a product over the
-// cluster puts eight SMs' loads in flight where one CTA per 32 rows left each SM streaming
-// its 256 KB share alone. Grid: (row groups x terms, cluster, workspaces); workspaces from
-// *n_active on exit (the whole cluster alike).
+// The sweep step over NR right-hand sides, one read of A for all of them. Bound by reading A once (K = 512: 4.2 MB per workspace and term): eight rows
+// per CTA, thread (r, g) takes the columns j = g (mod 32), 16 of them in flight at a time, issued
+// before the right-hand sides are staged in shared memory; two CTAs keep 128 KB in flight per SM.
+// The partial sums are added in a fixed order. A cluster of eight CTAs per 32 rows, which had each
+// SM wait for its cluster's barriers and remote sums, read at 2.4 TB/s with 22 workspaces active.
+// Grid: (row groups x terms, workspaces); workspaces from *n_active on exit.
 constexpr int kMaxRhs = 8;
-constexpr int kSkCluster = 8;
+constexpr int kChunk = 512;  // columns per round: 16 per thread
 
-__global__ void __cluster_dims__(1, kSkCluster, 1) __launch_bounds__(256)
-    k_sweep_multi(int n, int nr, const char* base, int64_t stride, char* vectors, int64_t vstride,
+template <int NR>
+__global__ void __launch_bounds__(256, 2)
+    k_sweep_multi(int n, const char* base, int64_t stride, char* vectors, int64_t vstride,
                   const int* zmap, const int* n_active, SweepTerms terms) {
   extern __shared__ __align__(16) unsigned char sk_smem[];
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  if ((int)blockIdx.z >= *n_active) return;  // uniform over the cluster
+  __shared__ double2 part[8][NR][8];
+  double2* xs = reinterpret_cast<double2*>(sk_smem);  // NR x min(n, kChunk)
+  const int64_t z = zmap[blockIdx.y];
+  if ((int)blockIdx.y >= *n_active) return;
   const SweepTerm t = terms.t[blockIdx.x % terms.n];
   const int group = blockIdx.x / terms.n;
-  const int64_t z = zmap[blockIdx.z];
-  const char* ws = base + stride * z;
+  char* ws = const_cast<char*>(base) + stride * z;
   char* vs = vectors + vstride * z;
-  const double2* A = reinterpret_cast<const double2*>(ws + t.a);
-  const double2* B = place<const double2>(vs, t.x);
-  const int rank = (int)cluster.block_rank();
-  const int share = (((n + kSkCluster - 1) / kSkCluster) + 7) / 8 * 8;  // columns per CTA
-  const int j0 = rank * share, j1 = min(n, j0 + share);
-  const int cols = t.a >= 0 ? max(j1 - j0, 0) : 0;
-  double2* Bs = reinterpret_cast<double2*>(sk_smem);  // cols x nr (this CTA's rows of B)
-  double2* part = Bs + (size_t)share * nr;            // 8 x 32 x nr, then the CTA's 32 x nr
-  const int total = cols * nr;
-  for (int e0 = 0; e0 < total; e0 += 8 * 256) {  // eight loads in flight per thread
-    double2 b[8];
+  const int tid = threadIdx.x, r = tid & 7, g = tid >> 3, lane = tid & 31;
+  const int i = group * 8 + r;
+  const int pitch = min(n, kChunk);
+  double sr[NR], si[NR];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = e0 + 256 * u + (int)threadIdx.x;
-      if (e < total) {
-        const int q = e / cols, j = e - q * cols;
-        b[u] = ldg_inflight(B + j0 + j + (int64_t)n * q);
-      }
+  for (int q = 0; q < NR; ++q) sr[q] = si[q] = 0.0;
+  const double2* A = place<const double2>(ws, t.a) + i;
+  const double2* x = place<const double2>(vs, t.x);
+  for (int c0 = 0; c0 < n; c0 += kChunk) {
+    const int cols = min(kChunk, n - c0);
+    double2 a[kChunk / 32];
+#pragma unroll
+    for (int u = 0; u < kChunk / 32; ++u) {
+      a[u] = make_double2(0.0, 0.0);
+      if (i < n && g + 32 * u < cols) a[u] = ldg_inflight(A + (int64_t)n * (c0 + g + 32 * u));
     }
+    if (c0 > 0) __syncthreads();  // the previous columns' right-hand sides have been used
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = e0 + 256 * u + (int)threadIdx.x;
-      if (e < total) Bs[e] = b[u];
-    }
-  }
-  __syncthreads();
-  const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int i = group * 32 + r;
-  double sr[kMaxRhs], si[kMaxRhs];
+    for (int q = 0; q < NR; ++q)
+      for (int j = tid; j < cols; j += 256) xs[pitch * q + j] = x[c0 + j + (int64_t)n * q];
+    __syncthreads();
 #pragma unroll
-  for (int q = 0; q < kMaxRhs; ++q) sr[q] = si[q] = 0.0;
-  if (i < n) {
-    constexpr int kUnroll = 8;
-    int j = g;
-    for (; j + 8 * (kUnroll - 1) < cols; j += 8 * kUnroll) {
-      double2 a[kUnroll];
+    for (int u = 0; u < kChunk / 32; ++u)
+      if (g + 32 * u < cols) {
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-        a[u] = ldg_inflight(A + i + (int64_t)n * (j0 + j + 8 * u));
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-#pragma unroll
-        for (int q = 0; q < kMaxRhs; ++q) {
-          if (q < nr) {
-            const double2 v = Bs[j + 8 * u + cols * q];
-            sr[q] = fma(a[u].x, v.x, fma(-a[u].y, v.y, sr[q]));
-            si[q] = fma(a[u].x, v.y, fma(a[u].y, v.x, si[q]));
-          }
-        }
-    }
-    for (; j < cols; j += 8) {
-      const double2 a = A[i + (int64_t)n * (j0 + j)];
-#pragma unroll
-      for (int q = 0; q < kMaxRhs; ++q) {
-        if (q < nr) {
-          const double2 v = Bs[j + cols * q];
-          sr[q] = fma(a.x, v.x, fma(-a.y, v.y, sr[q]));
-          si[q] = fma(a.x, v.y, fma(a.y, v.x, si[q]));
+        for (int q = 0; q < NR; ++q) {
+          const double2 v = xs[pitch * q + g + 32 * u];
+          sr[q] = fma(a[u].x, v.x, fma(-a[u].y, v.y, sr[q]));
+          si[q] = fma(a[u].x, v.y, fma(a[u].y, v.x, si[q]));
         }
       }
-    }
   }
 #pragma unroll
-  for (int q = 0; q < kMaxRhs; ++q)
-    if (q < nr) part[(q * 8 + g) * 32 + r] = make_double2(sr[q], si[q]);
+  for (int q = 0; q < NR; ++q) {
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      sr[q] += __shfl_xor_sync(0xffffffffu, sr[q], o);
+      si[q] += __shfl_xor_sync(0xffffffffu, si[q], o);
+    }
+    if (lane < 8) part[tid >> 5][q][lane] = make_double2(sr[q], si[q]);
+  }
   __syncthreads();
-  // the CTA's partial sums (warps in order) into part[q * 32 + r] (after the 8 x 32 x nr block)
-  double2* mine = part + 8 * 32 * nr;
-  for (int e = threadIdx.x; e < 32 * nr; e += 256) {
-    const int q = e >> 5, rr = e & 31;
+  const int row = group * 8 + (tid & 7), q = tid >> 3;
+  if (q < NR && row < n) {
     double tr = 0.0, ti = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      tr += part[(q * 8 + k) * 32 + rr].x;
-      ti += part[(q * 8 + k) * 32 + rr].y;
+      tr += part[k][q][tid & 7].x;
+      ti += part[k][q][tid & 7].y;
     }
-    mine[e] = make_double2(tr, ti);
-  }
-  cluster.sync();  // every CTA's partial sums are visible to the leader
-  if (rank == 0) {
-    for (int e = threadIdx.x; e < 32 * nr; e += 256) {
-      const int q = e >> 5, rr = e & 31;
-      const int row = group * 32 + rr;
-      double tr = 0.0, ti = 0.0;
-      for (int c = 0; c < kSkCluster; ++c) {
-        const double2* other = cluster.map_shared_rank(mine, c);
-        const double2 v = other[e];
-        tr += v.x;
-        ti += v.y;
-      }
-      if (row < n) {
-        double2* out = place<double2>(vs, t.y) + row + (int64_t)n * q;
-        double2 o = make_double2(t.alpha * tr, t.alpha * ti);
-        if (t.add) {
-          o.x += out->x;
-          o.y += out->y;
-        }
-        if (t.bd >= 0) {
-          const double2 b = bd_entry(reinterpret_cast<const double*>(ws + t.bd),
-                                     place<const double2>(vs, t.v) + (int64_t)n * q, row, false);
-          o.x -= b.x;
-          o.y -= b.y;
-        }
-        *out = o;
-      }
+    double2* out = place<double2>(vs, t.y) + row + (int64_t)n * q;
+    double2 o = make_double2(t.alpha * tr, t.alpha * ti);
+    if (t.add) {
+      o.x += out->x;
+      o.y += out->y;
     }
+    if (t.bd >= 0) {
+      const double2 b = bd_entry(place<const double>(ws, t.bd),
+                                 place<const double2>(vs, t.v) + (int64_t)n * q, row, false);
+      o.x -= b.x;
+      o.y -= b.y;
+    }
+    *out = o;
   }
-  cluster.sync();  // the leader has read every CTA's shared memory before any exits
+}
+
+template <int NR>
+int launch_sweep_multi(int n, char* base, int64_t stride, char* vectors, int64_t vstride,
+                       int workspaces, const int* zmap, const int* n_active,
+                       const SweepTerms& terms, cudaStream_t st) {
+  const int smem = (int)sizeof(double2) * NR * (n < kChunk ? n : kChunk);
+  if (cudaFuncSetAttribute(k_sweep_multi<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+      cudaSuccess)
+    return check_launch("sweep attribute");
+  k_sweep_multi<NR><<<dim3((n + 7) / 8 * terms.n, workspaces), 256, smem, st>>>(
+      n, base, stride, vectors, vstride, zmap, n_active, terms);
+  return check_launch("sweep product");
 }
 
 }  // namespace
@@ -775,16 +741,22 @@ int sweep_product_multi(int n, int nr, char* base, int64_t stride, char* vectors
                         const SweepTerms& terms, cudaStream_t st) {
   if (n % 4 != 0) return fail(EB_ERR_ARG, "sweep: block diagonals need n % 4 == 0");
   if (n <= 0 || workspaces <= 0 || nr <= 0 || terms.n <= 0) return 0;
-  if (nr > kMaxRhs) return fail(EB_ERR_ARG, "sweep: too many right-hand sides");
-  const int share = (((n + kSkCluster - 1) / kSkCluster) + 7) / 8 * 8;
-  const size_t smem = sizeof(double2) * ((size_t)share * nr + 9 * 32 * (size_t)nr);
-  if (smem > 200 * 1024) return fail(EB_ERR_ARG, "sweep: right-hand sides too large");
-  if (cudaFuncSetAttribute(k_sweep_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return check_launch("sweep attribute");
-  k_sweep_multi<<<dim3((n + 31) / 32 * terms.n, kSkCluster, workspaces), 256, smem, st>>>(
-      n, nr, base, stride, vectors, vstride, zmap, n_active, terms);
-  return check_launch("sweep product");
+  for (int k = 0; k < terms.n; ++k)
+    if (terms.t[k].a < 0 || terms.t[k].a2 >= 0) return fail(EB_ERR_ARG, "sweep: one matrix per term");
+  auto run = [&](auto launch) {
+    return launch(n, base, stride, vectors, vstride, workspaces, zmap, n_active, terms, st);
+  };
+  switch (nr) {
+    case 1: return run(launch_sweep_multi<1>);
+    case 2: return run(launch_sweep_multi<2>);
+    case 3: return run(launch_sweep_multi<3>);
+    case 4: return run(launch_sweep_multi<4>);
+    case 5: return run(launch_sweep_multi<5>);
+    case 6: return run(launch_sweep_multi<6>);
+    case 7: return run(launch_sweep_multi<7>);
+    case kMaxRhs: return run(launch_sweep_multi<kMaxRhs>);
+    default: return fail(EB_ERR_ARG, "sweep: too many right-hand sides");
+  }
 }
 
 }  // namespace dense
