@@ -125,8 +125,9 @@ __device__ void angular_rev(const Smem& S, const Instance& in, int fr, int fc,
   add_raw(A.u[2], rb);
   add_raw(A.u[3], rrb);
   if (len > 0.0) {
-    nxb += lenb * nbx / len;
-    nzb += lenb * nbz / len;
+    const double t = quot_(lenb, len);
+    nxb += t * nbx;
+    nzb += t * nbz;
   }
   A.n[0] += nxb + vnb * gx;
   A.n[1] += nzb + vnb * gz;
@@ -258,8 +259,9 @@ __device__ void radial_rev(const Smem& S, const Instance& in, int fm, int fr, in
     add_raw(A.u[2], Rb);
   }
   if (len > 0.0) {
-    nxb += lenb * nix / len;
-    nzb += lenb * niz / len;
+    const double t = quot_(lenb, len);
+    nxb += t * nix;
+    nzb += t * niz;
   }
   A.n[0] += nxb + vnb * gx;
   A.n[1] += nzb + vnb * gz;
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
       area = abs_c((fox - bix) * (boz - fiz) - (foz - biz) * (box - fix)) / 2.0;
       const double* w = Wi + 4 * cstride * (m + (int64_t)M * wrap_n(n0 + c));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) q[k] = -__ldg(w + cstride * k + h) / area;
+      for (int k = 0; k < 4; ++k) q[k] = -quot_(__ldg(w + cstride * k + h), area);
     }
     S.area[e] = area;
 #pragma unroll
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
       const double box = S.x[vidx(r + 1, c)], boz = S.z[vidx(r + 1, c)];
       const double cross = (fox - bix) * (boz - fiz) - (foz - biz) * (box - fix);
       // the slots hold q . F = -(w . F) / area, so (w . S) / area^2 = -ws / area
-      a = -ws / ar * sgn_c(cross) / 2.0;
+      a = -quot_(ws, ar) * sgn_c(cross) / 2.0;
     }
     S.ac[e] = a;
   }

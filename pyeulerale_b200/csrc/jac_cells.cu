@@ -86,7 +86,7 @@ struct CellGeometry {
     b = edge(3, 0);
     cross = (x[2].x - x[0].x) * (x[3].y - x[1].y) - (x[2].y - x[0].y) * (x[3].x - x[1].x);
   }
-  __device__ __forceinline__ double inv_area() const { return 1.0 / (abs_c(cross) / 2.0); }
+  __device__ __forceinline__ double inv_area() const { return recip_(abs_c(cross) / 2.0); }
   __device__ __forceinline__ Wall wall() const { return make_wall(i.nx, i.nz, i.gx, i.gz); }
 };
 

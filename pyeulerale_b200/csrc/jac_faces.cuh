@@ -35,7 +35,7 @@ __device__ __forceinline__ State make_state(double rho, double j1, double j2, do
   s.u[1] = j1;
   s.u[2] = j2;
   s.u[3] = e;
-  s.ir = 1.0 / rho;
+  s.ir = recip_(rho);
   s.p = kGm1 * (e - (j1 * j1 + j2 * j2) * s.ir * 0.5);
   s.vx = j1 * s.ir;
   s.vz = j2 * s.ir;
@@ -54,14 +54,14 @@ struct Wall {  // a wall face: normal, grid velocity, n.g and 1 / |n|^2
   double nx, nz, gx, gz, gn, inn;
 };
 __device__ __forceinline__ Wall make_wall(double nx, double nz, double gx, double gz) {
-  return Wall{nx, nz, gx, gz, nx * gx + nz * gz, 1.0 / (nx * nx + nz * nz)};
+  return Wall{nx, nz, gx, gz, nx * gx + nz * gz, recip_(nx * nx + nz * nz)};
 }
 // make_wall_ghost_state, f90:231-240.
 __device__ __forceinline__ State wall_ghost_of(const State& s, const Wall& w) {
   const double proj = w.nx * (s.u[1] - w.gx * s.u[0]) + w.nz * (s.u[2] - w.gz * s.u[0]);
   const double nn = w.nx * w.nx + w.nz * w.nz;
-  return make_state(s.u[0], s.u[1] - 2.0 * w.nx * proj / nn, s.u[2] - 2.0 * w.nz * proj / nn,
-                    s.u[3]);
+  return make_state(s.u[0], s.u[1] - quot_(2.0 * w.nx * proj, nn),
+                    s.u[2] - quot_(2.0 * w.nz * proj, nn), s.u[3]);
 }
 // make_farfield_ghost_state, f90:269-274: 2 U_inf - U.
 __device__ __forceinline__ State farfield_ghost_of(const State& s, const Instance& in) {
@@ -88,7 +88,7 @@ struct FaceDerivatives {
   double g_ll, g_l, g_r, g_rr;  // dS/dp of the four states
   double c2, c4;
   bool lam_l;                   // lambda is l's (else r's)
-  double sgn, c, len;           // that state's sign of the normal velocity and speed of sound
+  double sgn, c, len, ilen;     // that state's sign of the normal velocity and speed of sound; |n|
 
   __device__ __forceinline__ FaceDerivatives(const State& ll, const State& l, const State& r,
                                              const State& rr, const FaceGeometry& f, bool diss,
@@ -99,6 +99,7 @@ struct FaceDerivatives {
     vl = (nx * l.u[1] + nz * l.u[2]) * l.ir;
     vr = (nx * r.u[1] + nz * r.u[2]) * r.ir;
     len = sqrt_(nx * nx + nz * nz);
+    ilen = recip_(len);
     const double cl = sqrt_(kGamma * l.p * l.ir), cr = sqrt_(kGamma * r.p * r.ir);
     const double al = abs_c(vl) + cl * len, ar = abs_c(vr) + cr * len;
     lam_l = al > ar + 1e-8;
@@ -107,11 +108,11 @@ struct FaceDerivatives {
     sgn = (lam_l ? vl : vr) < 0.0 ? -1.0 : 1.0;
     const double num_l = ll.p - 2.0 * l.p + r.p, den_l = ll.p + 2.0 * l.p + r.p;
     const double num_r = l.p - 2.0 * r.p + rr.p, den_r = l.p + 2.0 * r.p + rr.p;
-    const double sl = abs_c(num_l) / den_l, sr = abs_c(num_r) / den_r;
+    const double sl = quot_(abs_c(num_l), den_l), sr = quot_(abs_c(num_r), den_r);
     const bool s_l = sl > sr + 1e-8;
     const double S = s_l ? sl : sr;
     const double sg = (s_l ? num_l : num_r) < 0.0 ? -1.0 : 1.0;
-    const double inv = 1.0 / (s_l ? den_l : den_r);
+    const double inv = recip_(s_l ? den_l : den_r);
     const double outer = (sg - S) * inv, centre = -2.0 * (sg + S) * inv;
     g_ll = s_l ? outer : 0.0;
     g_l = s_l ? centre : outer;
@@ -140,7 +141,7 @@ struct FaceDerivatives {
     const double v = Left ? vl : vr, g = Left ? g_l : g_r;
     const bool lam = Left == lam_l;
     // dlambda = sgn dv + len dc, dc = c / (2 p) dp - c / (2 rho) e_0
-    const double lp = lam ? 0.5 * len * c / s.p : 0.0, le = lam ? -0.5 * len * c * s.ir : 0.0;
+    const double lp = lam ? quot_(0.5 * len * c, s.p) : 0.0, le = lam ? -0.5 * len * c * s.ir : 0.0;
     const double lv = lam ? sgn : 0.0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -172,7 +173,7 @@ struct FaceDerivatives {
     double d = 0.5 * fma(l.u[k], ul - g, r.u[k] * (ur - g));
     if (k == (X ? 1 : 2)) d += 0.5 * (l.p + r.p);
     if (k == 3) d += 0.5 * fma(l.p, ul, r.p * ur);
-    const double lam = fma(sgn, lam_l ? ul : ur, c * (X ? nx : nz) / len);
+    const double lam = fma(sgn, lam_l ? ul : ur, c * (X ? nx : nz) * ilen);
     return fma(h[k], lam, d);
   }
 };

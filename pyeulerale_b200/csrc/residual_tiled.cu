@@ -214,7 +214,7 @@ __device__ __forceinline__ void tile_compute(TileSmem<T>& S, const Instance& in,
                       const T& boz) {
     const T fox = S.x[vidx(r + 1, c + 1)], foz = S.z[vidx(r + 1, c + 1)];
     const T area = abs_c((fox - bix) * (boz - fiz) - (foz - biz) * (box - fix)) / 2.0;
-    return T(1.0 / area);
+    return recip_(area);
   };
   if (own) {
     if constexpr (Pre) {

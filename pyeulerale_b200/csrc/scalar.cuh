@@ -21,6 +21,54 @@
 
 namespace eb {
 
+// ---- quotients and roots of doubles ---------------------------------------------------------
+// The stencil kernels spend up to a dozen divisions and roots per cell; the built-in ones end in a
+// branch to a path for subnormal and extreme operands. These start from the hardware's
+// approximations and refine them by Newton's iteration (the third-order form y (1 + e + e^2) for
+// 1 / b; the coupled Newton step for the root and its inverse), with a last correction by the
+// remainder, which leaves half a unit in the last place and a little. Zeros, infinities and NaN
+// among the divisors and radicands give what the built-in operations give; subnormal ones count
+// as zero.
+EB_HD double recip_(double b) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);  // NaN for zero and infinite b
+  double r = fma(y, fma(e, e, e), y);
+  r = fma(r, fma(-b, r, 1.0), r);
+  return e == e ? r : y;
+#else
+  return 1.0 / b;
+#endif
+}
+EB_HD double quot_(double a, double b) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);
+  const double r = fma(y, fma(e, e, e), y);
+  double q = a * r;
+  q = fma(fma(-b, q, a), r, q);
+  return e == e ? q : a * y;
+#else
+  return a / b;
+#endif
+}
+EB_HD double sqrt_(double x) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(x));
+  double g = x * y, h = 0.5 * y;
+  const double r = fma(-g, h, 0.5);  // NaN for zero, infinite and negative x
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  g = fma(fma(-g, g, x), h, g);
+  return r == r ? g : (x < 0.0 ? y : x);
+#else
+  return ::sqrt(x);
+#endif
+}
+
 template <class T, int K>
 struct Dual {
   T v;
@@ -74,8 +122,12 @@ EB_HD double value(const Dual<T, K>& x) {
   return value(x.v);
 }
 
-// Quotients and roots keep their values' division; the derivatives share one reciprocal per operand
-// (a division per component made up most of the nested duals' time).
+// Quotients and roots of any scalars; a dual's derivatives share one reciprocal per operand (a
+// division per component made up most of the nested duals' time).
+template <class A, class B>
+EB_HD promote_t<A, B> quot_(const A& a, const B& b);
+template <class T, int K>
+EB_HD Dual<T, K> recip_(const Dual<T, K>& b);
 
 // ---- Dual (op) Dual ------------------------------------------------------------------------
 template <class T, int K>
@@ -113,8 +165,8 @@ EB_HD Dual<T, K> operator*(const Dual<T, K>& a, const Dual<T, K>& b) {
 template <class T, int K>
 EB_HD Dual<T, K> operator/(const Dual<T, K>& a, const Dual<T, K>& b) {
   Dual<T, K> r;
-  r.v = a.v / b.v;
-  const T inv = 1.0 / b.v;
+  r.v = quot_(a.v, b.v);
+  const T inv = recip_(b.v);
 #pragma unroll
   for (int i = 0; i < K; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * inv;
   return r;
@@ -168,8 +220,8 @@ EB_HD Dual<T, K> operator*(const S& a, const Dual<T, K>& b) {
 template <class T, int K, class S, EB_LOWER(S, T)>
 EB_HD Dual<T, K> operator/(const Dual<T, K>& a, const S& b) {
   Dual<T, K> r;
-  r.v = a.v / b;
-  const S inv = 1.0 / b;
+  r.v = quot_(a.v, b);
+  const S inv = recip_(b);
 #pragma unroll
   for (int i = 0; i < K; ++i) r.d[i] = a.d[i] * inv;
   return r;
@@ -177,21 +229,34 @@ EB_HD Dual<T, K> operator/(const Dual<T, K>& a, const S& b) {
 template <class T, int K, class S, EB_LOWER(S, T)>
 EB_HD Dual<T, K> operator/(const S& a, const Dual<T, K>& b) {
   Dual<T, K> r;
-  r.v = a / b.v;
-  const T slope = -r.v * (1.0 / b.v);
+  r.v = quot_(a, b.v);
+  const T slope = -r.v * recip_(b.v);
 #pragma unroll
   for (int i = 0; i < K; ++i) r.d[i] = slope * b.d[i];
   return r;
 }
 #undef EB_LOWER
 
+template <class A, class B>
+EB_HD promote_t<A, B> quot_(const A& a, const B& b) {
+  return a / b;
+}
+template <class T, int K>
+EB_HD Dual<T, K> recip_(const Dual<T, K>& b) {
+  Dual<T, K> r;
+  r.v = recip_(b.v);
+  const T slope = -r.v * r.v;
+#pragma unroll
+  for (int i = 0; i < K; ++i) r.d[i] = slope * b.d[i];
+  return r;
+}
+
 // ---- elementary functions ------------------------------------------------------------------
-EB_HD double sqrt_(double x) { return ::sqrt(x); }
 template <class T, int K>
 EB_HD Dual<T, K> sqrt_(const Dual<T, K>& a) {
   Dual<T, K> r;
   r.v = sqrt_(a.v);
-  const T slope = 0.5 / r.v;
+  const T slope = 0.5 * recip_(r.v);
 #pragma unroll
   for (int i = 0; i < K; ++i) r.d[i] = a.d[i] * slope;
   return r;

@@ -51,7 +51,7 @@ __device__ __forceinline__ St<T> derive(const T& rho, const T& j1, const T& j2, 
   s.j1 = j1;
   s.j2 = j2;
   s.e = e;
-  s.ir = 1.0 / rho;
+  s.ir = recip_(rho);
   s.p = kGm1 * (e - (j1 * j1 + j2 * j2) * s.ir * 0.5);
   s.cs = sqrt_(kGamma * s.p * s.ir);
   return s;
@@ -60,7 +60,7 @@ __device__ __forceinline__ St<T> derive(const T& rho, const T& j1, const T& j2, 
 // The JST pressure sensor |pa - 2 pb + pc| / (pa + 2 pb + pc) (f90:208-211).
 template <class A, class B, class C>
 __device__ __forceinline__ auto sensor(const A& pa, const B& pb, const C& pc) {
-  return abs_c(pa - 2.0 * pb + pc) / (pa + 2.0 * pb + pc);
+  return quot_(abs_c(pa - 2.0 * pb + pc), pa + 2.0 * pb + pc);
 }
 
 // max_c(0, c) (f90:111-120 with x = 0): 0 only if 0 > Re c + 1e-8.
@@ -77,8 +77,8 @@ __device__ __forceinline__ St<promote_t<TS, TG>> wall_ghost_st(const St<TS>& s, 
   using R = promote_t<TS, TG>;
   const R proj = nx * (s.j1 - gx * s.rho) + nz * (s.j2 - gz * s.rho);
   const TG nn = nx * nx + nz * nz;
-  return derive<R>(lift<R>(s.rho), s.j1 - 2.0 * nx * proj / nn, s.j2 - 2.0 * nz * proj / nn,
-                   lift<R>(s.e));
+  return derive<R>(lift<R>(s.rho), s.j1 - quot_(2.0 * nx * proj, nn),
+                   s.j2 - quot_(2.0 * nz * proj, nn), lift<R>(s.e));
 }
 
 // Far-field ghost (make_farfield_ghost_state, f90:269-274): 2 U_inf - U.

@@ -25,7 +25,7 @@ __device__ __forceinline__ double sgn_c(double x) { return x < 0.0 ? -1.0 : 1.0;
 // adjoints of p, ir and cs of state s into b's conserved components (and clears them).
 __device__ __forceinline__ void derive_rev(const Sd& s, Sd& b) {
   if (b.cs != 0.0) {
-    const double t = b.cs * kGamma / (2.0 * s.cs);
+    const double t = quot_(b.cs * kGamma, 2.0 * s.cs);
     b.p += t * s.ir;
     b.ir += t * s.p;
   }
@@ -41,7 +41,8 @@ __device__ __forceinline__ void derive_rev(const Sd& s, Sd& b) {
 __device__ __forceinline__ void sensor_rev(double pa, double pb, double pc, double sb,
                                            double& pab, double& pbb, double& pcb) {
   const double n = pa - 2.0 * pb + pc, d = pa + 2.0 * pb + pc;
-  const double nb = sb * sgn_c(n) / d, db = -sb * fabs(n) / (d * d);
+  const double s = quot_(sb, d);
+  const double nb = s * sgn_c(n), db = -quot_(s * fabs(n), d);
   pab += nb + db;
   pbb += 2.0 * (db - nb);
   pcb += nb + db;
@@ -192,7 +193,7 @@ __device__ __forceinline__ void wall_ghost_rev(const Sd& s, double nx, double nz
   derive_rev(g, gb);
   const double proj = nx * (s.j1 - gx * s.rho) + nz * (s.j2 - gz * s.rho);
   const double nn = nx * nx + nz * nz;
-  const double a = 2.0 * proj / nn;  // g.j1 = s.j1 - nx a, g.j2 = s.j2 - nz a
+  const double a = quot_(2.0 * proj, nn);  // g.j1 = s.j1 - nx a, g.j2 = s.j2 - nz a
   sb.rho += gb.rho;
   sb.j1 += gb.j1;
   sb.j2 += gb.j2;
@@ -200,7 +201,7 @@ __device__ __forceinline__ void wall_ghost_rev(const Sd& s, double nx, double nz
   const double ab = -(gb.j1 * nx + gb.j2 * nz);
   nxb -= gb.j1 * a;
   nzb -= gb.j2 * a;
-  const double projb = 2.0 * ab / nn, nnb = -a * ab / nn;
+  const double projb = quot_(2.0 * ab, nn), nnb = -quot_(a * ab, nn);
   nxb += 2.0 * nx * nnb + projb * (s.j1 - gx * s.rho);
   nzb += 2.0 * nz * nnb + projb * (s.j2 - gz * s.rho);
   sb.j1 += projb * nx;
