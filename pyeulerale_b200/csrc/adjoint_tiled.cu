@@ -15,9 +15,10 @@
 // halo, then evaluates in reverse every face whose stencil reaches an owned state or whose
 // geometry or cells touch an owned vertex: angular faces of rows [-1, kTM) x columns
 // [-1, kTN + 2), radial faces of rows [-1, kTM + 2) x columns [-1, kTN]. A face's adjoints for
-// its four stencil states are added to the owned ones stencil position by stencil position,
-// with a barrier between positions (within one position and direction no two faces reach the
-// same state); its normal / grid-velocity adjoints and w . F for its two cells go to per-face
+// its four stencil states go to one plane per stencil position and direction (within one no two
+// faces reach the same state), which the owned states sum at the end (adding them to one plane
+// took a barrier per position, 24 per tile: about 520 us on 64 instances of 128 x 128, 366 with the
+// planes); its normal / grid-velocity adjoints and w . F for its two cells go to per-face
 // and per-cell slots, from which every owned vertex gathers its faces and cells in a fixed
 // order. The angular index is periodic for the states; vertex column N is a variable of its own
 // (cell N-1's forward corners) distinct from column 0 (cell 0's backward corners), so geometry
@@ -35,7 +36,7 @@
 namespace eb {
 namespace adj {
 
-constexpr int kTM = 32, kTN = 8, kThreads = 256;
+constexpr int kTM = 32, kTN = 8;
 constexpr int kSR = kTM + 6, kSC = kTN + 6;        // staged states: rows, columns [-3, k + 3)
 constexpr int kStaged = kSR * kSC;
 constexpr int kVR = kTM + 5, kVC = kTN + 5;        // staged vertices: [-2, k + 3)
@@ -59,7 +60,7 @@ struct Smem {
   double gr[4][kNR];          // radial faces
   double gw[4][kRC];          // the wall-ghost use of the wall face (radial faces of row 1)
   double ac[kECells];         // area adjoint x sign(cross) / 2 of the cell
-  double gu[4][kTN][kTM];     // owned states' adjoints
+  double gu[8][4][kTN][kTM];  // owned states' adjoints, one plane per direction and stencil position
 };
 
 __device__ __forceinline__ int sidx(int r, int c) { return (c + 3) * kSR + (r + 3); }
@@ -286,10 +287,11 @@ __device__ __forceinline__ void clear(FaceAdj& A) {
   A.wl = A.wr = 0.0;
 }
 
-// MinBlocks = 2: capped at 128 registers (with spills) so that two CTAs share an SM;
-// MinBlocks = 1: no cap, one CTA per SM. The same code, so the two give identical results.
-template <int MinBlocks>
-__global__ void __launch_bounds__(kThreads, MinBlocks)
+// One CTA per SM (its planes take the shared memory). 384 threads: the 713 faces of a full tile
+// in two rounds at 168 registers; 256 threads: three rounds, uncapped. The same code, so the two
+// give identical results.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
     k_residual_adjoint(Table t, const double* X, const double* V, const double* U,
                        const double* W, int cstride, double* gU, double* gX, double* gV) {
   extern __shared__ __align__(16) unsigned char adj_smem[];
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
     S.vx[e] = vv.x;
     S.vz[e] = vv.y;
   }
-  for (int e = tid; e < 4 * kTM * kTN; e += kThreads) (&S.gu[0][0][0])[e] = 0.0;
+  for (int e = tid; e < 32 * kTM * kTN; e += kThreads) (&S.gu[0][0][0][0])[e] = 0.0;
   for (int e = tid; e < 4 * kNA; e += kThreads) (&S.ga[0][0])[e] = 0.0;
   for (int e = tid; e < 4 * kNR; e += kThreads) (&S.gr[0][0])[e] = 0.0;
   for (int e = tid; e < 4 * kRC; e += kThreads) (&S.gw[0][0])[e] = 0.0;
@@ -373,8 +375,8 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
 
   // 3. faces in reverse, one face per thread and round. The face lists span the tile's part
   // inside the grid (tm x tn cells): angular faces of rows [-1, tm) x columns [-1, tn + 2),
-  // radial faces of rows [-1, tm + 2) x columns [-1, tn], the full lists (kNA + kNR faces, three
-  // rounds) for a full tile. The faces a partial tile leaves out reach no owned state, vertex or
+  // radial faces of rows [-1, tm + 2) x columns [-1, tn], the full lists (kNA + kNR faces) for a
+  // full tile. The faces a partial tile leaves out reach no owned state, vertex or
   // cell; their slots keep the zeros of phase 1.
   const int tm = min(kTM, M - m0), tn = min(kTN, N - n0);
   const int a_rows = tm + 1, r_rows = tm + 3;
@@ -450,20 +452,16 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
       if (fr >= -1 && fr < kTM && fc >= -1 && fc < kTN) S.wF[2][eidx(fr, fc)] = A.wl;
       if (fr - 1 >= -1 && fr - 1 < kTM && fc >= -1 && fc < kTN) S.wF[3][eidx(fr - 1, fc)] = A.wr;
     }
-    // state adjoints, one stencil position and direction at a time
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
+    // state adjoints: a cell is at one stencil position of one face per direction only, so each
+    // position has a plane of its own and no two faces write the same entry
+    if (have)
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        __syncthreads();
-        if (have && (dir == 0 ? angular : radial)) {
-          const int sr = dir == 0 ? fr : fr + 1 - k, sc = dir == 0 ? fc + 1 - k : fc;
-          if (sr >= 0 && sr < kTM && sc >= 0 && sc < kTN)
+        const int sr = angular ? fr : fr + 1 - k, sc = angular ? fc + 1 - k : fc;
+        if (sr >= 0 && sr < kTM && sc >= 0 && sc < kTN)
 #pragma unroll
-            for (int v = 0; v < 4; ++v) S.gu[v][sc][sr] += A.u[k][v];
-        }
+          for (int v = 0; v < 4; ++v) S.gu[(angular ? 0 : 4) + k][v][sc][sr] = A.u[k][v];
       }
-    }
   }
   __syncthreads();
 
@@ -496,7 +494,12 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
     if (m < M && n < N) {
       double* o = gU + 4 * cstride * (cell_base + m + (int64_t)M * n);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) o[cstride * v + h] = S.gu[v][c][r];
+      for (int v = 0; v < 4; ++v) {
+        double sum = S.gu[0][v][c][r];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) sum += S.gu[k][v][c][r];
+        o[cstride * v + h] = sum;
+      }
     }
   }
   // 6. owned vertices: rows [0, kTM) of the tile (and row M), columns [0, kTN) (and column N)
@@ -689,15 +692,16 @@ extern "C" int eb_apply_odes_adjoint(const eb_batch* b, const double* X, const d
   cudaStream_t st = EB_STREAM(stream);
   if (d_states || d_vertices || d_velocities) {
     auto launch = [&](int v) {
-      auto kernel = v == 0 ? adj::k_residual_adjoint<2> : adj::k_residual_adjoint<1>;
+      const int threads = v == 0 ? 384 : 256;
+      auto kernel = v == 0 ? adj::k_residual_adjoint<384> : adj::k_residual_adjoint<256>;
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(adj::Smem)) != cudaSuccess)
         return check_launch("apply_odes_adjoint attribute");
-      kernel<<<dim3(cs * adj::tiles(dim, dim), b->n_inst), adj::kThreads, sizeof(adj::Smem),
-               st>>>(t, X, V, U, w, cs, d_states, d_vertices, d_velocities);
+      kernel<<<dim3(cs * adj::tiles(dim, dim), b->n_inst), threads, sizeof(adj::Smem), st>>>(
+          t, X, V, U, w, cs, d_states, d_vertices, d_velocities);
       return check_launch("apply_odes_adjoint");
     };
-    static const char* const kNames[2] = {"2 CTAs/SM (128 registers)", "1 CTA/SM"};
+    static const char* const kNames[2] = {"1 CTA/SM of 384 threads", "1 CTA/SM of 256 threads"};
     if (int rc = tune::launch_tuned(is_complex ? "residual_adjoint complex" : "residual_adjoint",
                                     b->n_cells, dim, 2, 0, kNames, st, launch))
       return rc;
