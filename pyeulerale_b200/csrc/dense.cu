@@ -44,6 +44,8 @@ struct Operands {
   char* c;
   int64_t sa, sb, sc;  // bytes
   Products set;        // set.n == 0: strided
+  int gap0 = 0, gap1 = 0;  // columns of C left out (whole tiles)
+  __device__ __forceinline__ int column(int n0) const { return n0 < gap0 ? n0 : n0 + gap1 - gap0; }
   template <class T>
   __device__ __forceinline__ void of(int64_t z, const T*& A, const T*& B, T*& C) const {
     int64_t oa = sa * z, ob = sb * z, oc = sc * z;
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(kGemmThreads)
   const double2 *A, *B;
   double2* C;
   ops.of(blockIdx.z, A, B, C);
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
+  const int m0 = blockIdx.x * kBM, n0 = ops.column(blockIdx.y * kBN);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // the warp's 32 x 32 sub-tile
   const int fr = lane >> 2, fc = lane & 3;                 // fragment row / column indices
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(kGemmThreads)
   double2* C;
   ops.of(blockIdx.z, A, B, C);
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+  const int m0 = blockIdx.x * kBM, n0 = ops.column(blockIdx.y * BN);
   const int lane = tid & 31, warp = tid >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
   const int fr = lane >> 2, fc = lane & 3;
@@ -358,7 +360,7 @@ __global__ void __launch_bounds__(kGemmThreads)
   double* C;
   ops.of(blockIdx.z, A, B, C);
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+  const int m0 = blockIdx.x * kBM, n0 = ops.column(blockIdx.y * BN);
   const int lane = tid & 31, warp = tid >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
   const int fr = lane >> 2, fc = lane & 3;
@@ -441,7 +443,7 @@ int launch_zgemm(int M, int N, int K, double alpha, double beta, const Operands&
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return check_launch("zgemm attribute");
-  const dim3 grid((M + kBM - 1) / kBM, (N + bn - 1) / bn, batch);
+  const dim3 grid((M + kBM - 1) / kBM, (N - (ops.gap1 - ops.gap0) + bn - 1) / bn, batch);
   kernel<<<grid, kGemmThreads, smem, st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
   return check_launch("zgemm");
 }
@@ -459,8 +461,12 @@ int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A
 }
 
 int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
-              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st) {
-  const Operands ops{base, base, base, stride, stride, stride, set};
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st,
+              int gap0, int gap1) {
+  if (gap0 % kBN != 0 || gap1 % kBN != 0 || gap1 < gap0 || gap1 > N)
+    return fail(EB_ERR_ARG, "zgemm: bad gap");
+  if (gap1 - gap0 == N) return 0;
+  const Operands ops{base, base, base, stride, stride, stride, set, gap0, gap1};
   return launch_zgemm(M, N, K, alpha, beta, ops, lda, ldb, ldc, workspaces * set.n, -1, st);
 }
 

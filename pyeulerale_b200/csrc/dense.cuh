@@ -34,9 +34,11 @@ struct Products {
     c[n++] = pc;
   }
 };
-// C = alpha A B + beta C for every entry of every workspace (complex).
+// C = alpha A B + beta C for every entry of every workspace (complex); the columns [gap0, gap1) of
+// C, multiples of 64, are left out.
 int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
-              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st);
+              int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st,
+              int gap0 = 0, int gap1 = 0);
 
 // The same with real matrices; the dimensions and leading dimensions are multiples of 4.
 int dgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,

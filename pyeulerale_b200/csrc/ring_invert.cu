@@ -18,6 +18,7 @@
 // resident); each gives up after kPollLimit polls, records it in info and ends the launch's
 // work on that system.
 
+#include "gj_step.cuh"
 #include "ring_invert.cuh"
 
 #include <cuComplex.h>
@@ -35,58 +36,8 @@ int check_launch(const char* what);
 namespace rl {
 namespace {
 
-constexpr int kMaxRows = 1024;
-constexpr int kMaxWarps = 16;
 constexpr int kPollLimit = 1 << 22;  // about three seconds
 
-__device__ __forceinline__ double mul(double a, double b) { return a * b; }
-__device__ __forceinline__ cuDoubleComplex mul(cuDoubleComplex a, cuDoubleComplex b) {
-  return make_cuDoubleComplex(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double neg(double a) { return -a; }
-__device__ __forceinline__ cuDoubleComplex neg(cuDoubleComplex a) {
-  return make_cuDoubleComplex(-a.x, -a.y);
-}
-// c + a b
-__device__ __forceinline__ double fmadd(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ cuDoubleComplex fmadd(cuDoubleComplex a, cuDoubleComplex b,
-                                                 cuDoubleComplex c) {
-  return make_cuDoubleComplex(fma(a.x, b.x, fma(-a.y, b.y, c.x)),
-                              fma(a.x, b.y, fma(a.y, b.x, c.y)));
-}
-// c - a b
-__device__ __forceinline__ double fmsub(double a, double b, double c) { return fma(-a, b, c); }
-__device__ __forceinline__ cuDoubleComplex fmsub(cuDoubleComplex a, cuDoubleComplex b,
-                                                 cuDoubleComplex c) {
-  return make_cuDoubleComplex(fma(-a.x, b.x, fma(a.y, b.y, c.x)),
-                              fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
-}
-// 1 / a of a normal number: the hardware's approximation (error e below 2^-19) and one step of
-// the third-order Newton iteration y (1 + e + e^2), without the branches of a division, so that
-// it runs in the shadow of the pivot search.
-__device__ __forceinline__ double recip(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
-  const double e = fma(-a, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ cuDoubleComplex recip(cuDoubleComplex a) {
-  const double d = recip(a.x * a.x + a.y * a.y);
-  return make_cuDoubleComplex(a.x * d, -a.y * d);
-}
-// a non-negative number ordered like the modulus
-__device__ __forceinline__ double size_of(double a) { return fabs(a); }
-__device__ __forceinline__ double size_of(cuDoubleComplex a) { return a.x * a.x + a.y * a.y; }
-template <class T>
-__device__ __forceinline__ T zero_of();
-template <>
-__device__ __forceinline__ double zero_of<double>() {
-  return 0.0;
-}
-template <>
-__device__ __forceinline__ cuDoubleComplex zero_of<cuDoubleComplex>() {
-  return make_cuDoubleComplex(0.0, 0.0);
-}
 // Loads past L1: the panels are written by other SMs during the launch.
 __device__ __forceinline__ double load_l2(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ cuDoubleComplex load_l2(const cuDoubleComplex* p) {
@@ -103,14 +54,6 @@ __device__ __forceinline__ void store_release(unsigned long long* p, unsigned lo
   asm volatile("fence.acq_rel.gpu;\n st.release.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v)
                : "memory");
 }
-// Barrier `id` of `n` threads (a multiple of 32): wait, or arrive without waiting.
-__device__ __forceinline__ void bar_sync(int id, int n) {
-  asm volatile("barrier.cta.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(int id, int n) {
-  asm volatile("barrier.cta.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
-}
-
 constexpr int kSub = 4;  // steps published together
 // The word published for a group of kSub steps: the launch's epoch, whether the steps found
 // their pivots, and the pivot rows (ten bits each).
@@ -128,14 +71,11 @@ __device__ __forceinline__ int row_of(unsigned long long w, int k) {
   return (int)((w >> (10 * (kSub - 1 - k))) & 0x3FFull);
 }
 
-template <class T, int NC>
+template <class T, int NC, int Warps>
 struct Shared {
-  T cand[2][kMaxWarps][NC];      // each warp's best row of a step
-  T cand_inv[2][kMaxWarps];      // the reciprocal of its pivot entry
-  unsigned cand_key[2][kMaxWarps];
+  StepShared<T, NC, Warps> step;
   T rows[kSub][NC];              // the pivot rows of a group of steps in this CTA's columns
   unsigned long long word;       // the group's published word (0: the wait gave up)
-  int own[NC];                   // this CTA's own pivot rows
   int ok;                        // its own steps found their pivots so far
   int stop;
 };
@@ -151,11 +91,12 @@ __global__ void __launch_bounds__(Threads + 32, 1)
     k_ring_invert(int K, int z0, char* base, int64_t stride, InvertAt at, int epoch) {
   constexpr bool kReal = sizeof(T) == sizeof(double);
   constexpr int nt = Threads, kWarps = Threads / 32;  // compute threads and warps
-  constexpr int kStepBar = 1, kGroupBar = 2;  // kGroupBar + q: group q of this CTA's steps
+  constexpr int kGroupBar = 2;  // kGroupBar + q: group q of this CTA's steps
   constexpr int kGroups = NC / kSub;
   extern __shared__ __align__(16) unsigned char ri_smem[];
-  Shared<T, NC>& S = *reinterpret_cast<Shared<T, NC>*>(ri_smem);
-  T* stage = reinterpret_cast<T*>(ri_smem + sizeof(Shared<T, NC>));  // NC columns of K
+  using Sh = Shared<T, NC, Threads / 32>;
+  Sh& S = *reinterpret_cast<Sh*>(ri_smem);
+  T* stage = reinterpret_cast<T*>(ri_smem + sizeof(Sh));  // NC columns of K
   char* ws = base + stride * (z0 + blockIdx.y);
   auto place = [&](size_t off) { return ws + off; };
   const T* in = reinterpret_cast<const T*>(place(at.in));
@@ -180,7 +121,7 @@ __global__ void __launch_bounds__(Threads + 32, 1)
 #pragma unroll 8
       for (int i = lane; i < words; i += 32) __stcg(to + i, from[i]);
       __syncwarp();
-      if (lane == 0) store_release(flags + c0 / kSub + q, pack(epoch, S.ok != 0, S.own + kSub * q));
+      if (lane == 0) store_release(flags + c0 / kSub + q, pack(epoch, S.ok != 0, S.step.own + kSub * q));
       if (S.ok == 0) return;
     }
     bar_arrive(kGroupBar + kGroups, nt + 32);
@@ -198,106 +139,29 @@ __global__ void __launch_bounds__(Threads + 32, 1)
     for (int k = 0; k < NC; ++k)
       a[r][k] = i < K && k < width ? in[(size_t)K * (c0 + k) + i] : zero_of<T>();
   }
-  // this thread's best remaining entry of column a[.][0]: its key (ordered like the modulus to
-  // one part in 2^10, the row in the low ten bits; 0: none) and its reciprocal
-  unsigned mine = 0u;
-  T inv_mine = zero_of<T>();
-  auto candidate = [&]() {
-    T pivot = a[0][0];
-    mine = 0u;
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const unsigned key = left[r] ? ((unsigned)__double2hiint(size_of(a[r][0])) & ~0x3FFu) |
-                                         (unsigned)(kMaxRows - 1 - (tid + r * nt))
-                                   : 0u;
-      if (r == 0 || key > mine) {
-        mine = key;
-        pivot = a[r][0];
-      }
-    }
-    inv_mine = recip(pivot);
-  };
   for (int p = 0; p < panels; ++p) {
     if (p == j) {
-      // A rolled loop: each CTA runs it once, so unrolled steps would all be fetched cold (the
-      // unrolled form took 950 cycles per step). The columns rotate by one per step instead: the
-      // step's column is a[.][0], its result goes to the last place.
-      candidate();
-      bool ok = true;
-#pragma unroll 1
-      for (int jj = 0; jj < width; ++jj) {
-        const int par = jj & 1;
-        const unsigned best = __reduce_max_sync(0xffffffffu, mine);
-        if (mine == best) {  // this thread's row is the warp's best: stage it
-          // (best = 0, no row left: every lane stages, and the step fails if all warps say so)
-          const int brow = kMaxRows - 1 - (int)(best & 0x3FFu);
+      const bool ok = eliminate(
+          S.step, a, left, pos, width, c0, K, tid,
+          [&](int jj) {  // hand the finished group's columns to the other CTAs
 #pragma unroll
-          for (int r = 0; r < ROWS; ++r)
-            if (brow == tid + r * nt) {
+            for (int r = 0; r < ROWS; ++r) {
+              const int i = tid + r * nt;
+              if (i < K) {
 #pragma unroll
-              for (int k = 0; k < NC; ++k) S.cand[par][warp][k] = a[r][k];
+                for (int k = 0; k < kSub; ++k)
+                  stage[K * (jj - (kSub - 1) + k) + i] = a[r][NC - kSub + k];
+              }
             }
-          S.cand_inv[par][warp] = inv_mine;
-          S.cand_key[par][warp] = best;
-        }
-        bar_sync(kStepBar, nt);
-        unsigned kb = 0u;
-#pragma unroll
-        for (int q = 0; q < kWarps; ++q) kb = max(kb, S.cand_key[par][q]);
-        const int prow = kMaxRows - 1 - (int)(kb & 0x3FFu);
-        const unsigned size = kb & ~0x3FFu;
-        ok = size != 0u && size < 0x7FF00000u && prow < K;
-        if (!ok) {  // the same in every compute thread
-          if (tid == 0) {
-            S.ok = 0;
-            atomicExch(info, 1);
-          }
-          bar_arrive(kGroupBar + jj / kSub, nt + 32);
-          break;
-        }
-        const int w = (prow % nt) >> 5;  // the warp that holds row prow
-        const T inv = S.cand_inv[par][w];
-        const T* row = S.cand[par][w];
-        if (tid == 0) S.own[jj] = prow;
-        T f[ROWS];
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) f[r] = mul(a[r][0], inv);
-        if (warp == w) {
-#pragma unroll
-          for (int r = 0; r < ROWS; ++r)
-            if (tid + r * nt == prow) {  // the pivot row becomes inv times itself
-              left[r] = false;
-              pos[r] = c0 + jj;
-              f[r] = neg(inv);
-#pragma unroll
-              for (int k = 1; k < NC; ++k) a[r][k] = zero_of<T>();
+            bar_arrive(kGroupBar + jj / kSub, nt + 32);
+          },
+          [&](int jj) {
+            if (tid == 0) {
+              S.ok = 0;
+              atomicExch(info, 1);
             }
-        }
-        // the next step's column first: its search runs under the other columns' updates
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) a[r][0] = fmsub(f[r], row[1], a[r][1]);
-        candidate();
-#pragma unroll
-        for (int k = 2; k < NC; ++k) {
-          const T b = row[k];
-#pragma unroll
-          for (int r = 0; r < ROWS; ++r) a[r][k - 1] = fmsub(f[r], b, a[r][k]);
-        }
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) a[r][NC - 1] = neg(f[r]);
-        if (jj % kSub == kSub - 1) {  // hand the group's columns to the other CTAs
-#pragma unroll
-          for (int r = 0; r < ROWS; ++r) {
-            const int i = tid + r * nt;
-            if (i < K) {
-#pragma unroll
-              for (int k = 0; k < kSub; ++k)
-                stage[K * (jj - (kSub - 1) + k) + i] = a[r][NC - kSub + k];
-            }
-          }
-          bar_arrive(kGroupBar + jj / kSub, nt + 32);
-        }
-      }
+            bar_arrive(kGroupBar + jj / kSub, nt + 32);
+          });
       if (!ok) return;
       continue;
     }
@@ -370,7 +234,7 @@ __global__ void __launch_bounds__(Threads + 32, 1)
   bar_sync(kStepBar, nt);
   cuDoubleComplex* out = reinterpret_cast<cuDoubleComplex*>(place(at.out));
   for (int k = 0; k < width; ++k) {
-    const size_t col = (size_t)K * S.own[k];
+    const size_t col = (size_t)K * S.step.own[k];
     for (int i = tid; i < K; i += nt) {
       const T v = stage[(size_t)K * k + i];
       if constexpr (kReal) {
@@ -388,7 +252,7 @@ int launch(int K, int systems, char* base, int64_t stride, const InvertAt& at, i
            cudaStream_t st) {
   auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
   constexpr int threads = Threads + 32;
-  const int smem = (int)(sizeof(Shared<T, NC>) + sizeof(T) * NC * (size_t)K);
+  const int smem = (int)(sizeof(Shared<T, NC, Threads / 32>) + sizeof(T) * NC * (size_t)K);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return check_launch("ring_invert attribute");

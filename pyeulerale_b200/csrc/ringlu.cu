@@ -54,6 +54,7 @@
 
 #include "../../include/euler_b200.h"
 #include "dense.cuh"
+#include "gj_step.cuh"
 #include "physics.cuh"
 #include "ring_invert.cuh"
 
@@ -106,7 +107,7 @@ inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 // Rings of at most 1024 unknowns are supported.
 inline bool ring_supported(int K) { return K <= 1024; }
 
-// Blocked inversion: panels of 16 columns (8 where a panel thread holds two rows), column
+// Blocked inversion: panels of 16 columns (8 where a panel thread holds four rows), column
 // blocks whose trailing update is one ZGEMM.
 inline int panel_width(int K) { return K <= 512 ? 16 : 8; }
 constexpr int kGjBlock = 64;
@@ -231,20 +232,6 @@ __global__ void k_assemble(int M, int N, const double* J, const double* shift,
   }
 }
 
-__device__ __forceinline__ cuDoubleComplex cmul(cuDoubleComplex a, cuDoubleComplex b) {
-  return make_cuDoubleComplex(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-// acc + a b
-__device__ __forceinline__ cuDoubleComplex cfma(cuDoubleComplex a, cuDoubleComplex b,
-                                                cuDoubleComplex acc) {
-  return make_cuDoubleComplex(fma(a.x, b.x, fma(-a.y, b.y, acc.x)), fma(a.x, b.y, fma(a.y, b.x, acc.y)));
-}
-// acc - a b
-__device__ __forceinline__ cuDoubleComplex cfms(cuDoubleComplex a, cuDoubleComplex b,
-                                                cuDoubleComplex acc) {
-  return make_cuDoubleComplex(fma(-a.x, b.x, fma(a.y, b.y, acc.x)), fma(-a.x, b.y, fma(-a.y, b.x, acc.y)));
-}
-
 // The workspaces of a launch, one per shift.
 struct Systems {
   char* base;
@@ -257,45 +244,24 @@ __device__ __forceinline__ T* at(const Systems& g, size_t off) {
 }
 
 // Gauss-Jordan panel: elimination steps j0 .. j0+NB-1 on the panel columns of the K x K block
-// `in`, result written to the same columns of `out` (grid: 1 x shifts, 512 threads). Thread t keeps rows t + 512 r (r < ROWS) of the panel
-// in registers. A step: every warp finds its best row among the rows not chosen yet (largest
-// modulus, ties to the smaller row) and stages it in shared memory; after one barrier every
-// warp reduces the warp candidates itself, so all threads know the pivot row p and its values,
-// and eliminate the pivot column from their rows (row p: scaled by the pivot's inverse), which
-// also yields their candidates for the next step. The staging buffers alternate between steps,
-// so one barrier per step suffices. Records the pivot row of each step in perm and flags a zero
-// or non-finite pivot in info[0].
-// Maximum of a 64-bit key over the warp as two 32-bit warp reductions: the high words, then
-// the low words of the lanes that hold the maximal high word (the exact 64-bit maximum).
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long key) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned H = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned L = __reduce_max_sync(0xffffffffu, hi == H ? lo : 0u);
-  return ((unsigned long long)H << 32) | L;
-}
-
-constexpr int kPanelThreads = 512;
-constexpr int kMaxK = 1024;
+// `in`, result written to the same columns of `out` (grid: 1 x shifts). Thread t keeps rows
+// t + kPanelThreads r (r < ROWS) of the panel in registers; the steps are those of gj_step.cuh.
+// Records the pivot row of each step in perm and flags a zero or non-finite pivot in info[0].
+// (One row per thread on 512 threads, with 64-bit keys, a division per step and the row updated
+// before the next search, took 24.7 us per panel of 16 columns at K = 512; this form 19.6 us.)
+constexpr int kPanelThreads = 256;
 template <int NB, int ROWS>
 __global__ void __launch_bounds__(kPanelThreads, 1)
-    k_gj_panel(int K, int j0, Systems sys, size_t off_in, size_t off_out, size_t off_perm, size_t off_info) {
-  constexpr int kWarps = kPanelThreads / 32;
-  __shared__ cuDoubleComplex cand[2][kWarps][NB];
-  __shared__ cuDoubleComplex cand_inv[2][kWarps];  // 1 / (the candidate's pivot value)
-  __shared__ unsigned long long cand_key[2][kWarps];
-  __shared__ unsigned char chosen[kMaxK];
+    k_gj_panel(int K, int j0, Systems sys, size_t off_in, size_t off_out, size_t off_perm,
+               size_t off_info) {
+  __shared__ StepShared<cuDoubleComplex, NB, kPanelThreads / 32> S;
+  __shared__ unsigned char chosen[kMaxRows];
   const cuDoubleComplex* in = at<cuDoubleComplex>(sys, off_in);
   cuDoubleComplex* out = at<cuDoubleComplex>(sys, off_out);
   int* perm = at<int>(sys, off_perm);
   int* info = at<int>(sys, off_info);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   if (*info != 0) return;  // an earlier panel met a singular pivot
-  for (int i = tid; i < K; i += kPanelThreads) chosen[i] = 0;
-  __syncthreads();
-  for (int j = tid; j < j0; j += kPanelThreads) {
-    const int pj = perm[j];
-    if (pj >= 0 && pj < K) chosen[pj] = 1;
-  }
   cuDoubleComplex a[ROWS][NB];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
@@ -304,100 +270,28 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
     for (int k = 0; k < NB; ++k)
       a[r][k] = i < K ? in[(size_t)K * (j0 + k) + i] : make_cuDoubleComplex(0.0, 0.0);
   }
+  for (int i = tid; i < K; i += kPanelThreads) chosen[i] = 0;
   __syncthreads();
-  double best = -1.0;
-  int bi = kMaxK;
+  for (int j = tid; j < j0; j += kPanelThreads) {
+    const int pj = perm[j];
+    if (pj >= 0 && pj < K) chosen[pj] = 1;
+  }
+  __syncthreads();
+  bool left[ROWS];
+  int pos[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     const int i = tid + r * kPanelThreads;
-    if (i < K && !chosen[i]) {
-      const double v = a[r][0].x * a[r][0].x + a[r][0].y * a[r][0].y;
-      if (v > best) {
-        best = v;
-        bi = i;
-      }
-    }
+    left[r] = i < K && !chosen[i];
+    pos[r] = 0;
   }
-#pragma unroll 1
-  for (int jj = 0; jj < NB; ++jj) {
-    const int par = jj & 1;
-    // Arg-max as a max of 64-bit keys: the bits of |a|^2 (>= 0, so ordered like the values)
-    // with the low 10 mantissa bits replaced by 1023 - row, so equal (to 2^-42 relative) moduli
-    // go to the smaller row; 0 is "no candidate".
-    unsigned long long key =
-        bi < kMaxK ? (((unsigned long long)__double_as_longlong(best) & ~0x3FFull) |
-                      (unsigned long long)(kMaxK - 1 - bi))
-                   : 0ull;
-    const unsigned long long mine = key;
-    // the reciprocal of this thread's candidate pivot, formed while the arg-max runs (the
-    // winner stages it with its row, which takes the division off the step's critical path)
-    cuDoubleComplex cinv = make_cuDoubleComplex(0.0, 0.0);
-    if (bi < kMaxK) {
-      cuDoubleComplex c0 = a[0][0];
-#pragma unroll
-      for (int r = 1; r < ROWS; ++r)
-        if (bi == tid + r * kPanelThreads) c0 = a[r][0];
-      const double d = 1.0 / (c0.x * c0.x + c0.y * c0.y);
-      cinv = make_cuDoubleComplex(c0.x * d, -c0.y * d);
-    }
-    key = warp_max_u64(key);
-    if (key != 0ull && mine == key) {  // this thread owns the warp's best row: stage it
-      const int wi = kMaxK - 1 - (int)(key & 0x3FFull);
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r)
-        if (wi == tid + r * kPanelThreads) {
-#pragma unroll
-          for (int k = 0; k < NB; ++k) cand[par][warp][k] = a[r][k];
-        }
-      cand_inv[par][warp] = cinv;
-    }
-    if (lane == 0) cand_key[par][warp] = key;
-    __syncthreads();
-    const unsigned long long kb = warp_max_u64(lane < kWarps ? cand_key[par][lane] : 0ull);
-    const int p = kMaxK - 1 - (int)(kb & 0x3FFull);
-    const int w = (p % kPanelThreads) / 32;  // the warp of the thread that owns row p
-    const double v = __longlong_as_double((long long)(kb & ~0x3FFull));
-    if (!(kb != 0ull && v > 0.0 && v <= 1.7e308 && p < K)) {  // the same decision in every thread
-      if (tid == 0) atomicExch(info, 1);
-      return;
-    }
-    if (tid == 0) {
-      perm[j0 + jj] = p;
-      chosen[p] = 1;
-    }
-    // Each row is kept rotated by jj columns: the pivot column of this step is a[.][0] and the
-    // next one a[.][1]; after the elimination the row rotates by one more column, so after NB
-    // steps it is back in order. The staged pivot row is rotated the same way.
-    const cuDoubleComplex* prow = cand[par][w];
-    const cuDoubleComplex inv = cand_inv[par][w];
-    best = -1.0;
-    bi = kMaxK;
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const int i = tid + r * kPanelThreads;
-      if (i == p) {
-#pragma unroll
-        for (int k = 1; k < NB; ++k) a[r][k] = cmul(a[r][k], inv);
-        a[r][0] = inv;
-      } else {
-        const cuDoubleComplex fi = cmul(a[r][0], inv);
-#pragma unroll
-        for (int k = 1; k < NB; ++k) a[r][k] = cfms(fi, prow[k], a[r][k]);
-        a[r][0] = make_cuDoubleComplex(-fi.x, -fi.y);
-      }
-      if (jj + 1 < NB && i < K && i != p && !chosen[i]) {
-        const double cv = a[r][1].x * a[r][1].x + a[r][1].y * a[r][1].y;
-        if (cv > best) {
-          best = cv;
-          bi = i;
-        }
-      }
-      const cuDoubleComplex first = a[r][0];
-#pragma unroll
-      for (int k = 0; k + 1 < NB; ++k) a[r][k] = a[r][k + 1];
-      a[r][NB - 1] = first;
-    }
+  const bool ok = eliminate(S, a, left, pos, NB, j0, K, tid, [](int) {}, [](int) {});
+  if (!ok) {
+    if (tid == 0) atomicExch(info, 1);
+    return;
   }
+  __syncthreads();
+  if (tid < NB) perm[j0 + tid] = S.own[tid];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     const int i = tid + r * kPanelThreads;
@@ -484,7 +378,7 @@ __global__ void __launch_bounds__(256, 3) k_gj_update(int K, int j0, int c_lo, i
   for (int k = 0; k < NB; ++k) {
     const cuDoubleComplex g = G[k][r];
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) acc[q] = cfma(g, R[k][cb + 4 * q], acc[q]);
+    for (int q = 0; q < kPer; ++q) acc[q] = fmadd(g, R[k][cb + 4 * q], acc[q]);
   }
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
@@ -799,19 +693,20 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
   if (rc != EB_OK) return rc;
   Handle& side = g_handle[side_lane];
   constexpr int64_t kB = sizeof(cuDoubleComplex);
-  auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int b0) {
+  // the block's update of the columns [c_lo, c_hi) without [gap0, gap1)
+  auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int gap0, int gap1, int b0) {
     if (c_hi <= c_lo) return EB_OK;
     dense::Products p;
     p.add(D + kB * K * b0, L.off_Rp + kB * kGjBlock * c_lo, D + kB * K * c_lo);
     return dense::zgemm_set(K, c_hi - c_lo, kGjBlock, 1.0, 1.0, g.base, g.stride, g.S, p, K,
-                            kGjBlock, K, hh);
+                            kGjBlock, K, hh, gap0, gap1);
   };
   bool side_busy = false;
   for (int b0 = 0; b0 < K; b0 += kGjBlock) {
     for (int q = 0; q < kGjBlock / nb; ++q) {
       const size_t in = q & 1 ? L.off_T : D, out = q & 1 ? D : L.off_T;
-      if (nb == 16) gj_pass<16, 1>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
-      else gj_pass<8, 2>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
+      if (nb == 16) gj_pass<16, 2>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
+      else gj_pass<8, 4>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
     }
     if (K == kGjBlock) break;
     if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
@@ -819,12 +714,11 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
     k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, kGjBlock, g.systems(), D, L.off_Rp,
                                                       L.off_perm, L.off_info);
     const int n0 = b0 + kGjBlock, n1 = std::min(K, b0 + 2 * kGjBlock);  // the next block
-    if ((rc = update(st, n0, n1, b0)) != EB_OK) return rc;
+    if ((rc = update(st, n0, n1, 0, 0, b0)) != EB_OK) return rc;
     if (cudaEventRecord(side.start, st) != cudaSuccess ||
         cudaStreamWaitEvent(side.stream, side.start, 0) != cudaSuccess)
       return check_launch("ringlu side fork");
-    if ((rc = update(hs, 0, b0, b0)) != EB_OK) return rc;
-    if ((rc = update(hs, n1, K, b0)) != EB_OK) return rc;
+    if ((rc = update(hs, 0, K, b0, n1, b0)) != EB_OK) return rc;
     if (cudaEventRecord(side.done, side.stream) != cudaSuccess) return check_launch("ringlu side");
     side_busy = true;
   }
