@@ -211,14 +211,13 @@ __global__ void __launch_bounds__(kGemmThreads)
 // ---- cp.async variants --------------------------------------------------------------------
 // pitches in complex elements: A rows [k][m] 2 modulo 8, B rows [n][k] 4 modulo 8, so that the
 // 16-byte fragment loads of each quarter-warp fall on distinct banks
-constexpr int kPitchA = kBM + 2;
 constexpr int kPitchB = kBK + 4;
 
 // BN: tile columns (64: warps of 32 x 32; 32: warps of 32 x 16, half the registers and shared
 // memory, four CTAs per SM, twice the tiles); Stages: slices in flight.
-template <int BN, int Stages>
+template <int BN, int Stages, int BM = kBM>
 struct AsyncSmem {
-  double2 a[Stages][kBK][kPitchA];
+  double2 a[Stages][kBK][BM + 2];
   double2 b[Stages][BN][kPitchB];
 };
 
@@ -237,25 +236,26 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(Pending) : "memory");
 }
 
-template <int BN, int Stages>
+template <int BN, int Stages, int BM = kBM>
 __global__ void __launch_bounds__(kGemmThreads)
     k_zgemm_nn_async(int M, int N, int K, double alpha, Operands ops, int lda, int ldb,
                      double beta, int ldc) {
-  constexpr int NJ = BN / 16;                        // 8-column fragments per warp
+  constexpr int NI = BM / 16, NJ = BN / 16;          // 8-row and 8-column fragments per warp
+  constexpr int kAPerT = BM * kBK / kGemmThreads;   // A elements per thread and slice
   constexpr int kBPerT = kBK * BN / kGemmThreads;   // B elements per thread and slice
   extern __shared__ __align__(16) unsigned char zg_smem[];
-  AsyncSmem<BN, Stages>& S = *reinterpret_cast<AsyncSmem<BN, Stages>*>(zg_smem);
+  AsyncSmem<BN, Stages, BM>& S = *reinterpret_cast<AsyncSmem<BN, Stages, BM>*>(zg_smem);
   const double2 *A, *B;
   double2* C;
   ops.of(blockIdx.z, A, B, C);
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * kBM, n0 = ops.column(blockIdx.y * BN);
+  const int m0 = blockIdx.x * BM, n0 = ops.column(blockIdx.y * BN);
   const int lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
+  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
   const int fr = lane >> 2, fc = lane & 3;
-  double re[4][NJ][2], im[4][NJ][2];
+  double re[NI][NJ][2], im[NI][NJ][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
   const int slices = (K + kBK - 1) / kBK;
@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(kGemmThreads)
     if (s < slices) {
       const int buf = s % Stages, k0 = s * kBK;
 #pragma unroll
-      for (int q = 0; q < kAPer; ++q) {  // A: consecutive threads along m
-        const int e = tid + kGemmThreads * q, m = e % kBM, k = e / kBM;
+      for (int q = 0; q < kAPerT; ++q) {  // A: consecutive threads along m
+        const int e = tid + kGemmThreads * q, m = e % BM, k = e / BM;
         const int gm = m0 + m, gk = k0 + k;
         const bool ok = gm < M && gk < K;
         cp_async16(&S.a[buf][k][m], ok ? A + gm + (int64_t)lda * gk : A, ok);
@@ -289,24 +289,24 @@ __global__ void __launch_bounds__(kGemmThreads)
     const int buf = s % Stages;
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 4) {
-      double2 a[4], b[NJ];
-      double a_n[4];
+      double2 a[NI], b[NJ];
+      double a_n[NI];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < NI; ++i) {
         a[i] = S.a[buf][kk + fc][wm + 8 * i + fr];
         a_n[i] = -a[i].y;
       }
 #pragma unroll
       for (int j = 0; j < NJ; ++j) b[j] = S.b[buf][wn + 8 * j + fr][kk + fc];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
           mma884(re[i][j], a[i].x, b[j].x);
           mma884(im[i][j], a[i].x, b[j].y);
         }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
           mma884(re[i][j], a_n[i], b[j].y);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kGemmThreads)
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
@@ -339,34 +339,43 @@ __global__ void __launch_bounds__(kGemmThreads)
 
 namespace {
 
+// Fewer 64 x 32 tiles than SMs: the products go in 32 x 16 tiles (the same sums in the same order),
+// four times as many CTAs with a quarter of the work per slice (a pair of real 256^3 products:
+// 6.6 us, 11.5 in 64 x 32 tiles).
+inline bool few_tiles(int M, int N, int batch) {
+  return (int64_t)((M + 63) / 64) * ((N + 31) / 32) * batch < 148;
+}
+
 // ---- real matrices ----------------------------------------------------------------------------
 // The cp.async ring on 64 x 32 tiles with real elements: a copy moves two (the dimensions are
 // multiples of 4, so a pair never straddles an edge), pitches 4 modulo 16 doubles keep the
 // fragment loads of each half-warp on distinct banks. K = 512: 128 tiles per product, two
 // products (or shifts) fill the SMs.
 constexpr int kRealBN = 32, kRealStages = 3;
+template <int BM, int BN>
 struct RealSmem {
-  double a[kRealStages][kBK][kPadM];
-  double b[kRealStages][kRealBN][kPadK];
+  double a[kRealStages][kBK][BM + 4];
+  double b[kRealStages][BN][kPadK];
 };
 
+template <int BM, int BN>
 __global__ void __launch_bounds__(kGemmThreads)
     k_dgemm_nn(int M, int N, int K, double alpha, Operands ops, int lda, int ldb, double beta,
                int ldc) {
-  constexpr int BN = kRealBN, Stages = kRealStages, NJ = BN / 16;
+  constexpr int Stages = kRealStages, NI = BM / 16, NJ = BN / 16;
   extern __shared__ __align__(16) unsigned char dg_smem[];
-  RealSmem& S = *reinterpret_cast<RealSmem*>(dg_smem);
+  RealSmem<BM, BN>& S = *reinterpret_cast<RealSmem<BM, BN>*>(dg_smem);
   const double *A, *B;
   double* C;
   ops.of(blockIdx.z, A, B, C);
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * kBM, n0 = ops.column(blockIdx.y * BN);
+  const int m0 = blockIdx.x * BM, n0 = ops.column(blockIdx.y * BN);
   const int lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
+  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
   const int fr = lane >> 2, fc = lane & 3;
-  double acc[4][NJ][2];
+  double acc[NI][NJ][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   const int slices = (K + kBK - 1) / kBK;
@@ -374,8 +383,8 @@ __global__ void __launch_bounds__(kGemmThreads)
     if (s < slices) {
       const int buf = s % Stages, k0 = s * kBK;
 #pragma unroll
-      for (int q = 0; q < kBM * kBK / 2 / kGemmThreads; ++q) {
-        const int e = tid + kGemmThreads * q, m = 2 * (e % (kBM / 2)), k = e / (kBM / 2);
+      for (int q = 0; q < BM * kBK / 2 / kGemmThreads; ++q) {
+        const int e = tid + kGemmThreads * q, m = 2 * (e % (BM / 2)), k = e / (BM / 2);
         const int gm = m0 + m, gk = k0 + k;
         const bool ok = gm < M && gk < K;
         cp_async16(&S.a[buf][k][m], ok ? A + gm + (int64_t)lda * gk : A, ok);
@@ -399,20 +408,20 @@ __global__ void __launch_bounds__(kGemmThreads)
     const int buf = s % Stages;
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 4) {
-      double a[4], b[NJ];
+      double a[NI], b[NJ];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = S.a[buf][kk + fc][wm + 8 * i + fr];
+      for (int i = 0; i < NI; ++i) a[i] = S.a[buf][kk + fc][wm + 8 * i + fr];
 #pragma unroll
       for (int j = 0; j < NJ; ++j) b[j] = S.b[buf][wn + 8 * j + fr][kk + fc];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) mma884(acc[i][j], a[i], b[j]);
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
@@ -433,17 +442,20 @@ int launch_zgemm(int M, int N, int K, double alpha, double beta, const Operands&
     const char* e = std::getenv("EB_ZGEMM");
     variant = (e && e[0] == 'v' && e[1] >= '0' && e[1] <= '2') ? e[1] - '0' : kDefaultVariant;
   }
-  auto kernel = variant == kAsync      ? k_zgemm_nn_async<64, 3>
+  const bool small = variant == kAsyncNarrow && few_tiles(M, N - (ops.gap1 - ops.gap0), batch);
+  auto kernel = variant == kAsync ? k_zgemm_nn_async<64, 3>
+                : small           ? k_zgemm_nn_async<16, 3, 32>
                 : variant == kAsyncNarrow ? k_zgemm_nn_async<32, 2>
                                           : k_zgemm_nn;
-  const int smem = variant == kAsync        ? (int)sizeof(AsyncSmem<64, 3>)
+  const int smem = variant == kAsync ? (int)sizeof(AsyncSmem<64, 3>)
+                   : small           ? (int)sizeof(AsyncSmem<16, 3, 32>)
                    : variant == kAsyncNarrow ? (int)sizeof(AsyncSmem<32, 2>)
                                              : (int)sizeof(GemmSmem);
-  const int bn = variant == kAsyncNarrow ? 32 : kBN;
+  const int bm = small ? 32 : kBM, bn = small ? 16 : variant == kAsyncNarrow ? 32 : kBN;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return check_launch("zgemm attribute");
-  const dim3 grid((M + kBM - 1) / kBM, (N - (ops.gap1 - ops.gap0) + bn - 1) / bn, batch);
+  const dim3 grid((M + bm - 1) / bm, (N - (ops.gap1 - ops.gap0) + bn - 1) / bn, batch);
   kernel<<<grid, kGemmThreads, smem, st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
   return check_launch("zgemm");
 }
@@ -475,12 +487,17 @@ int dgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_
   if (M <= 0 || N <= 0 || workspaces * set.n <= 0) return 0;
   if ((M | N | K | lda | ldb | ldc) % 4 != 0) return fail(EB_ERR_ARG, "dgemm: sizes must be multiples of 4");
   const Operands ops{base, base, base, stride, stride, stride, set};
-  if (cudaFuncSetAttribute(k_dgemm_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(RealSmem)) != cudaSuccess)
-    return check_launch("dgemm attribute");
-  const dim3 grid((M + kBM - 1) / kBM, (N + kRealBN - 1) / kRealBN, workspaces * set.n);
-  k_dgemm_nn<<<grid, kGemmThreads, sizeof(RealSmem), st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
-  return check_launch("dgemm");
+  auto run = [&](auto kernel, int bm, int bn, size_t smem) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return check_launch("dgemm attribute");
+    const dim3 grid((M + bm - 1) / bm, (N + bn - 1) / bn, workspaces * set.n);
+    kernel<<<grid, kGemmThreads, smem, st>>>(M, N, K, alpha, ops, lda, ldb, beta, ldc);
+    return check_launch("dgemm");
+  };
+  if (few_tiles(M, N, workspaces * set.n))
+    return run(k_dgemm_nn<32, 16>, 32, 16, sizeof(RealSmem<32, 16>));
+  return run(k_dgemm_nn<kBM, kRealBN>, kBM, kRealBN, sizeof(RealSmem<kBM, kRealBN>));
 }
 
 namespace {
@@ -498,6 +515,32 @@ __device__ __forceinline__ double2 bd_entry(const double* bd, const double2* v, 
     o.y = fma(w, u[k].y, o.y);
   }
   return o;
+}
+
+// Programmatic dependent launch: a step's kernel starts while the step before it still runs, issues
+// its loads of the factors (which no step writes) and only then waits for that step's results. (The
+// sweeps over several right-hand sides let the next step start first thing: the 64-shift sweep of
+// the 129x129 grid takes 876 ms so, 892 with the next step let in after the wait, 924 without.)
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void wait_previous() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem,
+                             cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <class T>
@@ -535,27 +578,30 @@ __global__ void __launch_bounds__(256) k_sweep_n(int n, char* base, int64_t stri
   const int r = threadIdx.x & 7, g = threadIdx.x >> 3, lane = threadIdx.x & 31;
   const int i = group * 8 + r;
   double sr = 0.0, si = 0.0;
-  if (i < n && t.a >= 0) {
-    const double2* A = place<const double2>(ws, t.a) + i;
-    const double2* x = place<const double2>(ws, t.x);
-    constexpr int kUnroll = 8;  // column loads in flight per thread (ldg_inflight)
-    int j = g;
-    for (; j + 32 * (kUnroll - 1) < n; j += 32 * kUnroll) {
-      double2 a[kUnroll];
+  const bool active = i < n && t.a >= 0;
+  const double2* A = place<const double2>(ws, t.a) + i;
+  const double2* x = place<const double2>(ws, t.x);
+  constexpr int kUnroll = 16;  // column loads in flight per thread (ldg_inflight)
+  bool waited = false;
+  for (int j = g; j < n || !waited; j += 32 * kUnroll) {
+    double2 a[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(A + (int64_t)n * (j + 32 * u));
+    for (int u = 0; u < kUnroll; ++u) {
+      a[u] = make_double2(0.0, 0.0);
+      if (active && j + 32 * u < n) a[u] = ldg_inflight(A + (int64_t)n * (j + 32 * u));
+    }
+    if (!waited) {
+      wait_previous();
+      let_next_start();
+    }
+    waited = true;
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kUnroll; ++u)
+      if (active && j + 32 * u < n) {
         const double2 v = x[j + 32 * u];
         sr = fma(a[u].x, v.x, fma(-a[u].y, v.y, sr));
         si = fma(a[u].x, v.y, fma(a[u].y, v.x, si));
       }
-    }
-    for (; j < n; j += 32) {
-      const double2 a = ldg_inflight(A + (int64_t)n * j), v = x[j];
-      sr = fma(a.x, v.x, fma(-a.y, v.y, sr));
-      si = fma(a.x, v.y, fma(a.y, v.x, si));
-    }
   }
 #pragma unroll
   for (int o = 8; o < 32; o <<= 1) {
@@ -587,6 +633,17 @@ __global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stri
   char* ws = base + stride * blockIdx.y;
   const int lane = threadIdx.x & 31;
   const int j = group * 8 + (threadIdx.x >> 5);
+  // the first rows of the first matrix before the wait (512 rows: all of a column at K = 512)
+  constexpr int kAhead = 16;
+  double2 ahead[kAhead];
+  const double2* first = place<const double2>(ws, t.a) + (int64_t)n * j;
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    ahead[u] = make_double2(0.0, 0.0);
+    if (t.a >= 0 && j < n && lane + 32 * u < n) ahead[u] = ldg_inflight(first + lane + 32 * u);
+  }
+  wait_previous();
+  let_next_start();
   for (int i = threadIdx.x; i < n; i += 256) {
     if (t.a >= 0) xs[i] = place<const double2>(ws, t.x)[i];
     if (t.a2 >= 0)
@@ -595,31 +652,39 @@ __global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stri
   __syncthreads();
   if (j >= n) return;
   double sr = 0.0, si = 0.0;
-  auto dot = [&](const double2* col, const double2* v, double alpha) {
-    double tr = 0.0, ti = 0.0;
+  auto add = [&](const double2 a, const double2 w, double& tr, double& ti) {  // conj(a) w
+    tr = fma(a.x, w.x, fma(a.y, w.y, tr));
+    ti = fma(a.x, w.y, fma(-a.y, w.x, ti));
+  };
+  auto dot = [&](const double2* col, const double2* v, int from, double& tr, double& ti) {
     constexpr int kUnroll = 8;  // row loads in flight per lane (ldg_inflight)
-    int i = lane;
-    for (; i + 32 * (kUnroll - 1) < n; i += 32 * kUnroll) {  // conj(a) v
+    for (int i = from + lane; i < n; i += 32 * kUnroll) {
       double2 a[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) a[u] = ldg_inflight(col + i + 32 * u);
-#pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
-        const double2 w = v[i + 32 * u];
-        tr = fma(a[u].x, w.x, fma(a[u].y, w.y, tr));
-        ti = fma(a[u].x, w.y, fma(-a[u].y, w.x, ti));
+        a[u] = make_double2(0.0, 0.0);
+        if (i + 32 * u < n) a[u] = ldg_inflight(col + i + 32 * u);
       }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (i + 32 * u < n) add(a[u], v[i + 32 * u], tr, ti);
     }
-    for (; i < n; i += 32) {
-      const double2 a = ldg_inflight(col + i), w = v[i];
-      tr = fma(a.x, w.x, fma(a.y, w.y, tr));
-      ti = fma(a.x, w.y, fma(-a.y, w.x, ti));
-    }
-    sr = fma(alpha, tr, sr);
-    si = fma(alpha, ti, si);
   };
-  if (t.a >= 0) dot(place<const double2>(ws, t.a) + (int64_t)n * j, xs, t.alpha);
-  if (t.a2 >= 0) dot(place<const double2>(ws, t.a2) + (int64_t)n * j, xs + n, -1.0);
+  if (t.a >= 0) {
+    double tr = 0.0, ti = 0.0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (lane + 32 * u < n) add(ahead[u], xs[lane + 32 * u], tr, ti);
+    dot(first, xs, 32 * kAhead, tr, ti);
+    sr = fma(t.alpha, tr, sr);
+    si = fma(t.alpha, ti, si);
+  }
+  if (t.a2 >= 0) {
+    double tr = 0.0, ti = 0.0;
+    dot(place<const double2>(ws, t.a2) + (int64_t)n * j, xs + n, 0, tr, ti);
+    sr -= tr;
+    si -= ti;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     sr += __shfl_xor_sync(0xffffffffu, sr, o);
@@ -653,6 +718,7 @@ __global__ void __launch_bounds__(256, 2)
   const int tid = threadIdx.x, r = tid & 7, g = tid >> 3, lane = tid & 31;
   const int i = group * 8 + r;
   const int pitch = min(n, kChunk);
+  let_next_start();
   double sr[NR], si[NR];
 #pragma unroll
   for (int q = 0; q < NR; ++q) sr[q] = si[q] = 0.0;
@@ -666,7 +732,11 @@ __global__ void __launch_bounds__(256, 2)
       a[u] = make_double2(0.0, 0.0);
       if (i < n && g + 32 * u < cols) a[u] = ldg_inflight(A + (int64_t)n * (c0 + g + 32 * u));
     }
-    if (c0 > 0) __syncthreads();  // the previous columns' right-hand sides have been used
+    if (c0 == 0) {
+      wait_previous();
+    } else {
+      __syncthreads();  // the previous columns' right-hand sides have been used
+    }
 #pragma unroll
     for (int q = 0; q < NR; ++q)
       for (int j = tid; j < cols; j += 256) xs[pitch * q + j] = x[c0 + j + (int64_t)n * q];
@@ -724,9 +794,11 @@ int launch_sweep_multi(int n, char* base, int64_t stride, char* vectors, int64_t
   if (cudaFuncSetAttribute(k_sweep_multi<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return check_launch("sweep attribute");
-  k_sweep_multi<NR><<<dim3((n + 7) / 8 * terms.n, workspaces), 256, smem, st>>>(
-      n, base, stride, vectors, vstride, zmap, n_active, terms);
-  return check_launch("sweep product");
+  if (launch_dependent(k_sweep_multi<NR>, dim3((n + 7) / 8 * terms.n, workspaces), 256, smem, st, n,
+                       (const char*)base, stride, vectors, vstride, zmap, n_active, terms) !=
+      cudaSuccess)
+    return check_launch("sweep product");
+  return EB_OK;
 }
 
 }  // namespace
@@ -735,11 +807,11 @@ int sweep_product(int conj_trans, int n, char* base, int64_t stride, int workspa
                   const SweepTerms& terms, cudaStream_t st) {
   if (n <= 0 || workspaces <= 0 || terms.n <= 0) return 0;
   const dim3 grid((n + 7) / 8 * terms.n, workspaces);
-  if (conj_trans)
-    k_sweep_h<<<grid, 256, 2 * sizeof(double2) * (size_t)n, st>>>(n, base, stride, terms);
-  else
-    k_sweep_n<<<grid, 256, 0, st>>>(n, base, stride, terms);
-  return check_launch("sweep product");
+  const cudaError_t e =
+      conj_trans ? launch_dependent(k_sweep_h, grid, 256, 2 * sizeof(double2) * (size_t)n, st, n,
+                                    base, stride, terms)
+                 : launch_dependent(k_sweep_n, grid, 256, 0, st, n, base, stride, terms);
+  return e == cudaSuccess ? EB_OK : check_launch("sweep product");
 }
 
 int sweep_product_multi(int n, int nr, char* base, int64_t stride, char* vectors, int64_t vstride,
