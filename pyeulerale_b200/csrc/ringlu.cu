@@ -110,14 +110,21 @@ inline bool ring_supported(int K) { return K <= 1024; }
 // Blocked inversion: panels of 16 columns (8 where a panel thread holds four rows), column
 // blocks whose trailing update is one ZGEMM.
 inline int panel_width(int K) { return K <= 512 ? 16 : 8; }
-constexpr int kGjBlock = 64;
-// The blocked form needs whole column blocks and enough shifts per stream to fill the GPU with
-// its panels (one SM per shift): with one shift of the 129x129 grid (K = 512) it took 1.25 ms
-// per ring, with 16 per stream 0.175 ms per ring and shift; the cooperative launch takes 0.56 ms
-// per inversion, two shifts at a time (ring_invert.cu).
-constexpr int kGjBlockMinShifts = 8;
-inline bool blocked_inversion(int K, int shifts_per_stream) {
-  return K % kGjBlock == 0 && shifts_per_stream >= kGjBlockMinShifts;
+// Width of the column blocks: 128 where it divides K >= 512 (23 factorisations at K = 512 with the
+// GMRES on them: 847 ms, 876 with blocks of 64, whose trailing updates are half as deep), else 64.
+constexpr int kGjBlock = 64, kGjBlockWide = 128;
+inline int gj_block(int K) {
+  return K >= 512 && K % kGjBlockWide == 0 ? kGjBlockWide : kGjBlock;
+}
+// The blocked form needs whole column blocks, two shifts for its two streams, and enough work to
+// fill the GPU beside its panels (one SM per shift); the cooperative form holds only so many blocks
+// at a time (ring_invert.cu). Measured per ring, cooperative against blocked: K = 128, 24 shifts
+// 212 us against 322; K = 256, 10 shifts 624 against 635, 16 shifts 729 against 717, 24 shifts 1060
+// against 862; K = 512, 2 shifts 791 against 1121, 3 shifts 1455 against 1280, 12 shifts 4471
+// against 2392; K = 1024, 2 shifts 5518 against 4123. The line, shifts K^2 = 3 512^2, lies along
+// the crossings.
+inline bool blocked_inversion(int K, int shifts) {
+  return K % kGjBlock == 0 && shifts >= 2 && (int64_t)shifts * K * K >= 3 * 512 * 512;
 }
 
 // Byte offsets in a workspace.
@@ -155,7 +162,7 @@ Layout plan(int M, int N) {
   L.off_L2 = take(L.blk);
   L.off_Cr = take(L.blk);
   L.off_Br = take(L.blk);
-  L.off_Rp = take(sizeof(cuDoubleComplex) * (size_t)kGjBlock * L.K);
+  L.off_Rp = take(sizeof(cuDoubleComplex) * (size_t)kGjBlockWide * L.K);
   L.off_perm = take(sizeof(int) * (size_t)L.K);
   L.off_info = take(sizeof(int) * 4);
   L.off_flags = take(sizeof(uint64_t) * kInvertFlags);
@@ -674,12 +681,12 @@ void gj_pass(const Group& g, int j0, int c_lo, int c_hi, size_t in, size_t out, 
 
 // D <- D^-1 for every shift by Gauss-Jordan with implicit row pivoting (D: a K x K block's
 // place): for a few shifts one cooperative launch (ring_invert.cu), for many the blocked form,
-// whose columns go in blocks of kGjBlock: the panels of a block update only the block's columns
+// whose columns go in blocks of gj_block(K): the panels of a block update only the block's columns
 // (ping-pong with the scratch block T, an even number of passes, so the block ends in D), and the
-// rest of D takes the block's combined rank-kGjBlock update as ZGEMMs (tensor-core DMMA).
+// rest of D takes the block's combined update of that rank as ZGEMMs (tensor-core DMMA).
 int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
-  const int K = L.K, nb = panel_width(K);
+  const int K = L.K, nb = panel_width(K), BW = gj_block(K);
   if (!g.blocked) {
     const InvertAt where{D, L.off_T, D, L.off_L2 + L.blk / 2, L.off_flags, L.off_info};
     return ring_invert(K, g.S, g.base, g.stride, where, epoch, g.real, st);
@@ -697,23 +704,23 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
   auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int gap0, int gap1, int b0) {
     if (c_hi <= c_lo) return EB_OK;
     dense::Products p;
-    p.add(D + kB * K * b0, L.off_Rp + kB * kGjBlock * c_lo, D + kB * K * c_lo);
-    return dense::zgemm_set(K, c_hi - c_lo, kGjBlock, 1.0, 1.0, g.base, g.stride, g.S, p, K,
-                            kGjBlock, K, hh, gap0, gap1);
+    p.add(D + kB * K * b0, L.off_Rp + kB * BW * c_lo, D + kB * K * c_lo);
+    return dense::zgemm_set(K, c_hi - c_lo, BW, 1.0, 1.0, g.base, g.stride, g.S, p, K,
+                            BW, K, hh, gap0, gap1);
   };
   bool side_busy = false;
-  for (int b0 = 0; b0 < K; b0 += kGjBlock) {
-    for (int q = 0; q < kGjBlock / nb; ++q) {
+  for (int b0 = 0; b0 < K; b0 += BW) {
+    for (int q = 0; q < BW / nb; ++q) {
       const size_t in = q & 1 ? L.off_T : D, out = q & 1 ? D : L.off_T;
-      if (nb == 16) gj_pass<16, 2>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
-      else gj_pass<8, 4>(g, b0 + q * nb, b0, b0 + kGjBlock, in, out, st);
+      if (nb == 16) gj_pass<16, 2>(g, b0 + q * nb, b0, b0 + BW, in, out, st);
+      else gj_pass<8, 4>(g, b0 + q * nb, b0, b0 + BW, in, out, st);
     }
-    if (K == kGjBlock) break;
+    if (K == BW) break;
     if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
       return check_launch("ringlu side join");
-    k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, kGjBlock, g.systems(), D, L.off_Rp,
+    k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, BW, g.systems(), D, L.off_Rp,
                                                       L.off_perm, L.off_info);
-    const int n0 = b0 + kGjBlock, n1 = std::min(K, b0 + 2 * kGjBlock);  // the next block
+    const int n0 = b0 + BW, n1 = std::min(K, b0 + 2 * BW);  // the next block
     if ((rc = update(st, n0, n1, 0, 0, b0)) != EB_OK) return rc;
     if (cudaEventRecord(side.start, st) != cudaSuccess ||
         cudaStreamWaitEvent(side.stream, side.start, 0) != cudaSuccess)
@@ -1058,7 +1065,7 @@ int issue_factor(const Group& g, const double* const* J, cudaStream_t st) {
         reinterpret_cast<double*>(w + L.off_C2));
   }
   if ((rc = check_launch("ringlu assemble")) != EB_OK) return rc;
-  if (g.real || !blocked_inversion(L.K, (n_shifts + 1) / 2)) {
+  if (g.real || !blocked_inversion(L.K, n_shifts)) {
     // one stream: the inversions are cooperative launches, which never run two at a time here
     auto all = [&](auto begin, auto ring) {
       int code = begin(g, st);
