@@ -10,8 +10,10 @@
 // whole 512-byte rows (written by the threads themselves, a store touched 32 lines for 16 bytes
 // each). A block sum keeps the reference's face order, ((F_b + F_f) + F_i) + F_o.
 //
-// Measured on 282,000 cells of uneven grids: states 567 us before (dual numbers, tiles staged in
-// shared memory, at one CTA per SM), vertices 594 us, velocities 263 us, mach 34 us.
+// Measured on 282,000 cells of uneven grids against dual numbers (tiles staged in shared memory, at
+// one CTA per SM): states 567 -> 95 us (3.4 TB/s of 6.5 copied), vertices 594 -> 58 us, velocities
+// 263 -> 35 us, mach 34 -> 7.5 us. What is left is latency: the registers of a face's derivatives
+// leave eight to twelve warps per SM.
 
 #include "autotune.cuh"
 #include "common.cuh"
@@ -20,117 +22,10 @@
 namespace eb {
 namespace {
 
-// A warp's outputs of D doubles per cell, in rows padded by 16 bytes, so that the threads' 16-byte
-// accesses to their own rows fall on distinct banks.
-template <int D>
-struct WarpRows {
-  double2 v[32][D / 2 + 1];
-};
-
-// Thread `lane` hands over `mine`; the warp writes the rows of its first `valid` cells to `out`
-// (the first cell's place).
-template <int D>
-__device__ __forceinline__ void write_rows(WarpRows<D>& S, const double (&mine)[D], int lane,
-                                           int valid, double* out) {
-#pragma unroll
-  for (int e = 0; e < D / 2; ++e) S.v[lane][e] = make_double2(mine[2 * e], mine[2 * e + 1]);
-  __syncwarp();
-  constexpr int kPer = D / 2;
-  double2* o = reinterpret_cast<double2*>(out);
-#pragma unroll
-  for (int e = 0; e < kPer; ++e) {
-    const int f = 32 * e + lane;
-    if (f < valid * kPer) o[f] = S.v[f / kPer][f % kPer];
-  }
-  __syncwarp();
-}
-
-struct CellAt {  // a cell's place in its instance
-  int m, n;
-  int64_t M, N;
-  const double *U, *X, *V;
-
-  __device__ __forceinline__ State state(int dm, int dn) const {
-    int c = n + dn;
-    c = c < 0 ? c + (int)N : c >= (int)N ? c - (int)N : c;
-    const double2* q = reinterpret_cast<const double2*>(U + 4 * (m + dm + M * c));
-    const double2 a = __ldg(q), b = __ldg(q + 1);
-    return make_state(a.x, a.y, b.x, b.y);
-  }
-  // The corners in the order backward-inward, forward-inward, forward-outward, backward-outward.
-  __device__ __forceinline__ double2 corner(const double* A, int k) const {
-    const int64_t v = m + (k >= 2) + (M + 1) * (n + (k == 1 || k == 2));
-    return __ldg(reinterpret_cast<const double2*>(A + 2 * v));
-  }
-};
-
-struct CellGeometry {
-  double2 x[4];
-  FaceGeometry b, f, i, o;  // faces between corners 3-0, 1-2, 0-1 and 2-3 (outward normals)
-  double cross;     // signed area times 2
-
-  __device__ __forceinline__ explicit CellGeometry(const CellAt& at) {
-    double2 w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      x[k] = at.corner(at.X, k);
-      w[k] = at.V ? at.corner(at.V, k) : make_double2(0.0, 0.0);
-    }
-    auto edge = [&](int p, int q) {
-      return FaceGeometry{x[q].y - x[p].y, x[p].x - x[q].x, (w[p].x + w[q].x) / 2.0,
-                  (w[p].y + w[q].y) / 2.0};
-    };
-    i = edge(0, 1);
-    f = edge(1, 2);
-    o = edge(2, 3);
-    b = edge(3, 0);
-    cross = (x[2].x - x[0].x) * (x[3].y - x[1].y) - (x[2].y - x[0].y) * (x[3].x - x[1].x);
-  }
-  __device__ __forceinline__ double inv_area() const { return recip_(abs_c(cross) / 2.0); }
-  __device__ __forceinline__ Wall wall() const { return make_wall(i.nx, i.nz, i.gx, i.gz); }
-};
-
-// The radial line of a cell, boundary rows included (make_ode's five cases, f90:401-436): the
-// inner face has the line (o, c, i, ii), the outer one (i, c, o, oo), with ghost states past the
-// ends and the dissipation off on the faces whose line would reach past a ghost.
-struct RadialLine {
-  State i, o, ii, oo;
-  bool diss_i, diss_o;
-  __device__ __forceinline__ RadialLine(const CellAt& at, const State& c, const CellGeometry& g,
-                                        const Instance& in) {
-    const int m = at.m, M = (int)at.M;
-    diss_i = m >= 2;
-    diss_o = m <= M - 3;
-    i = m > 0 ? at.state(-1, 0) : wall_ghost_of(c, g.wall());
-    o = m < M - 1 ? at.state(1, 0) : farfield_ghost_of(c, in);
-    ii = diss_i ? at.state(-2, 0) : c;
-    oo = diss_o ? at.state(2, 0) : c;
-  }
-};
-
-__device__ __forceinline__ void clear(double (&a)[16]) {
-#pragma unroll
-  for (int e = 0; e < 16; ++e) a[e] = 0.0;
-}
-
-// Calls body(local cell, lane, valid cells of the warp) for the cells of this thread's instance.
-// Whole warps stay in the loop together; the body's cell is clamped to the instance.
-template <class Body>
-__device__ __forceinline__ void for_cells(const Instance& in, Body body) {
-  const int64_t cells = (int64_t)in.M * in.N;
-  const int lane = threadIdx.x & 31;
-  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); first < cells;
-       first += (int64_t)gridDim.x * blockDim.x) {
-    const int valid = (int)min((int64_t)32, cells - first);
-    body(first, min(first + lane, cells - 1), lane, valid);
-  }
-}
-
-__device__ __forceinline__ CellAt cell_at(const Instance& in, int64_t local, const double* X,
-                                          const double* V, const double* U) {
-  return CellAt{(int)(local % in.M), (int)(local / in.M), in.M, in.N, U + 4 * in.cell_offset,
-                X + 2 * in.vert_offset, V ? V + 2 * in.vert_offset : nullptr};
-}
+using Cell_ = CellAt<double, kDirNone>;
+using Geometry_ = CellGeometry<double>;
+using Line_ = RadialLine<double>;
+using Face_ = FaceDerivatives<double>;
 
 template <int Warps>
 __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
@@ -140,9 +35,9 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
   WarpRows<16>& S = rows[threadIdx.x >> 5];
   const int64_t slot = 16 * (int64_t)in.M * in.N;
   for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
-    const CellAt at = cell_at(in, local, X, V, U);
+    const Cell_ at(in, local, X, V, U, nullptr);
     const int m = at.m, M = in.M;
-    const CellGeometry geo(at);
+    const Geometry_ geo(at);
     const double s = -geo.inv_area();
     double* out = J + 144 * in.cell_offset + 16 * first;
     auto store = [&](int k, double (&a)[16], bool active) {
@@ -152,13 +47,13 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
     };
     double centre[16], a[16];
     clear(centre);
-    const State c = at.state(0, 0);
+    const State<double> c = at.state(0, 0);
     {  // angular faces: b (line f, c, b, bb), then f (line b, c, f, ff)
-      const State fw = at.state(0, 1), bw = at.state(0, -1);
+      const State<double> fw = at.state(0, 1), bw = at.state(0, -1);
       double Qb[4], gb, c4b;  // face b's block of its outer state f
       {
-        const State bb = at.state(0, -2);
-        const FaceDerivatives d(fw, c, bw, bb, geo.b, true, in);
+        const State<double> bb = at.state(0, -2);
+        const Face_ d(fw, c, bw, bb, geo.b, true, in);
         add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
         clear(a);
         add_outer(a, d.Q, d.g_rr, d.c4, bb);
@@ -170,8 +65,8 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
         gb = d.g_ll;
         c4b = d.c4;
       }
-      const State ff = at.state(0, 2);
-      const FaceDerivatives d(bw, c, fw, ff, geo.f, true, in);
+      const State<double> ff = at.state(0, 2);
+      const Face_ d(bw, c, fw, ff, geo.f, true, in);
       add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
       add_outer(a, d.Q, d.g_ll, -d.c4, bw);
       store(kB, a, true);
@@ -185,10 +80,10 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
     }
     // radial faces: i (line o, c, i, ii), then o (line i, c, o, oo); a ghost's block goes to the
     // cell itself, through the ghost's derivative
-    const RadialLine line(at, c, geo, in);
+    const Line_ line(at, c, geo, in);
     double Qi[4], gi, c4i;  // face i's block of its outer state o
     {
-      const FaceDerivatives d(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+      const Face_ d(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
       add_block(centre, d.of<true>(c), c, d.nx, d.nz, d.vl);
       clear(a);
       add_outer(a, d.Q, d.g_rr, d.c4, line.ii);
@@ -200,7 +95,7 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
       gi = d.g_ll;
       c4i = d.c4;
     }
-    const FaceDerivatives d(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+    const Face_ d(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
     if (m == 0) through_wall(centre, a, geo.wall());
     if (m == M - 1) {  // face i's outer state is the far-field ghost: minus its block
       double e[16];
@@ -233,40 +128,34 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
   });
 }
 
-// The derivative of the wall ghost's momentum by the wall's normal (x then z) or grid velocity,
-// contracted with dF_k by the momentum: e1, e2 -> the derivatives of F_k.
-__device__ __forceinline__ double2 ghost_by_normal(const Wall& w, const State& c, double e1,
-                                                   double e2) {
-  const double mx = c.u[1] - w.gx * c.u[0], mz = c.u[2] - w.gz * c.u[0];
-  const double t = w.nx * mx + w.nz * mz, en = fma(e1, w.nx, e2 * w.nz);
-  const double q = 2.0 * w.inn, r = q * en;
-  return make_double2(fma(r, 2.0 * t * w.nx * w.inn - mx, -q * t * e1),
-                      fma(r, 2.0 * t * w.nz * w.inn - mz, -q * t * e2));
-}
-__device__ __forceinline__ double2 ghost_by_velocity(const Wall& w, const State& c, double e1,
-                                                     double e2) {
+// The same by the wall's grid velocity (see ghost_by_normal).
+__device__ __forceinline__ P2<double> ghost_by_velocity(const Wall<double>& w,
+                                                        const State<double>& c, double e1,
+                                                        double e2) {
   const double a = 2.0 * w.inn * c.u[0] * fma(e1, w.nx, e2 * w.nz);
-  return make_double2(a * w.nx, a * w.nz);
+  return P2<double>{a * w.nx, a * w.nz};
 }
 
-// d(odes)/d(vertices) (Velo = false) or d(odes)/d(velocities): four corners' 4 x 2 blocks.
+// d(odes)/d(vertices) (Velo = false) or d(odes)/d(velocities): four corners' 4 x 2 blocks. The
+// vertices' kernel holds four faces' derivatives by their normals at once: at two CTAs per SM (255
+// registers) it takes 58 us, at three (168, 900 bytes spilled) 67 us; the velocities' fits three.
 template <bool Velo>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, Velo ? 3 : 2)
     k_jac_corners_cells(Table t, const double* X, const double* V, const double* U, double* J) {
   __shared__ WarpRows<8> rows[4];
   const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
   WarpRows<8>& S = rows[threadIdx.x >> 5];
   const int64_t slot = 8 * (int64_t)in.M * in.N;
   for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
-    const CellAt at = cell_at(in, local, X, V, U);
+    const Cell_ at(in, local, X, V, U, nullptr);
     const int m = at.m;
-    const CellGeometry geo(at);
+    const Geometry_ geo(at);
     const double ia = geo.inv_area();
-    const State c = at.state(0, 0);
+    const State<double> c = at.state(0, 0);
     // per face (b, f, i, o): dF_k by its normal, or by its grid velocity
     double gx[4][4], gz[4][4], sum[4];
-    auto face = [&](int q, const State& ll, const State& r, const State& rr, const FaceGeometry& f,
-                    bool diss) {
+    auto face = [&](int q, const State<double>& ll, const State<double>& r,
+                    const State<double>& rr, const FaceGeometry<double>& f, bool diss) {
       if constexpr (Velo) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -275,7 +164,7 @@ __global__ void __launch_bounds__(128, 3)
           gz[q][k] = a * f.nz;
         }
       } else {
-        const FaceDerivatives d(ll, c, r, rr, f, diss, in);
+        const Face_ d(ll, c, r, rr, f, diss, in);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           gx[q][k] = d.by_normal<true>(c, r, f, k);
@@ -286,7 +175,7 @@ __global__ void __launch_bounds__(128, 3)
       }
     };
     {
-      const State fw = at.state(0, 1), bw = at.state(0, -1);
+      const State<double> fw = at.state(0, 1), bw = at.state(0, -1);
       if constexpr (Velo) {
         face(0, c, bw, c, geo.b, true);
         face(1, c, fw, c, geo.f, true);
@@ -295,16 +184,16 @@ __global__ void __launch_bounds__(128, 3)
         face(1, bw, fw, at.state(0, 2), geo.f, true);
       }
     }
-    const RadialLine line(at, c, geo, in);
+    const Line_ line(at, c, geo, in);
     face(2, line.o, line.i, line.ii, geo.i, line.diss_i);
     face(3, line.i, line.o, line.oo, geo.o, line.diss_o);
     if (m == 0) {  // the wall ghost is on both radial lines and moves with the inner face
-      const Wall w = geo.wall();
+      const Wall<double> w = geo.wall();
       double e[16], dp[4];
       clear(e);
-      const FaceDerivatives di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+      const Face_ di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
       add_block(e, di.of<false>(line.i), line.i, di.nx, di.nz, di.vr);
-      const FaceDerivatives dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+      const Face_ dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
       grad_p(line.i, dp);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -312,9 +201,9 @@ __global__ void __launch_bounds__(128, 3)
         const double q = dO.Q[k] * dO.g_ll;
         const double e1 = e[k + 4] + fma(q, dp[1], k == 1 ? -dO.c4 : 0.0);
         const double e2 = e[k + 8] + fma(q, dp[2], k == 2 ? -dO.c4 : 0.0);
-        const double2 a = Velo ? ghost_by_velocity(w, c, e1, e2) : ghost_by_normal(w, c, e1, e2);
+        const P2<double> a = Velo ? ghost_by_velocity(w, c, e1, e2) : ghost_by_normal(w, c, e1, e2);
         gx[2][k] += a.x;
-        gz[2][k] += a.y;
+        gz[2][k] += a.z;
       }
     }
     double* out = J + 32 * in.cell_offset + 8 * first;
@@ -333,8 +222,8 @@ __global__ void __launch_bounds__(128, 3)
         }
       } else {
         // cross = (x2 - x0) (z3 - z1) - (z2 - z0) (x3 - x1), by corner k's coordinates
-        const double2 p = geo.x[(k + 1) & 3], q = geo.x[(k + 3) & 3];
-        double ax = p.y - q.y, az = q.x - p.x;
+        const P2<double> p = geo.x[(k + 1) & 3], q = geo.x[(k + 3) & 3];
+        double ax = p.z - q.z, az = q.x - p.x;
         ax *= sa;
         az *= sa;
 #pragma unroll
@@ -368,18 +257,18 @@ __global__ void __launch_bounds__(128)
   for (int n = (blockIdx.x - zero_blocks) * blockDim.x + threadIdx.x; n < in.N;
        n += (gridDim.x - zero_blocks) * blockDim.x) {
     const int64_t local = in.M - 1 + (int64_t)in.M * n;
-    const CellAt at = cell_at(in, local, X, V, U);
-    const CellGeometry geo(at);
-    const State c = at.state(0, 0);
-    const RadialLine line(at, c, geo, in);
-    const FaceDerivatives di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
-    const FaceDerivatives dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
+    const Cell_ at(in, local, X, V, U, nullptr);
+    const Geometry_ geo(at);
+    const State<double> c = at.state(0, 0);
+    const Line_ line(at, c, geo, in);
+    const Face_ di(line.o, c, line.i, line.ii, geo.i, line.diss_i, in);
+    const Face_ dO(line.i, c, line.o, line.oo, geo.o, line.diss_o, in);
     double e[16];
     clear(e);
     add_outer(e, di.Q, di.g_ll, -di.c4, line.o);
     add_block(e, dO.of<false>(line.o), line.o, dO.nx, dO.nz, dO.vr);
-    const double root = sqrt_(kGamma), speed = in.mach * root;
-    const double d[4] = {0.0, 2.0 * root * in.cos_aoa, 2.0 * root * in.sin_aoa, 2.0 * speed * root};
+    double d[4];
+    ghost_by_mach(in, d);
     const double s = -geo.inv_area();
 #pragma unroll
     for (int k = 0; k < 4; ++k)

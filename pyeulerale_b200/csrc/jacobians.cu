@@ -1,6 +1,7 @@
 // C ABI of the first-order Jacobians, replacing the complex-step procedures of
 // src/spatial_discretization.f90: the residual's by the closed-form kernels of jac_cells.cu, the
-// forces' by the dual-number kernels of jacobian_kernels.cuh with B = double.
+// forces' by the dual-number kernels of jacobian_kernels.cuh with B = double; and the residual's by
+// the states in dual numbers, for comparison.
 
 #include "jacobian_kernels.cuh"
 
@@ -14,6 +15,63 @@ int launch_jac_corners(const eb_batch* b, bool velocities, const double* X, cons
                        const double* U, double* J, cudaStream_t st);
 int launch_jac_mach(const eb_batch* b, const double* X, const double* V, const double* U,
                     double* J, cudaStream_t st);
+
+namespace {
+
+// Face flux kept out of line: the dual-number states Jacobian evaluates it in a loop with a wide
+// type, and inlining every case makes the kernel very large.
+template <class R, class SP, class TX, class TV, class TM>
+__device__ __noinline__ S4<R> face_call(int q, int flag, const SP& u, const Geometry<TX, TV>& g,
+                                        const TM& mach, const Instance& in) {
+  return face<R>(q, flag, u, g, mach, in);
+}
+
+// State provider for the states Jacobian: the states of slot `seed_slot` carry the identity
+// tangent, every other state a zero tangent.
+struct SeededStates {
+  const Plain* p;
+  int seed_slot;
+  EB_HD S4<Dual<double, 4>> operator()(int s) const {
+    S4<Dual<double, 4>> r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r.v[k] = seed<double, 4>(p->u[s].v[k], s == seed_slot ? k : -1);
+    return r;
+  }
+};
+
+// d(odes)/d(states) blocks (compute_odes_wrt_states, f90:666-750) by dual numbers. Each slot's
+// block sums only the faces that read that slot (others contribute exactly zero). Grid z: slots.
+__global__ void __launch_bounds__(128) k_jac_states(Table t, const double* X, const double* V,
+                                                    const double* U, double* J) {
+  using R = Dual<double, 4>;
+  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;  // grid y = instance
+  const int64_t cells = (int64_t)in.M * in.N;
+  for (int64_t local = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; local < cells;
+       local += (int64_t)gridDim.x * blockDim.x) {
+    Plain p;
+    load_plain(in, local, X, V, U, p);
+    const Geometry<double, double> geo = geometry(p.x, p.w);
+    const int s = blockIdx.z;
+    double* out = J + 144 * in.cell_offset + 16 * local + 16 * cells * s;
+    double acc[4][4] = {};
+    const bool active = slot_active(s, p.m, in.M);
+    const SeededStates prov{&p, s};
+    for (int q = 0; q < 4; ++q) {
+      if (!active || !face_uses_slot(q, p.flag, s)) continue;
+      const S4<R> f = face_call<R>(q, p.flag, prov, geo, in.mach, in);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[r][i] = acc[r][i] + f.v[r].d[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) out[r + 4 * i] = active ? -acc[r][i] / geo.area : 0.0;
+  }
+}
+
+}  // namespace
 }  // namespace eb
 
 extern "C" {
@@ -45,8 +103,7 @@ int eb_compute_odes_wrt_states_untiled(const eb_batch* b, const double* X, const
   dim3 jgrid;
   if (int rc = per_instance_grid(b, false, 1, 128, jgrid)) return rc;
   jgrid.z = 9;
-  k_jac_states<double, kDirNone><<<jgrid, 128, 0, EB_STREAM(stream)>>>(
-      t, b->n_cells, X, V, U, nullptr, J, nullptr, nullptr);
+  k_jac_states<<<jgrid, 128, 0, EB_STREAM(stream)>>>(t, X, V, U, J);
   return check_launch("compute_odes_wrt_states_untiled");
 }
 
