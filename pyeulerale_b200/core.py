@@ -46,10 +46,13 @@ class _Staging:
     A transfer from ordinary host memory waits for the driver's own copies; through a pinned buffer
     the host writes (or reads) the values once, in whatever layout its array has, and the transfer
     runs on the stream. A buffer is written again only after its previous transfer has finished.
+    The buffers start as parts of one pinned allocation of ``numel`` values each (a pinned
+    allocation costs about half a millisecond whatever its size); a larger array replaces its own.
     """
 
-    def __init__(self, torch, count: int = 4) -> None:
+    def __init__(self, torch, numel: int, count: int = 4) -> None:
         self._torch = torch
+        self._numel = numel
         self._ring = [[None, torch.cuda.Event()] for _ in range(count)]
         self._next = 0
 
@@ -57,6 +60,11 @@ class _Staging:
         slot = self._ring[self._next]
         self._next = (self._next + 1) % len(self._ring)
         slot[1].synchronize()
+        if slot[0] is None and n <= self._numel:
+            whole = self._torch.empty(len(self._ring) * self._numel, dtype=self._torch.float64,
+                                      pin_memory=True)
+            for one, part in zip(self._ring, whole.split(self._numel)):
+                one[0] = part if one[0] is None else one[0]
         if slot[0] is None or slot[0].numel() < n:
             slot[0] = self._torch.empty(n, dtype=self._torch.float64, pin_memory=True)
         return slot[0][:n], slot[1]
@@ -159,7 +167,7 @@ class SpatialDiscretization:
         self._dJF_u = torch.zeros(8 * N, **f64)
         self._dJF_x = torch.zeros(8 * N, **f64)
         self._mirrors: dict[str, np.ndarray] = {}
-        self._staging = _Staging(torch)
+        self._staging = _Staging(torch, 8 * max(nc, nv))  # a complex state, or two of vertices
         self._lu_stale = True
         self.set_free_stream_state()
 
