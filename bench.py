@@ -801,9 +801,9 @@ def run_b200(args) -> None:
             "jacobian_states": {"value": world * cells / t_jac, "unit": "cells/s",
                                 "achieved_gbs": BYTES_PER_CELL_JAC_STATES * cells / t_jac / 1e9,
                                 "bytes_per_cell": BYTES_PER_CELL_JAC_STATES,
-                                "kernel": "k_jac_states_tiled",
+                                "kernel": "k_jac_states_cells",
                                 "untiled": {"value": world * cells / t_jac_plain,
-                                            "kernel": "k_jac_states (one thread per cell)"}},
+                                            "kernel": "k_jac_states (dual numbers)"}},
             "tangent": {"value": world * cells / t_tan, "unit": "cells/s",
                         "achieved_gbs": BYTES_PER_CELL_TANGENT * cells / t_tan / 1e9,
                         "bytes_per_cell": BYTES_PER_CELL_TANGENT,

@@ -110,12 +110,11 @@ int eb_compute_odes_wrt_mach(const eb_batch* b, const double* X, const double* V
                              const double* U, double* J, void* stream);
 /* compute_odes_wrt_states, f90:666-750. J: (4, 4, M, N, 9) per instance, 144*cell_offset.
  * Blocks the reference does not compute (slots reaching past the radial boundary) are 0.
- * Tiled kernel: each face evaluated once for both cells, per seeded stencil state. */
+ * One thread per cell, each of its faces differentiated in closed form. */
 int eb_compute_odes_wrt_states(const eb_batch* b, const double* X, const double* V,
                                const double* U, double* J, void* stream);
-/* The same Jacobian by the plain one-thread-per-cell kernel (each slot's block from that cell's
- * own face evaluations, as the reference's per-cell complex step); a baseline for the tiled
- * kernel. */
+/* The same Jacobian by dual numbers (each slot's block from that cell's own face evaluations, as
+ * the reference's per-cell complex step); a baseline for the closed-form kernel. */
 int eb_compute_odes_wrt_states_untiled(const eb_batch* b, const double* X, const double* V,
                                        const double* U, double* J, void* stream);
 /* compute_odes_wrt_vertices, f90:933-993. J: (4, 2, M, N, 4) per instance, 32*cell_offset. */
@@ -270,8 +269,8 @@ int eb_gmres_solve_anchored(const eb_batch* b, const double* J, int n_sys, const
 
 /* Device workspace (bytes) holding the block-LU factors of one M x N instance: 3 M dense
  * (4N)^2 complex super-blocks (Dinv, L1, C1' per ring: 768 M N^2 bytes; 1.6 GB at 129x129,
- * 12.9 GB at 257x257, 25.8 GB at 513x257), the rings' real 4 x 4 block diagonals (B2, C2), two
- * scratch super-blocks, pivots and solve vectors. */
+ * 12.9 GB at 257x257, 25.8 GB at 513x257), the rings' real 4 x 4 block diagonals (B1, B2, C1,
+ * C2), four scratch super-blocks, pivots, the inversion's flags and solve vectors. */
 int64_t eb_ringlu_workspace_bytes(int M, int N);
 
 /* Factors A = J - shift I (J: d(odes)/d(states) of the single instance in `b`) by block
@@ -333,7 +332,8 @@ int eb_fp64_mma_probe(int64_t iterations, int sms, double* sink, void* stream);
  * complex double (interleaved), column-major, no transposes, A_z = A + z stride_a complex
  * elements (likewise B, C); alpha and beta real, beta == 0 does not read C. variant: -1 the
  * default (2), 0 the register-staged double buffer, 1 the cp.async three-stage ring on 64 x 64
- * tiles, 2 a two-stage ring on 64 x 32 tiles (identical results). In the reference the dense products of its solves are SuperLU's and BLAS's
+ * tiles, 2 a two-stage ring on 64 x 32 tiles, 32 x 16 where those are too few to fill the GPU
+ * (identical results). In the reference the dense products of its solves are SuperLU's and BLAS's
  * (core.py:533-599). */
 int eb_zgemm_strided_batched(int M, int N, int K, double alpha, const double* A, int lda,
                              int64_t stride_a, const double* B, int ldb, int64_t stride_b,
@@ -342,8 +342,8 @@ int eb_zgemm_strided_batched(int M, int N, int K, double alpha, const double* A,
 
 /* ---- launch-variant autotuner -------------------------------------------------------------- */
 
-/* Kernels with several launch variants of identical results (the states Jacobian: dual width 4
- * at one CTA per SM or width 2 at two) time each variant on the first call for a problem size
+/* Kernels with several launch variants of identical results (the states Jacobian: four or two
+ * warps per CTA) time each variant on the first call for a problem size
  * and keep the fastest (EB_AUTOTUNE=0, or a stream being captured: the default variant, untimed).
  * Writes the choices and their times as text into buf (len bytes, NUL-terminated) and returns
  * the report's full length. No counterpart in the reference (which has no GPU kernels). */

@@ -1,18 +1,22 @@
-// Dense complex double products of the ring-block LU (ringlu.cu): strided-batched
-// C = alpha A B + beta C (column-major, no transposes) on the FP64 tensor-core instruction
-// mma.sync.m8n8k4.f64, and strided-batched matrix-vector products y = alpha op(A) x + beta y with
-// op(A) = A or A^H. alpha and beta are real (the LU uses +-1 and 0 / 1).
+// Dense double products of the ring-block LU (ringlu.cu): strided-batched C = alpha A B + beta C
+// (column-major, no transposes; complex, or real where every shift is real) on the FP64
+// tensor-core instruction mma.sync.m8n8k4.f64, and the matrix-vector products of its sweeps.
+// alpha and beta are real (the LU uses +-1 and 0 / 1).
 //
-// GEMM: a CTA computes a kBM x kBN tile of C for one batch entry with four warps, each a 32 x 32
-// sub-tile as 4 x 4 products of 8 x 8 (m8n8k4 fragments; real and imaginary parts in separate
-// accumulators: re += Ar Br - Ai Bi, im += Ar Bi + Ai Br, four real MMAs per complex product).
-// The kBK-deep slices of A and B go through shared memory as separate real / imaginary planes,
-// two slices in flight (the next slice's global loads are issued before the current slice's
-// MMAs). Edges (sizes not multiples of the tile) load zeros and store under bounds checks.
-// A second variant (kAsync) moves the slices with cp.async into a three-stage ring of shared
-// buffers that keep each complex element's two parts together (one 16-byte fragment load gives
-// both), with no register staging; it issues the same MMAs in the same order, so the two
-// variants give identical results.
+// GEMM: a CTA computes a tile of C for one batch entry with four warps, each a sub-tile of 8 x 8
+// products (m8n8k4 fragments; complex: real and imaginary parts in separate accumulators, re +=
+// Ar Br - Ai Bi, im += Ar Bi + Ai Br, four real MMAs per complex product). The kBK-deep slices of A
+// and B go through shared memory, two slices in flight (the next slice's loads are issued before
+// the current slice's MMAs). Edges (sizes not multiples of the tile) load zeros and store under
+// bounds checks. The default moves the slices with cp.async into a ring of shared buffers that keep
+// each complex element's two parts together (one 16-byte fragment load gives both) on 64 x 32
+// tiles, or 32 x 16 where those would leave SMs idle; a register-staged variant and one on 64 x 64
+// tiles issue the same MMAs in the same order, so all give identical results.
+//
+// Sweep products: y (+)= -sum of blocks times vectors for one right-hand side (k_sweep_n, and
+// k_sweep_h for the adjoint's A^H), or for several that share the block (k_sweep_multi). A ring's
+// terms go in one launch, and the launches of a sweep start early (programmatic dependent
+// launches): each loads its matrix while the one before it finishes.
 
 #include <cuda_runtime.h>
 
