@@ -11,13 +11,15 @@
 // each). A block sum keeps the reference's face order, ((F_b + F_f) + F_i) + F_o.
 //
 // Measured on 282,000 cells of uneven grids against dual numbers (tiles staged in shared memory, at
-// one CTA per SM): states 567 -> 95 us (3.4 TB/s of 6.5 copied), vertices 594 -> 58 us, velocities
-// 263 -> 35 us, mach 34 -> 7.5 us. What is left is latency: the registers of a face's derivatives
+// one CTA per SM): states 567 -> 80 us (4.1 TB/s of 6.5 copied), vertices 594 -> 45 us, velocities
+// 263 -> 26 us, mach 34 -> 7.5 us. What is left is latency: the registers of a face's derivatives
 // leave eight to twelve warps per SM.
 
 #include "autotune.cuh"
 #include "common.cuh"
 #include "jac_faces.cuh"
+
+#include <algorithm>
 
 namespace eb {
 namespace {
@@ -27,14 +29,56 @@ using Geometry_ = CellGeometry<double>;
 using Line_ = RadialLine<double>;
 using Face_ = FaceDerivatives<double>;
 
+// Calls body(instance, warp's first cell, thread's cell, lane, valid cells of the warp) for a batch's
+// cells, 32 to a warp. Grid y = instance, or one row for all: then the warps' cells of all
+// instances, each rounded up to whole warps, are one range, and a warp finds its instance by the
+// sums of the table's sizes. Whole warps stay in the loop together; the thread's cell is clamped to
+// the instance.
+template <class Body>
+__device__ __forceinline__ void for_batch_cells(const Table& t, Body body) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const bool flat = t.dev != nullptr && (int)gridDim.y < t.n;
+  for (int64_t w = blockIdx.x * (int64_t)warps + (threadIdx.x >> 5);;
+       w += (int64_t)gridDim.x * warps) {
+    int64_t part = w;  // the warp's place among its instance's
+    int at = blockIdx.y;
+    if (flat) {
+      int base = 0;
+      for (; base < t.n; base += 32) {
+        int64_t sum = 0;
+        if (base + lane < t.n)
+          sum = ((int64_t)t.dev[base + lane].M * t.dev[base + lane].N + 31) / 32;
+        const int64_t own = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+          const int64_t before = __shfl_up_sync(0xffffffffu, sum, d);
+          if (lane >= d) sum += before;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, sum > part);
+        if (past != 0u) {
+          const int k = __ffs(past) - 1;
+          part -= __shfl_sync(0xffffffffu, sum - own, k);
+          at = base + k;
+          break;
+        }
+        part -= __shfl_sync(0xffffffffu, sum, 31);
+      }
+      if (base >= t.n) return;
+    }
+    const Instance in = t.dev ? t.dev[at] : t.single;
+    const int64_t cells = (int64_t)in.M * in.N, first = 32 * part;
+    if (first >= cells) return;
+    body(in, first, min(first + lane, cells - 1), lane, (int)min((int64_t)32, cells - first));
+  }
+}
+
 template <int Warps>
 __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
     k_jac_states_cells(Table t, const double* X, const double* V, const double* U, double* J) {
   __shared__ WarpRows<16> rows[Warps];
-  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
   WarpRows<16>& S = rows[threadIdx.x >> 5];
-  const int64_t slot = 16 * (int64_t)in.M * in.N;
-  for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
+  for_batch_cells(t, [&](const Instance& in, int64_t first, int64_t local, int lane, int valid) {
+    const int64_t slot = 16 * (int64_t)in.M * in.N;
     const Cell_ at(in, local, X, V, U, nullptr);
     const int m = at.m, M = in.M;
     const Geometry_ geo(at);
@@ -138,15 +182,14 @@ __device__ __forceinline__ P2<double> ghost_by_velocity(const Wall<double>& w,
 
 // d(odes)/d(vertices) (Velo = false) or d(odes)/d(velocities): four corners' 4 x 2 blocks. The
 // vertices' kernel holds four faces' derivatives by their normals at once: at two CTAs per SM (255
-// registers) it takes 58 us, at three (168, 900 bytes spilled) 67 us; the velocities' fits three.
+// registers) it took 58 us, at three (168, 900 bytes spilled) 67 us (a grid row per instance); the velocities' fits three.
 template <bool Velo>
 __global__ void __launch_bounds__(128, Velo ? 3 : 2)
     k_jac_corners_cells(Table t, const double* X, const double* V, const double* U, double* J) {
   __shared__ WarpRows<8> rows[4];
-  const Instance in = t.dev ? t.dev[blockIdx.y] : t.single;
   WarpRows<8>& S = rows[threadIdx.x >> 5];
-  const int64_t slot = 8 * (int64_t)in.M * in.N;
-  for_cells(in, [&](int64_t first, int64_t local, int lane, int valid) {
+  for_batch_cells(t, [&](const Instance& in, int64_t first, int64_t local, int lane, int valid) {
+    const int64_t slot = 8 * (int64_t)in.M * in.N;
     const Cell_ at(in, local, X, V, U, nullptr);
     const int m = at.m;
     const Geometry_ geo(at);
@@ -276,11 +319,27 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// Grid of a kernel that goes through for_batch_cells. One grid row per instance, sized by the table's
+// largest dimension squared, leaves an uneven batch most of its blocks without cells, and each
+// still takes registers until it has read its instance's entry: 21 grids of 282,000 cells, 512 x 21
+// blocks for 2,200 with cells, 207 us for the six Jacobians, 170 us as one flat range. The search
+// reads the table in rounds of 32, so the flat range is for batches of up to four rounds that fill
+// less than three quarters of the rows.
+int cells_grid(const eb_batch* b, int threads, dim3& grid) {
+  if (int rc = per_instance_grid(b, false, 1, threads, grid)) return rc;
+  const int64_t square = (int64_t)b->max_dim * b->max_dim;
+  if (b->n_inst > 1 && b->n_inst <= 128 && 4 * b->n_cells <= 3 * square * b->n_inst) {
+    const int64_t blocks = b->n_cells / threads + b->n_inst;
+    grid = dim3((unsigned)std::min<int64_t>(blocks, 148 * 64 * 8), 1);
+  }
+  return EB_OK;
+}
+
 template <int Warps>
 int launch_states(const eb_batch* b, const Table& t, const double* X, const double* V,
                   const double* U, double* J, cudaStream_t st) {
   dim3 grid;
-  if (int rc = per_instance_grid(b, false, 1, 32 * Warps, grid)) return rc;
+  if (int rc = cells_grid(b, 32 * Warps, grid)) return rc;
   k_jac_states_cells<Warps><<<grid, 32 * Warps, 0, st>>>(t, X, V, U, J);
   return check_launch("compute_odes_wrt_states");
 }
@@ -302,7 +361,7 @@ int launch_jac_corners(const eb_batch* b, bool velocities, const double* X, cons
                        const double* U, double* J, cudaStream_t st) {
   const Table t = make_table(b);
   dim3 grid;
-  if (int rc = per_instance_grid(b, false, 1, 128, grid)) return rc;
+  if (int rc = cells_grid(b, 128, grid)) return rc;
   if (velocities) k_jac_corners_cells<true><<<grid, 128, 0, st>>>(t, X, V, U, J);
   else k_jac_corners_cells<false><<<grid, 128, 0, st>>>(t, X, V, U, J);
   return check_launch(velocities ? "compute_odes_wrt_velocities" : "compute_odes_wrt_vertices");

@@ -51,3 +51,26 @@ def test_batch_equals_single_launches(cuda):
             gpu.call(name, gpu.X, gpu.V, gpu.U, one)
             parts.append(one)
         np.testing.assert_array_equal(J.cpu().numpy(), cuda.cat(parts).cpu().numpy())
+
+
+@pytest.mark.parametrize("count", [2, 33, 128, 129])
+def test_many_uneven_instances(cuda, count):
+    """Batches below, at and above the rounds of the flat range's search: every cell is written with
+    what its own launch writes."""
+    from pyeulerale_b200.batch import InstanceSet, InstanceSpec
+
+    kinds = [_case(M, N) for M, N in SIZES[:3] + SIZES[4:]]
+    cases = [kinds[(7 * k) % 5 if k else 3] for k in range(count)]
+    inst = InstanceSet([InstanceSpec(c["X"], c["mach"], c["aoa"]) for c in cases])
+    pack = lambda k: cuda.from_numpy(  # noqa: E731
+        np.concatenate([np.asarray(c[k]).ravel(order="F") for c in cases])).cuda()
+    X, V, U = pack("X"), pack("V"), pack("U")
+    for name, per_cell in KEYS.values():
+        J = cuda.full((per_cell * inst.n_cells,), float("nan"), dtype=cuda.float64, device="cuda")
+        inst.call(name, X, V, U, J)
+        parts = {}
+        for c in kinds:
+            gpu = Gpu(cuda, c)
+            parts[id(c)] = gpu.empty(per_cell * gpu.M * gpu.N)
+            gpu.call(name, gpu.X, gpu.V, gpu.U, parts[id(c)])
+        assert cuda.equal(J, cuda.cat([parts[id(c)] for c in cases]))
