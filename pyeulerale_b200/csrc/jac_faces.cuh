@@ -114,26 +114,45 @@ struct Block {
 };
 
 // A face's flux in its cell's orientation, differentiated. diss = false: the central flux of the
-// faces next to the boundaries (f90:197, 219); ll and rr need then only be finite.
+// faces next to the boundaries (f90:197, 219). Nothing of the dissipation is formed there: r may be a
+// ghost state, whose pressure and density can be negative (2 U_inf - U of a cell at twice the free
+// stream's; the reflection at a fast wall), so that it has no speed of sound; ll and rr are not
+// used.
 template <class T>
 struct FaceDerivatives {
   T nx, nz, vn, vl, vr;
   T Q[4], h[4];                 // dF/dS, dF/dlambda (zero without dissipation)
   T g_ll, g_l, g_r, g_rr;       // dS/dp of the four states
   T c2, c4;
+  bool diss;
   bool lam_l;                   // lambda is l's (else r's)
   double sgn;                   // the sign of that state's normal velocity
   T c, len, ilen;               // its speed of sound; |n| and its inverse
 
   __device__ __forceinline__ FaceDerivatives(const State<T>& ll, const State<T>& l,
                                              const State<T>& r, const State<T>& rr,
-                                             const FaceGeometry<T>& f, bool diss,
-                                             const Instance& in) {
+                                             const FaceGeometry<T>& f, bool diss_,
+                                             const Instance& in)
+      : diss(diss_) {
     nx = f.nx;
     nz = f.nz;
     vn = f.gx * nx + f.gz * nz;
     vl = (nx * l.u[1] + nz * l.u[2]) * l.ir;
     vr = (nx * r.u[1] + nz * r.u[2]) * r.ir;
+    if (diss) {
+      dissipation(ll, l, r, rr, in);
+    } else {
+      lam_l = false;
+      sgn = 0.0;
+      g_ll = g_l = g_r = g_rr = c2 = c4 = c = len = ilen = lift<T>(0.0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) Q[k] = h[k] = lift<T>(0.0);
+    }
+  }
+
+  __device__ __forceinline__ void dissipation(const State<T>& ll, const State<T>& l,
+                                              const State<T>& r, const State<T>& rr,
+                                              const Instance& in) {
     len = sqrt_(nx * nx + nz * nz);
     ilen = recip_(len);
     const T cl = sqrt_(kGamma * l.p * l.ir), cr = sqrt_(kGamma * r.p * r.ir);
@@ -157,14 +176,13 @@ struct FaceDerivatives {
     c2 = in.k2 * S * lam;
     c4 = in.k4 * lam - in.c4 * c2;
     const bool active = !(0.0 > value(c4) + 1e-8);  // max_c(0, c4)
-    const double on = diss ? 1.0 : 0.0, on4 = active ? on : 0.0;
-    c2 = c2 * on;
+    const double on4 = active ? 1.0 : 0.0;
     c4 = c4 * on4;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const T d1 = r.u[k] - l.u[k];
       const T d3 = mad(3.0, l.u[k] - r.u[k], rr.u[k] - ll.u[k]);
-      const T by_c2 = -mad(on4 * in.c4, d3, on * d1);  // dF/dc2 (through c4 as well)
+      const T by_c2 = -mad(on4 * in.c4, d3, d1);  // dF/dc2 (through c4 as well)
       Q[k] = by_c2 * (in.k2 * lam);
       h[k] = mad(by_c2, in.k2 * S, on4 * in.k4 * d3);
     }
@@ -175,7 +193,7 @@ struct FaceDerivatives {
   __device__ __forceinline__ Block<T> of(const State<T>& s) const {
     Block<T> b;
     const T v = Left ? vl : vr, g = Left ? g_l : g_r;
-    const bool lam = Left == lam_l;
+    const bool lam = diss && Left == lam_l;
     // dlambda = sgn dv + len dc, dc = c / (2 p) dp - c / (2 rho) e_0
     const T zero = lift<T>(0.0);
     const T lp = lam ? quot_(0.5 * len * c, s.p) : zero, le = lam ? -0.5 * len * c * s.ir : zero;
@@ -197,6 +215,7 @@ struct FaceDerivatives {
     const T n = k == 1 ? nx : k == 2 ? nz : lift<T>(0.0);
     T f = 0.5 * (mad(l.u[k], vl - vn, r.u[k] * (vr - vn)) + n * (l.p + r.p));
     if (k == 3) f = f + 0.5 * mad(l.p, vl, r.p * vr);
+    if (!diss) return f;
     const T d1 = r.u[k] - l.u[k];
     const T d3 = mad(3.0, l.u[k] - r.u[k], rr.u[k] - ll.u[k]);
     return mad(c4, d3, mad(-c2, d1, f));
@@ -210,6 +229,7 @@ struct FaceDerivatives {
     T d = 0.5 * mad(l.u[k], ul - g, r.u[k] * (ur - g));
     if (k == (X ? 1 : 2)) d = d + 0.5 * (l.p + r.p);
     if (k == 3) d = d + 0.5 * mad(l.p, ul, r.p * ur);
+    if (!diss) return d;
     const T lam = mad(sgn, lam_l ? ul : ur, c * (X ? nx : nz) * ilen);
     return mad(h[k], lam, d);
   }
