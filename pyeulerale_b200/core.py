@@ -40,54 +40,35 @@ def _torch():
     return torch
 
 
-class _Staging:
-    """Pinned host buffers between the host arrays and the device, one ring per solver.
+# Transfers go through pinned buffers: one from ordinary host memory waits for the driver's own
+# copies; with a pinned buffer the host writes (or reads) the values once, in whatever layout its
+# array has, and the transfer runs on the stream. Every transfer takes a buffer of its own from
+# PyTorch's pinned allocator, which hands a buffer out again only after the transfers recorded on it
+# have finished: threads and streams that share a solver share no buffer, and a new solver finds
+# the buffers that earlier ones returned (a first pinned allocation takes about half a millisecond).
 
-    A transfer from ordinary host memory waits for the driver's own copies; through a pinned buffer
-    the host writes (or reads) the values once, in whatever layout its array has, and the transfer
-    runs on the stream. A buffer is written again only after its previous transfer has finished.
-    The buffers start as parts of one pinned allocation of ``numel`` values each (a pinned
-    allocation costs about half a millisecond whatever its size); a larger array replaces its own.
-    """
+def _pinned(torch, numel: int):
+    return torch.empty(numel, dtype=torch.float64, pin_memory=True)
 
-    def __init__(self, torch, numel: int, count: int = 4) -> None:
-        self._torch = torch
-        self._numel = numel
-        self._ring = [[None, torch.cuda.Event()] for _ in range(count)]
-        self._next = 0
 
-    def _buffer(self, n: int):
-        slot = self._ring[self._next]
-        self._next = (self._next + 1) % len(self._ring)
-        slot[1].synchronize()
-        if slot[0] is None and n <= self._numel:
-            whole = self._torch.empty(len(self._ring) * self._numel, dtype=self._torch.float64,
-                                      pin_memory=True)
-            for one, part in zip(self._ring, whole.split(self._numel)):
-                one[0] = part if one[0] is None else one[0]
-        if slot[0] is None or slot[0].numel() < n:
-            slot[0] = self._torch.empty(n, dtype=self._torch.float64, pin_memory=True)
-        return slot[0][:n], slot[1]
+def _to_device(torch, array: np.ndarray, dtype, dst=None):
+    """``array`` as ``dtype`` in Fortran order on the device (flat float64, in ``dst`` if given)."""
+    n = array.size * (2 if dtype is complex else 1)
+    buf = _pinned(torch, n)
+    buf.numpy().view(dtype).reshape(array.shape, order="F")[...] = array
+    if dst is None:
+        dst = torch.empty(n, dtype=torch.float64, device="cuda")
+    dst.copy_(buf, non_blocking=True)
+    return dst
 
-    def to_device(self, array: np.ndarray, dtype, dst=None):
-        """``array`` as ``dtype`` in Fortran order on the device (flat float64, in ``dst`` if given)."""
-        n = array.size * (2 if dtype is complex else 1)
-        buf, event = self._buffer(n)
-        buf.numpy().view(dtype).reshape(array.shape, order="F")[...] = array
-        if dst is None:
-            dst = self._torch.empty(n, dtype=self._torch.float64, device="cuda")
-        dst.copy_(buf, non_blocking=True)
-        event.record()
-        return dst
 
-    def to_host(self, src, dtype, out: np.ndarray) -> np.ndarray:
-        """Flat float64 device values, as ``dtype`` in Fortran order, into ``out``."""
-        buf, event = self._buffer(src.numel())
-        buf.copy_(src, non_blocking=True)
-        event.record()
-        event.synchronize()
-        out[...] = buf.numpy().view(dtype).reshape(out.shape, order="F")
-        return out
+def _to_host(torch, src, dtype, out: np.ndarray) -> np.ndarray:
+    """Flat float64 device values, as ``dtype`` in Fortran order, into ``out``."""
+    buf = _pinned(torch, src.numel())
+    buf.copy_(src, non_blocking=True)
+    torch.cuda.current_stream().synchronize()
+    out[...] = buf.numpy().view(dtype).reshape(out.shape, order="F")
+    return out
 
 
 class SpatialDiscretization:
@@ -167,7 +148,6 @@ class SpatialDiscretization:
         self._dJF_u = torch.zeros(8 * N, **f64)
         self._dJF_x = torch.zeros(8 * N, **f64)
         self._mirrors: dict[str, np.ndarray] = {}
-        self._staging = _Staging(torch, 8 * max(nc, nv))  # a complex state, or two of vertices
         self._lu_stale = True
         self.set_free_stream_state()
 
@@ -310,18 +290,18 @@ class SpatialDiscretization:
         return _lib.single_batch(inst)
 
     def _upload(self, velocities: bool = True) -> None:
-        self._staging.to_device(self._vertices.real, float, self._dX)
+        _to_device(self._torch, self._vertices.real, float, self._dX)
         if velocities:
-            self._staging.to_device(self._velocities.real, float, self._dV)
-        self._staging.to_device(self._states.real, float, self._dU)
+            _to_device(self._torch, self._velocities.real, float, self._dV)
+        _to_device(self._torch, self._states.real, float, self._dU)
 
     def _cvec(self, array: np.ndarray):
         """Complex host array -> interleaved device float64 vector."""
-        return self._staging.to_device(np.asarray(array), complex)
+        return _to_device(self._torch, np.asarray(array), complex)
 
-    def _store(self, out: np.ndarray, dev, shape: tuple) -> np.ndarray:
+    def _store(self, out: np.ndarray, dev) -> np.ndarray:
         """Interleaved complex device vector -> host array ``out`` of that shape."""
-        return self._staging.to_host(dev, complex, out)
+        return _to_host(self._torch, dev, complex, out)
 
     def _stream(self) -> int:
         return self._torch.cuda.current_stream().cuda_stream
@@ -334,19 +314,19 @@ class SpatialDiscretization:
     def set_free_stream_state(self) -> None:
         """Sets ``states`` to free-stream (core.py:265-268)."""
         self._call("eb_set_free_stream_state", ptr(self._dU))
-        self._staging.to_host(self._dU, float, self._states)
+        _to_host(self._torch, self._dU, float, self._states)
 
     def compute_odes(self) -> None:
         """Computes ``odes`` from ``states``, ``vertices`` and ``velocities`` (core.py:270-276)."""
         self._upload()
         self._call("eb_compute_odes", ptr(self._dX), ptr(self._dV), ptr(self._dU), ptr(self._dR))
-        self._staging.to_host(self._dR, float, self._odes)
+        _to_host(self._torch, self._dR, float, self._odes)
 
     def compute_forces(self) -> None:
         """Computes ``forces`` from ``states`` and ``vertices`` (core.py:601-608)."""
         self._upload(velocities=False)
         self._call("eb_compute_forces", ptr(self._dX), ptr(self._dU), ptr(self._dF), None)
-        self._staging.to_host(self._dF, float, self._forces)
+        _to_host(self._torch, self._dF, float, self._forces)
 
     def linearize(self) -> None:
         """Computes the Jacobians on the device (core.py:278-292)."""
@@ -370,7 +350,7 @@ class SpatialDiscretization:
         self._call(name, ptr(jac), ptr(x), ptr(y))
         if out is None:
             out = np.empty(out_shape, dtype=complex, order="F")
-        return self._store(out, y, out_shape)
+        return self._store(out, y)
 
     def apply_odes_wrt_mach_fwd(self, d_mach: np.ndarray, d_odes: np.ndarray | None = None):
         """``dR/dMa . dMa`` (core.py:294-319)."""
@@ -547,7 +527,7 @@ class SpatialDiscretization:
         self._call(apply_rev, ptr(J_im), ptr(w), ptr(y_im))
         y_re[0::2] -= y_im[1::2]  # y_re + i y_im
         y_re[1::2] += y_im[0::2]
-        return self._store(np.empty(out_shape, dtype=complex, order="F"), y_re, out_shape)
+        return self._store(np.empty(out_shape, dtype=complex, order="F"), y_re)
 
     def _grad_out(self, out, shape, result):
         if out is not None:
@@ -778,4 +758,4 @@ class SpatialDiscretization:
         dcp = torch.empty(2 * self._nc(), dtype=torch.float64, device="cuda")
         self._call("eb_apply_pressure_coefficients_wrt_states_fwd", ptr(self._dU),
                    ptr(self._cvec(d_states)), ptr(dcp))
-        return self._store(d_pressure_coefficients, dcp, shape)
+        return self._store(d_pressure_coefficients, dcp)
