@@ -328,6 +328,11 @@ int eb_fp64_fma_probe(int64_t iterations, int sms, double* sink, void* stream);
  * mma.sync.m8n8k4.f64 (512 flops each). No counterpart in the reference. */
 int eb_fp64_mma_probe(int64_t iterations, int sms, double* sink, void* stream);
 
+/* The kernels' own scalar operations, for comparison with the built-in ones: out (4 x n) receives
+ * a[i] / b[i], 1 / b[i] and sqrt(b[i]) as the stencil kernels form them, and 1 / b[i] as the ring
+ * LU's pivot steps do (for normal b below 2^1022). No counterpart in the reference. */
+int eb_scalar_probe(int64_t n, const double* a, const double* b, double* out, void* stream);
+
 /* The ring LU's dense product as a library call: C_z = alpha A_z B_z + beta C_z for z < batch,
  * complex double (interleaved), column-major, no transposes, A_z = A + z stride_a complex
  * elements (likewise B, C); alpha and beta real, beta == 0 does not read C. variant: -1 the

@@ -33,17 +33,24 @@ __device__ __forceinline__ cuDoubleComplex fmsub(cuDoubleComplex a, cuDoubleComp
   return make_cuDoubleComplex(fma(-a.x, b.x, fma(a.y, b.y, c.x)),
                               fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
 }
-// 1 / a of a normal number: the hardware's approximation (error e below 2^-19) and one step of
-// the third-order Newton iteration y (1 + e + e^2), without the branches of a division, so that
-// it runs in the shadow of the pivot search.
+// 1 / a of a normal number below 2^1022: two Newton-Raphson steps y <- y + y (1 - a y), each of which
+// squares the relative error, from the hardware's approximation (2^-19 or better), without the
+// branches of a division, so that it runs in the shadow of the pivot search. eliminate() forms
+// the reciprocals of other pivots again, by division.
 __device__ __forceinline__ double recip(double a) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
-  const double e = fma(-a, y, 1.0);
-  return fma(y, fma(e, e, e), y);
+  y = fma(y, fma(-a, y, 1.0), y);
+  return fma(y, fma(-a, y, 1.0), y);
 }
 __device__ __forceinline__ cuDoubleComplex recip(cuDoubleComplex a) {
   const double d = recip(a.x * a.x + a.y * a.y);
+  return make_cuDoubleComplex(a.x * d, -a.y * d);
+}
+// 1 / a by division.
+__device__ __forceinline__ double recip_any(double a) { return 1.0 / a; }
+__device__ __forceinline__ cuDoubleComplex recip_any(cuDoubleComplex a) {
+  const double d = 1.0 / (a.x * a.x + a.y * a.y);
   return make_cuDoubleComplex(a.x * d, -a.y * d);
 }
 // a non-negative number ordered like the modulus
@@ -144,8 +151,9 @@ __device__ __forceinline__ bool eliminate(StepShared<T, NC, Warps>& S, T (&a)[RO
       return false;
     }
     const int w = (prow % nt) >> 5;  // the warp that holds row prow
-    const T inv = S.cand_inv[par][w];
     const T* row = S.cand[par][w];
+    T inv = S.cand_inv[par][w];
+    if (size < 0x00100000u || size >= 0x7FD00000u) inv = recip_any(row[0]);
     if (tid == 0) S.own[jj] = prow;
     T f[ROWS];
 #pragma unroll

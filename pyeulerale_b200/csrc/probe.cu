@@ -1,15 +1,17 @@
-// FP64 throughput probes: the denominators of the FP64 roofline fractions the bench reports for
+// Probes. FP64 throughput: the denominators of the FP64 roofline fractions the bench reports for
 // the stencil kernels (DFMA) and the dense ring-LU products (DMMA); the HBM denominator is a
 // measured copy bandwidth, these are its FP64 counterparts. In the DFMA probe every thread runs
 // kChains independent chains of fused multiply-adds, enough to cover the pipeline latency, on a
 // grid of eight 256-thread CTAs per SM; the chains' sum goes to `sink` so that no work is
-// optimised away.
+// optimised away. And the scalar operations that replace built-in ones, for comparison with those.
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "../../include/euler_b200.h"
+#include "gj_step.cuh"
+#include "scalar.cuh"
 
 namespace eb {
 
@@ -59,6 +61,18 @@ __global__ void __launch_bounds__(256) k_fp64_mma(int64_t iterations, double* si
   if (s == 12345.678) sink[0] = s;  // practically never true; keeps the accumulators live
 }
 
+// The stencil kernels' quotient, reciprocal and root and the ring LU's pivot reciprocal.
+__global__ void __launch_bounds__(256) k_scalars(int64_t n, const double* a, const double* b,
+                                                 double* out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    out[i] = quot_(a[i], b[i]);
+    out[n + i] = recip_(b[i]);
+    out[2 * n + i] = sqrt_(b[i]);
+    out[3 * n + i] = rl::recip(b[i]);
+  }
+}
+
 }  // namespace
 }  // namespace eb
 
@@ -73,4 +87,11 @@ extern "C" int eb_fp64_fma_probe(int64_t iterations, int sms, double* sink, void
   eb::k_fp64_fma<<<8 * sms, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       iterations, 0.999999999, 1e-9, sink);
   return eb::check_launch("fma probe");
+}
+
+extern "C" int eb_scalar_probe(int64_t n, const double* a, const double* b, double* out,
+                               void* stream) {
+  if (n < 1 || !a || !b || !out) return eb::fail(EB_ERR_ARG, "scalar probe: bad arguments");
+  eb::k_scalars<<<592, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, a, b, out);
+  return eb::check_launch("scalar probe");
 }
