@@ -54,7 +54,6 @@ __device__ __forceinline__ void store_release(unsigned long long* p, unsigned lo
   asm volatile("fence.acq_rel.gpu;\n st.release.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v)
                : "memory");
 }
-constexpr int kSub = 4;  // steps published together
 // The word published for a group of kSub steps: the launch's epoch, whether the steps found
 // their pivots, and the pivot rows (ten bits each).
 __device__ __forceinline__ unsigned long long pack(int epoch, bool ok, const int* piv) {
@@ -72,12 +71,13 @@ __device__ __forceinline__ int row_of(unsigned long long w, int k) {
 }
 
 template <class T, int NC, int Warps>
-struct Shared {
+struct alignas(16) Shared {  // (the staged columns behind it are copied in pairs of doubles)
   StepShared<T, NC, Warps> step;
   T rows[kSub][NC];              // the pivot rows of a group of steps in this CTA's columns
   unsigned long long word;       // the group's published word (0: the wait gave up)
-  int ok;                        // its own steps found their pivots so far
-  int stop;
+  int bad;                       // the group of its own steps that met no pivot (else kGroups)
+  int failed;                    // info at the start: an earlier block of the system failed
+  int ended;                     // the work ended before its own steps
 };
 
 // Grid: (ceil(K / NC), systems); block: the compute threads, ceil(K / ROWS) rounded up to whole
@@ -106,23 +106,26 @@ __global__ void __launch_bounds__(Threads + 32, 1)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int j = blockIdx.x, panels = gridDim.x, c0 = j * NC, width = min(NC, K - c0);
   if (tid == 0) {  // info may be set during this launch: one thread's view is the CTA's
-    S.stop = *info;
-    S.ok = 1;
+    S.failed = *info;
+    S.bad = kGroups;
+    S.ended = 0;
   }
   __syncthreads();
-  if (S.stop != 0) return;
+  if (S.failed != 0) return;
   if (warp == kWarps) {  // the publishing warp: copies the groups from shared memory
     const int words = kSub * K * (int)sizeof(T) / 16;
     for (int q = 0; q < width / kSub; ++q) {
       bar_sync(kGroupBar + q, nt + 32);
-      if (S.stop != 0) return;
+      if (S.ended != 0) return;
       const double2* from = reinterpret_cast<const double2*>(stage + (size_t)K * kSub * q);
       double2* to = reinterpret_cast<double2*>(pub + (size_t)K * (c0 + kSub * q));
 #pragma unroll 8
       for (int i = lane; i < words; i += 32) __stcg(to + i, from[i]);
       __syncwarp();
-      if (lane == 0) store_release(flags + c0 / kSub + q, pack(epoch, S.ok != 0, S.step.own + kSub * q));
-      if (S.ok == 0) return;
+      // the compute threads may be in a later group by now: its failure leaves q < bad as it is
+      const bool ok = q < *(volatile int*)&S.bad;
+      if (lane == 0) store_release(flags + c0 / kSub + q, pack(epoch, ok, S.step.own + kSub * q));
+      if (!ok) return;
     }
     bar_arrive(kGroupBar + kGroups, nt + 32);
     return;
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(Threads + 32, 1)
           },
           [&](int jj) {
             if (tid == 0) {
-              S.ok = 0;
+              S.bad = jj / kSub;
               atomicExch(info, 1);
             }
             bar_arrive(kGroupBar + jj / kSub, nt + 32);
@@ -182,9 +185,11 @@ __global__ void __launch_bounds__(Threads + 32, 1)
       }
       bar_sync(kStepBar, nt);
       const unsigned long long word = S.word;
-      if (word == 0ull) {  // the publishing warp of this CTA ends as well
-        if (tid == 0) S.stop = 1;
-        for (int o = 0; p < j && o < 1; ++o) bar_arrive(kGroupBar, nt + 32);
+      if (word == 0ull) {
+        if (p < j) {  // the publishing warp waits for this CTA's first group: it ends as well
+          if (tid == 0) S.ended = 1;
+          bar_arrive(kGroupBar, nt + 32);
+        }
         return;
       }
       T g[ROWS][kSub];

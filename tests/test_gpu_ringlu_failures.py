@@ -1,0 +1,40 @@
+"""Failing factorisations of the ring LU: zero pivots at any step of any CTA's columns (GPU)."""
+
+from __future__ import annotations
+
+import pytest
+
+from helpers import crandn
+from test_gpu_ringlu_sizes import _setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("step", [0, 3, 4, 5, 6, 9, 14, 15, 16, 22, 63, 110, 159])
+@pytest.mark.parametrize("shift", [0.0, 0.5j])
+def test_zero_pivot(cuda, step, shift):
+    """The first ring's block is the identity but for a zero pivot at one step: a zero column, or at a
+    complex shift i w the second column of [[0, -w], [w, 0]]. The failing step is published, so the
+    status is that of a singular block, not that of a wait that ran out."""
+    from pyeulerale_b200 import _lib, solver
+
+    M, N = 4, 40
+    if shift and step % 4 == 0:
+        step += 1  # the pair's two columns are in one cell
+    gpu, J, rng = _setup(cuda, M, N, 4)
+    bad = cuda.zeros_like(J)
+    own = bad[:16 * M * N].reshape(N, M, 4, 4)  # [cell, ring, column, row] of the own-cell blocks
+    own[:] = cuda.eye(4, dtype=cuda.float64, device="cuda")
+    n, k = divmod(step, 4)
+    own[n, 0, k] = 0.0
+    if shift:
+        w = shift.imag
+        own[n, 0, k - 1] = 0.0
+        own[n, 0, k, k - 1], own[n, 0, k - 1, k] = -w, w
+    lu = solver.RingLU(gpu.batch, tol=1e-10)
+    with pytest.raises(_lib.EulerB200Error) as e:
+        lu.factor(bad, shift)
+    assert e.value.code == _lib.EB_ERR_NAN
+    lu.factor(J, shift)
+    _, rel = lu.solve(gpu.dev(crandn(rng, (4, M, N))))
+    assert rel <= 1e-10
