@@ -276,7 +276,7 @@ int64_t eb_ringlu_workspace_bytes(int M, int N);
 /* Factors A = J - shift I (J: d(odes)/d(states) of the single instance in `b`) by block
  * Gaussian elimination over the radial rings, pivoting inside each ring block. The factors
  * serve eb_ringlu_solve for both A and A^H. Synchronises `stream`; EB_ERR_NAN if a ring block
- * is singular. */
+ * is singular, EB_ERR_CUDA if a CTA's wait for another one's pivots ran out. */
 int eb_ringlu_factor(const eb_batch* b, const double* J, double shift_re, double shift_im,
                      void* workspace, int64_t workspace_bytes, void* stream);
 
@@ -333,6 +333,11 @@ int eb_fp64_mma_probe(int64_t iterations, int sms, double* sink, void* stream);
  * LU's pivot steps do (for normal b below 2^1022). No counterpart in the reference. */
 int eb_scalar_probe(int64_t n, const double* a, const double* b, double* out, void* stream);
 
+/* The wait of the ring LU's inversion, on a flag that nothing sets: polls it `polls` times (1 to 2^22)
+ * and returns what a factorisation returns then. scratch: 16 bytes of device memory. Synchronises
+ * `stream`. No counterpart in the reference. */
+int eb_ringlu_wait_probe(int polls, void* scratch, void* stream);
+
 /* The ring LU's dense product as a library call: C_z = alpha A_z B_z + beta C_z for z < batch,
  * complex double (interleaved), column-major, no transposes, A_z = A + z stride_a complex
  * elements (likewise B, C); alpha and beta real, beta == 0 does not read C. variant: -1 the
@@ -369,8 +374,9 @@ int64_t eb_ptc_workspace_bytes(int M, int N, int max_steps);
  * CUDA graph; the control values stay on the device and the host reads one stop flag per step.
  * On return U is the final state, R and J its residual and Jacobian (of the state before the
  * last update when max_steps ends the loop), history (HOST, 2 max_steps) the pairs (max|R|,
- * rel) of the steps and *n_steps their count. EB_ERR_NAN if rel became non-finite or a ring block was singular;
- * reaching max_steps is not an error (as in the example driver). Synchronises `stream`. */
+ * rel) of the steps and *n_steps their count. EB_ERR_NAN if rel became non-finite or a ring block
+ * was singular; reaching max_steps is not an error (as in the example driver). Synchronises
+ * `stream`. */
 int eb_ptc_run(const eb_batch* b, const double* X, const double* V, double* U, double* R,
                double* J, double ser, double rtol, int max_steps, void* workspace,
                int64_t workspace_bytes, double* history, int* n_steps, void* stream);

@@ -112,6 +112,7 @@ _SIGNATURES: dict[str, list] = {
     "eb_fp64_fma_probe": ["i64", "i", "p", "s"],
     "eb_fp64_mma_probe": ["i64", "i", "p", "s"],
     "eb_scalar_probe": ["i64", "p", "p", "p", "s"],
+    "eb_ringlu_wait_probe": ["i", "p", "s"],
     "eb_zgemm_strided_batched": ["i", "i", "i", "d", "p", "i", "i64", "p", "i", "i64", "d", "p",
                                  "i", "i64", "i", "i", "s"],
     "eb_odes_wrt_mach_dir": ["b", "p", "p", "p", "i", "p", "p", "p", "s"],

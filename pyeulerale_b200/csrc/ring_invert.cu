@@ -15,8 +15,8 @@
 // K = 512 took 1150 us, of K = 128 about 300 us, complex.
 //
 // The waits are polls of a flag in global memory by CTAs of one cooperative launch (all are
-// resident); each gives up after kPollLimit polls, records it in info and ends the launch's
-// work on that system.
+// resident); each gives up after kPollLimit polls, records it in info (kRanOut) and ends the
+// launch's work on that system.
 
 #include "gj_step.cuh"
 #include "ring_invert.cuh"
@@ -68,6 +68,22 @@ __device__ __forceinline__ bool is_epoch(unsigned long long w, int epoch) {
 __device__ __forceinline__ bool is_ok(unsigned long long w) { return (w >> (10 * kSub)) & 1ull; }
 __device__ __forceinline__ int row_of(unsigned long long w, int k) {
   return (int)((w >> (10 * (kSub - 1 - k))) & 0x3FFull);
+}
+
+// Polls until the flag holds a word of this launch; false once `limit` polls have not seen one.
+__device__ __forceinline__ bool wait_word(const unsigned long long* flag, int epoch, int limit,
+                                          unsigned long long& w) {
+  for (int n = 0; n < limit; ++n) {
+    w = load_acquire(flag);
+    if (is_epoch(w, epoch)) return true;
+  }
+  return false;
+}
+
+// Waits on a flag that nothing sets.
+__global__ void k_wait_probe(const unsigned long long* flag, int* info, int polls) {
+  unsigned long long w;
+  if (!wait_word(flag, 1, polls, w)) atomicCAS(info, 0, kRanOut);
 }
 
 template <class T, int NC, int Warps>
@@ -161,7 +177,7 @@ __global__ void __launch_bounds__(Threads + 32, 1)
           [&](int jj) {
             if (tid == 0) {
               S.bad = jj / kSub;
-              atomicExch(info, 1);
+              atomicCAS(info, 0, kSingular);
             }
             bar_arrive(kGroupBar + jj / kSub, nt + 32);
           });
@@ -172,15 +188,11 @@ __global__ void __launch_bounds__(Threads + 32, 1)
     for (int q = 0; q < groups; ++q) {
       const int g0 = p * NC + q * kSub;  // the group's first step
       if (warp == 0) {
-        unsigned long long w = 0ull;
-        int n = 0;
-        for (; n < kPollLimit; ++n) {
-          w = load_acquire(flags + g0 / kSub);
-          if (is_epoch(w, epoch)) break;
-        }
+        unsigned long long w;
+        const bool came = wait_word(flags + g0 / kSub, epoch, kPollLimit, w);
         if (lane == 0) {
-          if (n == kPollLimit) atomicExch(info, 2);
-          S.word = n < kPollLimit && is_ok(w) ? w : 0ull;
+          if (!came) atomicCAS(info, 0, kRanOut);
+          S.word = came && is_ok(w) ? w : 0ull;
         }
       }
       bar_sync(kStepBar, nt);
@@ -304,5 +316,27 @@ int ring_invert(int K, int systems, char* base, int64_t stride, const InvertAt& 
                     : run(launch<cuDoubleComplex, 8, 2, 512>);
 }
 
+int info_status(int info) {
+  if (info == kRanOut)
+    return fail(EB_ERR_CUDA, "ringlu: an inversion's wait for another CTA's pivots ran out");
+  return info ? fail(EB_ERR_NAN, "ringlu: singular or non-finite ring block") : EB_OK;
+}
+
 }  // namespace rl
 }  // namespace eb
+
+extern "C" int eb_ringlu_wait_probe(int polls, void* scratch, void* stream) {
+  using namespace eb;
+  if (polls < 1 || polls > rl::kPollLimit || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 15))
+    return fail(EB_ERR_ARG, "wait probe: bad arguments");
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto* flag = static_cast<unsigned long long*>(scratch);
+  int* info = reinterpret_cast<int*>(flag + 1);
+  int seen = 0;
+  if (cudaMemsetAsync(scratch, 0, 16, st) != cudaSuccess) return check_launch("wait probe");
+  rl::k_wait_probe<<<1, 32, 0, st>>>(flag, info, polls);
+  if (cudaMemcpyAsync(&seen, info, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return check_launch("wait probe");
+  return rl::info_status(seen);
+}

@@ -16,8 +16,12 @@ struct InvertAt {
   size_t out;    // the inverse, complex (may be `in`)
   size_t real;   // the inverse again as real numbers (real scalar type only)
   size_t flags;  // uint64[kInvertFlags], zero before the first launch of a factorisation
-  size_t info;   // int: 0, or non-zero once a pivot was zero or not finite
+  size_t info;   // int: 0, or the first of the states below
 };
+constexpr int kSingular = 1;  // a pivot was zero or not finite
+constexpr int kRanOut = 2;    // a wait for another CTA's pivots ran out
+// The EB_* status of an info value, with its error text.
+int info_status(int info);
 constexpr int kInvertFlags = 256;  // K / 4 groups of steps at most
 
 // Inverts the block of every system (workspaces at base + stride s), of order K (at most 1024, a

@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
   }
   const bool ok = eliminate(S, a, left, pos, NB, j0, K, tid, [](int) {}, [](int) {});
   if (!ok) {
-    if (tid == 0) atomicExch(info, 1);
+    if (tid == 0) atomicExch(info, kSingular);
     return;
   }
   __syncthreads();
@@ -1199,7 +1199,7 @@ int eb_ringlu_factor_many(const eb_batch* b, const double* const* J, int n_shift
     return check_launch("ringlu info");
   if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch("ringlu info");
   for (int i : info)
-    if (i != 0) return fail(EB_ERR_NAN, "ringlu: singular or non-finite ring block");
+    if ((rc = info_status(i)) != EB_OK) return rc;
   return EB_OK;
 }
 
@@ -1303,7 +1303,7 @@ struct PtcCtl {
   int run;                       // the loop had not stopped when this step began
   int done;                      // stopped: rel <= rtol, rel not finite, or a singular block
   int steps;                     // relative norms recorded
-  int status;                    // EB_OK or EB_ERR_NAN
+  int status;                    // EB_OK, EB_ERR_NAN or EB_ERR_CUDA (a wait ran out)
 };
 
 struct PtcLayout {
@@ -1421,14 +1421,14 @@ __global__ void __launch_bounds__(128) k_ptc_refine_rhs(int M, int N, const doub
   }
 }
 
-// U += Re(xs + correction); a singular ring block (LU info) stops the loop instead
+// U += Re(xs + correction); a failed factorisation (LU info) stops the loop instead
 __global__ void k_ptc_update(int M, int N, const cuDoubleComplex* x_ring, const double* xs,
                              const int* lu_info, PtcCtl* c, double* U) {
   if (c->done) return;
   if (*lu_info != 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       c->done = 1;
-      c->status = EB_ERR_NAN;
+      c->status = *lu_info == kRanOut ? EB_ERR_CUDA : EB_ERR_NAN;
     }
     return;
   }
@@ -1626,6 +1626,7 @@ int eb_ptc_run(const eb_batch* b, const double* X, const double* V, double* U, d
                           cudaMemcpyDeviceToHost) != cudaSuccess)
     return check_launch("ptc history");
   *n_steps = n;
+  if (hc.status == EB_ERR_CUDA) return info_status(kRanOut);
   if (hc.status != EB_OK)
     return fail(hc.status, "ptc: non-finite residual or singular ring block");
   return EB_OK;

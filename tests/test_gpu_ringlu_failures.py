@@ -1,4 +1,5 @@
-"""Failing factorisations of the ring LU: zero pivots at any step of any CTA's columns (GPU)."""
+"""Failing factorisations of the ring LU: zero pivots at any step of any CTA's columns, and a wait that
+runs out (GPU)."""
 
 from __future__ import annotations
 
@@ -38,3 +39,13 @@ def test_zero_pivot(cuda, step, shift):
     lu.factor(J, shift)
     _, rel = lu.solve(gpu.dev(crandn(rng, (4, M, N))))
     assert rel <= 1e-10
+
+
+def test_wait_runs_out(cuda):
+    from pyeulerale_b200 import _lib
+
+    scratch = cuda.zeros(2, dtype=cuda.int64, device="cuda")
+    with pytest.raises(_lib.EulerB200Error) as e:
+        _lib.call("eb_ringlu_wait_probe", 1000, scratch.data_ptr(), None)
+    assert e.value.code == _lib.EB_ERR_CUDA and "ran out" in str(e.value)
+    cuda.cuda.synchronize()
