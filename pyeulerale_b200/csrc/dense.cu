@@ -795,8 +795,10 @@ int launch_sweep_multi(int n, char* base, int64_t stride, char* vectors, int64_t
                        int workspaces, const int* zmap, const int* n_active,
                        const SweepTerms& terms, cudaStream_t st) {
   const int smem = (int)sizeof(double2) * NR * (n < kChunk ? n : kChunk);
-  if (cudaFuncSetAttribute(k_sweep_multi<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
+  // the limit is the kernel's, not the launch's: always the most it can need, so that another
+  // thread's smaller sweep does not lower it under this launch
+  if (cudaFuncSetAttribute(k_sweep_multi<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(double2) * NR * kChunk) != cudaSuccess)
     return check_launch("sweep attribute");
   if (launch_dependent(k_sweep_multi<NR>, dim3((n + 7) / 8 * terms.n, workspaces), 256, smem, st, n,
                        (const char*)base, stride, vectors, vstride, zmap, n_active, terms) !=

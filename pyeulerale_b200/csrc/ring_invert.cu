@@ -269,9 +269,14 @@ int launch(int K, int systems, char* base, int64_t stride, const InvertAt& at, i
            cudaStream_t st) {
   auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
   constexpr int threads = Threads + 32;
-  const int smem = (int)(sizeof(Shared<T, NC, Threads / 32>) + sizeof(T) * NC * (size_t)K);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
+  auto bytes = [](int k) {
+    return (int)(sizeof(Shared<T, NC, Threads / 32>) + sizeof(T) * NC * (size_t)k);
+  };
+  const int smem = bytes(K);
+  // the limit is the kernel's, not the launch's: always the most this variant can need, so that
+  // another thread's smaller block does not lower it under this launch
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           bytes(ROWS * Threads)) != cudaSuccess)
     return check_launch("ring_invert attribute");
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -1,7 +1,9 @@
-"""Failing factorisations of the ring LU: zero pivots at any step of any CTA's columns, and a wait that
-runs out (GPU)."""
+"""Failing factorisations of the ring LU: zero pivots at any step of any CTA's columns, a wait that runs
+out, and threads that factor grids of different sizes (GPU)."""
 
 from __future__ import annotations
+
+from concurrent.futures import ThreadPoolExecutor
 
 import pytest
 
@@ -49,3 +51,26 @@ def test_wait_runs_out(cuda):
         _lib.call("eb_ringlu_wait_probe", 1000, scratch.data_ptr(), None)
     assert e.value.code == _lib.EB_ERR_CUDA and "ran out" in str(e.value)
     cuda.cuda.synchronize()
+
+
+def test_threads_of_different_sizes(cuda, monkeypatch):
+    """Two kernels serve ranges of sizes: neither thread's factorisations and sweeps are refused because
+    of the other's smaller ones."""
+    from pyeulerale_b200 import solver
+
+    monkeypatch.setenv("EB_RINGLU_GRAPHS", "0")
+    jobs = []
+    for N in (66, 128, 70, 120):
+        gpu, J, rng = _setup(cuda, 5, N, N)
+        jobs.append((solver.RingLU(gpu.batch, tol=1e-10), J, gpu.dev(crandn(rng, (4, 5, N)))))
+
+    def work(job):
+        lu, J, rhs = job
+        worst = 0.0
+        for k in range(40):
+            lu.factor(J, 0.3j)
+            worst = max(worst, lu.solve(rhs)[1])
+        return worst
+
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        assert max(pool.map(work, jobs)) <= 1e-10
