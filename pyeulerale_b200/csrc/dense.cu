@@ -479,7 +479,7 @@ int zgemm_nn_batched(int M, int N, int K, double alpha, const cuDoubleComplex* A
 int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
               int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st,
               int gap0, int gap1) {
-  if (gap0 % kBN != 0 || gap1 % kBN != 0 || gap1 < gap0 || gap1 > N)
+  if (gap0 % kBN != 0 || gap1 < gap0 || gap1 > N)
     return fail(EB_ERR_ARG, "zgemm: bad gap");
   if (gap1 - gap0 == N) return 0;
   const Operands ops{base, base, base, stride, stride, stride, set, gap0, gap1};

@@ -35,7 +35,7 @@ struct Products {
   }
 };
 // C = alpha A B + beta C for every entry of every workspace (complex); the columns [gap0, gap1) of
-// C, multiples of 64, are left out.
+// C, gap0 a multiple of 64, are left out.
 int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
               int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st,
               int gap0 = 0, int gap1 = 0);

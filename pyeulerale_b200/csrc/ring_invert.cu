@@ -264,37 +264,65 @@ __global__ void __launch_bounds__(Threads + 32, 1)
   }
 }
 
+// The kernel variant of a block order, and the launches with it.
 template <class T, int NC, int ROWS, int Threads>
-int launch(int K, int systems, char* base, int64_t stride, const InvertAt& at, int epoch,
-           cudaStream_t st) {
-  auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
-  constexpr int threads = Threads + 32;
-  auto bytes = [](int k) {
-    return (int)(sizeof(Shared<T, NC, Threads / 32>) + sizeof(T) * NC * (size_t)k);
-  };
-  const int smem = bytes(K);
-  // the limit is the kernel's, not the launch's: always the most this variant can need, so that
-  // another thread's smaller block does not lower it under this launch
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes(ROWS * Threads)) != cudaSuccess)
-    return check_launch("ring_invert attribute");
-  int dev = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
-    return check_launch("ring_invert occupancy");
-  const int panels = (K + NC - 1) / NC;
-  const int fit = sms * per_sm / panels;  // systems whose CTAs are resident together
-  if (fit < 1) return fail(EB_ERR_CUDA, "ring_invert: the device cannot hold one block's CTAs");
-  for (int z0 = 0; z0 < systems; z0 += fit) {
-    const dim3 grid(panels, std::min(fit, systems - z0));
-    void* args[] = {(void*)&K,      (void*)&z0, (void*)&base,
-                    (void*)&stride, (void*)&at, (void*)&epoch};
-    if (cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(threads), args, smem, st) !=
-        cudaSuccess)
-      return check_launch("ring_invert");
+struct Variant {
+  static constexpr int kThreads = Threads + 32;
+  static int bytes(int K) {
+    return (int)(sizeof(Shared<T, NC, Threads / 32>) + sizeof(T) * NC * (size_t)K);
   }
-  return EB_OK;
+  // The number of systems whose CTAs are resident together, or a negative EB_* status.
+  static int resident(int K) {
+    auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
+    // the limit is the kernel's, not the launch's: always the most this variant can need, so that
+    // another thread's smaller block does not lower it under this launch
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             bytes(ROWS * Threads)) != cudaSuccess)
+      return check_launch("ring_invert attribute");
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, bytes(K)) !=
+            cudaSuccess)
+      return check_launch("ring_invert occupancy");
+    const int fit = sms * per_sm / ((K + NC - 1) / NC);
+    return fit < 1 ? fail(EB_ERR_CUDA, "ring_invert: the device cannot hold one block's CTAs") : fit;
+  }
+  static int launch(int K, int systems, char* base, int64_t stride, const InvertAt& at, int epoch,
+                    cudaStream_t st) {
+    auto kernel = k_ring_invert<T, NC, ROWS, Threads>;
+    const int fit = resident(K);
+    if (fit < 0) return fit;
+    for (int z0 = 0; z0 < systems; z0 += fit) {
+      const dim3 grid((K + NC - 1) / NC, std::min(fit, systems - z0));
+      void* args[] = {(void*)&K,      (void*)&z0, (void*)&base,
+                      (void*)&stride, (void*)&at, (void*)&epoch};
+      if (cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(kThreads), args, bytes(K),
+                                      st) != cudaSuccess)
+        return check_launch("ring_invert");
+    }
+    return EB_OK;
+  }
+};
+
+// Calls run with the variant for blocks of order K. Rows per thread: 128 compute threads (one warp per
+// scheduler: the step's latency grows with the warps that share one) as long as a thread's rows
+// fit its registers; above K = 512 more threads, which caps them (K = 1024 real: 1174 us at four
+// rows, 1262 at two; complex: 2246 us at two rows and 512 threads, 2453 at four and 256).
+template <class Run>
+int with_variant(int K, bool real, Run run) {
+  using Z = cuDoubleComplex;
+  if (real)
+    return K <= 128   ? run(Variant<double, 16, 1, 128>())
+           : K <= 256 ? run(Variant<double, 16, 2, 128>())
+           : K <= 512 ? run(Variant<double, 16, 4, 128>())
+           : K <= 768 ? run(Variant<double, 16, 3, 256>())
+                      : run(Variant<double, 16, 4, 256>());
+  return K <= 128   ? run(Variant<Z, 8, 1, 128>())
+         : K <= 256 ? run(Variant<Z, 8, 2, 128>())
+         : K <= 512 ? run(Variant<Z, 8, 4, 128>())
+         : K <= 768 ? run(Variant<Z, 8, 3, 256>())
+                    : run(Variant<Z, 8, 2, 512>());
 }
 
 }  // namespace
@@ -303,22 +331,13 @@ int ring_invert(int K, int systems, char* base, int64_t stride, const InvertAt& 
                 bool real, cudaStream_t st) {
   if (K < 4 || K > kMaxRows || K % 4 != 0 || systems < 1 || epoch < 1)
     return fail(EB_ERR_ARG, "ring_invert: bad sizes");
-  auto run = [&](auto kernel) { return kernel(K, systems, base, stride, at, epoch, st); };
-  // Rows per thread: 128 compute threads (one warp per scheduler: the step's latency grows with the
-  // warps that share one) as long as a thread's rows fit its registers; above K = 512 more
-  // threads, which caps them (K = 1024 real: 1174 us at four rows, 1262 at two; complex: 2246 us at
-  // two rows and 512 threads, 2453 at four and 256).
-  if (real)
-    return K <= 128   ? run(launch<double, 16, 1, 128>)
-           : K <= 256 ? run(launch<double, 16, 2, 128>)
-           : K <= 512 ? run(launch<double, 16, 4, 128>)
-           : K <= 768 ? run(launch<double, 16, 3, 256>)
-                      : run(launch<double, 16, 4, 256>);
-  return K <= 128   ? run(launch<cuDoubleComplex, 8, 1, 128>)
-         : K <= 256 ? run(launch<cuDoubleComplex, 8, 2, 128>)
-         : K <= 512 ? run(launch<cuDoubleComplex, 8, 4, 128>)
-         : K <= 768 ? run(launch<cuDoubleComplex, 8, 3, 256>)
-                    : run(launch<cuDoubleComplex, 8, 2, 512>);
+  return with_variant(K, real, [&](auto variant) {
+    return variant.launch(K, systems, base, stride, at, epoch, st);
+  });
+}
+
+int ring_invert_resident(int K, bool real) {
+  return with_variant(K, real, [&](auto variant) { return variant.resident(K); });
 }
 
 int info_status(int info) {

@@ -29,6 +29,8 @@ constexpr int kInvertFlags = 256;  // K / 4 groups of steps at most
 // real: the blocks hold real numbers. Returns an EB_* status.
 int ring_invert(int K, int systems, char* base, int64_t stride, const InvertAt& at, int epoch,
                 bool real, cudaStream_t st);
+// The number of systems that one launch of it holds (later ones wait), or a negative EB_* status.
+int ring_invert_resident(int K, bool real);
 
 }  // namespace rl
 }  // namespace eb

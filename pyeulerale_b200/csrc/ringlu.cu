@@ -107,24 +107,42 @@ inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 // Rings of at most 1024 unknowns are supported.
 inline bool ring_supported(int K) { return K <= 1024; }
 
-// Blocked inversion: panels of 16 columns (8 where a panel thread holds four rows), column
-// blocks whose trailing update is one ZGEMM.
-inline int panel_width(int K) { return K <= 512 ? 16 : 8; }
-// Width of the column blocks: 128 where it divides K >= 512 (23 factorisations at K = 512 with the
-// GMRES on them: 847 ms, 876 with blocks of 64, whose trailing updates are half as deep), else 64.
+// Blocked inversion: column blocks whose trailing update is one ZGEMM, 128 wide where that divides
+// K >= 512 (23 factorisations at K = 512 with the GMRES on them: 847 ms, 876 with blocks of 64,
+// whose trailing updates are half as deep), else 64, the last one with what is left of K (a
+// remainder of 4 joins the block before it).
 constexpr int kGjBlock = 64, kGjBlockWide = 128;
-inline int gj_block(int K) {
-  return K >= 512 && K % kGjBlockWide == 0 ? kGjBlockWide : kGjBlock;
+inline int block_end(int K, int b0) {
+  const int BW = K >= 512 && K % kGjBlockWide == 0 ? kGjBlockWide : kGjBlock;
+  return K - b0 - BW < 8 ? K : b0 + BW;
 }
-// The blocked form needs whole column blocks, two shifts for its two streams, and enough work to
-// fill the GPU beside its panels (one SM per shift); the cooperative form holds only so many blocks
-// at a time (ring_invert.cu). Measured per ring, cooperative against blocked: K = 128, 24 shifts
-// 212 us against 322; K = 256, 10 shifts 624 against 635, 16 shifts 729 against 717, 24 shifts 1060
-// against 862; K = 512, 2 shifts 791 against 1121, 3 shifts 1455 against 1280, 12 shifts 4471
-// against 2392; K = 1024, 2 shifts 5518 against 4123. The line, shifts K^2 = 3 512^2, lies along
-// the crossings.
+// The panels of a block: 16 columns each (8 where a panel thread holds four rows), then 8 and 4 for
+// what is left; an even number (each panel moves the block between its place and a scratch block),
+// the first one split in two for that if need be. width: a multiple of 4, at least 8.
+struct Panels {
+  int n = 0, width[kGjBlockWide / 8 + 2];
+};
+inline Panels panels_of(int K, int width) {
+  Panels p;
+  for (int nb = K <= 512 ? 16 : 8; nb >= 4; nb /= 2)
+    for (; width >= nb; width -= nb) p.width[p.n++] = nb;
+  if (p.n % 2 != 0) {
+    p.width[0] /= 2;
+    p.width[p.n++] = p.width[0];
+  }
+  return p;
+}
+// The cooperative form holds only so many blocks at a time (ring_invert.cu), the others wait for
+// their launch; the blocked form, which needs two shifts for its two streams, fills the GPU with the
+// GEMMs beside its panels (one SM per shift) whatever their number. Measured per ring in us,
+// cooperative against blocked, in one launch: K = 256, 8 shifts 370, 581; K = 400, 2 shifts 589, 857;
+// K = 512, 2 shifts 780, 1096; in two: K = 160, 24 shifts 479, 468; K = 256, 16 shifts 720, 721;
+// K = 320, 4 shifts 821, 693; K = 512, 3 shifts 1438, 1231; K = 1024, 2 shifts 5417, 4039; in three:
+// K = 256, 24 shifts 1069, 864; K = 512, 5 shifts 2194, 1456. So the second launch is the line, and
+// up to K = 256, where it costs no more than the blocked form's, the third.
 inline bool blocked_inversion(int K, int shifts) {
-  return K % kGjBlock == 0 && shifts >= 2 && (int64_t)shifts * K * K >= 3 * 512 * 512;
+  const int fit = ring_invert_resident(K, false);  // (an error shows again in ring_invert)
+  return shifts >= 2 && fit > 0 && shifts > (K <= 256 ? 2 : 1) * (int64_t)fit;
 }
 
 // Byte offsets in a workspace.
@@ -678,15 +696,27 @@ void gj_pass(const Group& g, int j0, int c_lo, int c_hi, size_t in, size_t out, 
   k_gj_update<NB><<<dim3(tiles, g.S), 256, 0, st>>>(K, j0, c_lo, c_hi, g.systems(), in, out,
                                                     L.off_perm, L.off_info);
 }
+// The panels of the column block [b0, b1), which ends where it began (D; T: a scratch block).
+void gj_block(const Group& g, int b0, int b1, size_t D, cudaStream_t st) {
+  const Panels p = panels_of(g.L.K, b1 - b0);
+  const bool wide = g.L.K > 512;
+  for (int q = 0, j0 = b0; q < p.n; j0 += p.width[q++]) {
+    const size_t in = q & 1 ? g.L.off_T : D, out = q & 1 ? D : g.L.off_T;
+    if (p.width[q] == 16) gj_pass<16, 2>(g, j0, b0, b1, in, out, st);
+    else if (p.width[q] == 8 && !wide) gj_pass<8, 2>(g, j0, b0, b1, in, out, st);
+    else if (p.width[q] == 8) gj_pass<8, 4>(g, j0, b0, b1, in, out, st);
+    else if (!wide) gj_pass<4, 2>(g, j0, b0, b1, in, out, st);
+    else gj_pass<4, 4>(g, j0, b0, b1, in, out, st);
+  }
+}
 
 // D <- D^-1 for every shift by Gauss-Jordan with implicit row pivoting (D: a K x K block's
-// place): for a few shifts one cooperative launch (ring_invert.cu), for many the blocked form,
-// whose columns go in blocks of gj_block(K): the panels of a block update only the block's columns
-// (ping-pong with the scratch block T, an even number of passes, so the block ends in D), and the
-// rest of D takes the block's combined update of that rank as ZGEMMs (tensor-core DMMA).
+// place): for a few shifts one cooperative launch (ring_invert.cu), for many the blocked form: the
+// panels of a column block update only the block's columns, and the rest of D takes the block's
+// combined update of that rank as ZGEMMs (tensor-core DMMA).
 int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) {
   const Layout& L = g.L;
-  const int K = L.K, nb = panel_width(K), BW = gj_block(K);
+  const int K = L.K;
   if (!g.blocked) {
     const InvertAt where{D, L.off_T, D, L.off_L2 + L.blk / 2, L.off_flags, L.off_info};
     return ring_invert(K, g.S, g.base, g.stride, where, epoch, g.real, st);
@@ -700,32 +730,30 @@ int invert(const Group& g, size_t D, int epoch, cudaStream_t st, int side_lane) 
   if (rc != EB_OK) return rc;
   Handle& side = g_handle[side_lane];
   constexpr int64_t kB = sizeof(cuDoubleComplex);
-  // the block's update of the columns [c_lo, c_hi) without [gap0, gap1)
-  auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int gap0, int gap1, int b0) {
+  // the update of the columns [c_lo, c_hi) without [gap0, gap1) by the block [b0, b1)
+  auto update = [&](cudaStream_t hh, int c_lo, int c_hi, int gap0, int gap1, int b0, int b1) {
     if (c_hi <= c_lo) return EB_OK;
+    const int BW = b1 - b0;
     dense::Products p;
     p.add(D + kB * K * b0, L.off_Rp + kB * BW * c_lo, D + kB * K * c_lo);
     return dense::zgemm_set(K, c_hi - c_lo, BW, 1.0, 1.0, g.base, g.stride, g.S, p, K,
                             BW, K, hh, gap0, gap1);
   };
   bool side_busy = false;
-  for (int b0 = 0; b0 < K; b0 += BW) {
-    for (int q = 0; q < BW / nb; ++q) {
-      const size_t in = q & 1 ? L.off_T : D, out = q & 1 ? D : L.off_T;
-      if (nb == 16) gj_pass<16, 2>(g, b0 + q * nb, b0, b0 + BW, in, out, st);
-      else gj_pass<8, 4>(g, b0 + q * nb, b0, b0 + BW, in, out, st);
-    }
-    if (K == BW) break;
+  for (int b0 = 0, b1; b0 < K; b0 = b1) {
+    b1 = block_end(K, b0);
+    gj_block(g, b0, b1, D, st);
+    if (b1 - b0 == K) break;
     if (side_busy && cudaStreamWaitEvent(st, side.done, 0) != cudaSuccess)
       return check_launch("ringlu side join");
-    k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, BW, g.systems(), D, L.off_Rp,
+    k_gj_take_pivot_rows<<<dim3(K, g.S), 64, 0, st>>>(K, b0, b1 - b0, g.systems(), D, L.off_Rp,
                                                       L.off_perm, L.off_info);
-    const int n0 = b0 + BW, n1 = std::min(K, b0 + 2 * BW);  // the next block
-    if ((rc = update(st, n0, n1, 0, 0, b0)) != EB_OK) return rc;
+    const int n1 = b1 < K ? block_end(K, b1) : K;  // the next block: [b1, n1)
+    if ((rc = update(st, b1, n1, 0, 0, b0, b1)) != EB_OK) return rc;
     if (cudaEventRecord(side.start, st) != cudaSuccess ||
         cudaStreamWaitEvent(side.stream, side.start, 0) != cudaSuccess)
       return check_launch("ringlu side fork");
-    if ((rc = update(hs, 0, K, b0, n1, b0)) != EB_OK) return rc;
+    if ((rc = update(hs, 0, K, b0, n1, b0, b1)) != EB_OK) return rc;
     if (cudaEventRecord(side.done, side.stream) != cudaSuccess) return check_launch("ringlu side");
     side_busy = true;
   }
