@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(32 * Warps, Warps == 4 ? 3 : 4)
 __device__ __forceinline__ P2<double> ghost_by_velocity(const Wall<double>& w,
                                                         const State<double>& c, double e1,
                                                         double e2) {
-  const double a = 2.0 * w.inn * c.u[0] * fma(e1, w.nx, e2 * w.nz);
+  const double a = quot_(2.0 * c.u[0] * fma(e1, w.nx, e2 * w.nz), fma(w.nx, w.nx, w.nz * w.nz));
   return P2<double>{a * w.nx, a * w.nz};
 }
 
@@ -195,17 +195,14 @@ __global__ void __launch_bounds__(128, Velo ? 3 : 2)
     const Geometry_ geo(at);
     const double ia = geo.inv_area();
     const State<double> c = at.state(0, 0);
-    // per face (b, f, i, o): dF_k by its normal, or by its grid velocity
-    double gx[4][4], gz[4][4], sum[4];
+    // per face (b, f, i, o): dF_k by its normal; or by its grid velocity, mean[k] times the normal,
+    // and what the wall face's moves through the ghost
+    double gx[4][4], gz[4][4], sum[4], mean[4][4], wx[4], wz[4];
     auto face = [&](int q, const State<double>& ll, const State<double>& r,
                     const State<double>& rr, const FaceGeometry<double>& f, bool diss) {
       if constexpr (Velo) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const double a = -0.5 * (c.u[k] + r.u[k]);
-          gx[q][k] = a * f.nx;
-          gz[q][k] = a * f.nz;
-        }
+        for (int k = 0; k < 4; ++k) mean[q][k] = -0.5 * (c.u[k] + r.u[k]);
       } else {
         const Face_ d(ll, c, r, rr, f, diss, in);
 #pragma unroll
@@ -230,6 +227,8 @@ __global__ void __launch_bounds__(128, Velo ? 3 : 2)
     const Line_ line(at, c, geo, in);
     face(2, line.o, line.i, line.ii, geo.i, line.diss_i);
     face(3, line.i, line.o, line.oo, geo.o, line.diss_o);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) wx[k] = wz[k] = 0.0;
     if (m == 0) {  // the wall ghost is on both radial lines and moves with the inner face
       const Wall<double> w = geo.wall();
       double e[16], dp[4];
@@ -245,8 +244,13 @@ __global__ void __launch_bounds__(128, Velo ? 3 : 2)
         const double e1 = e[k + 4] + fma(q, dp[1], k == 1 ? -dO.c4 : 0.0);
         const double e2 = e[k + 8] + fma(q, dp[2], k == 2 ? -dO.c4 : 0.0);
         const P2<double> a = Velo ? ghost_by_velocity(w, c, e1, e2) : ghost_by_normal(w, c, e1, e2);
-        gx[2][k] += a.x;
-        gz[2][k] += a.z;
+        if constexpr (Velo) {
+          wx[k] = a.x;
+          wz[k] = a.z;
+        } else {
+          gx[2][k] += a.x;
+          gz[2][k] += a.z;
+        }
       }
     }
     double* out = J + 32 * in.cell_offset + 8 * first;
@@ -258,10 +262,22 @@ __global__ void __launch_bounds__(128, Velo ? 3 : 2)
       const int into = k == 0 ? 0 : k == 1 ? 2 : k == 2 ? 1 : 3;
       double a[8];
       if constexpr (Velo) {
+        const FaceGeometry<double> faces[4] = {geo.b, geo.f, geo.i, geo.o};
+        const FaceGeometry<double>&p = faces[from], &q = faces[into];
+        const bool wall = from == 2 || into == 2;
+        // -v / (2 area), corrected by its remainder: the entries' own roundings are so few that the
+        // inverse area's shows (errors of 1.9e-16 of the largest entries' root mean square, now 1.7)
+        const double twice = fabs(geo.cross), half = 0.5 * ia;
+        auto by_area = [&](double v) {
+          const double t = v * half;
+          return -fma(fma(-twice, t, v), half, t);
+        };
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          a[r] = -ia * 0.5 * (gx[from][r] + gx[into][r]);
-          a[r + 4] = -ia * 0.5 * (gz[from][r] + gz[into][r]);
+          const double x = fma(mean[from][r], p.nx, mean[into][r] * q.nx);
+          const double z = fma(mean[from][r], p.nz, mean[into][r] * q.nz);
+          a[r] = by_area(wall ? x + wx[r] : x);
+          a[r + 4] = by_area(wall ? z + wz[r] : z);
         }
       } else {
         // cross = (x2 - x0) (z3 - z1) - (z2 - z0) (x3 - x1), by corner k's coordinates
