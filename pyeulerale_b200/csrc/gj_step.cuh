@@ -35,8 +35,9 @@ __device__ __forceinline__ cuDoubleComplex fmsub(cuDoubleComplex a, cuDoubleComp
 }
 // 1 / a of a normal number below 2^1022: two Newton-Raphson steps y <- y + y (1 - a y), each of which
 // squares the relative error, from the hardware's approximation (2^-19 or better), without the
-// branches of a division, so that it runs in the shadow of the pivot search. eliminate() forms
-// the reciprocals of other pivots again, by division.
+// branches of a division, so that it runs in the shadow of the pivot search. (Bringing the other
+// numbers into that range by a power of two, or dividing by them where a row is staged, took 3 %
+// of a ring's time.)
 __device__ __forceinline__ double recip(double a) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
@@ -45,12 +46,6 @@ __device__ __forceinline__ double recip(double a) {
 }
 __device__ __forceinline__ cuDoubleComplex recip(cuDoubleComplex a) {
   const double d = recip(a.x * a.x + a.y * a.y);
-  return make_cuDoubleComplex(a.x * d, -a.y * d);
-}
-// 1 / a by division.
-__device__ __forceinline__ double recip_any(double a) { return 1.0 / a; }
-__device__ __forceinline__ cuDoubleComplex recip_any(cuDoubleComplex a) {
-  const double d = 1.0 / (a.x * a.x + a.y * a.y);
   return make_cuDoubleComplex(a.x * d, -a.y * d);
 }
 // a non-negative number ordered like the modulus
@@ -86,17 +81,17 @@ struct StepShared {
   int own[NC];              // the pivot rows
 };
 
-// `width` elimination steps (a multiple of kSub, at most NC) on the columns a: thread tid of the
-// 32 Warps that call it holds rows tid + 32 Warps r (r < ROWS, rows from K on are zero), left[r]
-// tells the rows not chosen yet. A step takes the largest modulus among those (to one part in
-// 2^10; ties go to the smaller row) as the pivot: every warp stages its best row, one barrier,
-// every thread finds the winner and eliminates the column from its rows, the next step's column
-// first, so that its search runs under the other columns' updates. S.own[jj] and pos[r] = c0 +
-// jj record step jj's row. Calls done(jj) after each group of kSub steps (their columns are then
-// a[.][NC - kSub ..]), failed(jj) and returns false at a zero or non-finite pivot (alike in all
-// threads). The columns rotate by one per step: the step's column is a[.][0], its result goes to
-// the last place, so after NC steps they are in order, after fewer column k is at NC - width + k.
-// (The loop stays rolled: each CTA runs it once, and unrolled steps, all fetched cold, took 950
+// `width` elimination steps (a multiple of kSub, at most NC) on the columns a: thread tid of the 32
+// Warps that call it holds rows tid + 32 Warps r (r < ROWS, rows from K on are zero), left[r] tells
+// the rows not chosen yet. A step takes the largest modulus among those (to one part in 2^10; ties
+// go to the smaller row) as the pivot: every warp stages its best row, one barrier, every thread
+// finds the winner and eliminates the column from its rows, the next step's column first, so that
+// its search runs under the other columns' updates. S.own[jj] and pos[r] = c0 + jj record step jj's
+// row. Calls done(jj) after each group of kSub steps (their columns are then a[.][NC - kSub ..]),
+// failed(jj) and returns false at a zero or non-finite pivot or one outside recip's range (alike in
+// all threads). The columns rotate by one per step: the step's column is a[.][0], its result goes
+// to the last place, so after NC steps they are in order, after fewer column k is at NC - width +
+// k. (The loop stays rolled: each CTA runs it once, and unrolled steps, all fetched cold, took 950
 // cycles each; 512 to 930 cycles by rows per thread in this form.)
 template <class T, int NC, int ROWS, int Warps, class Done, class Failed>
 __device__ __forceinline__ bool eliminate(StepShared<T, NC, Warps>& S, T (&a)[ROWS][NC],
@@ -146,14 +141,15 @@ __device__ __forceinline__ bool eliminate(StepShared<T, NC, Warps>& S, T (&a)[RO
     for (int q = 0; q < Warps; ++q) kb = max(kb, S.cand_key[par][q]);
     const int prow = kMaxRows - 1 - (int)(kb & 0x3FFu);
     const unsigned size = kb & ~0x3FFu;
-    if (!(size != 0u && size < 0x7FF00000u && prow < K)) {  // the same in every thread
+    // the same in every thread: zero, not finite, or out of recip's range (size_of: the modulus of
+    // a real number, its square of a complex one)
+    if (size - 0x00100000u >= 0x7FC00000u || prow >= K) {
       failed(jj);
       return false;
     }
     const int w = (prow % nt) >> 5;  // the warp that holds row prow
+    const T inv = S.cand_inv[par][w];
     const T* row = S.cand[par][w];
-    T inv = S.cand_inv[par][w];
-    if (size < 0x00100000u || size >= 0x7FD00000u) inv = recip_any(row[0]);
     if (tid == 0) S.own[jj] = prow;
     T f[ROWS];
 #pragma unroll
