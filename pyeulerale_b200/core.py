@@ -7,12 +7,13 @@ Fortran-ordered complex128 host arrays that the user modifies in place, every ``
 ``linearize`` call reads them, and results are written back to host arrays. The work runs on
 the GPU through the C ABI (``include/euler_b200.h``):
 
-* residual, forces and all Jacobians are forward-mode dual-number kernels (no complex step);
+* residual and forces are stencil kernels, the residual's Jacobians are formed in closed form and
+  the forces' by dual numbers (no complex step);
 * Jacobian products are stencil gathers on the device-resident Jacobians;
 * the resolvent ``(dR/dU - shift I)^-1`` is a direct block LU over the grid's radial rings on
   the device, refined to the solve tolerance (the reference factorises with SuperLU on every
   call); complex GMRES with a block-Jacobi preconditioner is the alternative solver;
-* the 13 second-order routines are exact directional derivatives of the Jacobians (nested
+* the 13 second-order routines are exact directional derivatives of the Jacobians (evaluated in
   duals) instead of the reference's central differences of complex-step Jacobians, so they
   agree with the reference to its finite-difference truncation error.
 

@@ -339,10 +339,6 @@ __global__ void __launch_bounds__(kGemmThreads)
       }
 }
 
-}  // namespace
-
-namespace {
-
 // Fewer 64 x 32 tiles than SMs: the products go in 32 x 16 tiles (the same sums in the same order),
 // four times as many CTAs with a quarter of the work per slice (a pair of real 256^3 products:
 // 6.6 us, 11.5 in 64 x 32 tiles).
@@ -697,10 +693,10 @@ __global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stri
   if (lane == 0) finish_row(t, ws, j, sr, si, true);
 }
 
-// The sweep step over NR right-hand sides, one read of A for all of them. Bound by reading A once (K = 512: 4.2 MB per workspace and term): eight rows
-// per CTA, thread (r, g) takes the columns j = g (mod 32), 16 of them in flight at a time, issued
-// before the right-hand sides are staged in shared memory; two CTAs keep 128 KB in flight per SM.
-// The partial sums are added in a fixed order. A cluster of eight CTAs per 32 rows, which had each
+// The sweep step over NR right-hand sides, one read of A for all of them. Bound by reading A once
+// (K = 512: 4.2 MB per workspace and term): eight rows per CTA, thread (r, g) takes the columns
+// j = g (mod 32), 16 of them in flight at a time, issued before the right-hand sides are staged in
+// shared memory; two CTAs keep 128 KB in flight per SM. The partial sums are added in a fixed order. A cluster of eight CTAs per 32 rows, which had each
 // SM wait for its cluster's barriers and remote sums, read at 2.4 TB/s with 22 workspaces active.
 // Grid: (row groups x terms, workspaces); workspaces from *n_active on exit.
 constexpr int kMaxRhs = 8;

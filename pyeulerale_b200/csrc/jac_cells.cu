@@ -181,8 +181,9 @@ __device__ __forceinline__ P2<double> ghost_by_velocity(const Wall<double>& w,
 }
 
 // d(odes)/d(vertices) (Velo = false) or d(odes)/d(velocities): four corners' 4 x 2 blocks. The
-// vertices' kernel holds four faces' derivatives by their normals at once: at two CTAs per SM (255
-// registers) it took 58 us, at three (168, 900 bytes spilled) 67 us (a grid row per instance); the velocities' fits three.
+// vertices' kernel holds four faces' derivatives by their normals at once: at two CTAs per SM (252
+// registers) it took 58 us, at three (168, 900 bytes spilled) 67 us (a grid row per instance); the
+// velocities' fits three.
 template <bool Velo>
 __global__ void __launch_bounds__(128, Velo ? 3 : 2)
     k_jac_corners_cells(Table t, const double* X, const double* V, const double* U, double* J) {
@@ -265,8 +266,8 @@ __global__ void __launch_bounds__(128, Velo ? 3 : 2)
         const FaceGeometry<double> faces[4] = {geo.b, geo.f, geo.i, geo.o};
         const FaceGeometry<double>&p = faces[from], &q = faces[into];
         const bool wall = from == 2 || into == 2;
-        // -v / (2 area), corrected by its remainder: the entries' own roundings are so few that the
-        // inverse area's shows (errors of 1.9e-16 of the largest entries' root mean square, now 1.7)
+        // -v / (2 area), corrected by its remainder: an entry has so few roundings of its own that the
+        // inverse area's shows (error 1.83e-16 of the entries, root mean squares, 1.75 so)
         const double twice = fabs(geo.cross), half = 0.5 * ia;
         auto by_area = [&](double v) {
           const double t = v * half;

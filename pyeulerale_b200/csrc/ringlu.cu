@@ -150,8 +150,8 @@ struct Layout {
   int M, N, K;
   size_t blk;   // bytes of one K x K complex block
   size_t bdr;   // bytes of one ring's block diagonal (N real 4 x 4 blocks)
-  size_t off_D, off_L1, off_C1, off_B1d, off_C1d, off_B2, off_C2, off_T, off_L2, off_Cr, off_Br, off_Rp, off_perm,
-      off_info, off_flags, off_acc, off_shift;
+  size_t off_D, off_L1, off_C1, off_B1d, off_C1d, off_B2, off_C2, off_T, off_L2, off_Cr, off_Br,
+      off_Rp, off_perm, off_info, off_flags, off_acc, off_shift;
   size_t off_y, off_x, off_r, off_w;
   size_t total;
 };
