@@ -315,7 +315,10 @@ class SpatialDiscretization:
     def set_free_stream_state(self) -> None:
         """Sets ``states`` to free-stream (core.py:265-268)."""
         self._call("eb_set_free_stream_state", ptr(self._dU))
-        _to_host(self._torch, self._dU, float, self._states)
+        # without a pinned buffer: every solver is constructed with this call, and a process's first
+        # pinned buffer costs a millisecond
+        host = self._dU.cpu().numpy()
+        self._states[...] = np.reshape(host, self._states.shape, order="F")
 
     def compute_odes(self) -> None:
         """Computes ``odes`` from ``states``, ``vertices`` and ``velocities`` (core.py:270-276)."""
