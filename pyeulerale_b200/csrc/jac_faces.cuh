@@ -114,10 +114,10 @@ struct Block {
 };
 
 // A face's flux in its cell's orientation, differentiated. diss = false: the central flux of the
-// faces next to the boundaries (f90:197, 219). Nothing of the dissipation is formed there: r may be a
-// ghost state, whose pressure and density can be negative (2 U_inf - U of a cell at twice the free
-// stream's; the reflection at a fast wall), so that it has no speed of sound; ll and rr are not
-// used.
+// faces next to the boundaries (f90:197, 219). r may be a ghost state there, whose pressure and
+// density can be negative (2 U_inf - U of a cell at twice the free stream's; the reflection at a fast
+// wall): it has no speed of sound, and what the dissipation is formed from is replaced by zeros. ll
+// and rr need then only be finite.
 template <class T>
 struct FaceDerivatives {
   T nx, nz, vn, vl, vr;
@@ -139,44 +139,31 @@ struct FaceDerivatives {
     vn = f.gx * nx + f.gz * nz;
     vl = (nx * l.u[1] + nz * l.u[2]) * l.ir;
     vr = (nx * r.u[1] + nz * r.u[2]) * r.ir;
-    if (diss) {
-      dissipation(ll, l, r, rr, in);
-    } else {
-      lam_l = false;
-      sgn = 0.0;
-      g_ll = g_l = g_r = g_rr = c2 = c4 = c = len = ilen = lift<T>(0.0);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) Q[k] = h[k] = lift<T>(0.0);
-    }
-  }
-
-  __device__ __forceinline__ void dissipation(const State<T>& ll, const State<T>& l,
-                                              const State<T>& r, const State<T>& rr,
-                                              const Instance& in) {
+    const T zero = lift<T>(0.0);
     len = sqrt_(nx * nx + nz * nz);
-    ilen = recip_(len);
+    ilen = diss ? recip_(len) : zero;
     const T cl = sqrt_(kGamma * l.p * l.ir), cr = sqrt_(kGamma * r.p * r.ir);
     const T al = abs_c(vl) + cl * len, ar = abs_c(vr) + cr * len;
     lam_l = value(al) > value(ar) + 1e-8;
-    const T lam = lam_l ? al : ar;
-    c = lam_l ? cl : cr;
+    const T lam = !diss ? zero : lam_l ? al : ar;
+    c = !diss ? zero : lam_l ? cl : cr;
     sgn = value(lam_l ? vl : vr) < 0.0 ? -1.0 : 1.0;
     const T num_l = ll.p - 2.0 * l.p + r.p, den_l = ll.p + 2.0 * l.p + r.p;
     const T num_r = l.p - 2.0 * r.p + rr.p, den_r = l.p + 2.0 * r.p + rr.p;
     const T sl = quot_(abs_c(num_l), den_l), sr = quot_(abs_c(num_r), den_r);
     const bool s_l = value(sl) > value(sr) + 1e-8;
-    const T S = s_l ? sl : sr;
+    const T S = !diss ? zero : s_l ? sl : sr;
     const double sg = value(s_l ? num_l : num_r) < 0.0 ? -1.0 : 1.0;
-    const T inv = recip_(s_l ? den_l : den_r);
+    const T inv = recip_(!diss ? lift<T>(1.0) : s_l ? den_l : den_r);
     const T outer = (sg - S) * inv, centre = -2.0 * (sg + S) * inv;
-    g_ll = s_l ? outer : lift<T>(0.0);
+    g_ll = s_l ? outer : zero;
     g_l = s_l ? centre : outer;
     g_r = s_l ? outer : centre;
-    g_rr = s_l ? lift<T>(0.0) : outer;
+    g_rr = s_l ? zero : outer;
     c2 = in.k2 * S * lam;
     c4 = in.k4 * lam - in.c4 * c2;
     const bool active = !(0.0 > value(c4) + 1e-8);  // max_c(0, c4)
-    const double on4 = active ? 1.0 : 0.0;
+    const double on4 = diss && active ? 1.0 : 0.0;
     c4 = c4 * on4;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -215,7 +202,6 @@ struct FaceDerivatives {
     const T n = k == 1 ? nx : k == 2 ? nz : lift<T>(0.0);
     T f = 0.5 * (mad(l.u[k], vl - vn, r.u[k] * (vr - vn)) + n * (l.p + r.p));
     if (k == 3) f = f + 0.5 * mad(l.p, vl, r.p * vr);
-    if (!diss) return f;
     const T d1 = r.u[k] - l.u[k];
     const T d3 = mad(3.0, l.u[k] - r.u[k], rr.u[k] - ll.u[k]);
     return mad(c4, d3, mad(-c2, d1, f));
@@ -229,7 +215,6 @@ struct FaceDerivatives {
     T d = 0.5 * mad(l.u[k], ul - g, r.u[k] * (ur - g));
     if (k == (X ? 1 : 2)) d = d + 0.5 * (l.p + r.p);
     if (k == 3) d = d + 0.5 * mad(l.p, ul, r.p * ur);
-    if (!diss) return d;
     const T lam = mad(sgn, lam_l ? ul : ur, c * (X ? nx : nz) * ilen);
     return mad(h[k], lam, d);
   }

@@ -8,8 +8,9 @@
 // carried fifteen. What bounds them is FP64 arithmetic in few threads (a block of one cell
 // evaluates one to four faces of about 1,000 operations); the grid's z is the slot or the corner, since a
 // 128 x 128 grid with a thread per cell alone would leave an SM four warps.
-// Measured on a 128 x 128 grid, directions of the states: states Jacobian 382 us nested, 56 us now
-// (1240 us before each slot had its threads); vertices Jacobian 208 us nested, 44 us now (427 us).
+// Measured on a 128 x 128 grid, directions of the states, inputs not in L2: states Jacobian 382 us
+// nested, 61 us now (1240 us before each slot had its threads); vertices Jacobian 208 us nested, 53 us
+// now (427 us).
 
 #include "jac_faces.cuh"
 #include "jacobian_kernels.cuh"
