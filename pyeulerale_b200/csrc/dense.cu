@@ -565,30 +565,37 @@ __device__ __forceinline__ void finish_row(const SweepTerm& t, char* ws, int i, 
   *y = o;
 }
 
-// Sweep step, op(A) = A. What bounds a step is latency: a few dependent loads and one launch, so
-// a product is spread thin, eight rows per CTA (K = 512: 64 CTAs of 64 KB each; with 32 rows per
-// CTA each of 16 SMs streamed 256 KB). Thread (r, g) sums the columns j = g (mod 32) of row r;
-// the partial sums are added in a fixed order. Grid: (row groups x terms, workspaces).
-__global__ void __launch_bounds__(256) k_sweep_n(int n, char* base, int64_t stride,
-                                                 SweepTerms terms) {
-  __shared__ double2 part[8][8];
+// Sweep step, op(A) = A. For few workspaces what bounds a step is latency, a few dependent loads and
+// one launch, so a product is spread thin, eight rows per CTA (K = 512: 64 CTAs of 64 KB each; with
+// 32 rows per CTA each of 16 SMs streamed 256 KB); many are bound by reading their matrices, 32 rows
+// per CTA, whose warps read 512 bytes at a time. Thread (r, g) sums the columns j = g (mod
+// kSweepThreads / Rows) of row r, eight loads in flight, four CTAs per SM, so that the next step's
+// CTAs find room beside this one's (sixteen loads at three CTAs per SM: a solve at K = 512 with 12
+// rings took 328 us, 273 so; 32 shifts 3391, 2553 with 32 rows, 2783 with eight). The partial sums are
+// added in a fixed order. Grid: (row groups x terms, workspaces).
+constexpr int kSweepThreads = 256;
+template <int Rows>
+__global__ void __launch_bounds__(kSweepThreads, 4) k_sweep_n(int n, char* base, int64_t stride,
+                                                              SweepTerms terms) {
+  constexpr int kGroups = kSweepThreads / Rows;  // columns taken at a time
+  __shared__ double2 part[8][Rows];
   const SweepTerm t = terms.t[blockIdx.x % terms.n];
   const int group = blockIdx.x / terms.n;
   char* ws = base + stride * blockIdx.y;
-  const int r = threadIdx.x & 7, g = threadIdx.x >> 3, lane = threadIdx.x & 31;
-  const int i = group * 8 + r;
+  const int r = threadIdx.x % Rows, g = threadIdx.x / Rows, lane = threadIdx.x & 31;
+  const int i = group * Rows + r;
   double sr = 0.0, si = 0.0;
   const bool active = i < n && t.a >= 0;
   const double2* A = place<const double2>(ws, t.a) + i;
   const double2* x = place<const double2>(ws, t.x);
-  constexpr int kUnroll = 16;  // column loads in flight per thread (ldg_inflight)
+  constexpr int kUnroll = 8;  // column loads in flight per thread (ldg_inflight)
   bool waited = false;
-  for (int j = g; j < n || !waited; j += 32 * kUnroll) {
+  for (int j = g; j < n || !waited; j += kGroups * kUnroll) {
     double2 a[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       a[u] = make_double2(0.0, 0.0);
-      if (active && j + 32 * u < n) a[u] = ldg_inflight(A + (int64_t)n * (j + 32 * u));
+      if (active && j + kGroups * u < n) a[u] = ldg_inflight(A + (int64_t)n * (j + kGroups * u));
     }
     if (!waited) {
       wait_previous();
@@ -597,20 +604,20 @@ __global__ void __launch_bounds__(256) k_sweep_n(int n, char* base, int64_t stri
     waited = true;
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u)
-      if (active && j + 32 * u < n) {
-        const double2 v = x[j + 32 * u];
+      if (active && j + kGroups * u < n) {
+        const double2 v = x[j + kGroups * u];
         sr = fma(a[u].x, v.x, fma(-a[u].y, v.y, sr));
         si = fma(a[u].x, v.y, fma(a[u].y, v.x, si));
       }
   }
 #pragma unroll
-  for (int o = 8; o < 32; o <<= 1) {
+  for (int o = Rows; o < 32; o <<= 1) {
     sr += __shfl_xor_sync(0xffffffffu, sr, o);
     si += __shfl_xor_sync(0xffffffffu, si, o);
   }
-  if (lane < 8) part[threadIdx.x >> 5][lane] = make_double2(sr, si);
+  if (lane < Rows) part[threadIdx.x >> 5][lane] = make_double2(sr, si);
   __syncthreads();
-  if (threadIdx.x < 8 && i < n) {
+  if (threadIdx.x < Rows && i < n) {
     double tr = 0.0, ti = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -803,16 +810,27 @@ int launch_sweep_multi(int n, char* base, int64_t stride, char* vectors, int64_t
   return EB_OK;
 }
 
+// Rows per CTA of a forward step: eight until their CTAs for one term fill the 592 places (four per
+// SM) one and a half times. Solves over 12 rings in us, eight rows against 32: K = 320, 12 shifts 872,
+// 967, 24 shifts 1675, 1596; K = 512, 8 shifts 760, 979, 16 shifts 1452, 1454, 24 shifts 2130, 2059;
+// K = 1024, 4 shifts 836, 1300, 8 shifts 1598, 1657.
+inline int sweep_rows(int n, int workspaces) {
+  return (int64_t)((n + 7) / 8) * workspaces > 6 * 148 ? 32 : 8;
+}
+
 }  // namespace
 
 int sweep_product(int conj_trans, int n, char* base, int64_t stride, int workspaces,
                   const SweepTerms& terms, cudaStream_t st) {
   if (n <= 0 || workspaces <= 0 || terms.n <= 0) return 0;
-  const dim3 grid((n + 7) / 8 * terms.n, workspaces);
-  const cudaError_t e =
-      conj_trans ? launch_dependent(k_sweep_h, grid, 256, 2 * sizeof(double2) * (size_t)n, st, n,
-                                    base, stride, terms)
-                 : launch_dependent(k_sweep_n, grid, 256, 0, st, n, base, stride, terms);
+  const int rows = conj_trans ? 8 : sweep_rows(n, workspaces);
+  const dim3 grid((n + rows - 1) / rows * terms.n, workspaces);
+  auto launch = [&](auto kernel, size_t smem) {
+    return launch_dependent(kernel, grid, kSweepThreads, smem, st, n, base, stride, terms);
+  };
+  const cudaError_t e = conj_trans   ? launch(k_sweep_h, 2 * sizeof(double2) * (size_t)n)
+                        : rows == 32 ? launch(k_sweep_n<32>, 0)
+                                     : launch(k_sweep_n<8>, 0);
   return e == cudaSuccess ? EB_OK : check_launch("sweep product");
 }
 
