@@ -400,21 +400,56 @@ __global__ void k_apply_mach_fwd(Table t, const double* J, const double* dm, dou
   }
 }
 
-// apply_odes_wrt_mach_rev, f90:632-650: a cluster of kMachCluster CTAs per instance, warp-shuffle
-// sums, the CTAs' sums added in rank order by the cluster's leader (a single CTA streamed the 1.5 MB
-// of a 128 x 128 instance in 28 us).
-constexpr int kMachCluster = 8;
-__global__ void __cluster_dims__(kMachCluster, 1, 1) __launch_bounds__(512)
-    k_apply_mach_rev(Table t, const double* J, const double* w, double* dm) {
+// apply_odes_wrt_mach_rev, f90:632-650. A single CTA streams the 1.5 MB of a 128 x 128 instance in
+// 25 us, a cluster of eight in 9; but clusters start one after the other, about 0.1 us each, and many
+// instances keep the GPU busy with a CTA each. Clusters: the first n_large clusters take one instance of
+// more than `small` cells each, as long as there are any, their CTAs' sums added in rank order by the
+// leader; the CTAs of the other clusters take one instance each, if it is not of those (small < 0: all
+// are large, a cluster each). Else: a CTA per instance of at most `small` cells. Warp-shuffle sums.
+constexpr int kMachCluster = 8, kMachThreads = 512;
+
+// The c-th instance of more than `small` cells (-1: there are not as many), for a whole CTA.
+__device__ __forceinline__ int large_instance(const Table& t, int64_t small, int c) {
+  constexpr int kWarps = kMachThreads / 32;
+  __shared__ unsigned words[kWarps];
+  const int tid = threadIdx.x;
+  for (int base = 0; base < t.n; base += kMachThreads) {
+    const bool large =
+        base + tid < t.n && (int64_t)t.dev[base + tid].M * t.dev[base + tid].N > small;
+    const unsigned word = __ballot_sync(0xffffffffu, large);
+    if ((tid & 31) == 0) words[tid >> 5] = word;
+    __syncthreads();
+    int found = -1;
+    for (int w = 0; w < kWarps && found < 0; ++w) {
+      const int k = __popc(words[w]);
+      if (c < k) found = base + 32 * w + (int)__fns(words[w], 0, c + 1);
+      else c -= k;
+    }
+    __syncthreads();
+    if (found >= 0) return found;
+  }
+  return -1;
+}
+
+template <bool Clusters>
+__device__ __forceinline__ void apply_mach_rev(const Table& t, int n_large, int64_t small,
+                                               const double* J, const double* w, double* dm) {
   namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank(), inst = blockIdx.x / kMachCluster;
+  const int place = Clusters ? blockIdx.x / kMachCluster : blockIdx.x;
+  const int rank = Clusters ? blockIdx.x % kMachCluster : 0;
+  const bool spread = Clusters && place < n_large;
+  const int inst = !Clusters || small < 0 ? place
+                   : spread               ? large_instance(t, small, place)
+                                          : (place - n_large) * kMachCluster + rank;
+  if (inst < 0 || inst >= t.n) return;
   const Instance in = t.dev ? t.dev[inst] : t.single;
   const int64_t cells = (int64_t)in.M * in.N;
+  if (!spread && cells > small) return;
+  const int first = spread ? rank : 0, step = spread ? kMachCluster * kMachThreads : kMachThreads;
   double sr = 0.0, si = 0.0;
   // 16-byte loads, and the cell loop unrolled so that several cells' loads are in flight
 #pragma unroll 4
-  for (int64_t c = rank * blockDim.x + threadIdx.x; c < cells; c += kMachCluster * blockDim.x) {
+  for (int64_t c = first * kMachThreads + threadIdx.x; c < cells; c += step) {
     const int64_t g = in.cell_offset + c;
     const double2 j01 = __ldg(reinterpret_cast<const double2*>(J + 4 * g));
     const double2 j23 = __ldg(reinterpret_cast<const double2*>(J + 4 * g + 2));
@@ -444,16 +479,33 @@ __global__ void __cluster_dims__(kMachCluster, 1, 1) __launch_bounds__(512)
   __shared__ double total[2];
   if (threadIdx.x < 2) {
     double a = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) a += red[threadIdx.x][k];
+    for (int k = 0; k < kMachThreads / 32; ++k) a += red[threadIdx.x][k];
     total[threadIdx.x] = a;
+    if (!spread) dm[2 * inst + threadIdx.x] = a;
   }
-  cluster.sync();
-  if (rank == 0 && threadIdx.x < 2) {
-    double a = 0.0;
-    for (int k = 0; k < kMachCluster; ++k) a += *cluster.map_shared_rank(&total[threadIdx.x], k);
-    dm[2 * inst + threadIdx.x] = a;
+  if (!spread) return;
+  if constexpr (Clusters) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (rank == 0 && threadIdx.x < 2) {
+      double a = 0.0;
+      for (int k = 0; k < kMachCluster; ++k) a += *cluster.map_shared_rank(&total[threadIdx.x], k);
+      dm[2 * inst + threadIdx.x] = a;
+    }
+    cluster.sync();  // the leader has read every CTA's sums before any exits
   }
-  cluster.sync();  // the leader has read every CTA's sums before any exits
+}
+__global__ void __cluster_dims__(kMachCluster, 1, 1) __launch_bounds__(kMachThreads)
+    k_apply_mach_rev_clusters(Table t, int n_large, int64_t small, const double* J, const double* w,
+                              double* dm) {
+  apply_mach_rev<true>(t, n_large, small, J, w, dm);
+  // beside the launch of the other instances it may have started early: over only after that one
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+__global__ void __launch_bounds__(kMachThreads)
+    k_apply_mach_rev(Table t, int64_t small, const double* J, const double* w, double* dm) {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  apply_mach_rev<false>(t, 0, small, J, w, dm);
 }
 
 // apply_forces_wrt_states_fwd, f90:1333-1348.
@@ -772,7 +824,41 @@ int eb_apply_odes_wrt_mach_rev(const eb_batch* b, const double* J, const double*
   EB_ALIGNED(J, d_odes, d_mach);
   if (!J || !d_mach || !d_odes) return fail(EB_ERR_ARG, "null array");
   const Table t = make_table(b);
-  k_apply_mach_rev<<<kMachCluster * b->n_inst, 512, 0, EB_STREAM(stream)>>>(t, J, d_odes, d_mach);
+  // A cluster pays from 100 cells per instance of the batch on (48 instances of 64 x 64 cells: 10.8 us in
+  // clusters, 10.1 alone; 90 x 90: 12.9, 15.1; 16 of 45 x 45: 6.7, 8.6), and only for instances of more
+  // than a 72nd of all cells (those that all CTAs cannot share evenly; 100 of 128 x 128: 40, 35). The
+  // sizes are on the device, so the bounds that the host knows decide: no instance can be that large,
+  // or a launch of clusters that look for such instances, and of the others' CTAs. Beyond 74
+  // instances, whose clusters do not fit the GPU together, the others get a launch of their own
+  // (eight to a cluster, 100 of 128 x 128 crowd on few SMs: 59 us).
+  const int n = b->n_inst;
+  const int64_t square = n > 1 || b->d_table ? (int64_t)b->max_dim * b->max_dim : b->n_cells;
+  const bool equal = b->n_cells == n * square;  // every instance has as many cells
+  const int64_t largest = std::min(square, b->n_cells - 20 * (int64_t)(n - 1));
+  int64_t small = std::max<int64_t>({512, 100 * (int64_t)n, b->n_cells / 72});
+  const int n_large = largest <= small ? 0
+                      : equal          ? n
+                                       : (int)std::min<int64_t>(n, b->n_cells / (small + 1));
+  if (equal) small = -1;
+  const bool apart = n_large == 0 || (n > 74 && !equal);
+  const int clusters = n_large + (apart || equal ? 0 : (n + 7) / 8);
+  cudaStream_t st = EB_STREAM(stream);
+  if (apart)
+    k_apply_mach_rev<<<n, kMachThreads, 0, st>>>(t, n_large ? small : INT64_MAX, J, d_odes, d_mach);
+  if (n_large > 0) {
+    cudaLaunchAttribute beside;  // the two launches share nothing: the clusters need not wait
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMachCluster * clusters);
+    cfg.blockDim = dim3(kMachThreads);
+    cfg.stream = st;
+    cfg.attrs = &beside;
+    cfg.numAttrs = apart ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, k_apply_mach_rev_clusters, t, n_large, small, J, d_odes, d_mach) !=
+        cudaSuccess)
+      return check_launch("apply_odes_wrt_mach_rev");
+  }
   return check_launch("apply_odes_wrt_mach_rev");
 }
 
