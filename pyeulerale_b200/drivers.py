@@ -137,10 +137,12 @@ def _batched_solves(instances, J, shifts_of, rhs_of, out_of, adjoint: bool, work
     instances of one grid size together per factorisation call, as many per call as the
     ``workspace`` (one uint8 device tensor) holds. If a call fails (a singular or non-finite
     system, a solve that misses ``tol``), its systems are retried one at a time and those that
-    still fail are passed to ``on_fail`` (or re-raised without one)."""
+    still fail are passed to ``on_fail`` (or re-raised without one). Other errors, such as an
+    inversion's wait that ran out, are raised."""
     from . import _lib
     from .solver import RingLUMany, ringlu_workspace_bytes
 
+    numerical = (_lib.EB_ERR_NAN, _lib.EB_ERR_NOCONV)
     groups = _shape_groups(instances)
     for (M, N), members in groups.items():
         todo = [i for i in members if i in shifts_of]
@@ -165,12 +167,14 @@ def _batched_solves(instances, J, shifts_of, rhs_of, out_of, adjoint: bool, work
             chunk = todo[c0:c0 + cap]
             try:
                 run(chunk)
-            except _lib.EulerB200Error:
+            except _lib.EulerB200Error as error:
+                if error.code not in numerical:
+                    raise
                 for i in chunk:
                     try:
                         run([i])
-                    except _lib.EulerB200Error:
-                        if on_fail is None:
+                    except _lib.EulerB200Error as alone:
+                        if on_fail is None or alone.code not in numerical:
                             raise
                         on_fail(i)
 
