@@ -485,7 +485,8 @@ int zgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_
 int dgemm_set(int M, int N, int K, double alpha, double beta, char* base, int64_t stride,
               int workspaces, const Products& set, int lda, int ldb, int ldc, cudaStream_t st) {
   if (M <= 0 || N <= 0 || workspaces * set.n <= 0) return 0;
-  if ((M | N | K | lda | ldb | ldc) % 4 != 0) return fail(EB_ERR_ARG, "dgemm: sizes must be multiples of 4");
+  if ((M | N | K | lda | ldb | ldc) % 4 != 0)
+    return fail(EB_ERR_ARG, "dgemm: sizes must be multiples of 4");
   const Operands ops{base, base, base, stride, stride, stride, set};
   auto run = [&](auto kernel, int bm, int bn, size_t smem) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -703,8 +704,9 @@ __global__ void __launch_bounds__(256) k_sweep_h(int n, char* base, int64_t stri
 // The sweep step over NR right-hand sides, one read of A for all of them. Bound by reading A once
 // (K = 512: 4.2 MB per workspace and term): eight rows per CTA, thread (r, g) takes the columns
 // j = g (mod 32), 16 of them in flight at a time, issued before the right-hand sides are staged in
-// shared memory; two CTAs keep 128 KB in flight per SM. The partial sums are added in a fixed order. A cluster of eight CTAs per 32 rows, which had each
-// SM wait for its cluster's barriers and remote sums, read at 2.4 TB/s with 22 workspaces active.
+// shared memory; two CTAs keep 128 KB in flight per SM. The partial sums are added in a fixed order.
+// A cluster of eight CTAs per 32 rows, which had each SM wait for its cluster's barriers and remote
+// sums, read at 2.4 TB/s with 22 workspaces active.
 // Grid: (row groups x terms, workspaces); workspaces from *n_active on exit.
 constexpr int kMaxRhs = 8;
 constexpr int kChunk = 512;  // columns per round: 16 per thread

@@ -824,13 +824,13 @@ int eb_apply_odes_wrt_mach_rev(const eb_batch* b, const double* J, const double*
   EB_ALIGNED(J, d_odes, d_mach);
   if (!J || !d_mach || !d_odes) return fail(EB_ERR_ARG, "null array");
   const Table t = make_table(b);
-  // A cluster pays from 100 cells per instance of the batch on (48 instances of 64 x 64 cells: 10.8 us in
-  // clusters, 10.1 alone; 90 x 90: 12.9, 15.1; 16 of 45 x 45: 6.7, 8.6), and only for instances of more
-  // than a 72nd of all cells (those that all CTAs cannot share evenly; 100 of 128 x 128: 40, 35). The
-  // sizes are on the device, so the bounds that the host knows decide: no instance can be that large,
-  // or a launch of clusters that look for such instances, and of the others' CTAs. Beyond 74
-  // instances, whose clusters do not fit the GPU together, the others get a launch of their own
-  // (eight to a cluster, 100 of 128 x 128 crowd on few SMs: 59 us).
+  // A cluster pays from 100 cells per instance of the batch on (48 instances of 64 x 64 cells: 10.8
+  // us in clusters, 10.1 alone; 90 x 90: 12.9, 15.1; 16 of 45 x 45: 6.7, 8.6), and only for
+  // instances of more than a 72nd of all cells (those that all CTAs cannot share evenly; 100 of 128
+  // x 128: 40, 35). The sizes are on the device, so the bounds that the host knows decide: no
+  // instance can be that large, or a launch of clusters that look for such instances, and of the
+  // others' CTAs. Beyond 74 instances, whose clusters do not fit the GPU together, the others get a
+  // launch of their own (eight to a cluster, 100 of 128 x 128 crowd on few SMs: 59 us).
   const int n = b->n_inst;
   const int64_t square = n > 1 || b->d_table ? (int64_t)b->max_dim * b->max_dim : b->n_cells;
   const bool equal = b->n_cells == n * square;  // every instance has as many cells

@@ -1,5 +1,5 @@
-"""apply_odes_wrt_mach_rev over batches: instances with a cluster of CTAs each, with a CTA each, and both in
-one launch (GPU).
+"""apply_odes_wrt_mach_rev over batches: instances with a cluster of CTAs each, with a CTA each, and
+both in one call (GPU).
 
 Tolerance: both sides add the same products in another order, so they differ by a few units of the sum
 of their absolute values: 1e-13 of it is left for up to 20,000 cells of four terms."""
